@@ -11,6 +11,7 @@
 #include <stdint.h>
 
 #include "kernels.cuh"
+#include "kernels_mlp.cuh"
 
 namespace mgsb {
 
@@ -1020,6 +1021,347 @@ __global__ void __launch_bounds__(1024) k_coarse_vcycle_dsm(const CoarseArgs A) 
         const int r0 = first_row(F), cnt = own_rows(F);
         for (int li = threadIdx.x; li < cnt; li += blockDim.x) A.lv[F].e[q[F].off + r0 + li] = loc(F, ec[F], li);
     }
+}
+
+// ---------------------------------------------------------------------------
+// The same part of the V-cycle with the operators of levels F..L-1 resident in
+// the cluster's shared memory too, and the vectors exchanged by remote stores.
+// What bounds k_coarse_vcycle_dsm is the latency of a phase (2-2.5 us): slice
+// pointers, columns, a division that finds each column's owner, remote loads,
+// which move 5 bytes a clock per SM (16-byte random loads, measured), and code
+// and parameters that every phase touches for the first time.  A cluster barrier
+// costs 500-650 clocks.  Here
+//   - CTA `rank` owns whole slices of 4 rows of every level; their entries (row of
+//     the vector read and coefficient, 32 lanes wide) and a list of the phases lie
+//     in memory as one image per CTA, laid out by the host as the kernel reads it,
+//     and arrive in one bulk copy issued before the dependency wait (no kernel
+//     writes the image);
+//   - a phase's entries go from there to registers while the barrier before it is
+//     waited for;
+//   - of each level a CTA holds the window of rows that its rows read (own rows,
+//     their neighbours, children and parents; contiguous in the numbering), and
+//     the owner of a row stores it into every window that holds it: each of the
+//     row's 8 lanes has the sum after the shuffles and serves two CTAs.  A phase
+//     then gathers from its own shared memory only;
+//   - the coarsest right-hand side and correction are whole in every CTA, and
+//     the inverse's rows and the frame's diagonals are fetched behind the first
+//     phases.
+// Same lanes, order and arithmetic per row as the cluster kernel: the same bits.
+// ---------------------------------------------------------------------------
+constexpr int kMaxCluster = 16;
+constexpr int kStagedStaticSmem = 1024;   // the barrier, and the alignment of the dynamic part
+constexpr int kStagedThreads = 512;       // at most: 128 registers a thread hold a phase's operator entries
+constexpr int kStagedHeld = 6;            // entries of a lane held in registers; longer rows read the rest in a loop
+
+enum StagedKind : int {
+    kStRestrict,   // right-hand side = restriction of the finer residual, correction = dinv of it
+    kStWhole,      // coarsest right-hand side, to every CTA
+    kStSweep,
+    kStResidual,
+    kStProlongSweep,   // prolongation and the first sweep from the descent's residual (k_prolong_sweep)
+    kStProlong,        // prolongation alone
+    kStDense           // coarsest solve
+};
+
+struct StagedPhase {   // offsets: bytes in the CTA's dynamic shared memory
+    int kind;
+    int out;                   // to global memory (the last phase) instead of into the windows
+    int many, first, rb, re;   // own slices, first row of the first, own rows
+    int ptr, idx, val;         // first step of each slice; per step 32 rows of the vector read, and coefficients
+    int src;                   // the vector that the entries (and the parents) read; -1: gsrc, with 4-byte indices
+    int self, lo;              // the level's correction, and its window's first row
+    int rhs, rhs0;             // what the sweep subtracts from, and the row at its start
+    int dd;                    // own D, then own dinv
+    int par;                   // per own row: 4 parents (rows of src), 4 weights
+    int dst;
+    int win;                   // int2[kMaxCluster]: every CTA's window of the level (first row, rows)
+    int zero;                  // no pre-smoothing: the correction starts from zero
+    int pad;
+    const float4* gsrc;
+    float4* gout;
+};
+struct StagedLoad {   // this frame's diagonals of the own rows of a level
+    int rb, count, dd, pad;
+    const float *dfull, *dinv;
+};
+struct StagedHead {
+    int loads, load_at;
+    int coarse_off, coarse_n, coarse_rb, coarse_re;   // coarsest level: the body's rows, own rows
+    int pad[2];
+};
+struct StagedPlan {
+    const unsigned char* image;   // [(body * cluster + rank) * image_bytes]: StagedHead, phases, loads, windows, entries
+    int image_bytes;
+    int ainv;                     // the own rows of the coarsest inverse
+    int phases, phase_at;         // the same in every CTA
+    int bytes, block;
+};
+
+__device__ __forceinline__ void cluster_st(uint32_t a, float4 v) {
+    asm volatile("st.shared::cluster.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(a), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
+                 : "memory");
+}
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t a, int rank) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async8(uint32_t dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
+}
+
+// e_i = sum_k Ainv_ik r_k of the coarsest level, one row per warp, in T.
+template <typename T>
+__device__ __forceinline__ float4 staged_dense_row(const T* a, int n, int lane, const float4* r) {
+    T ax = 0, ay = 0, az = 0;
+#pragma unroll 5
+    for (int k = lane; k < n; k += 32) {
+        const float4 v = r[k];
+        ax = fma(a[k], (T)v.x, ax);
+        ay = fma(a[k], (T)v.y, ay);
+        az = fma(a[k], (T)v.z, az);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        ax += __shfl_xor_sync(0xffffffffu, ax, o);
+        ay += __shfl_xor_sync(0xffffffffu, ay, o);
+        az += __shfl_xor_sync(0xffffffffu, az, o);
+    }
+    return make_float4((float)ax, (float)ay, (float)az, 0.f);
+}
+
+// What a slice of 4 rows (8 lanes per row) needs of the image in one phase, in registers.
+struct StagedSlice {
+    int row, li;   // this lane's row and its place among the own rows (0 when the row is not one)
+    bool valid;
+    int t, T;      // this lane's first and last step
+    int idx[kStagedHeld];
+    float val[kStagedHeld];
+    uint32_t d0, d1;   // where the row goes in this lane's two CTAs; 0: it does not
+};
+
+__device__ __forceinline__ void staged_load(StagedSlice& s, const StagedPhase& P, const unsigned char* smb, int g, int lane,
+                                            uint32_t peer0, uint32_t peer1) {
+    constexpr int S = 32 / kLanesC;
+    s.row = P.first + g * S + lane % S;
+    s.valid = s.row >= P.rb && s.row < P.re;
+    s.li = s.valid ? s.row - P.rb : 0;
+    const int2* win = reinterpret_cast<const int2*>(smb + P.win) + lane / S;
+    const int2 w0 = win[0], w1 = win[kLanesC];
+    s.d0 = s.valid && (unsigned)(s.row - w0.x) < (unsigned)w0.y ? peer0 + P.dst + 16 * (s.row - w0.x) : 0u;
+    s.d1 = s.valid && (unsigned)(s.row - w1.x) < (unsigned)w1.y ? peer1 + P.dst + 16 * (s.row - w1.x) : 0u;
+    s.t = s.T = 0;
+    if (P.kind == kStProlong) return;
+    const int* ptr = reinterpret_cast<const int*>(smb + P.ptr);
+    s.t = ptr[g];
+    s.T = ptr[g + 1];
+    const bool wide = P.src < 0;
+#pragma unroll
+    for (int k = 0; k < kStagedHeld; ++k) {
+        const int e = min(s.t + k, s.T - 1) * 32 + lane;   // past the end: the last entry with coefficient 0
+        s.idx[k] = wide ? reinterpret_cast<const int*>(smb + P.idx)[e] : (int)reinterpret_cast<const uint16_t*>(smb + P.idx)[e];
+        s.val[k] = s.t + k < s.T ? reinterpret_cast<const float*>(smb + P.val)[e] : 0.f;
+    }
+}
+
+// Sum of the slice's entries, reduced over each row's lanes.
+__device__ __forceinline__ float4 staged_sum(const StagedSlice& s, const StagedPhase& P, const unsigned char* smb, int lane) {
+    constexpr int S = 32 / kLanesC;
+    float4 v[kStagedHeld];
+    if (P.src < 0) {
+        const float4* x = P.gsrc;
+#pragma unroll
+        for (int k = 0; k < kStagedHeld; ++k) v[k] = __ldg(x + s.idx[k]);
+    } else {
+        const float4* x = reinterpret_cast<const float4*>(smb + P.src);
+#pragma unroll
+        for (int k = 0; k < kStagedHeld; ++k) v[k] = x[s.idx[k]];
+    }
+    float ax = 0.f, ay = 0.f, az = 0.f;
+#pragma unroll
+    for (int k = 0; k < kStagedHeld; ++k) {
+        ax = fmaf(s.val[k], v[k].x, ax);
+        ay = fmaf(s.val[k], v[k].y, ay);
+        az = fmaf(s.val[k], v[k].z, az);
+    }
+    for (int t = s.t + kStagedHeld; t < s.T; ++t) {
+        const int e = t * 32 + lane;
+        const float a = reinterpret_cast<const float*>(smb + P.val)[e];
+        const float4 x = P.src < 0 ? __ldg(P.gsrc + reinterpret_cast<const int*>(smb + P.idx)[e])
+                                   : reinterpret_cast<const float4*>(smb + P.src)[reinterpret_cast<const uint16_t*>(smb + P.idx)[e]];
+        ax = fmaf(a, x.x, ax);
+        ay = fmaf(a, x.y, ay);
+        az = fmaf(a, x.z, az);
+    }
+#pragma unroll
+    for (int o = S; o < 32; o <<= 1) {
+        ax += __shfl_xor_sync(0xffffffffu, ax, o);
+        ay += __shfl_xor_sync(0xffffffffu, ay, o);
+        az += __shfl_xor_sync(0xffffffffu, az, o);
+    }
+    return make_float4(ax, ay, az, 0.f);
+}
+
+__device__ __forceinline__ void staged_store(const StagedSlice& s, const StagedPhase& P, int lane, float4 q) {
+    if (P.out) {
+        if (s.valid && lane < 32 / kLanesC) P.gout[s.row] = q;
+        return;
+    }
+    if (s.d0) cluster_st(s.d0, q);
+    if (s.d1) cluster_st(s.d1, q);
+}
+
+// The slice's rows from their sum, for the phases that restrict.
+__device__ __forceinline__ void staged_restricted(const StagedSlice& s, const StagedPhase& P, unsigned char* smb, int lane,
+                                                  float4 r) {
+    if (P.kind == kStRestrict) {
+        if (s.valid && lane < 32 / kLanesC) reinterpret_cast<float4*>(smb + P.rhs)[s.li] = r;
+        const float di = P.zero ? 0.f : reinterpret_cast<const float*>(smb + P.dd)[P.re - P.rb + s.li];
+        r = make_float4(di * r.x, di * r.y, di * r.z, 0.f);   // the first sweep from zero
+    }
+    staged_store(s, P, lane, r);
+}
+
+__global__ void __launch_bounds__(kStagedThreads, 1) k_coarse_vcycle_staged(const StagedPlan Q, const float* __restrict__ Ainv,
+                                                                         const double* __restrict__ Ainv64,
+                                                                         const int32_t* __restrict__ dense_off) {
+    pdl_trigger();
+    extern __shared__ __align__(128) unsigned char smb[];
+    __shared__ __align__(8) uint64_t bar;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int cs = (int)cluster.num_blocks();
+    const int rank = (int)cluster.block_rank();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+    constexpr int S = 32 / kLanesC;
+    const int sub = lane / S;
+    if (threadIdx.x == 0) {
+        mbar_init(&bar, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        mbar_expect_tx(&bar, (uint32_t)Q.image_bytes);
+        bulk_g2s(smb, Q.image + (size_t)blockIdx.x * Q.image_bytes, (uint32_t)Q.image_bytes, &bar);
+    }
+    __syncthreads();
+    cluster_arrive();   // matched below: every CTA of the cluster runs before it is written to
+    // this lane's two CTAs (of up to 16; a CTA beyond the cluster has an empty window): their shared memory
+    const uint32_t base = smem_u32(smb);
+    const uint32_t peer0 = cluster_addr(base, sub < cs ? sub : rank),
+                   peer1 = cluster_addr(base, sub + kLanesC < cs ? sub + kLanesC : rank);
+    const int dense0 = __ldg(dense_off + blockIdx.x / cs);
+    // the image; when it does not arrive the CTA takes part in the barriers only, and the frame ends non-finite
+    const bool ok = mbar_wait(&bar, 0, kMaxPolls);
+    const StagedHead& head = *reinterpret_cast<const StagedHead*>(smb);
+    const int nc = head.coarse_n;
+    auto phase = [&](int p) -> const StagedPhase& {
+        return *reinterpret_cast<const StagedPhase*>(smb + Q.phase_at + p * sizeof(StagedPhase));
+    };
+    StagedSlice s;
+    float4 sum = f4z();
+    const bool busy = ok && warp < phase(0).many;
+    if (busy) staged_load(s, phase(0), smb, warp, lane, peer0, peer1);
+    pdl_wait();
+    if (ok) {   // this frame's data: diagonals, and the inverse's rows behind the first phases
+        for (int i = 0; i < head.loads; ++i) {
+            const StagedLoad& d = reinterpret_cast<const StagedLoad*>(smb + head.load_at)[i];
+            for (int r = threadIdx.x; r < d.count; r += blockDim.x) {
+                cp_async4(base + d.dd + 4 * r, d.dfull + d.rb + r);
+                cp_async4(base + d.dd + 4 * (d.count + r), d.dinv + d.rb + r);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        const size_t first = (size_t)(head.coarse_rb - head.coarse_off) * nc + dense0;
+        const int many = (head.coarse_re - head.coarse_rb) * nc;
+        if (Ainv64)
+            for (int i = threadIdx.x; i < many; i += blockDim.x) cp_async8(base + Q.ainv + 8 * i, Ainv64 + first + i);
+        else
+            for (int i = threadIdx.x; i < many; i += blockDim.x) cp_async4(base + Q.ainv + 4 * i, Ainv + first + i);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        if (busy) sum = staged_sum(s, phase(0), smb, lane);   // the first phase's rows, while the diagonals arrive
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+    }
+    cluster_wait();
+    __syncthreads();   // the diagonals of this CTA
+    for (int p = 0; p < Q.phases; ++p) {
+        const StagedPhase& P = phase(p);
+        const int kind = ok ? P.kind : -1;
+        if (kind == kStRestrict || kind == kStWhole) {
+            for (int g = warp; g < P.many; g += nwarp) {
+                if (g != warp) staged_load(s, P, smb, g, lane, peer0, peer1);
+                staged_restricted(s, P, smb, lane, p == 0 && g == warp ? sum : staged_sum(s, P, smb, lane));
+            }
+            if (kind == kStWhole) asm volatile("cp.async.wait_all;" ::: "memory");
+        } else if (kind == kStSweep || kind == kStResidual) {
+            for (int g = warp; g < P.many; g += nwarp) {
+                if (g != warp) staged_load(s, P, smb, g, lane, peer0, peer1);
+                const float4 x = reinterpret_cast<const float4*>(smb + P.self)[s.valid ? s.row - P.lo : 0];
+                const float4 b = reinterpret_cast<const float4*>(smb + P.rhs)[s.li];
+                const float D = reinterpret_cast<const float*>(smb + P.dd)[s.li];
+                const float w = reinterpret_cast<const float*>(smb + P.dd)[P.re - P.rb + s.li];
+                const float4 a = staged_sum(s, P, smb, lane);
+                const float rx = b.x - fmaf(D, x.x, a.x), ry = b.y - fmaf(D, x.y, a.y), rz = b.z - fmaf(D, x.z, a.z);
+                staged_store(s, P, lane, kind == kStResidual
+                                             ? make_float4(rx, ry, rz, 0.f)
+                                             : make_float4(fmaf(w, rx, x.x), fmaf(w, ry, x.y), fmaf(w, rz, x.z), 0.f));
+            }
+        } else if (kind == kStProlongSweep || kind == kStProlong) {
+            for (int g = warp; g < P.many; g += nwarp) {
+                if (g != warp) staged_load(s, P, smb, g, lane, peer0, peer1);
+                const float4* ec = reinterpret_cast<const float4*>(smb + P.src);
+                const int4 id = reinterpret_cast<const int4*>(smb + P.par)[2 * s.li];
+                const float4 pw = reinterpret_cast<const float4*>(smb + P.par)[2 * s.li + 1];
+                const float4 c0 = ec[id.x], c1 = ec[id.y], c2 = ec[id.z], c3 = ec[id.w];
+                const float4 pe = make_float4(pw.x * c0.x + pw.y * c1.x + pw.z * c2.x + pw.w * c3.x,
+                                              pw.x * c0.y + pw.y * c1.y + pw.z * c2.y + pw.w * c3.y,
+                                              pw.x * c0.z + pw.y * c1.z + pw.z * c2.z + pw.w * c3.z, 0.f);
+                float4 x = reinterpret_cast<const float4*>(smb + P.self)[s.valid ? s.row - P.lo : 0];
+                if (kind == kStProlongSweep) {
+                    // A (x + pe) = A x + D pe + OP e: the sweep from the residual at x
+                    const float4 b = reinterpret_cast<const float4*>(smb + P.rhs)[s.valid ? s.row - P.rhs0 : 0];
+                    const float D = reinterpret_cast<const float*>(smb + P.dd)[s.li];
+                    const float w = reinterpret_cast<const float*>(smb + P.dd)[P.re - P.rb + s.li];
+                    const float4 a = staged_sum(s, P, smb, lane);
+                    const float rx = b.x - fmaf(D, pe.x, a.x), ry = b.y - fmaf(D, pe.y, a.y), rz = b.z - fmaf(D, pe.z, a.z);
+                    x.x += pe.x;
+                    x.y += pe.y;
+                    x.z += pe.z;
+                    x = make_float4(fmaf(w, rx, x.x), fmaf(w, ry, x.y), fmaf(w, rz, x.z), 0.f);
+                } else {
+                    __syncwarp();   // in place: every lane of the row has read it
+                    x.x += pe.x;
+                    x.y += pe.y;
+                    x.z += pe.z;
+                }
+                staged_store(s, P, lane, x);
+            }
+        } else if (kind == kStDense) {
+            // coarsest: e = A^-1 r for the own rows, to every CTA (or out, when it is the only level)
+            for (int i = warp; i < P.re - P.rb; i += nwarp) {
+                const float4* rf = reinterpret_cast<const float4*>(smb + P.src);
+                const size_t at = (size_t)i * nc;
+                const float4 e = Ainv64 ? staged_dense_row(reinterpret_cast<const double*>(smb + Q.ainv) + at, nc, lane, rf)
+                                        : staged_dense_row(reinterpret_cast<const float*>(smb + Q.ainv) + at, nc, lane, rf);
+                const int row = P.rb + i;
+                if (P.out) {
+                    if (lane == 0) P.gout[row] = e;
+                } else if (lane % S == 0) {
+                    const int to = P.dst + 16 * (row - head.coarse_off);
+                    if (sub < cs) cluster_st(peer0 + to, e);
+                    if (sub + kLanesC < cs) cluster_st(peer1 + to, e);
+                }
+            }
+        }
+        if (p + 1 == Q.phases) break;
+        cluster_arrive();
+        // the next phase's operator, behind the barrier
+        if (ok && warp < phase(p + 1).many) staged_load(s, phase(p + 1), smb, warp, lane, peer0, peer1);
+        cluster_wait();
+    }
+    // no remote store follows the last barrier; a copy that never arrived is waited for again before the CTA ends
+    if (!ok) mbar_wait(&bar, 0, kMaxPolls);
 }
 
 // ---------------------------------------------------------------------------

@@ -331,8 +331,8 @@ bool build_plan(std::vector<PlanBody>& bodies, const mgsb_params& p, Plan& P, st
         ld.nnz = (int)col.size();
         {
             // OP of the finer level: row i = sum over its neighbours j of a_ij * (prolongation row j),
-            // accumulated in FP64 (weights as stored), columns ascending; padding on the body's
-            // first row of this level; every column checked to lie in the row's body
+            // accumulated in FP64 (weights as stored), columns ascending; padding on the row's
+            // first parent, which the kernels read anyway; every column checked to lie in the row's body
             PlanLevel& fl = P.levels[l - 1];
             std::vector<int32_t> optr(nfin + 1, 0), ocol, pad(nfin, 0);
             std::vector<double> oval, acc(n, 0.0);
@@ -362,7 +362,7 @@ bool build_plan(std::vector<PlanBody>& bodies, const mgsb_params& p, Plan& P, st
                     mark[c] = 0;
                 }
                 optr[i + 1] = (int32_t)ocol.size();
-                pad[i] = loff[prev_body[i]];
+                pad[i] = ld.pid[i].x;
             }
             build_ell(optr, ocol, oval, nfin, fl.S, fl.op_slice_ptr, fl.op_col, fl.op_val, &pad);
             std::vector<int32_t> body_of_level(n, 0);

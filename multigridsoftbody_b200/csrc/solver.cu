@@ -79,6 +79,14 @@ struct LevelDev {
 
 }  // namespace
 
+// Host copies of a coarse level's structure, from which the staged cluster kernel's images are built.
+struct LevelHost {
+    std::vector<int32_t> slice_ptr, ell_col, op_slice_ptr, op_col, rptr, rcol;
+    std::vector<float> ell_val, op_val, rw;
+    std::vector<int4> pid;   // per row of this level: parents on the next coarser level
+    std::vector<float4> pw;
+};
+
 struct mgsb_solver {
     mgsb_params p{};
     int device = 0;
@@ -182,6 +190,14 @@ struct mgsb_solver {
     int cluster = 1;
     int fuse_l0 = 1;
     int coarse_block = 512;
+    // k_coarse_vcycle_staged: its layout for this shape (bytes 0: it does not fit), the CTAs' images and
+    // whether the device's copy is older than the host's
+    StagedPlan staged{};
+    std::vector<LevelHost> coarse_host;   // one entry per level of the hierarchy that is set up
+    std::vector<unsigned char> staged_image;
+    unsigned char* staged_dev = nullptr;
+    size_t staged_cap = 0;
+    bool staged_stale = false;
     int split = 1;   // first level of the cluster kernel; levels 1..split-1 run grid-wide
     bool pdl = true;  // programmatic dependent launch between consecutive kernels
     bool fuse_prolong = true;   // prolongation + first post-sweep as one kernel (k_prolong_sweep)
@@ -245,6 +261,7 @@ mgsb_solver::~mgsb_solver() {
         if (stage_ev[k]) cudaEventDestroy(stage_ev[k]);
     }
     if (readback) cudaFreeHost(readback);
+    if (staged_dev) cudaFree(staged_dev);
     if (aux_stream) cudaStreamDestroy(aux_stream);
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
@@ -313,7 +330,6 @@ constexpr int kFallbackL0Sweeps = 2;
 // Shape of the coarse V-cycle kernel: explicit tuning if set, else by size
 // (level-0 work fused for bodies up to 40k vertices; ~2.5k rows per CTA).
 size_t coarse_smem_bytes(const mgsb_solver* h, int cs, int split);
-
 // Largest body's rows on a coarse level below which it stays in the cluster
 // kernel by default; larger levels run as grid-wide kernels over all SMs.
 constexpr int kClusterLevelRows = 1024;
@@ -353,6 +369,8 @@ void apply_tuning(mgsb_solver* h) {
         h->cluster = std::min(cap, std::max(1, (h->maxv[h->split] + 63) / 64));
         while (h->cluster < 16 && coarse_smem_bytes(h, h->cluster, h->split) > (size_t)h->max_smem_optin) ++h->cluster;
     }
+    h->staged = StagedPlan{};
+    h->staged_stale = true;   // planned for this shape before the next launch
 }
 
 void invalidate_graph(mgsb_solver* h) {
@@ -609,12 +627,32 @@ mgsb_status rebuild(mgsb_solver* h) {
         TRY(dupload(h, pool, &h->range, P.range));
         h->range_host = P.range;
         if (L > kMaxLevels) return set_err(h, MGSB_NOT_SUPPORTED, "at most %d levels", kMaxLevels);
+        h->coarse_host.assign(L, LevelHost{});
+        for (int l = 1; l < L; ++l) {   // the plan's arrays are not needed after their upload
+            PlanLevel& pl = P.levels[l];
+            LevelHost& H = h->coarse_host[l];
+            H.slice_ptr = std::move(pl.slice_ptr);
+            H.ell_col = std::move(pl.ell_col);
+            H.ell_val = std::move(pl.ell_val);
+            H.rptr = std::move(pl.rptr);
+            H.rcol = std::move(pl.rcol);
+            H.rw = std::move(pl.rw);
+            if (l == L - 1) break;
+            H.op_slice_ptr = std::move(pl.op_slice_ptr);
+            H.op_col = std::move(pl.op_col);
+            H.op_val = std::move(pl.op_val);
+            H.pid = std::move(P.levels[l + 1].pid);
+            H.pw = std::move(P.levels[l + 1].pw);
+        }
         CUDA_TRY(h, cudaFuncSetAttribute(k_coarse_vcycle_dsm, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         CUDA_TRY(h, cudaDeviceGetAttribute(&h->max_smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device));
         CUDA_TRY(h, cudaFuncSetAttribute(k_coarse_vcycle_dsm, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          h->max_smem_optin));
         CUDA_TRY(h, cudaFuncSetAttribute(k_coarse_vcycle_cta, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          h->max_smem_optin));
+        CUDA_TRY(h, cudaFuncSetAttribute(k_coarse_vcycle_staged, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        CUDA_TRY(h, cudaFuncSetAttribute(k_coarse_vcycle_staged, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         h->max_smem_optin - kStagedStaticSmem));
         CUDA_TRY(h, cudaFuncSetAttribute(k_coarse_apply, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          h->max_smem_optin));
         TRY(dupload(h, pool, &h->dense_off_d, P.dense_off));
@@ -822,6 +860,370 @@ size_t coarse_smem_bytes(const mgsb_solver* h, int cs, int split) {
     return (size_t)best * sizeof(float4);
 }
 
+// Layout and images of k_coarse_vcycle_staged for a cluster size and a first level.  The kernel is taken wherever a
+// CTA's image and vectors fit its shared memory; k_coarse_vcycle_dsm, which reads the operators from L2 in every
+// phase, runs the shapes that do not, numberings whose rows reach far among them.  Leaves h->staged.bytes 0 if it
+// does not fit or the device cannot schedule the cluster.
+void plan_staged(mgsb_solver* h, int cs, int split) {
+    constexpr int S = kSliceCoarse, G = kLanesC;
+    const int L = h->p.levels, lc = L - 1, nb = (int)h->bodies.size();
+    struct Entries {
+        std::vector<int> idx;
+        std::vector<float> val;
+    };
+    struct Part {   // one level of one CTA
+        int off = 0, n = 0, slices = 0, first = 0, rb = 0, re = 0;   // the body's rows, own slices and rows
+        int2 win{0, 0};
+        std::vector<int32_t> rp, ep, op;
+        Entries re_, ee, oe;
+        std::vector<int4> pid;
+        std::vector<float4> pw;
+    };
+    std::vector<Part> parts((size_t)nb * cs * L);
+    auto part = [&](int bi, int k, int l) -> Part& { return parts[((size_t)bi * cs + k) * L + l]; };
+    // shares and windows
+    for (int bi = 0; bi < nb; ++bi) {
+        for (int l = split; l < L; ++l) {
+            const int2 rg = h->range_host[(size_t)bi * L + l];
+            const int g0 = rg.x / S, g1 = (rg.x + rg.y + S - 1) / S, per = (g1 - g0 + cs - 1) / cs;
+            for (int k = 0; k < cs; ++k) {
+                Part& o = part(bi, k, l);
+                const int s0 = std::min(g1, g0 + k * per), s1 = std::min(g1, s0 + per);
+                o.off = rg.x;
+                o.n = rg.y;
+                o.slices = s1 - s0;
+                o.first = s0 * S;
+                o.rb = std::max(rg.x, s0 * S);
+                o.re = std::max(o.rb, std::min(rg.x + rg.y, s1 * S));
+            }
+        }
+        for (int l = split; l < L; ++l) {
+            const LevelHost& H = h->coarse_host[l];
+            for (int k = 0; k < cs; ++k) {
+                Part& o = part(bi, k, l);
+                int2 w{o.rb, o.re};
+                auto add = [&w](int c) { w = w.y > w.x ? int2{std::min(w.x, c), std::max(w.y, c + 1)} : int2{c, c + 1}; };
+                if (l == lc) {
+                    w = int2{o.off, o.off + o.n};
+                } else {
+                    for (int i = o.rb; i < o.re; ++i)
+                        for (int e = H.slice_ptr[i / S] + i % S; e < H.slice_ptr[i / S + 1]; e += S) add(H.ell_col[e]);
+                    const LevelHost& N = h->coarse_host[l + 1];
+                    const Part& n = part(bi, k, l + 1);
+                    for (int e = N.rptr[n.rb]; e < N.rptr[n.re]; ++e) add(N.rcol[e]);
+                    if (l > split) {
+                        const LevelHost& U = h->coarse_host[l - 1];
+                        const Part& u = part(bi, k, l - 1);
+                        for (int i = u.rb; i < u.re; ++i) {
+                            for (int e = U.op_slice_ptr[i / S] + i % S; e < U.op_slice_ptr[i / S + 1]; e += S) add(U.op_col[e]);
+                            for (int c : {U.pid[i].x, U.pid[i].y, U.pid[i].z, U.pid[i].w}) add(c);
+                        }
+                    }
+                }
+                o.win = w;
+            }
+        }
+    }
+    // entries: slices of 4 rows, 8 lanes per row, 32 entries per step, at least one step per slice; a lane without an
+    // entry reads the vector's first row with coefficient 0
+    auto steps = [&](const Part& o, auto&& row_entries, std::vector<int32_t>& ptr, Entries& ent) {
+        std::vector<std::pair<int, float>> row[S];
+        ptr.assign(1, 0);
+        for (int g = 0; g < o.slices; ++g) {
+            int T = 1;
+            for (int r = 0; r < S; ++r) {
+                row[r].clear();
+                const int i = o.first + g * S + r;
+                if (i >= o.rb && i < o.re) row_entries(i, row[r]);
+                T = std::max(T, (int)(row[r].size() + G - 1) / G);
+            }
+            for (int t = 0; t < T; ++t)
+                for (int lane = 0; lane < 32; ++lane) {
+                    const size_t e = (size_t)(t * G + lane / S);
+                    const auto v = e < row[lane % S].size() ? row[lane % S][e] : std::make_pair(0, 0.f);
+                    ent.idx.push_back(v.first);
+                    ent.val.push_back(v.second);
+                }
+            ptr.push_back(ptr.back() + T);
+        }
+    };
+    auto at = [](const Part& w, int c) { return c - w.win.x; };
+    struct Most {
+        size_t W = 0, rows = 0, slices = 0, re = 0, ee = 0, oe = 0;
+    };
+    std::vector<Most> most(L);
+    size_t coarsest = 0, ainv = 0;
+    for (int bi = 0; bi < nb; ++bi)
+        for (int k = 0; k < cs; ++k)
+            for (int l = split; l < L; ++l) {
+                Part& o = part(bi, k, l);
+                const LevelHost& H = h->coarse_host[l];
+                using Row = std::vector<std::pair<int, float>>;
+                steps(o, [&](int i, Row& out) {
+                    for (int e = H.rptr[i]; e < H.rptr[i + 1]; ++e)
+                        out.emplace_back(l == split ? H.rcol[e] : at(part(bi, k, l - 1), H.rcol[e]), H.rw[e]);
+                }, o.rp, o.re_);
+                Most& m = most[l];
+                m.rows = std::max(m.rows, (size_t)(o.re - o.rb));
+                m.slices = std::max(m.slices, (size_t)o.slices);
+                m.re = std::max(m.re, o.re_.idx.size());
+                if (l == lc) {
+                    coarsest = std::max(coarsest, (size_t)o.n);
+                    ainv = std::max(ainv, (size_t)(o.re - o.rb) * o.n);
+                    continue;
+                }
+                const Part& n = part(bi, k, l + 1);
+                // the padding (a zero on the row itself, on its first parent) is left out: the row reads both anyway
+                steps(o, [&](int i, Row& out) {
+                    for (int e = H.slice_ptr[i / S] + i % S; e < H.slice_ptr[i / S + 1]; e += S)
+                        if (H.ell_col[e] != i) out.emplace_back(at(o, H.ell_col[e]), H.ell_val[e]);
+                }, o.ep, o.ee);
+                steps(o, [&](int i, Row& out) {
+                    for (int e = H.op_slice_ptr[i / S] + i % S; e < H.op_slice_ptr[i / S + 1]; e += S)
+                        if (H.op_val[e] != 0.f || H.op_col[e] != H.pid[i].x) out.emplace_back(at(n, H.op_col[e]), H.op_val[e]);
+                }, o.op, o.oe);
+                for (int i = o.rb; i < o.re; ++i) {
+                    const int4 id = H.pid[i];
+                    o.pid.push_back(int4{at(n, id.x), at(n, id.y), at(n, id.z), at(n, id.w)});
+                    o.pw.push_back(H.pw[i]);
+                }
+                m.W = std::max(m.W, (size_t)(o.win.y - o.win.x));
+                m.ee = std::max(m.ee, o.ee.idx.size());
+                m.oe = std::max(m.oe, o.oe.idx.size());
+            }
+    // the layout, the same in every CTA: the image, then what the kernel writes
+    struct At {
+        int win, rp, ri, rv, ep, ei, ev, op, oi, ov, par, r, e, e2, res, dd;
+    };
+    std::vector<At> lay(L);
+    StagedPlan q{};
+    size_t bytes = 0;
+    auto room = [&](size_t b) {
+        const size_t a = bytes;
+        bytes += (b + 15) / 16 * 16;
+        return (int)std::min<size_t>(a, 1u << 30);
+    };
+    const int pre = h->p.pre_sweeps, post = h->p.post_sweeps;
+    const bool fused = h->fuse_prolong && post > 0;
+    const int levels = lc - split;   // levels above the coarsest
+    const int most_phases = levels * (1 + std::max(pre, 1) + 1 + post) + 2;
+    room(sizeof(StagedHead));
+    const int phase_at = room(most_phases * sizeof(StagedPhase)), load_at = room(levels * sizeof(StagedLoad));
+    for (int l = split; l < L; ++l) {
+        At& s = lay[l];
+        const Most& m = most[l];
+        s.win = room(kMaxCluster * sizeof(int2));
+        s.rp = room(4 * (m.slices + 1));
+        s.ri = room((l == split ? 4 : 2) * m.re);
+        s.rv = room(4 * m.re);
+        if (l == lc) break;
+        s.ep = room(4 * (m.slices + 1));
+        s.ei = room(2 * m.ee);
+        s.ev = room(4 * m.ee);
+        s.op = room(4 * (m.slices + 1));
+        s.oi = room(2 * m.oe);
+        s.ov = room(4 * m.oe);
+        s.par = room(32 * m.rows);
+        if (m.W > 65536) return;   // 2-byte rows
+    }
+    if (coarsest > 65536) return;
+    const size_t image = bytes;
+    for (int l = split; l < L; ++l) {
+        At& s = lay[l];
+        const Most& m = most[l];
+        s.r = room(16 * (l == lc ? coarsest : m.rows));
+        s.e = room(16 * (l == lc ? coarsest : m.W));
+        if (l == lc) break;
+        s.e2 = room(16 * m.W);
+        s.res = room(16 * m.W);
+        s.dd = room(8 * m.rows);
+    }
+    q.ainv = room(ainv * (h->p.precision == MGSB_PRECISION_MIXED ? 8 : 4));
+    if (bytes > (size_t)(h->max_smem_optin - kStagedStaticSmem)) return;
+    q.image_bytes = (int)image;
+    q.phase_at = phase_at;
+    q.bytes = (int)bytes;
+    // a warp per slice of the largest share, and per row of the coarsest: phases are latency, barriers grow with warps
+    size_t warps = 4;
+    for (int l = split; l < L; ++l) warps = std::max(warps, l == lc ? most[l].rows : most[l].slices);
+    q.block = (int)std::min<size_t>(32 * warps, kStagedThreads);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)cs);
+    cfg.blockDim = dim3((unsigned)q.block);
+    cfg.dynamicSmemBytes = bytes;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)cs;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int nclusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&nclusters, k_coarse_vcycle_staged, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return;
+    }
+    if (nclusters < 1) return;
+    // the images
+    h->staged_image.assign((size_t)nb * cs * image, 0);
+    for (int bi = 0; bi < nb; ++bi)
+        for (int k = 0; k < cs; ++k) {
+            unsigned char* img = h->staged_image.data() + ((size_t)bi * cs + k) * image;
+            auto put = [&](int to, const auto& v) {
+                if (!v.empty()) std::memcpy(img + to, v.data(), v.size() * sizeof(v[0]));
+            };
+            auto put_entries = [&](int idx, int val, const Entries& e, bool wide) {
+                if (wide)
+                    put(idx, e.idx);
+                else
+                    put(idx, std::vector<uint16_t>(e.idx.begin(), e.idx.end()));
+                put(val, e.val);
+            };
+            std::vector<StagedPhase> ph;
+            std::vector<StagedLoad> loads;
+            auto phase = [&](int l, int kind) -> StagedPhase& {
+                const Part& o = part(bi, k, l);
+                StagedPhase P{};
+                P.kind = kind;
+                P.many = o.slices;
+                P.first = o.first;
+                P.rb = o.rb;
+                P.re = o.re;
+                P.lo = o.win.x;
+                P.win = lay[l].win;
+                P.dd = lay[l].dd;
+                P.par = lay[l].par;
+                ph.push_back(P);
+                return ph.back();
+            };
+            auto sweep = [&](int l, int from, int to, int kind) -> StagedPhase& {
+                StagedPhase& P = phase(l, kind);
+                P.ptr = lay[l].ep;
+                P.idx = lay[l].ei;
+                P.val = lay[l].ev;
+                P.src = P.self = from;
+                P.rhs = lay[l].r;
+                P.rhs0 = P.rb;
+                P.dst = to;
+                return P;
+            };
+            auto other = [&](int l, int v) { return v == lay[l].e ? lay[l].e2 : lay[l].e; };
+            std::vector<int> cur(L);
+            for (int l = split; l < L; ++l) {
+                const Part& o = part(bi, k, l);
+                for (int j = 0; j < cs; ++j) {
+                    const int2 w = part(bi, j, l).win, window{w.x, w.y - w.x};
+                    std::memcpy(img + lay[l].win + j * sizeof(int2), &window, sizeof window);
+                }
+                put(lay[l].rp, o.rp);
+                put_entries(lay[l].ri, lay[l].rv, o.re_, l == split);
+                StagedPhase& R = phase(l, l == lc ? kStWhole : kStRestrict);
+                R.ptr = lay[l].rp;
+                R.idx = lay[l].ri;
+                R.val = lay[l].rv;
+                R.src = l == split ? -1 : lay[l - 1].res;
+                R.gsrc = l == split ? h->lev[l - 1].res : nullptr;
+                R.rhs = lay[l].r;
+                R.dst = l == lc ? lay[l].r : lay[l].e;
+                cur[l] = lay[l].e;
+                if (l == lc) break;
+                put(lay[l].ep, o.ep);
+                put_entries(lay[l].ei, lay[l].ev, o.ee, false);
+                put(lay[l].op, o.op);
+                put_entries(lay[l].oi, lay[l].ov, o.oe, false);
+                for (size_t r = 0; r < o.pid.size(); ++r) {
+                    std::memcpy(img + lay[l].par + 32 * r, &o.pid[r], 16);
+                    std::memcpy(img + lay[l].par + 32 * r + 16, &o.pw[r], 16);
+                }
+                loads.push_back(StagedLoad{o.rb, o.re - o.rb, lay[l].dd, 0, h->lev[l].dfull, h->lev[l].dinv});
+                R.zero = pre == 0;
+                for (int j = 1; j < pre; ++j) {
+                    sweep(l, cur[l], other(l, cur[l]), kStSweep);
+                    cur[l] = other(l, cur[l]);
+                }
+                sweep(l, cur[l], lay[l].res, kStResidual);
+            }
+            {
+                StagedPhase& P = phase(lc, kStDense);
+                P.many = 0;   // no slices: a warp per row
+                P.src = lay[lc].r;
+                P.dst = lay[lc].e;
+            }
+            for (int l = lc - 1; l >= split; --l) {
+                StagedPhase& P = phase(l, fused ? kStProlongSweep : kStProlong);
+                P.ptr = lay[l].op;
+                P.idx = lay[l].oi;
+                P.val = lay[l].ov;
+                P.src = cur[l + 1];
+                P.self = cur[l];
+                P.rhs = lay[l].res;
+                P.rhs0 = P.lo;
+                P.dst = cur[l] = fused ? other(l, cur[l]) : cur[l];
+                for (int j = fused ? 1 : 0; j < post; ++j) {
+                    sweep(l, cur[l], other(l, cur[l]), kStSweep);
+                    cur[l] = other(l, cur[l]);
+                }
+            }
+            ph.back().out = 1;
+            ph.back().gout = h->lev[split].e;
+            const Part& c = part(bi, k, lc);
+            const StagedHead head{(int)loads.size(), load_at, c.off, c.n, c.rb, c.re, {0, 0}};
+            q.phases = (int)ph.size();
+            std::memcpy(img, &head, sizeof head);
+            put(phase_at, ph);
+            put(load_at, loads);
+        }
+    h->staged = q;
+}
+
+// The staged kernel's plan and images for the current shape, if they are not there yet; the copy goes on the stream:
+// after the frames that ran with another shape's.
+// One body: the kernel with the operators in shared memory, over more CTAs than apply_tuning's rule takes (the remote
+// stores cost less than the issue slots of many warps in one SM: 16 CTAs against 8 and 4 take 9.5, 11.0 and 15.2 us
+// per V-cycle at 496 rows, 8.0, 8.0 and 8.6 us at 189 rows).  Many bodies fill the SMs without it: 128 beams of up to
+// 189 rows take 13.5 us with two CTAs each and 14.8 us with their images copied first.
+mgsb_status ready_staged(mgsb_solver* h) {
+    if (!h->staged_stale) return MGSB_OK;
+    h->staged = StagedPlan{};
+    h->staged_image.clear();
+    if (is_mg(h) && !h->fuse_l0 && !h->dense_op && h->bodies.size() == 1 && (int)h->coarse_host.size() == h->p.levels) {
+        if (h->tune_cluster > 1) {
+            plan_staged(h, h->cluster, h->split);
+        } else if (h->tune_cluster == 0) {
+            const int most = std::min(kMaxCluster, (h->maxv[h->split] + 15) / 16);
+            for (int cs : {16, 8, 4, 2}) {
+                if (cs > most && cs > 2) continue;
+                plan_staged(h, cs, h->split);
+                if (!h->staged.bytes) continue;
+                h->cluster = cs;
+                break;
+            }
+        }
+    }
+    if (h->staged.bytes) {
+        CUDA_TRY(h, cudaSetDevice(h->device));
+        const size_t n = h->staged_image.size();
+        if (n > h->staged_cap) {
+            CUDA_TRY(h, cudaStreamSynchronize(h->stream));
+            if (h->staged_dev) cudaFree(h->staged_dev);
+            h->staged_dev = nullptr;
+            h->staged_cap = 0;
+            if (cudaMalloc((void**)&h->staged_dev, n) != cudaSuccess) {
+                cudaGetLastError();
+                h->staged = StagedPlan{};
+                return set_err(h, MGSB_OUT_OF_MEMORY, "cudaMalloc(%zu) of the coarse kernel's images failed", n);
+            }
+            h->staged_cap = n;
+        }
+        CUDA_TRY(h, cudaMemcpyAsync(h->staged_dev, h->staged_image.data(), n, cudaMemcpyHostToDevice, h->stream));
+        CUDA_TRY(h, cudaStreamSynchronize(h->stream));
+        h->staged_image = std::vector<unsigned char>();
+        h->staged.image = h->staged_dev;
+    }
+    h->staged_stale = false;
+    return MGSB_OK;
+}
+
 // Can the device co-schedule one cluster of this shape?
 bool coarse_shape_feasible(mgsb_solver* h, int cs, int block, int fused, int split) {
     const size_t smem = fused ? 0 : coarse_smem_bytes(h, cs, split);
@@ -950,8 +1352,10 @@ mgsb_status launch_coarse(mgsb_solver* h, const CoarseArgs& args_in) {
 mgsb_status launch_coarse_cluster(mgsb_solver* h, const CoarseArgs& args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(h->bodies.size() * h->cluster));
-    cfg.blockDim = dim3((unsigned)h->coarse_block);
-    cfg.dynamicSmemBytes = h->fuse_l0 ? 0 : coarse_smem_bytes(h, h->cluster, args.first);
+    cfg.blockDim = dim3((unsigned)(h->staged.bytes ? h->staged.block : h->coarse_block));
+    cfg.dynamicSmemBytes = h->fuse_l0       ? 0
+                           : h->staged.bytes ? (size_t)h->staged.bytes
+                                             : coarse_smem_bytes(h, h->cluster, args.first);
     if (cfg.dynamicSmemBytes > (size_t)h->max_smem_optin) {
         h->enqueue_status = set_err(h, MGSB_NOT_SUPPORTED,
                                     "coarse kernel shape (cluster %d, split %d) needs %zu B of shared memory per CTA (max %d)",
@@ -975,13 +1379,14 @@ mgsb_status launch_coarse_cluster(mgsb_solver* h, const CoarseArgs& args) {
     }
     // fused: global-memory kernel that also owns the level-0 residual and prolongation;
     // one CTA: every owned level in one CTA's shared memory; else the
-    // distributed-shared-memory kernel over the cluster
+    // distributed-shared-memory kernels over the cluster, with the operators staged where they fit
     const int reps = prof_begin(h, "k_coarse_vcycle");
     cudaError_t e = cudaSuccess;
     for (int r = 0; r < reps && e == cudaSuccess; ++r)
         e = h->fuse_l0 ? cudaLaunchKernelEx(&cfg, k_coarse_vcycle, args)
-            : one_cta  ? cudaLaunchKernelEx(&cfg, k_coarse_vcycle_cta, args)
-                       : cudaLaunchKernelEx(&cfg, k_coarse_vcycle_dsm, args);
+            : one_cta         ? cudaLaunchKernelEx(&cfg, k_coarse_vcycle_cta, args)
+            : h->staged.bytes ? cudaLaunchKernelEx(&cfg, k_coarse_vcycle_staged, h->staged, args.Ainv, args.Ainv64, args.dense_off)
+                              : cudaLaunchKernelEx(&cfg, k_coarse_vcycle_dsm, args);
     prof_end(h, "k_coarse_vcycle");
     ++h->launches;
     if (e != cudaSuccess) {
@@ -1538,7 +1943,7 @@ void enqueue_frame(mgsb_solver* h) {
 
 mgsb_status ensure_ready(mgsb_solver* h) {
     if (h->dirty) TRY(rebuild(h));
-    return MGSB_OK;
+    return ready_staged(h);
 }
 
 mgsb_status push_tool(mgsb_solver* h) {
@@ -2388,6 +2793,7 @@ mgsb_status mgsb_set_broad_phase(mgsb_solver* h, int32_t on) {
 mgsb_status mgsb_set_fused_prolongation(mgsb_solver* h, int32_t on) {
     if (!h || (on != 0 && on != 1)) return MGSB_INVALID_ARG;
     h->fuse_prolong = on != 0;
+    apply_tuning(h);   // the staged kernel's phases
     invalidate_graph(h);
     return MGSB_OK;
 }
@@ -2502,6 +2908,8 @@ mgsb_status mgsb_autotune(mgsb_solver* h, int32_t frames, int32_t* chosen) {
         h->coarse_block = c.block;
         apply_tuning(h);
         invalidate_graph(h);
+        if ((st = ready_staged(h)) != MGSB_OK) break;
+        if (h->staged.bytes && c.block != 512) continue;   // it picks its own block size
         cudaMemsetAsync(h->fac_valid, 0, h->bodies.size() * sizeof(int32_t), h->stream);
         restore();
         st = step_once(h);   // warm-up: capture + coarsest factorisation
@@ -2823,6 +3231,7 @@ extern "C" mgsb_status mgsb_smoother_pairs(mgsb_solver* h, int32_t sweeps, float
     if (h->fuse_l0)
         return set_err(h, MGSB_NOT_SUPPORTED, "pair generation uses the shared-memory coarse kernel (fuse_level0 = 0)");
     TRY(sync_check(h));
+    TRY(ready_staged(h));
     const int n0 = h->N0;
     auto& pool = h->pair_mem;
     if (!h->ls_xf) {
@@ -2934,6 +3343,7 @@ extern "C" mgsb_status mgsb_vcycle_residuals(mgsb_solver* h, int32_t cycles, int
     if (mode == 2 && !h->ls_net) return set_err(h, MGSB_INVALID_ARG, "no learned smoother attached");
     if (h->fuse_l0) return set_err(h, MGSB_NOT_SUPPORTED, "needs the shared-memory coarse kernel (fuse_level0 = 0)");
     TRY(sync_check(h));
+    TRY(ready_staged(h));
     const int n0 = h->N0;
     auto& pool = h->pair_mem;
     if (!h->ls_xf) {
