@@ -412,153 +412,369 @@ __global__ void __launch_bounds__(kMlpThreads) k_mlp_tc(int n, int ntiles, const
 }
 
 // ---------------------------------------------------------------------------
-// Training: forward + backward for a block of 128 samples (one thread per
-// sample for the per-sample passes), FP32 math with the same BF16 rounding of
-// the weights and activations as the tensor-core forward (straight-through in
-// the backward).  Loss = mean over samples and the 3 outputs of (y - t)^2.
-// Activations live in shared memory feature-major ([unit][sample], row stride
-// 129 against bank conflicts); the weight gradients are then formed
-// cooperatively as dot products over the block's samples, so every block
-// writes its gradient sum to grad_part[block][kMlpParams] without atomics, and
-// k_mlp_reduce sums the blocks in a fixed order (deterministic).
+// Training: forward + backward, FP32 math with the same BF16 rounding of the
+// weights and activations as the tensor-core forward (straight-through in the
+// backward).  Loss = mean over samples and the 3 outputs of (y - t)^2.
+//
+// A step is a chain of two launches.  k_mlp_fwd_bwd takes 32 samples per CTA (a
+// sample per lane, 8 hidden units per warp) and leaves the rows that the weight
+// gradients multiply -- features, dZ1, H1, dZ2, H2, dY -- in global scratch, a
+// row per unit over all samples.  k_mlp_grad gives each CTA a tile of
+// parameters: their rows arrive in shared memory by bulk copies, a thread forms
+// the dot products of one 128-sample block, and the blocks are added in
+// ascending order, without atomics (deterministic); the same thread then takes
+// the Adam step.  Both kernels fill the chip at 4,096 samples (128 and 127 CTAs
+// of 148 SMs); one CTA per 128 samples for everything, as before, left 116 SMs
+// idle: 100 steps on 200,000 pairs took 10.1 ms with its four small launches, and
+// take 3.2 ms (the upload of the pairs included).  Every sum runs in the order of
+// that form: the same bits.
 // ---------------------------------------------------------------------------
-constexpr int kTrainThreads = 128;
-constexpr int kTrainLd = kTrainThreads + 1;
-constexpr size_t kTrainSmem =
-    sizeof(float) * ((size_t)kMlpParams + (4 * kMlpHid + kMlpIn + kMlpOut) * (size_t)kTrainLd + kTrainThreads);
+constexpr int kTrainThreads = 256;            // 8 warps of 8 hidden units each
+constexpr int kTrainSamples = 32;             // per CTA
+constexpr int kGradBlock = 128;               // samples of one dot product
+constexpr int kGradLd = kGradBlock + 4;       // its place in a scratch row: 16-byte reads of 8 blocks miss no bank
+constexpr int kTrainChunk = 8192;             // samples of one launch pair at most (9 MB of scratch)
+// scratch rows
+constexpr int kActX = 0, kActZ1 = kActX + kMlpIn, kActH1 = kActZ1 + kMlpHid, kActZ2 = kActH1 + kMlpHid,
+              kActH2 = kActZ2 + kMlpHid, kActY = kActH2 + kMlpHid, kActRows = kActY + kMlpOut;
 
-__global__ void __launch_bounds__(kTrainThreads) k_mlp_fwd_bwd(int nb, const int32_t* __restrict__ idx,
-                                                               const float* __restrict__ X, const float* __restrict__ T,
-                                                               const float* __restrict__ prm, float* __restrict__ grad_part,
-                                                               float* __restrict__ loss_part, float inv_count) {
-    extern __shared__ float tsm[];
-    float* w = tsm;                                   // BF16-rounded weights, exact biases
-    float* Z1 = w + kMlpParams;                       // [64][129] pre-activations, then dZ1
-    float* H1 = Z1 + kMlpHid * kTrainLd;              // [64][129]
-    float* Z2 = H1 + kMlpHid * kTrainLd;              // [64][129] then dZ2
-    float* H2 = Z2 + kMlpHid * kTrainLd;              // [64][129]
-    float* Xs = H2 + kMlpHid * kTrainLd;              // [9][129]
-    float* dY = Xs + kMlpIn * kTrainLd;               // [3][129]
-    float* lsum = dY + kMlpOut * kTrainLd;            // [128]
-    for (int q = threadIdx.x; q < kMlpParams; q += blockDim.x) {
-        const bool is_bias = (q >= kOffB1 && q < kOffW2) || (q >= kOffB2 && q < kOffW3) || q >= kOffB3;
-        w[q] = is_bias ? prm[q] : bf16r(prm[q]);
+__host__ __device__ inline int train_blocks(int n) { return (n + kGradBlock - 1) / kGradBlock; }
+
+struct TrainSmem {
+    float w1[kMlpIn][kMlpHid];     // [k][j]
+    float w2t[kMlpHid][kMlpHid + 4];   // [k][j], forward (the transposing stores meet 4 to a bank)
+    float w2[kMlpHid][kMlpHid];    // [j][k], backward
+    float w3[kMlpOut][kMlpHid];
+    float b1[kMlpHid], b2[kMlpHid], b3[kMlpOut + 1];
+    float x[kMlpIn][kTrainSamples];
+    float h1[kMlpHid][kTrainSamples], h2[kMlpHid][kTrainSamples], z2[kMlpHid][kTrainSamples];
+    float d[kMlpOut][kTrainSamples], dy[kMlpOut][kTrainSamples];
+};
+
+// Row of sample s of a minibatch: s itself, or uniform in [0, n) from a counter-based hash (splitmix64).
+struct SampleOf {
+    int sampled, first, n;
+    uint64_t seed, step;
+    __device__ __forceinline__ int operator()(int s) const {
+        if (!sampled) return first + s;
+        uint64_t z = seed + (step * 0x9E3779B97F4A7C15ull) + (uint64_t)(first + s) * 0xBF58476D1CE4E5B9ull;
+        z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
+        z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
+        z ^= z >> 31;
+        return (int)(z % (uint64_t)n);
     }
-    __syncthreads();
-    const int s = threadIdx.x;
-    const int gs = blockIdx.x * blockDim.x + s;
+};
+
+// nb samples of this launch; ld: floats of a scratch row.  lsum[s]: the sample's squared error.
+__global__ void __launch_bounds__(kTrainThreads) k_mlp_fwd_bwd(int nb, SampleOf sample, const float* __restrict__ X,
+                                                               const float* __restrict__ T, const float* __restrict__ prm,
+                                                               float* __restrict__ act, int ld, float* __restrict__ lsum,
+                                                               float inv_count) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    extern __shared__ __align__(16) unsigned char train_smem[];
+    TrainSmem& S = *reinterpret_cast<TrainSmem*>(train_smem);
+    const int s = threadIdx.x & 31, warp = threadIdx.x >> 5, j0 = 8 * warp;
+    const int gs = blockIdx.x * kTrainSamples + s;
     const bool valid = gs < nb;
-    const int row = valid ? (idx ? idx[gs] : gs) : 0;
-    // ---- forward
-    float loss = 0.f;
-    for (int k = 0; k < kMlpIn; ++k) Xs[k * kTrainLd + s] = valid ? bf16r(X[(size_t)row * kMlpIn + k]) : 0.f;
-    for (int j = 0; j < kMlpHid; ++j) {
-        float a = w[kOffB1 + j];
-        for (int k = 0; k < kMlpIn; ++k) a = fmaf(w[kOffW1 + j * kMlpIn + k], Xs[k * kTrainLd + s], a);
-        Z1[j * kTrainLd + s] = a;
-        H1[j * kTrainLd + s] = bf16r(gelu(a));
+    // the samples are not written by any kernel of a training run: read before the wait
+    const int row = valid ? sample(gs) : 0;
+    for (int k = warp; k < kMlpIn; k += kTrainThreads / 32) S.x[k][s] = valid ? bf16r(X[(size_t)row * kMlpIn + k]) : 0.f;
+    const float target = valid && warp < kMlpOut ? T[(size_t)row * kMlpOut + warp] : 0.f;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    // weights, BF16-rounded, and exact biases
+    for (int q = threadIdx.x; q < kMlpHid * kMlpHid; q += kTrainThreads) {
+        const float w = bf16r(prm[kOffW2 + q]);
+        S.w2[q / kMlpHid][q % kMlpHid] = w;
+        S.w2t[q % kMlpHid][q / kMlpHid] = w;
     }
-    for (int j = 0; j < kMlpHid; ++j) {
-        float a = w[kOffB2 + j];
-        for (int k = 0; k < kMlpHid; ++k) a = fmaf(w[kOffW2 + j * kMlpHid + k], H1[k * kTrainLd + s], a);
-        Z2[j * kTrainLd + s] = a;
-        H2[j * kTrainLd + s] = bf16r(gelu(a));
+    for (int q = threadIdx.x; q < kMlpHid * kMlpIn; q += kTrainThreads) S.w1[q % kMlpIn][q / kMlpIn] = bf16r(prm[kOffW1 + q]);
+    if (threadIdx.x < kMlpOut * kMlpHid) S.w3[threadIdx.x / kMlpHid][threadIdx.x % kMlpHid] = bf16r(prm[kOffW3 + threadIdx.x]);
+    if (threadIdx.x < kMlpHid) {
+        S.b1[threadIdx.x] = prm[kOffB1 + threadIdx.x];
+        S.b2[threadIdx.x] = prm[kOffB2 + threadIdx.x];
     }
-    for (int o = 0; o < kMlpOut; ++o) {
-        float a = w[kOffB3 + o];
-        for (int k = 0; k < kMlpHid; ++k) a = fmaf(w[kOffW3 + o * kMlpHid + k], H2[k * kTrainLd + s], a);
-        const float d = valid ? a - T[(size_t)row * kMlpOut + o] : 0.f;
-        loss += d * d;
-        dY[o * kTrainLd + s] = 2.f * d * inv_count;
-    }
-    // ---- backward through layer 3 and 2 (own sample only)
-    for (int k = 0; k < kMlpHid; ++k) {
-        float a = 0.f;
-        for (int o = 0; o < kMlpOut; ++o) a = fmaf(dY[o * kTrainLd + s], w[kOffW3 + o * kMlpHid + k], a);
-        Z2[k * kTrainLd + s] = a * gelu_grad(Z2[k * kTrainLd + s]);   // dZ2
-    }
-    for (int k = 0; k < kMlpHid; ++k) {
-        float a = 0.f;
-        for (int j = 0; j < kMlpHid; ++j) a = fmaf(Z2[j * kTrainLd + s], w[kOffW2 + j * kMlpHid + k], a);
-        Z1[k * kTrainLd + s] = a * gelu_grad(Z1[k * kTrainLd + s]);   // dZ1
-    }
-    lsum[s] = loss;
+    if (threadIdx.x < kMlpOut) S.b3[threadIdx.x] = prm[kOffB3 + threadIdx.x];
     __syncthreads();
-    // ---- weight gradients: dot products over the block's samples
-    float* gp = grad_part + (size_t)blockIdx.x * kMlpParams;
-    for (int q = threadIdx.x; q < kMlpParams; q += blockDim.x) {
-        const float *u, *v = nullptr;
-        if (q < kOffB1) {
-            const int j = (q - kOffW1) / kMlpIn, i = (q - kOffW1) % kMlpIn;
-            u = Z1 + j * kTrainLd;
-            v = Xs + i * kTrainLd;
-        } else if (q < kOffW2) {
-            u = Z1 + (q - kOffB1) * kTrainLd;
-        } else if (q < kOffB2) {
-            const int j = (q - kOffW2) / kMlpHid, k = (q - kOffW2) % kMlpHid;
-            u = Z2 + j * kTrainLd;
-            v = H1 + k * kTrainLd;
-        } else if (q < kOffW3) {
-            u = Z2 + (q - kOffB2) * kTrainLd;
-        } else if (q < kOffB3) {
-            const int o = (q - kOffW3) / kMlpHid, k = (q - kOffW3) % kMlpHid;
-            u = dY + o * kTrainLd;
-            v = H2 + k * kTrainLd;
-        } else {
-            u = dY + (q - kOffB3) * kTrainLd;
+    auto row8 = [](const float* p, float (&w)[8]) {
+        const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
+        w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w;
+        w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
+    };
+    // place of this sample in the scratch rows
+    float* at = act + (size_t)(gs / kGradBlock) * kGradLd + gs % kGradBlock;
+    for (int k = warp; k < kMlpIn; k += kTrainThreads / 32) at[(size_t)(kActX + k) * ld] = S.x[k][s];
+    // ---- forward
+    float z1[8], z2[8], w[8];
+    row8(S.b1 + j0, z1);
+#pragma unroll
+    for (int k = 0; k < kMlpIn; ++k) {
+        row8(&S.w1[k][j0], w);
+        const float x = S.x[k][s];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) z1[u] = fmaf(w[u], x, z1[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+        const float h = bf16r(gelu(z1[u]));
+        S.h1[j0 + u][s] = h;
+        at[(size_t)(kActH1 + j0 + u) * ld] = h;
+    }
+    __syncthreads();
+    row8(S.b2 + j0, z2);
+#pragma unroll 8
+    for (int k = 0; k < kMlpHid; ++k) {
+        row8(&S.w2t[k][j0], w);
+        const float h = S.h1[k][s];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) z2[u] = fmaf(w[u], h, z2[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+        const float h = bf16r(gelu(z2[u]));
+        S.h2[j0 + u][s] = h;
+        at[(size_t)(kActH2 + j0 + u) * ld] = h;
+    }
+    __syncthreads();
+    if (warp < kMlpOut) {
+        float a = S.b3[warp];
+#pragma unroll 16
+        for (int k = 0; k < kMlpHid; ++k) a = fmaf(S.w3[warp][k], S.h2[k][s], a);
+        const float d = valid ? a - target : 0.f;
+        const float dy = 2.f * d * inv_count;
+        S.d[warp][s] = d;
+        S.dy[warp][s] = dy;
+        at[(size_t)(kActY + warp) * ld] = dy;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        float loss = 0.f;
+#pragma unroll
+        for (int o = 0; o < kMlpOut; ++o) {
+            const float d = S.d[o][s];
+            loss += d * d;
         }
+        lsum[gs] = loss;
+    }
+    // ---- backward through layers 3 and 2
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
         float a = 0.f;
-        if (v)
-            for (int t = 0; t < kTrainThreads; ++t) a = fmaf(u[t], v[t], a);
-        else
-            for (int t = 0; t < kTrainThreads; ++t) a += u[t];
-        gp[q] = a;
+#pragma unroll
+        for (int o = 0; o < kMlpOut; ++o) a = fmaf(S.dy[o][s], S.w3[o][j0 + u], a);
+        const float z = a * gelu_grad(z2[u]);
+        S.z2[j0 + u][s] = z;
+        at[(size_t)(kActZ2 + j0 + u) * ld] = z;
     }
-    if (threadIdx.x == 0) {
-        float t = 0.f;
-        for (int i = 0; i < kTrainThreads; ++i) t += lsum[i];
-        loss_part[blockIdx.x] = t;
+    __syncthreads();
+    float a1[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) a1[u] = 0.f;
+#pragma unroll 8
+    for (int j = 0; j < kMlpHid; ++j) {
+        row8(&S.w2[j][j0], w);
+        const float z = S.z2[j][s];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) a1[u] = fmaf(z, w[u], a1[u]);
     }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) at[(size_t)(kActZ1 + j0 + u) * ld] = a1[u] * gelu_grad(z1[u]);
 }
 
-// grad[q] = sum_b grad_part[b][q] (fixed order); loss = sum_b loss_part[b] * inv_count.
-__global__ void k_mlp_reduce(int nblk, const float* __restrict__ grad_part, const float* __restrict__ loss_part,
-                             float inv_count, float* __restrict__ grad, float* __restrict__ loss) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q < kMlpParams) {
-        float a = 0.f;
-        for (int b = 0; b < nblk; ++b) a += grad_part[(size_t)b * kMlpParams + q];
-        grad[q] = a;
-    }
-    if (q == 0) {
-        float l = 0.f;
-        for (int b = 0; b < nblk; ++b) l += loss_part[b];
-        *loss = l * inv_count;
-    }
-}
-
-// Adam (Kingma & Ba 2015) on the FP32 master parameters; step t >= 1.
-__global__ void k_adam(float* __restrict__ prm, const float* __restrict__ grad, float* __restrict__ m,
-                       float* __restrict__ v, float lr, float b1, float b2, float eps, float bc1, float bc2) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= kMlpParams) return;
-    const float gq = grad[q];
-    const float mq = b1 * m[q] + (1.f - b1) * gq;
-    const float vq = b2 * v[q] + (1.f - b2) * gq * gq;
+// Adam (Kingma & Ba 2015) on one FP32 master parameter.
+struct AdamStep {
+    float lr, b1, b2, eps, bc1, bc2;
+};
+__device__ __forceinline__ void adam(float gq, float* prm, float* m, float* v, int q, const AdamStep& A) {
+    const float mq = A.b1 * m[q] + (1.f - A.b1) * gq;
+    const float vq = A.b2 * v[q] + (1.f - A.b2) * gq * gq;
     m[q] = mq;
     v[q] = vq;
-    prm[q] -= lr * (mq / bc1) / (sqrtf(vq / bc2) + eps);
+    prm[q] -= A.lr * (mq / A.bc1) / (sqrtf(vq / A.bc2) + A.eps);
 }
 
-// Uniform sample indices in [0, n) from a counter-based hash (splitmix64).
-__global__ void k_sample_indices(int nb, int n, uint64_t seed, uint64_t step, int32_t* __restrict__ idx) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= nb) return;
-    uint64_t z = seed + (step * 0x9E3779B97F4A7C15ull) + (uint64_t)s * 0xBF58476D1CE4E5B9ull;
-    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
-    z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
-    z ^= z >> 31;
-    idx[s] = (int32_t)(z % (uint64_t)n);
+// Parameter tiles: rows u of one scratch group against rows v of another, 13 rows of shared memory at most.
+constexpr int kGradGroups = 32;   // blocks of 128 samples in shared memory at a time, a lane each
+constexpr int kGradThreads = 64;  // two halves of the tile, 32 blocks each
+constexpr int kGradRows = 13;
+constexpr int kTiles2 = 8 * 13;   // W2: 8 x 5 parameters of dZ2 x H1
+constexpr int kTiles1 = 16;       // W1: 4 x 9 of dZ1 x features
+constexpr int kTiles3 = 7;        // W3: 3 x 10 of dY x H2
+constexpr int kGradTiles = kTiles2 + kTiles1 + kTiles3;
+constexpr int kGradParams = 48;   // most parameters of a tile, biases included
+
+struct GradSmem {
+    alignas(128) float row[kGradRows][kGradGroups * kGradLd];
+    float part[kGradParams][kGradGroups + 1];
+    float loss[kGradGroups];
+    uint64_t bar;
+};
+
+// Dot products of MU rows u and MV rows v over one block of 128 samples, and the sums of the rows u.
+template <int MU, int MV>
+__device__ __forceinline__ void grad_dots(const float* const (&u)[MU], const float* const (&v)[MV], float (&dot)[MU][MV],
+                                          float (&sum)[MU]) {
+#pragma unroll
+    for (int i = 0; i < MU; ++i) {
+        sum[i] = 0.f;
+#pragma unroll
+        for (int j = 0; j < MV; ++j) dot[i][j] = 0.f;
+    }
+#pragma unroll 2
+    for (int t = 0; t < kGradBlock; t += 4) {
+        float a[MU][4], b[MV][4];
+#pragma unroll
+        for (int i = 0; i < MU; ++i) {
+            const float4 q = *reinterpret_cast<const float4*>(u[i] + t);
+            a[i][0] = q.x; a[i][1] = q.y; a[i][2] = q.z; a[i][3] = q.w;
+        }
+#pragma unroll
+        for (int j = 0; j < MV; ++j) {
+            const float4 q = *reinterpret_cast<const float4*>(v[j] + t);
+            b[j][0] = q.x; b[j][1] = q.y; b[j][2] = q.z; b[j][3] = q.w;
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+#pragma unroll
+            for (int i = 0; i < MU; ++i) {
+                sum[i] += a[i][k];
+#pragma unroll
+                for (int j = 0; j < MV; ++j) dot[i][j] = fmaf(a[i][k], b[j][k], dot[i][j]);
+            }
+    }
+}
+
+// One thread's share of a tile: rows u0.. and v0.. of S.row, block `lane`; parameter (i, j) of the tile's U x V goes to
+// part[i * V + j], the sums of the rows u to part[U * V + i].
+template <int MU, int MV>
+__device__ __forceinline__ void grad_tile(GradSmem& S, int lane, int u0, int v0, int U, int V, int i0, int j0, bool sums) {
+    const float *u[MU], *v[MV];
+#pragma unroll
+    for (int i = 0; i < MU; ++i) u[i] = S.row[u0 + i] + lane * kGradLd;
+#pragma unroll
+    for (int j = 0; j < MV; ++j) v[j] = S.row[v0 + j] + lane * kGradLd;
+    float dot[MU][MV], sum[MU];
+    grad_dots<MU, MV>(u, v, dot, sum);
+#pragma unroll
+    for (int i = 0; i < MU; ++i) {
+#pragma unroll
+        for (int j = 0; j < MV; ++j)
+            if (j0 + j < V) S.part[(i0 + i) * V + j0 + j][lane] = dot[i][j];   // else a row past a narrower tile
+        if (sums) S.part[U * V + i0 + i][lane] = sum[i];
+    }
+}
+
+// Gradient of a launch's nblk blocks of 128 samples, tile blockIdx.x.  acc: the sums of the launches before it (grad,
+// loss), else 0.  final: inv_count scales the loss, and with prm the Adam step is taken; else the sums stay in grad.
+__global__ void __launch_bounds__(kGradThreads) k_mlp_grad(int nblk, const float* __restrict__ act, int ld,
+                                                           const float* __restrict__ lsum, int acc, int final, float inv_count,
+                                                           float* __restrict__ grad, float* __restrict__ loss,
+                                                           float* __restrict__ loss_out, float* __restrict__ prm,
+                                                           float* __restrict__ m, float* __restrict__ v, AdamStep A,
+                                                           int32_t* __restrict__ err) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    extern __shared__ __align__(128) unsigned char grad_smem[];
+    GradSmem& S = *reinterpret_cast<GradSmem*>(grad_smem);
+    const int lane = threadIdx.x & 31, half = threadIdx.x >> 5;
+    // the tile: U rows from u_at against V rows from v_at; its first parameter and row stride; its biases
+    int U, V, u_at, v_at, q0, stride, bias = -1;
+    int tile = blockIdx.x;
+    const int kind = tile < kTiles2 ? 2 : tile < kTiles2 + kTiles1 ? 1 : 3;
+    if (kind == 2) {
+        const int r = tile / 13, c = tile % 13;
+        U = 8;
+        V = min(5, kMlpHid - 5 * c);
+        u_at = kActZ2 + 8 * r;
+        v_at = kActH1 + 5 * c;
+        q0 = kOffW2 + 8 * r * kMlpHid + 5 * c;
+        stride = kMlpHid;
+        if (c == 0) bias = kOffB2 + 8 * r;
+    } else if (kind == 1) {
+        tile -= kTiles2;
+        U = 4;
+        V = kMlpIn;
+        u_at = kActZ1 + 4 * tile;
+        v_at = kActX;
+        q0 = kOffW1 + 4 * tile * kMlpIn;
+        stride = kMlpIn;
+        bias = kOffB1 + 4 * tile;
+    } else {
+        tile -= kTiles2 + kTiles1;
+        U = kMlpOut;
+        V = min(10, kMlpHid - 10 * tile);
+        u_at = kActY;
+        v_at = kActH2 + 10 * tile;
+        q0 = kOffW3 + 10 * tile;
+        stride = kMlpHid;
+        if (tile == 0) bias = kOffB3;
+    }
+    const int many = U * V + (bias >= 0 ? U : 0);   // parameters of the tile
+    auto param = [&](int p) { return p < U * V ? q0 + p / V * stride + p % V : bias + p - U * V; };
+    if (threadIdx.x == 0) {
+        mbar_init(&S.bar, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    float g = 0.f, l = 0.f;   // this thread's parameter; thread 0 of the first tile: the loss
+    if (acc && threadIdx.x < many) g = grad[param(threadIdx.x)];
+    const bool loss_tile = blockIdx.x == gridDim.x - 1;   // the smallest
+    if (acc && loss_tile && threadIdx.x == 0) l = *loss;
+    bool ok = true;
+    uint32_t phase = 0;
+    for (int b0 = 0; b0 < nblk && ok; b0 += kGradGroups, phase ^= 1) {
+        const int nb = min(kGradGroups, nblk - b0);
+        if (threadIdx.x == 0) {
+            mbar_expect_tx(&S.bar, (uint32_t)((U + V) * nb * kGradLd * 4));
+            for (int r = 0; r < U + V; ++r)
+                bulk_g2s(S.row[r], act + (size_t)(r < U ? u_at + r : v_at + r - U) * ld + (size_t)b0 * kGradLd,
+                         (uint32_t)(nb * kGradLd * 4), &S.bar);
+        }
+        if (loss_tile && half == 1 && lane < nb) {   // the blocks' losses, in sample order
+            const float4* p = reinterpret_cast<const float4*>(lsum + (size_t)(b0 + lane) * kGradBlock);
+            float t = 0.f;
+#pragma unroll 8
+            for (int i = 0; i < kGradBlock / 4; ++i) {
+                const float4 q = __ldg(p + i);
+                t += q.x;
+                t += q.y;
+                t += q.z;
+                t += q.w;
+            }
+            S.loss[lane] = t;
+        }
+        ok = mbar_wait(&S.bar, phase, kMaxPolls);
+        if (ok && lane < nb) {
+            if (kind == 2)
+                grad_tile<4, 5>(S, lane, 4 * half, U, U, V, 4 * half, 0, bias >= 0);
+            else if (kind == 1)
+                grad_tile<2, 9>(S, lane, 2 * half, U, U, V, 2 * half, 0, true);
+            else
+                grad_tile<3, 5>(S, lane, 0, U + 5 * half, U, V, 0, 5 * half, bias >= 0 && half == 0);
+        }
+        __syncthreads();
+        if (ok && threadIdx.x < many)
+            for (int b = 0; b < nb; ++b) g += S.part[threadIdx.x][b];
+        if (loss_tile && threadIdx.x == 0)
+            for (int b = 0; b < nb; ++b) l += S.loss[b];
+        __syncthreads();
+    }
+    if (!ok) {   // report, and leave no copy in flight
+        if (threadIdx.x == 0) atomicExch(err, 1);
+        mbar_wait(&S.bar, phase ^ 1, kMaxPolls);
+        return;
+    }
+    if (threadIdx.x < many) {
+        const int q = param(threadIdx.x);
+        if (final && prm)
+            adam(g, prm, m, v, q, A);
+        else
+            grad[q] = g;
+    }
+    if (loss_tile && threadIdx.x == 0) {
+        if (final) l *= inv_count;
+        *loss = l;
+        if (final && loss_out) *loss_out = l;
+    }
 }
 
 }  // namespace

@@ -23,11 +23,9 @@ struct mgsb_mlp {
     float *prm = nullptr, *m = nullptr, *v = nullptr, *grad = nullptr, *loss = nullptr;
     uint8_t* img = nullptr;
     int adam_t = 0;
-    // growable scratch
-    float *grad_part = nullptr, *loss_part = nullptr;
-    int part_cap = 0;
-    int32_t* idx = nullptr;
-    int idx_cap = 0;
+    // growable scratch: the rows of a training launch (at most kTrainChunk samples) and its samples' errors
+    float *act = nullptr, *lsum = nullptr;
+    int act_cap = 0;   // blocks of 128 samples
     float *X = nullptr, *T = nullptr, *Y = nullptr;
     uint8_t* tiles = nullptr;
     size_t data_cap = 0;
@@ -38,8 +36,8 @@ struct mgsb_mlp {
 mgsb_mlp::~mgsb_mlp() {
     cudaSetDevice(device);
     if (stream) cudaStreamSynchronize(stream);
-    for (void* p : {(void*)prm, (void*)m, (void*)v, (void*)grad, (void*)loss, (void*)img, (void*)grad_part,
-                    (void*)loss_part, (void*)idx, (void*)X, (void*)T, (void*)Y, (void*)tiles, (void*)werr})
+    for (void* p : {(void*)prm, (void*)m, (void*)v, (void*)grad, (void*)loss, (void*)img, (void*)act,
+                    (void*)lsum, (void*)X, (void*)T, (void*)Y, (void*)tiles, (void*)werr})
         if (p) cudaFree(p);
     if (stream) cudaStreamDestroy(stream);
 }
@@ -84,19 +82,16 @@ mgsb_status ensure_data(mgsb_mlp* h, size_t n) {
     return MGSB_OK;
 }
 
-mgsb_status ensure_parts(mgsb_mlp* h, int nblk, int nidx) {
-    if (nblk > h->part_cap) {
-        if (h->grad_part) cudaFree(h->grad_part);
-        if (h->loss_part) cudaFree(h->loss_part);
-        MLP_CUDA(h, cudaMalloc(&h->grad_part, (size_t)nblk * kMlpParams * sizeof(float)));
-        MLP_CUDA(h, cudaMalloc(&h->loss_part, (size_t)nblk * sizeof(float)));
-        h->part_cap = nblk;
-    }
-    if (nidx > h->idx_cap) {
-        if (h->idx) cudaFree(h->idx);
-        MLP_CUDA(h, cudaMalloc(&h->idx, (size_t)nidx * sizeof(int32_t)));
-        h->idx_cap = nidx;
-    }
+mgsb_status ensure_act(mgsb_mlp* h, int samples) {
+    const int nblk = train_blocks(std::min(samples, kTrainChunk));
+    if (nblk <= h->act_cap) return MGSB_OK;
+    if (h->act) cudaFree(h->act);
+    if (h->lsum) cudaFree(h->lsum);
+    h->act = h->lsum = nullptr;
+    h->act_cap = 0;
+    MLP_CUDA(h, cudaMalloc(&h->act, (size_t)kActRows * nblk * kGradLd * sizeof(float)));
+    MLP_CUDA(h, cudaMalloc(&h->lsum, (size_t)nblk * kGradBlock * sizeof(float)));
+    h->act_cap = nblk;
     return MGSB_OK;
 }
 
@@ -106,16 +101,46 @@ mgsb_status repack(mgsb_mlp* h) {
     return MGSB_OK;
 }
 
-// Gradient of the mean squared error over `nb` samples (rows idx[] of X/T, or
-// rows 0..nb-1 when idx is null) into h->grad, loss into h->loss.
-mgsb_status launch_grad(mgsb_mlp* h, int nb, const int32_t* idx, const float* X, const float* T) {
-    const int nblk = (nb + kTrainThreads - 1) / kTrainThreads;
-    MLP_TRY(ensure_parts(h, nblk, 0));
+// Kernel launch that may start while the one before it finishes (both wait for it before they touch its results).
+template <typename... KArgs, typename... Args>
+cudaError_t launch_after(mgsb_mlp* h, void (*kernel)(KArgs...), int grid, int block, size_t smem, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = h->stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+// Mean squared error over `nb` samples (rows 0..nb-1 of X/T, or sampled), kTrainChunk of them per launch pair.  With
+// adam the parameters take the step and loss_out (optional) gets the loss; else the gradient is left in h->grad and
+// the loss in h->loss.
+mgsb_status launch_grad(mgsb_mlp* h, int nb, SampleOf sample, const AdamStep* step, float* loss_out) {
+    MLP_TRY(ensure_act(h, nb));
     const float inv = 1.f / (float)(nb * kMlpOut);
-    k_mlp_fwd_bwd<<<nblk, kTrainThreads, kTrainSmem, h->stream>>>(nb, idx, X, T, h->prm, h->grad_part, h->loss_part, inv);
-    k_mlp_reduce<<<(kMlpParams + 255) / 256, 256, 0, h->stream>>>(nblk, h->grad_part, h->loss_part, inv, h->grad, h->loss);
-    MLP_CUDA(h, cudaGetLastError());
+    for (int at = 0; at < nb; at += kTrainChunk) {
+        const int n = std::min(kTrainChunk, nb - at), nblk = train_blocks(n), ld = nblk * kGradLd;
+        sample.first = at;
+        MLP_CUDA(h, launch_after(h, k_mlp_fwd_bwd, nblk * (kGradBlock / kTrainSamples), kTrainThreads, sizeof(TrainSmem), n,
+                                 sample, (const float*)h->X, (const float*)h->T, (const float*)h->prm, h->act, ld, h->lsum, inv));
+        MLP_CUDA(h, launch_after(h, k_mlp_grad, kGradTiles, kGradThreads, sizeof(GradSmem), nblk, (const float*)h->act, ld,
+                                 (const float*)h->lsum, at > 0 ? 1 : 0, at + n == nb ? 1 : 0, inv, h->grad, h->loss, loss_out,
+                                 step ? h->prm : (float*)nullptr, h->m, h->v, step ? *step : AdamStep{}, h->werr));
+    }
     return MGSB_OK;
+}
+
+// The training kernels' bounded waits.
+mgsb_status check_waits(mgsb_mlp* h) {
+    int32_t werr = 0;
+    MLP_CUDA(h, cudaMemcpyAsync(&werr, h->werr, sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
+    MLP_CUDA(h, cudaStreamSynchronize(h->stream));
+    return werr ? mlp_err(h, MGSB_TIMEOUT, "network training: a bounded wait ran out") : MGSB_OK;
 }
 
 // Deterministic initialisation (uniform +-sqrt(6/(fan_in+fan_out)), zero biases).
@@ -165,7 +190,8 @@ mgsb_status mgsb_mlp_create(int32_t device, uint64_t seed, mgsb_mlp** out) {
     if (cudaMalloc(&h->prm, pb) || cudaMalloc(&h->m, pb) || cudaMalloc(&h->v, pb) || cudaMalloc(&h->grad, pb) ||
         cudaMalloc(&h->loss, sizeof(float)) || cudaMalloc(&h->img, kImgBytes) || cudaMalloc(&h->werr, sizeof(int32_t)))
         return fail(MGSB_OUT_OF_MEMORY);
-    if (cudaFuncSetAttribute(k_mlp_fwd_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrainSmem) ||
+    if (cudaFuncSetAttribute(k_mlp_fwd_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TrainSmem)) ||
+        cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GradSmem)) ||
         cudaFuncSetAttribute(k_mlp_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mlp_tc_smem()))
         return fail(MGSB_CUDA_ERROR);
     std::vector<float> p;
@@ -240,12 +266,12 @@ mgsb_status mgsb_mlp_loss_grad(mgsb_mlp* h, const float* x, const float* t, int3
     MLP_TRY(ensure_data(h, n));
     MLP_CUDA(h, cudaMemcpyAsync(h->X, x, (size_t)n * kMlpIn * sizeof(float), cudaMemcpyHostToDevice, h->stream));
     MLP_CUDA(h, cudaMemcpyAsync(h->T, t, (size_t)n * kMlpOut * sizeof(float), cudaMemcpyHostToDevice, h->stream));
-    MLP_TRY(launch_grad(h, n, nullptr, h->X, h->T));
+    MLP_CUDA(h, cudaMemsetAsync(h->werr, 0, sizeof(int32_t), h->stream));
+    MLP_TRY(launch_grad(h, n, SampleOf{0, 0, n, 0, 0}, nullptr, nullptr));
     if (grad)
         MLP_CUDA(h, cudaMemcpyAsync(grad, h->grad, kMlpParams * sizeof(float), cudaMemcpyDeviceToHost, h->stream));
     if (loss) MLP_CUDA(h, cudaMemcpyAsync(loss, h->loss, sizeof(float), cudaMemcpyDeviceToHost, h->stream));
-    MLP_CUDA(h, cudaStreamSynchronize(h->stream));
-    return MGSB_OK;
+    return check_waits(h);
 }
 
 mgsb_status mgsb_mlp_train(mgsb_mlp* h, const float* x, const float* t, int64_t n, int32_t steps, int32_t batch,
@@ -255,7 +281,8 @@ mgsb_status mgsb_mlp_train(mgsb_mlp* h, const float* x, const float* t, int64_t 
     MLP_TRY(ensure_data(h, (size_t)n));
     MLP_CUDA(h, cudaMemcpyAsync(h->X, x, (size_t)n * kMlpIn * sizeof(float), cudaMemcpyHostToDevice, h->stream));
     MLP_CUDA(h, cudaMemcpyAsync(h->T, t, (size_t)n * kMlpOut * sizeof(float), cudaMemcpyHostToDevice, h->stream));
-    MLP_TRY(ensure_parts(h, (batch + kTrainThreads - 1) / kTrainThreads, batch));
+    MLP_TRY(ensure_act(h, batch));
+    MLP_CUDA(h, cudaMemsetAsync(h->werr, 0, sizeof(int32_t), h->stream));
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     float* hist = nullptr;   // loss of every step, read back once at the end
     if (losses) MLP_CUDA(h, cudaMalloc(&hist, (size_t)steps * sizeof(float)));
@@ -266,19 +293,16 @@ mgsb_status mgsb_mlp_train(mgsb_mlp* h, const float* x, const float* t, int64_t 
     for (int s = 0; s < steps; ++s) {
         // cosine decay of the step size to 10 %
         const float lr_s = lr * (0.55f + 0.45f * std::cos(3.14159265f * (float)s / (float)steps));
-        k_sample_indices<<<(batch + 255) / 256, 256, 0, h->stream>>>(batch, (int)n, seed, (uint64_t)s, h->idx);
-        MLP_TRY(launch_grad(h, batch, h->idx, h->X, h->T));
         ++h->adam_t;
         const float bc1 = 1.f - std::pow(b1, (float)h->adam_t), bc2 = 1.f - std::pow(b2, (float)h->adam_t);
-        k_adam<<<(kMlpParams + 255) / 256, 256, 0, h->stream>>>(h->prm, h->grad, h->m, h->v, lr_s, b1, b2, eps, bc1, bc2);
-        if (losses) MLP_CUDA(h, cudaMemcpyAsync(hist + s, h->loss, sizeof(float), cudaMemcpyDeviceToDevice, h->stream));
+        const AdamStep step{lr_s, b1, b2, eps, bc1, bc2};
+        MLP_TRY(launch_grad(h, batch, SampleOf{1, 0, (int)n, seed, (uint64_t)s}, &step, losses ? hist + s : nullptr));
     }
     MLP_CUDA(h, cudaGetLastError());
     MLP_TRY(repack(h));
     if (losses)
         MLP_CUDA(h, cudaMemcpyAsync(losses, hist, (size_t)steps * sizeof(float), cudaMemcpyDeviceToHost, h->stream));
-    MLP_CUDA(h, cudaStreamSynchronize(h->stream));
-    return MGSB_OK;
+    return check_waits(h);
 }
 
 }  // extern "C"
