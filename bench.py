@@ -251,13 +251,14 @@ def algorithmic_bytes(kernel, solver, meshes, params):
     V = sum(m.num_verts for m in meshes)
     T = sum(m.num_tets for m in meshes)
     n0, nnz0 = solver.level_size(0)
-    if kernel == "k_mg_local":
-        # tet ids 16 + g vectors 40 + slot ids 16 + 4 slot writes 64; s and d 16 each per vertex
-        return 136 * T + 32 * V
+    if kernel in ("k_mg_local", "k_mg_local64"):
+        # per tet its corners 8, g vectors 40 and contributions 8; s and d 16 each per vertex (the blocks' vertex
+        # lists and slots, a few bytes per tet, depend on the mesh's order)
+        return 56 * T + 32 * V
     if kernel == "k_l0_sweep_rg":
         # average over one V-cycle's level-0 sweeps (the first also assembles the RHS)
         plain = 56 * n0 + 8 * nnz0
-        gather = plain + 16 * n0 + 4 * n0 + 16 * 4 * T   # b0, slot_ptr, slots
+        gather = plain + 16 * n0 + 4 * n0 + 16 * n0   # b0, slot_ptr, a slot per vertex at least
         k = params.pre_sweeps + params.post_sweeps
         return (gather + (k - 1) * plain) / k
     lb = LevelBytes(solver, params)
@@ -284,9 +285,9 @@ def algorithmic_bytes(kernel, solver, meshes, params):
         # FP64 outer residual: ELL value 8 + column 4 B per entry; per row the FP64 displacement (32), diagonal
         # (8), contact weight, Jacobi weight, fix flag (12), r32 and e out (32), the learned start residual (16)
         # and the right-hand side: read (32) or, in a PD iteration's first pass, assembled from b0 (32) and the
-        # row's slots (64 B per tet over the body) and written (32)
+        # row's slots (32 B each, one per vertex at least) and written (32)
         per_row = 32 + 8 + 12 + 32 + 16
-        first = 32 + 32 + 4 + 64 * T / max(n0, 1)
+        first = 32 + 32 + 4 + 32
         k = max(params.refinement_passes, 1)
         return 12 * nnz0 + n0 * (per_row + (first + (k - 1) * 32) / k)
     if kernel == "k_ls_sweep_tc":

@@ -3,8 +3,10 @@
 // Layout in HBM (all bodies of a batch concatenated per level):
 //   positions / RHS / corrections : float4 per vertex (xyz + pad, 16-B vector access)
 //   tets                          : int4 vertex ids + (float4, float4, float2) rest data
-//   per-(tet, corner) RHS slots   : float4, ordered by vertex (CSR), so the RHS
-//                                   gather is a contiguous segmented sum — no atomics
+//   RHS slots                     : float4 (double4 in the mixed kind), one per (tet,
+//                                   corner) or per (block of tets, vertex); slices of 8
+//                                   vertices, slot k of the 8 side by side, so the RHS
+//                                   gather reads whole lines — no atomics
 //   matrices                      : sliced ELL (32-row slices, column-major inside
 //                                   a slice), off-diagonal only; diagonal apart
 #pragma once
@@ -12,6 +14,7 @@
 #include <stdint.h>
 
 #include "device_math.cuh"
+#include "plan.hpp"
 
 namespace mgsb {
 
@@ -70,12 +73,18 @@ __global__ void __launch_bounds__(256) k_ref_local(int T, const int4* __restrict
                                                    const float4* __restrict__ invB, const float2* __restrict__ invC,
                                                    const float4* __restrict__ x, const int4* __restrict__ slot_of,
                                                    float4* __restrict__ slots, float stiffness, int drop_small = 1) {
-    pdl_enter();
+    pdl_trigger();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= T) return;
+    if (t >= T) {
+        pdl_wait();
+        return;
+    }
+    // the tet's set-up data is written by no kernel: loaded before the dependency wait
     const int4 id = __ldg(tets + t);
     const float4 a = __ldg(invA + t), b = __ldg(invB + t);
     const float2 c = __ldg(invC + t);
+    const int4 so = __ldg(slot_of + t);
+    pdl_wait();
     const float inv[9] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, c.x};
     const float vol = c.y;
     const float4 p0 = __ldg(x + id.x), p1 = __ldg(x + id.y), p2 = __ldg(x + id.z), p3 = __ldg(x + id.w);
@@ -100,7 +109,6 @@ __global__ void __launch_bounds__(256) k_ref_local(int T, const int4* __restrict
         Ac[r * 4 + 2] = inv[r + 3];
         Ac[r * 4 + 3] = inv[r + 6];
     }
-    const int4 so = __ldg(slot_of + t);
     const int sid[4] = {so.x, so.y, so.z, so.w};
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -124,23 +132,40 @@ __global__ void __launch_bounds__(256) k_ref_local(int T, const int4* __restrict
 // (DCDByPoint_sphere, PDSolver.cu:277-331), then the under-relaxed Jacobi
 // step with Chebyshev acceleration (calculatePOS, PDSolver.cu:192-235).
 // On the last iteration also v = (x - last)/dt (calculateV, PDSolver.cu:245).
-__global__ void __launch_bounds__(256) k_ref_vertex(
+// Latency bound: what no kernel of a frame writes (the slots' place, mass,
+// diagonal, fix flag; the spheres, copied before the frame) is read before the
+// dependency wait, and the slots, in whole lines, 12 loads in flight per thread.
+// Blocks of 64: a 20k-vertex body then covers every SM.
+constexpr int kRefVertexThreads = 64;
+__global__ void __launch_bounds__(kRefVertexThreads) k_ref_vertex(
     int n, float4* __restrict__ x, float4* __restrict__ prev, const float4* __restrict__ s, const float4* __restrict__ last,
     float4* __restrict__ v, const float* __restrict__ fixf, const float* __restrict__ mass, const float* __restrict__ vdiag,
-    const int32_t* __restrict__ slot_ptr, const float4* __restrict__ slots, const SphereSet* __restrict__ spheres,
+    const int32_t* __restrict__ slot_ptr, const float4* __restrict__ slots, const SphereSet* __restrict__ sphere_set,
     float kc, float dt, float omega, double relax, int last_iter, int32_t* __restrict__ cflag, float* __restrict__ cdepth,
     float* __restrict__ cenergy, int32_t* __restrict__ nonfinite, const int32_t* __restrict__ tri_ptr = nullptr,
     const int32_t* __restrict__ tri_idx = nullptr, const float4* __restrict__ tri_push = nullptr) {
-    pdl_enter();
+    pdl_trigger();
+    __shared__ SphereSet sphere_copy;
+    const SphereSet* spheres = &sphere_copy;
+    static_assert(sizeof(SphereSet) / 4 <= kRefVertexThreads, "a word per thread");
+    if (threadIdx.x < sizeof(SphereSet) / 4)
+        reinterpret_cast<int32_t*>(&sphere_copy)[threadIdx.x] = reinterpret_cast<const int32_t*>(sphere_set)[threadIdx.x];
+    __syncthreads();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    if (i >= n) {
+        pdl_wait();
+        return;
+    }
+    const int e0 = __ldg(slot_ptr + i / kSlotSlice) + i % kSlotSlice, e1 = __ldg(slot_ptr + i / kSlotSlice + 1);
+    const float fix = __ldg(fixf + i), vd = __ldg(vdiag + i), dc = __ldg(mass + i) / (dt * dt);
+    pdl_wait();
+    const float4 p4 = x[i], s4 = __ldg(s + i), pv4 = prev[i];
     float fx = 0.f, fy = 0.f, fz = 0.f;
-    const int e1 = __ldg(slot_ptr + i + 1);
-    for (int e = __ldg(slot_ptr + i); e < e1; ++e) {
+#pragma unroll 12
+    for (int e = e0; e < e1; e += kSlotSlice) {
         const float4 c = __ldg(slots + e);
         fx += c.x; fy += c.y; fz += c.z;
     }
-    const float4 p4 = x[i];
     const float p[3] = {p4.x, p4.y, p4.z};
     float cd[3] = {0.f, 0.f, 0.f}, cf[3] = {0.f, 0.f, 0.f};
     int flag = 0;
@@ -197,10 +222,6 @@ __global__ void __launch_bounds__(256) k_ref_vertex(
             ce += kc * pe * pe;
         }
     }
-    const float fix = __ldg(fixf + i);
-    const float dc = __ldg(mass + i) / (dt * dt);
-    const float vd = __ldg(vdiag + i);
-    const float4 s4 = __ldg(s + i), pv4 = prev[i];
     const float sv[3] = {s4.x, s4.y, s4.z}, pv[3] = {pv4.x, pv4.y, pv4.z};
     const float fe[3] = {fx, fy, fz};
     float nx[3];
@@ -566,58 +587,140 @@ __global__ void k_coarse_frame(int n, const int32_t* __restrict__ rptr, const in
 
 // Local step, one thread per tet, on x = s + d: F = sum_j x_j g_j^T from the
 // edge vectors (s_k - s_0) + (d_k - d_0), R = closest rotation; the RHS of
-// the displacement system gets w (R - F(s)) g_j in the four corner slots.
-__global__ void __launch_bounds__(256) k_mg_local(int T, const int4* __restrict__ tets, const float4* __restrict__ gA,
-                                                  const float4* __restrict__ gB, const float2* __restrict__ gC,
-                                                  const float4* __restrict__ s, const float4* __restrict__ d,
-                                                  const int4* __restrict__ slot_of, float4* __restrict__ slots) {
+// the displacement system gets w (R - F(s)) g_j at the four corners.
+// A block takes up to 256 consecutive tets of one body.  Its vertices' s and d
+// (120 on the beams, for 1,024 corners) are gathered once into shared memory,
+// and the corners' contributions are summed per vertex there, in a
+// fixed order, before one slot per vertex of the block leaves it: 64 bytes of slots per tet
+// that the next kernel gathers became 8 (and the corner and slot indices 20
+// instead of 32), the sums in Acc = float, or double in the mixed kind, which
+// keeps its right-hand side in FP64.
+// Measured, local step and the next kernel's gather together per PD iteration:
+// 128-body batch 47.3 + 37 us before, 57.1 + 17 us; 829,440 tets, mixed, 29.4 +
+// 31 us before, 33.9 + 14 us; 103,680 tets 5.8 + 7.5 us before, 6.2 + 3.6 us.
+// What bounds it: issue slots on many tets (64 % busy, 735 instructions per tet
+// of a warp, over half of them the polar iteration), latency on one body.
+struct LocalArgs {
+    const int4* block;
+    const ushort4* tet;
+    const int32_t *id, *slot;
+    const ushort2* range;
+    const uint16_t* ent;
+    const float4 *gA, *gB;
+    const float2* gC;
+    int most;   // vertices of the largest block
+};
+constexpr size_t local_smem_bytes(int most) {
+    return (size_t)most * 2 * sizeof(float4) + 4 * kLocalTets * (sizeof(float4) + sizeof(uint16_t));
+}
+
+template <typename Acc, typename Slot>
+__device__ __forceinline__ void mg_local(const LocalArgs& A, const float4* __restrict__ s, const float4* __restrict__ d,
+                                         Slot* __restrict__ slots) {
     pdl_trigger();
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= T) {
-        pdl_wait();
-        return;
+    extern __shared__ __align__(16) unsigned char local_smem[];
+    float4* ss = reinterpret_cast<float4*>(local_smem);
+    float4* sd = ss + A.most;
+    float4* sc = sd + A.most;   // the corners' contributions, corner-major
+    uint16_t* sent = reinterpret_cast<uint16_t*>(sc + 4 * kLocalTets);
+    // the block's set-up data is written by no kernel: loaded before the dependency wait, while the previous kernel runs
+    const int4 blk = __ldg(A.block + blockIdx.x);
+    const int t0 = blk.x, nt = blk.y, v0 = blk.z, nv = blk.w;
+    const int tid = threadIdx.x, t = t0 + tid;
+    const bool has = tid < nt;
+    ushort4 id = make_ushort4(0, 0, 0, 0);
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+    float2 c = make_float2(0.f, 0.f);
+    if (has) {
+        id = __ldg(A.tet + t);
+        a = __ldg(A.gA + t);
+        b = __ldg(A.gB + t);
+        c = __ldg(A.gC + t);
     }
-    // the tet's set-up data (vertices, shape gradients, weight, slots) is written by no kernel:
-    // loaded before the dependency wait, while the previous kernel runs
-    const int4 id = __ldg(tets + t);
-    const float4 a = __ldg(gA + t), b = __ldg(gB + t);
-    const float2 c = __ldg(gC + t);
-    const int4 so = __ldg(slot_of + t);
+    for (int q = tid; q < 2 * nt; q += kLocalTets)   // two entries at a time: a block's part starts at a multiple of 4
+        reinterpret_cast<uint32_t*>(sent)[q] = __ldg(reinterpret_cast<const uint32_t*>(A.ent + 4 * (size_t)t0) + q);
+    const int mine = tid < nv ? __ldg(A.id + v0 + tid) : 0;
+    const int pv = tid >> 1;   // the vertex whose contributions this thread and its neighbour sum
+    const int slot = pv < nv ? __ldg(A.slot + v0 + pv) : 0;
+    const ushort2 range = pv < nv ? __ldg(A.range + v0 + pv) : make_ushort2(0, 0);
     pdl_wait();
-    // g1 = (a.x a.y a.z), g2 = (a.w b.x b.y), g3 = (b.z b.w c.x), w = c.y
-    const float g1[3] = {a.x, a.y, a.z}, g2[3] = {a.w, b.x, b.y}, g3[3] = {b.z, b.w, c.x};
-    const float w = c.y;
-    const float4 s0 = __ldg(s + id.x), s1 = __ldg(s + id.y), s2 = __ldg(s + id.z), s3 = __ldg(s + id.w);
-    const float4 q0 = __ldg(d + id.x), q1 = __ldg(d + id.y), q2 = __ldg(d + id.z), q3 = __ldg(d + id.w);
-    const float e1[3] = {s1.x - s0.x, s1.y - s0.y, s1.z - s0.z};
-    const float e2[3] = {s2.x - s0.x, s2.y - s0.y, s2.z - s0.z};
-    const float e3[3] = {s3.x - s0.x, s3.y - s0.y, s3.z - s0.z};
-    const float f1[3] = {q1.x - q0.x, q1.y - q0.y, q1.z - q0.z};
-    const float f2[3] = {q2.x - q0.x, q2.y - q0.y, q2.z - q0.z};
-    const float f3[3] = {q3.x - q0.x, q3.y - q0.y, q3.z - q0.z};
-    float Fs[9], F[9];
-#pragma unroll
-    for (int r = 0; r < 3; ++r)
-#pragma unroll
-        for (int q = 0; q < 3; ++q) {
-            Fs[r * 3 + q] = e1[r] * g1[q] + e2[r] * g2[q] + e3[r] * g3[q];
-            F[r * 3 + q] = (e1[r] + f1[r]) * g1[q] + (e2[r] + f2[r]) * g2[q] + (e3[r] + f3[r]) * g3[q];
-        }
-    float R[9];
-    if (!polar_newton(F, R)) svd_rotation(F, R);   // the SVD only for inverted / degenerate tets
-#pragma unroll
-    for (int q = 0; q < 9; ++q) R[q] -= Fs[q];
-    float o1[3], o2[3], o3[3];
-#pragma unroll
-    for (int r = 0; r < 3; ++r) {
-        o1[r] = w * (R[r * 3 + 0] * g1[0] + R[r * 3 + 1] * g1[1] + R[r * 3 + 2] * g1[2]);
-        o2[r] = w * (R[r * 3 + 0] * g2[0] + R[r * 3 + 1] * g2[1] + R[r * 3 + 2] * g2[2]);
-        o3[r] = w * (R[r * 3 + 0] * g3[0] + R[r * 3 + 1] * g3[1] + R[r * 3 + 2] * g3[2]);
+    if (tid < nv) {
+        ss[tid] = __ldg(s + mine);
+        sd[tid] = __ldg(d + mine);
     }
-    slots[so.x] = make_float4(-(o1[0] + o2[0] + o3[0]), -(o1[1] + o2[1] + o3[1]), -(o1[2] + o2[2] + o3[2]), 0.f);
-    slots[so.y] = make_float4(o1[0], o1[1], o1[2], 0.f);
-    slots[so.z] = make_float4(o2[0], o2[1], o2[2], 0.f);
-    slots[so.w] = make_float4(o3[0], o3[1], o3[2], 0.f);
+    for (int v = tid + kLocalTets; v < nv; v += kLocalTets) {
+        const int i = __ldg(A.id + v0 + v);
+        ss[v] = __ldg(s + i);
+        sd[v] = __ldg(d + i);
+    }
+    __syncthreads();
+    if (has) {
+        // g1 = (a.x a.y a.z), g2 = (a.w b.x b.y), g3 = (b.z b.w c.x), w = c.y
+        const float g1[3] = {a.x, a.y, a.z}, g2[3] = {a.w, b.x, b.y}, g3[3] = {b.z, b.w, c.x};
+        const float w = c.y;
+        const float4 s0 = ss[id.x], s1 = ss[id.y], s2 = ss[id.z], s3 = ss[id.w];
+        const float4 q0 = sd[id.x], q1 = sd[id.y], q2 = sd[id.z], q3 = sd[id.w];
+        const float e1[3] = {s1.x - s0.x, s1.y - s0.y, s1.z - s0.z};
+        const float e2[3] = {s2.x - s0.x, s2.y - s0.y, s2.z - s0.z};
+        const float e3[3] = {s3.x - s0.x, s3.y - s0.y, s3.z - s0.z};
+        const float f1[3] = {q1.x - q0.x, q1.y - q0.y, q1.z - q0.z};
+        const float f2[3] = {q2.x - q0.x, q2.y - q0.y, q2.z - q0.z};
+        const float f3[3] = {q3.x - q0.x, q3.y - q0.y, q3.z - q0.z};
+        float Fs[9], F[9];
+#pragma unroll
+        for (int r = 0; r < 3; ++r)
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                Fs[r * 3 + q] = e1[r] * g1[q] + e2[r] * g2[q] + e3[r] * g3[q];
+                F[r * 3 + q] = (e1[r] + f1[r]) * g1[q] + (e2[r] + f2[r]) * g2[q] + (e3[r] + f3[r]) * g3[q];
+            }
+        float R[9];
+        if (!polar_newton(F, R)) svd_rotation(F, R);   // the SVD only for inverted / degenerate tets
+#pragma unroll
+        for (int q = 0; q < 9; ++q) R[q] -= Fs[q];
+        float o1[3], o2[3], o3[3];
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+            o1[r] = w * (R[r * 3 + 0] * g1[0] + R[r * 3 + 1] * g1[1] + R[r * 3 + 2] * g1[2]);
+            o2[r] = w * (R[r * 3 + 0] * g2[0] + R[r * 3 + 1] * g2[1] + R[r * 3 + 2] * g2[2]);
+            o3[r] = w * (R[r * 3 + 0] * g3[0] + R[r * 3 + 1] * g3[1] + R[r * 3 + 2] * g3[2]);
+        }
+        sc[tid] = make_float4(-(o1[0] + o2[0] + o3[0]), -(o1[1] + o2[1] + o3[1]), -(o1[2] + o2[2] + o3[2]), 0.f);
+        sc[tid + kLocalTets] = make_float4(o1[0], o1[1], o1[2], 0.f);
+        sc[tid + 2 * kLocalTets] = make_float4(o2[0], o2[1], o2[2], 0.f);
+        sc[tid + 3 * kLocalTets] = make_float4(o3[0], o3[1], o3[2], 0.f);
+    }
+    __syncthreads();
+    for (int v = pv; v < (nv + 15) / 16 * 16; v += kLocalTets / 2) {   // whole warps: two threads per vertex
+        const ushort2 rg = v == pv ? range : v < nv ? __ldg(A.range + v0 + v) : make_ushort2(0, 0);
+        Acc x = 0, y = 0, z = 0;
+#pragma unroll 4
+        for (int e = rg.x + (tid & 1); e < rg.y; e += 2) {
+            const float4 k = sc[sent[e]];
+            x += k.x;
+            y += k.y;
+            z += k.z;
+        }
+        x += __shfl_xor_sync(0xffffffffu, x, 1);
+        y += __shfl_xor_sync(0xffffffffu, y, 1);
+        z += __shfl_xor_sync(0xffffffffu, z, 1);
+        if (v >= nv || (tid & 1)) continue;
+        Slot q;
+        q.x = x;
+        q.y = y;
+        q.z = z;
+        q.w = 0;
+        slots[v == pv ? slot : __ldg(A.slot + v0 + v)] = q;
+    }
+}
+
+__global__ void __launch_bounds__(kLocalTets) k_mg_local(const LocalArgs A, const float4* __restrict__ s,
+                                                         const float4* __restrict__ d, float4* __restrict__ slots) {
+    mg_local<float>(A, s, d, slots);
+}
+__global__ void __launch_bounds__(kLocalTets) k_mg_local64(const LocalArgs A, const float4* __restrict__ s,
+                                                           const float4* __restrict__ d, double4* __restrict__ slots) {
+    mg_local<double>(A, s, d, slots);
 }
 
 // RHS assembly alone: b = b0 + sum of the vertex's slots.
@@ -627,8 +730,9 @@ __global__ void k_gather_rhs(int n, float4* __restrict__ b, const float4* __rest
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     float4 bi = __ldg(b0 + i);
-    const int e1 = __ldg(slot_ptr + i + 1);
-    for (int e = __ldg(slot_ptr + i); e < e1; ++e) {
+    const int e1 = __ldg(slot_ptr + i / kSlotSlice + 1);
+#pragma unroll 8
+    for (int e = __ldg(slot_ptr + i / kSlotSlice) + i % kSlotSlice; e < e1; e += kSlotSlice) {
         const float4 c = __ldg(slots + e);
         bi.x += c.x; bi.y += c.y; bi.z += c.z;
     }

@@ -44,8 +44,9 @@ __global__ void __launch_bounds__(kLsThreads) k_ls_residual(int n, const int32_t
     const bool valid = row < n;
     float4 bg = make_float4(0.f, 0.f, 0.f, 0.f);
     if (slots) {
-        const int beg = valid ? __ldg(slot_ptr + row) : 0, end = valid ? __ldg(slot_ptr + row + 1) : 0;
-        const float4 sl = rg_slot_sum<G>(valid, lane, beg, end, slots);
+        const bool slice = warp * S < n;
+        const int beg = slice ? __ldg(slot_ptr + warp) : 0, end = slice ? __ldg(slot_ptr + warp + 1) : 0;
+        const float4 sl = rg_slot_sum<G>(lane, beg, end, slots);
         const float4 bb = valid ? __ldg(b0 + row) : make_float4(0.f, 0.f, 0.f, 0.f);
         bg = make_float4(bb.x + sl.x, bb.y + sl.y, bb.z + sl.z, 0.f);
         if (valid && lane < S) bgather[row] = bg;

@@ -238,19 +238,19 @@ __device__ __forceinline__ float4 held_sum(const HeldEntries<K>& h, int lane, co
 constexpr int kHeldL0 = 4;   // level-0 entries held per lane (4 lanes per row: 16 per row)
 constexpr int kHeldC = 6;    // coarse-level entries held per lane (8 lanes per row: 48 per row)
 
-// Sum of the contiguous float4 slots [beg, end) split across the G lanes.
+// Sum of the RHS slots [beg, end) of a slice's 8 rows, each row's split across its G lanes (lane l takes the slots
+// l / 8, l / 8 + G, ... of row l % 8: 32 neighbouring slots per step).  The slots past a row's last are zero.
 template <int G>
-__device__ __forceinline__ float4 rg_slot_sum(bool valid, int lane, int beg, int end, const float4* __restrict__ slots) {
+__device__ __forceinline__ float4 rg_slot_sum(int lane, int beg, int end, const float4* __restrict__ slots) {
     constexpr int S = 32 / G;
+    static_assert(S == kSlotSlice, "a warp covers one slice of slots");
     float ax = 0.f, ay = 0.f, az = 0.f;
-    if (valid) {
-#pragma unroll 2
-        for (int q = beg + lane / S; q < end; q += G) {
-            const float4 t = __ldg(slots + q);
-            ax += t.x;
-            ay += t.y;
-            az += t.z;
-        }
+#pragma unroll 6
+    for (int q = beg + lane; q < end; q += 32) {
+        const float4 t = __ldg(slots + q);
+        ax += t.x;
+        ay += t.y;
+        az += t.z;
     }
 #pragma unroll
     for (int o = S; o < 32; o <<= 1) {
@@ -281,12 +281,13 @@ __global__ void __launch_bounds__(256) k_l0_sweep_rg(int n, const int32_t* __res
     const bool valid = row < n;
     HeldEntries<kHeldL0> he;
     hold_ell_row<G>(he, row, valid, lane, sp, col, val);
-    const int sbeg = (gather && valid) ? __ldg(slot_ptr + row) : 0, send = (gather && valid) ? __ldg(slot_ptr + row + 1) : 0;
+    const bool slice = gather && warp * S < n;
+    const int sbeg = slice ? __ldg(slot_ptr + warp) : 0, send = slice ? __ldg(slot_ptr + warp + 1) : 0;
     pdl_wait();
     if (gate && __ldg(gate) == 0) return;   // gated launches run only when the learned V-cycle was rejected
     float4 bi;
     if (gather) {
-        const float4 sl = rg_slot_sum<G>(valid, lane, sbeg, send, slots);
+        const float4 sl = rg_slot_sum<G>(lane, sbeg, send, slots);
         const float4 bb = valid ? __ldg(b0 + row) : f4z();
         bi = make_float4(bb.x + sl.x, bb.y + sl.y, bb.z + sl.z, 0.f);
         if (valid && lane < S) b[row] = bi;

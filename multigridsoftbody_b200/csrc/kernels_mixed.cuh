@@ -128,13 +128,14 @@ __global__ void __launch_bounds__(kMxThreads, 3) k_mx_residual(int n, const int3
                                                      const float* __restrict__ dinv, float4* __restrict__ r32,
                                                      float4* __restrict__ e, int first_sweep,
                                                      const double4* __restrict__ b0, const int32_t* __restrict__ slot_ptr,
-                                                     const float4* __restrict__ slots, const float* __restrict__ fixf,
+                                                     const double4* __restrict__ slots, const float* __restrict__ fixf,
                                                      float4* __restrict__ ls_r, float* __restrict__ part,
                                                      float* __restrict__ part_end) {
     pdl_trigger();
     __shared__ float red[kMxThreads / 32];
     constexpr int G = kLanesMx, RW = 32 / G;   // lanes per row, rows per warp
     constexpr int SH = 32 / kLanesL0;           // slice height of the level-0 sliced ELL
+    static_assert(RW == kSlotSlice, "a warp covers one slice of slots");
     const int lane = threadIdx.x & 31;
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int row = warp * RW + (lane % RW);
@@ -146,12 +147,12 @@ __global__ void __launch_bounds__(kMxThreads, 3) k_mx_residual(int n, const int3
     // entries finish in the tail loops.  The set-up structure (slot and ELL offsets, columns, FP64
     // values, the contact-free diagonal, the fix mask) is written by no kernel: it is loaded before
     // the dependency wait, while the previous kernel runs.
-    constexpr int kMxSlotsAhead = 6, kMxEllAhead = 4;
+    constexpr int kMxSlotsAhead = 2, kMxEllAhead = 4;
     int s_beg = 0, s_end = 0, q0 = 0, end = 0;
     if (valid) {
         if (b0) {
-            s_beg = __ldg(slot_ptr + row) + j;
-            s_end = __ldg(slot_ptr + row + 1);
+            s_beg = __ldg(slot_ptr + warp) + lane;   // 32 neighbouring slots per step
+            s_end = __ldg(slot_ptr + warp + 1);
         }
         const int slice = row / SH;
         q0 = __ldg(sp + slice) + j * SH + (row - slice * SH);
@@ -170,12 +171,12 @@ __global__ void __launch_bounds__(kMxThreads, 3) k_mx_residual(int n, const int3
     const double D0 = own ? __ldg(diag64 + row) : 0.0;
     const float fxown = own ? __ldg(fixf + row) : 0.f;
     pdl_wait();
-    float4 sl[kMxSlotsAhead];
+    double4 sl[kMxSlotsAhead];
     if (b0) {
 #pragma unroll
         for (int k = 0; k < kMxSlotsAhead; ++k) {
-            const int q = s_beg + k * G;
-            sl[k] = q < s_end ? __ldg(slots + q) : make_float4(0.f, 0.f, 0.f, 0.f);
+            const int q = s_beg + k * 32;
+            sl[k] = q < s_end ? slots[q] : d4z();
         }
     }
     // the row's own data, on the row's first lane
@@ -187,14 +188,14 @@ __global__ void __launch_bounds__(kMxThreads, 3) k_mx_residual(int n, const int3
         double sx = 0.0, sy = 0.0, sz = 0.0;
 #pragma unroll
         for (int k = 0; k < kMxSlotsAhead; ++k) {
-            if (s_beg + k * G < s_end) {
+            if (s_beg + k * 32 < s_end) {
                 sx += sl[k].x;
                 sy += sl[k].y;
                 sz += sl[k].z;
             }
         }
-        for (int q = s_beg + kMxSlotsAhead * G; q < s_end; q += G) {
-            const float4 t = __ldg(slots + q);
+        for (int q = s_beg + kMxSlotsAhead * 32; q < s_end; q += 32) {
+            const double4 t = slots[q];
             sx += t.x;
             sy += t.y;
             sz += t.z;

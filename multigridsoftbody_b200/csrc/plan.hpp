@@ -64,7 +64,15 @@ struct Plan {
     std::vector<int4> tets, slot_of;
     std::vector<float4> tA, tB;
     std::vector<float2> tC;
-    std::vector<int32_t> slot_ptr;
+    // Right-hand-side slots.  Reference kind: one per (tet, corner), slot_of.  Multigrid kinds: one per vertex of
+    // each block of up to kLocalTets consecutive tets of a body, which the local step sums over the block's tets.
+    std::vector<int32_t> slot_ptr;   // per slice of kSlotSlice vertices, its first slot
+    std::vector<int4> lblock;        // per block: first tet, tets, first entry of lv_*, vertices
+    std::vector<ushort4> ltet;       // per tet: its corners among the block's vertices
+    std::vector<int32_t> lv_id, lv_slot;   // per vertex of a block: vertex, slot
+    std::vector<ushort2> lv_range;         // and its contributions [x, y) in the block's part of lent
+    std::vector<uint16_t> lent;            // per block 4 x tets: contributions by vertex, corner * kLocalTets + tet
+    int max_local = 0;                     // most vertices of a block
     std::vector<PlanLevel> levels;            // [0] = finest (matrix only)
     std::vector<float> dense;                 // coarsest dense blocks (row-major per body)
     std::vector<double> dense64;              // the same in FP64
@@ -89,6 +97,8 @@ void build_ell(const std::vector<int32_t>& ptr, const std::vector<int32_t>& col,
                const std::vector<int32_t>* pad_col = nullptr);
 
 constexpr int kSliceL0 = 8;       // 4 lanes per row at level 0
+constexpr int kSlotSlice = 8;     // vertices whose RHS slots interleave (the height of a level-0 slice)
+constexpr int kLocalTets = 256;   // tets of a block of the multigrid kinds' local step
 constexpr int kSliceCoarse = 4;   // 8 lanes per row on coarse levels
 
 // Copies a mesh into a body (rest data, default material, no fixed vertex,

@@ -9,6 +9,7 @@
 #include <memory>
 #include <mutex>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/mgsb.h"
@@ -31,6 +32,7 @@ namespace {
 
 constexpr int kBlock = 256;
 inline int grid_for(int n) { return (n + kBlock - 1) / kBlock; }
+inline int grid_ref_vertex(int n) { return (n + kRefVertexThreads - 1) / kRefVertexThreads; }
 // blocks of kBlock threads for a row-group kernel (32/S lanes per row, slices of S rows)
 inline int grid_rows(int n, int S) { return ((n + S - 1) / S * 32 + kBlock - 1) / kBlock; }
 
@@ -144,7 +146,10 @@ struct mgsb_solver {
     int4* slot_of = nullptr;
     int32_t* slot_ptr = nullptr;
     float4* slots = nullptr;
-    // multigrid
+    // multigrid: the local step's blocks, and the mixed kind's slots
+    LocalArgs local{};
+    int local_blocks = 0;
+    double4* slots64 = nullptr;
     float4 *b = nullptr, *b0 = nullptr, *target = nullptr, *d = nullptr, *d2 = nullptr;
     // mixed precision (FP64 master state and outer residual)
     double4 *x64 = nullptr, *v64 = nullptr, *s64 = nullptr, *last64 = nullptr, *dd64 = nullptr, *b64 = nullptr,
@@ -532,19 +537,49 @@ mgsb_status rebuild(mgsb_solver* h) {
     Plan P;
     std::string perr;
     if (!build_plan(h->bodies, h->p, P, perr)) return set_err(h, MGSB_INVALID_ARG, "%s", perr.c_str());
-    const int N0 = P.N0, T = P.T;
+    const int N0 = P.N0;
     TRY(dupload(h, pool, &h->body_of, P.body_of));
     TRY(dupload(h, pool, &h->fixf, P.fixf));
     TRY(dupload(h, pool, &h->mass, P.mass));
     TRY(dupload(h, pool, &h->vdiag, P.diag));
     TRY(dupload(h, pool, &h->tets, P.tets));
-    TRY(dupload(h, pool, &h->slot_of, P.slot_of));
     TRY(dupload(h, pool, &h->tA, P.tA));
     TRY(dupload(h, pool, &h->tB, P.tB));
     TRY(dupload(h, pool, &h->tC, P.tC));
     TRY(dupload(h, pool, &h->slot_ptr, P.slot_ptr));
-    TRY(dalloc(h, pool, &h->slots, 4 * (size_t)T));
-    CUDA_TRY(h, cudaMemset(h->slots, 0, 4 * (size_t)T * sizeof(float4)));
+    if (mg && h->p.precision == MGSB_PRECISION_MIXED) {
+        TRY(dalloc(h, pool, &h->slots64, (size_t)P.slot_ptr.back()));
+        CUDA_TRY(h, cudaMemset(h->slots64, 0, (size_t)P.slot_ptr.back() * sizeof(double4)));
+    } else {
+        TRY(dalloc(h, pool, &h->slots, (size_t)P.slot_ptr.back()));
+        CUDA_TRY(h, cudaMemset(h->slots, 0, (size_t)P.slot_ptr.back() * sizeof(float4)));
+    }
+    if (mg) {
+        LocalArgs& A = h->local;
+        auto up = [&](auto& out, const auto& v) {
+            std::remove_const_t<std::remove_pointer_t<std::remove_reference_t<decltype(out)>>>* p = nullptr;
+            const mgsb_status st = dupload(h, pool, &p, v);
+            out = p;
+            return st;
+        };
+        TRY(up(A.block, P.lblock));
+        TRY(up(A.tet, P.ltet));
+        TRY(up(A.id, P.lv_id));
+        TRY(up(A.slot, P.lv_slot));
+        TRY(up(A.range, P.lv_range));
+        TRY(up(A.ent, P.lent));
+        A.gA = h->tA;
+        A.gB = h->tB;
+        A.gC = h->tC;
+        A.most = P.max_local;
+        CUDA_TRY(h, cudaFuncSetAttribute(k_mg_local, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)local_smem_bytes(4 * kLocalTets)));
+        CUDA_TRY(h, cudaFuncSetAttribute(k_mg_local64, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)local_smem_bytes(4 * kLocalTets)));
+        h->local_blocks = (int)P.lblock.size();
+    } else {
+        TRY(dupload(h, pool, &h->slot_of, P.slot_of));
+    }
     h->h_inv = P.h_inv;
     h->h_ac = P.h_ac;
     h->h_vol = P.h_vol;
@@ -832,7 +867,7 @@ void enqueue_ref_frame(mgsb_solver* h) {
         LAUNCH(h, k_ref_local, grid_for(T), kBlock, 0, T, h->tets, h->tA, h->tB, h->tC, h->x, h->slot_of, h->slots,
                p.volume_stiffness, 1);
         omega = 4 / (4 - p.cheb_rho * p.cheb_rho * omega);
-        LAUNCH(h, k_ref_vertex, grid_for(n), kBlock, 0, n, h->x, h->prev, h->s, h->last, h->v, h->fixf, h->mass,
+        LAUNCH(h, k_ref_vertex, grid_ref_vertex(n), kRefVertexThreads, 0, n, h->x, h->prev, h->s, h->last, h->v, h->fixf, h->mass,
                h->vdiag, h->slot_ptr, h->slots, h->spheres_dev, p.collision_stiffness, p.dt, omega,
                (double)p.relaxation, it == p.iterations - 1 ? 3 : 0, h->cflag, h->cdepth, h->cenergy,
                h->nonfinite, nullptr, nullptr, nullptr);
@@ -1750,7 +1785,7 @@ void fill_coarse_args(mgsb_solver* h, CoarseArgs& ca) {
 // followed by its residual check.
 float4* enqueue_mg_solve(mgsb_solver* h, bool learned, const LearnedFallback& fb) {
     const mgsb_params& p = h->p;
-    const int n0 = h->N0, T = h->T, L = p.levels;
+    const int n0 = h->N0, L = p.levels;
     const int nb = (int)h->bodies.size();
     const float om = p.jacobi_omega;
     std::vector<LevelDev>& lv = h->lev;
@@ -1773,7 +1808,7 @@ float4* enqueue_mg_solve(mgsb_solver* h, bool learned, const LearnedFallback& fb
     const int l0_pre = fallback ? std::max(p.pre_sweeps, kFallbackL0Sweeps) : p.pre_sweeps;
     const int l0_post = fallback ? std::max(p.post_sweeps, kFallbackL0Sweeps) : p.post_sweeps;
     for (int it = 0; it < p.iterations; ++it) {
-        LAUNCH(h, k_mg_local, grid_for(T), kBlock, 0, T, h->tets, h->tA, h->tB, h->tC, h->s, xa, h->slot_of, h->slots);
+        LAUNCH(h, k_mg_local, h->local_blocks, kLocalTets, local_smem_bytes(h->local.most), h->local, h->s, xa, h->slots);
         if (learned) {
             for (int pass = 0; pass < p.refinement_passes; ++pass) {
                 const int c = it * p.refinement_passes + pass;
@@ -1846,7 +1881,7 @@ void enqueue_mg_frame(mgsb_solver* h) {
 // inverse, then the PD iterations; the displacement ends in dd64 / d32.
 void enqueue_mixed_solve(mgsb_solver* h, bool learned, const LearnedFallback& fb) {
     const mgsb_params& p = h->p;
-    const int n0 = h->N0, T = h->T, L = p.levels;
+    const int n0 = h->N0, L = p.levels;
     const int nb = (int)h->bodies.size();
     const float om = p.jacobi_omega;
     std::vector<LevelDev>& lv = h->lev;
@@ -1873,7 +1908,8 @@ void enqueue_mixed_solve(mgsb_solver* h, bool learned, const LearnedFallback& fb
     const int l0_pre = fallback ? std::max(p.pre_sweeps, kFallbackL0Sweeps) : p.pre_sweeps;
     const int l0_post = fallback ? std::max(p.post_sweeps, kFallbackL0Sweeps) : p.post_sweeps;
     for (int it = 0; it < p.iterations; ++it) {
-        LAUNCH(h, k_mg_local, grid_for(T), kBlock, 0, T, h->tets, h->tA, h->tB, h->tC, h->s, h->d32, h->slot_of, h->slots);
+        LAUNCH(h, k_mg_local64, h->local_blocks, kLocalTets, local_smem_bytes(h->local.most), h->local, h->s, h->d32,
+               h->slots64);
         for (int pass = 0; pass < p.refinement_passes; ++pass) {
             float4* ea = h->d;
             float4* eb = h->d2;
@@ -1885,7 +1921,7 @@ void enqueue_mixed_solve(mgsb_solver* h, bool learned, const LearnedFallback& fb
             // this outer residual, against the right-hand side that cycle solved for
             LAUNCH(h, k_mx_residual, g0, kMxThreads, 0, n0, lv[0].slice_ptr, lv[0].ell_col, h->ell_val64, h->diag64, h->c0,
                    h->dd64, h->b64, lv[0].dinv, h->r32, ea, (l0_pre > 0 && !learned) ? 1 : 0,
-                   gather ? h->b0_64 : nullptr, gather ? h->slot_ptr : nullptr, gather ? h->slots : nullptr, h->fixf,
+                   gather ? h->b0_64 : nullptr, gather ? h->slot_ptr : nullptr, gather ? h->slots64 : nullptr, h->fixf,
                    learned ? h->ls_r : nullptr, learned ? h->ls_part0 + (size_t)c * h->ls_nblk : nullptr,
                    (learned && c > 0) ? h->ls_part1 + (size_t)(c - 1) * h->ls_nblk : nullptr);
             if (learned) {
@@ -3318,8 +3354,7 @@ extern "C" mgsb_status mgsb_smoother_pairs(mgsb_solver* h, int32_t sweeps, float
     // (3) the residual a further PD iteration would start from: the local step
     //     at the current displacement gives b' = b0 + slots, r3 = b' - A d.
     //     (the slots are rebuilt by the next frame's first local step)
-    k_mg_local<<<grid_for(h->T), kBlock, 0, st>>>(h->T, h->tets, h->tA, h->tB, h->tC, h->s, h->d_final, h->slot_of,
-                                                   h->slots);
+    k_mg_local<<<h->local_blocks, kLocalTets, local_smem_bytes(h->local.most), st>>>(h->local, h->s, h->d_final, h->slots);
     k_gather_rhs<<<grid_for(n0), kBlock, 0, st>>>(n0, h->ls_ec, h->b0, h->slot_ptr, h->slots);
     k_ls_residual<<<g0, kLsThreads, 0, st>>>(n0, l0.slice_ptr, l0.ell_col, l0.ell_val, l0.dfull, h->fixf, h->d_final,
                                              h->ls_ec, h->ls_save, nullptr, nullptr);
@@ -3493,7 +3528,7 @@ void enqueue_two_level_frame(mgsb_two_level* t) {
                pc.volume_stiffness, 0);
         LAUNCH(C, k_ref_tri_dcd, grid_for(t->ntri), kBlock, 0, t->ntri, t->tris, C->x, C->spheres_dev, t->push);
         omega = 4 / (4 - pc.cheb_rho * pc.cheb_rho * omega);
-        LAUNCH(C, k_ref_vertex, grid_for(t->nc), kBlock, 0, t->nc, C->x, C->prev, C->s, C->last, C->v, C->fixf, C->mass,
+        LAUNCH(C, k_ref_vertex, grid_ref_vertex(t->nc), kRefVertexThreads, 0, t->nc, C->x, C->prev, C->s, C->last, C->v, C->fixf, C->mass,
                C->vdiag, C->slot_ptr, C->slots, C->spheres_dev, pc.collision_stiffness, pc.dt, omega,
                (double)pc.relaxation, it == pc.iterations - 1 ? 2 : 0, C->cflag, C->cdepth, C->cenergy, C->nonfinite,
                t->tri_ptr, t->tri_idx, t->push);
@@ -3504,7 +3539,7 @@ void enqueue_two_level_frame(mgsb_two_level* t) {
         LAUNCH(F, k_ref_local, grid_for(F->T), kBlock, 0, F->T, F->tets, F->tA, F->tB, F->tC, F->x, F->slot_of, F->slots,
                pf.volume_stiffness, 0);
         omega = 4 / (4 - pf.cheb_rho * pf.cheb_rho * omega);
-        LAUNCH(F, k_ref_vertex, grid_for(t->nf), kBlock, 0, t->nf, F->x, F->prev, F->s, F->last, F->v, F->fixf, F->mass,
+        LAUNCH(F, k_ref_vertex, grid_ref_vertex(t->nf), kRefVertexThreads, 0, t->nf, F->x, F->prev, F->s, F->last, F->v, F->fixf, F->mass,
                F->vdiag, F->slot_ptr, F->slots, F->spheres_dev, pf.collision_stiffness, pf.dt, omega,
                (double)pf.relaxation, it == pf.iterations - 1 ? 2 : 0, F->cflag, F->cdepth, F->cenergy, F->nonfinite,
                nullptr, nullptr, nullptr);
