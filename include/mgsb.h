@@ -207,7 +207,7 @@ mgsb_status mgsb_get_normals(mgsb_solver* h, int32_t body, float* out /* [3*V] *
  * cudaMalloc while they run (a host that owns the GPU memory budget and forbids
  * driver allocations in its frame loop; a real-time thread that cannot take the
  * implicit synchronisation of cudaMalloc/cudaFree).  No counterpart in the
- * reference.  Scratch is a fixed 2 MiB device array inside the library, held by
+ * reference.  Scratch is a fixed 1 MiB device array inside the library, held by
  * every GPU that loads it until exit; a body may have at most 65,536 surface
  * triangles and 65,536 surface vertices, else MGSB_NOT_SUPPORTED.  A pending
  * set-up (after mgsb_set_fixed / mgsb_set_material) is not rebuilt here:

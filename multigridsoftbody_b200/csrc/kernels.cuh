@@ -524,15 +524,45 @@ __global__ void k_l0_frame(int n, const float4* __restrict__ s, const float* __r
     d[i] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
-// Positions as packed xyz (3 floats per vertex) for the zero-copy frame
-// readback; launched on its own after a frame, outside the frame's graph.
-__global__ void k_pack_xyz(int n, const float4* __restrict__ x, float* __restrict__ out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+// Readbacks straight into pinned host memory (or, packed on the device, for a
+// copy in pieces), the non-finite flag with them:
+// a launch and a synchronisation instead of up to three copies (each 2-4 us
+// between a frame's last kernel and the host, whatever its size).  4 rows per
+// thread, 16-byte stores that leave whole lines.  Launched on their own after a
+// frame, outside its graph.  out: n x 3 floats, then (flags set) n words; the
+// flag's word at nf_out.
+__global__ void __launch_bounds__(256) k_read_frame(int n, const float4* __restrict__ x, const int32_t* __restrict__ flags,
+                                                    const int32_t* __restrict__ nonfinite, float* __restrict__ out,
+                                                    int32_t* __restrict__ flags_out, int32_t* __restrict__ nf_out) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, i = 4 * t;
+    if (t == 0) *nf_out = *nonfinite;
     if (i >= n) return;
-    const float4 v = x[i];
-    out[3 * i] = v.x;
-    out[3 * i + 1] = v.y;
-    out[3 * i + 2] = v.z;
+    if (i + 4 <= n) {
+        const float4 a = x[i], b = x[i + 1], c = x[i + 2], d = x[i + 3];
+        float4* o = reinterpret_cast<float4*>(out) + 3 * (size_t)t;
+        o[0] = make_float4(a.x, a.y, a.z, b.x);
+        o[1] = make_float4(b.y, b.z, c.x, c.y);
+        o[2] = make_float4(c.z, d.x, d.y, d.z);
+        if (flags)   // flags_out follows 12 n bytes: 4-byte aligned only
+            for (int k = 0; k < 4; ++k) flags_out[i + k] = flags[i + k];
+        return;
+    }
+    for (int k = i; k < n; ++k) {
+        const float4 v = x[k];
+        out[3 * k] = v.x;
+        out[3 * k + 1] = v.y;
+        out[3 * k + 2] = v.z;
+        if (flags) flags_out[k] = flags[k];
+    }
+}
+
+// n words (contact flags, depths, float4 rows) and the flag.
+__global__ void __launch_bounds__(256) k_read_words(int n, const int32_t* __restrict__ src,
+                                                    const int32_t* __restrict__ nonfinite, int32_t* __restrict__ out,
+                                                    int32_t* __restrict__ nf_out) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0) *nf_out = *nonfinite;
+    if (i < n) out[i] = src[i];
 }
 
 // End of frame: x = s + d, v = v_predicted + d/dt (= (x - x_prev)/dt), and a

@@ -43,11 +43,14 @@ __global__ void __launch_bounds__(256) k_tri_normals(int nf, const int4* __restr
 
 // Per surface vertex j: sum of its triangles' normals (vertex->triangle CSR,
 // triangle ids local to the body), divided by the length when it exceeds
-// FLT_EPSILON (AvgOutsideTetVertNormal).
+// FLT_EPSILON (AvgOutsideTetVertNormal).  out (and the non-finite flag's copy)
+// may be pinned host memory.
 __global__ void __launch_bounds__(256) k_vert_normals(int nsv, const int32_t* __restrict__ ptr,
                                                       const int32_t* __restrict__ fidx, const float4* __restrict__ fn,
-                                                      float4* __restrict__ out) {
+                                                      float4* __restrict__ out, const int32_t* __restrict__ nonfinite,
+                                                      int32_t* __restrict__ nf_out) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j == 0) *nf_out = *nonfinite;
     if (j >= nsv) return;
     float sx = 0.f, sy = 0.f, sz = 0.f;
     const int e1 = __ldg(ptr + j + 1);
@@ -213,8 +216,11 @@ __global__ void __launch_bounds__(kEnergyThreads) k_energy_partial(EnergyArgs a,
 
 // out[k] = sum over blocks of partial k (fixed order); out[4] = sqrt.
 __global__ void __launch_bounds__(kEnergyThreads) k_energy_final(const double* __restrict__ partial, int nblk,
-                                                                 double* __restrict__ out) {
+                                                                 double* __restrict__ out,
+                                                                 const int32_t* __restrict__ nonfinite,
+                                                                 int32_t* __restrict__ nf_out) {
     __shared__ double red[kEnergyThreads / 32];
+    if (threadIdx.x == 0) *nf_out = *nonfinite;
     for (int k = 0; k < kEnergyTerms; ++k) {
         double v = 0.0;
         for (int j = threadIdx.x; j < nblk; j += blockDim.x) v += partial[k * nblk + j];

@@ -94,21 +94,6 @@ __device__ __forceinline__ float ls_row_features(int row, float sx, float sy, fl
     return (fx != 0.f && s > 0.f) ? s / D : 0.f;
 }
 
-// 16 BF16 features (9 used) of one row into a K-major interleaved tile.
-__device__ __forceinline__ void ls_store_tile_row(uint8_t* tile, int row_in_tile, const float (&f)[kMlpIn]) {
-    uint32_t w[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const float lo = 2 * i < kMlpIn ? f[2 * i] : 0.f;
-        const float hi = 2 * i + 1 < kMlpIn ? f[2 * i + 1] : 0.f;
-        const __nv_bfloat162 two = __floats2bfloat162_rn(lo, hi);
-        w[i] = *reinterpret_cast<const uint32_t*>(&two);
-    }
-    uint8_t* base = tile + interleaved_offset(row_in_tile, 0, kMlpInPad);
-    *reinterpret_cast<uint4*>(base) = make_uint4(w[0], w[1], w[2], w[3]);
-    *reinterpret_cast<uint4*>(base + 128) = make_uint4(w[4], w[5], w[6], w[7]);
-}
-
 // Features of every row into the BF16 tensor-core tiles and the update scale
 // s_i / D_i (0 for fixed vertices or a zero residual); optionally the FP32
 // features row-major into xf[n][9].  4 lanes per row.
@@ -151,7 +136,7 @@ __global__ void __launch_bounds__(kLsThreads) k_ls_features(int n, const int32_t
     if (!valid || lane >= S) return;
     float f[kMlpIn];
     scale[row] = ls_row_features(row, sx, sy, sz, sa, sd, dfull, diag0, fixf, r, f);
-    if (tiles) ls_store_tile_row(tiles + (size_t)(row / kMlpTile) * kTileBytes, row % kMlpTile, f);
+    if (tiles) mlp_store_features(tiles + (size_t)(row / kMlpTile) * kTileBytes, row % kMlpTile, f);
     if (xf)
         for (int k = 0; k < kMlpIn; ++k) xf[(size_t)row * kMlpIn + k] = f[k];
 }
@@ -356,7 +341,7 @@ __global__ void __launch_bounds__(kMlpThreads) k_ls_sweep_tc(int n, int ntiles, 
                 f[8] = bz * is;
                 sc = (fxr != 0.f && s > 0.f) ? s / Dr : 0.f;
             }
-            ls_store_tile_row(Sm.x, rt, f);
+            mlp_store_features(Sm.x, rt, f);
         }
         fence_async_shared();
         tc_fence_before();

@@ -94,18 +94,6 @@ __global__ void k_mlp_pack(const float* __restrict__ prm, uint8_t* __restrict__ 
     if (t < kMlpOutPad) bias[2 * kMlpHid + t] = t < kMlpOut ? prm[kOffB3 + t] : 0.f;
 }
 
-// Row-major FP32 features [n][9] -> BF16 interleaved tiles (rows padded to a
-// multiple of 128 with zeros).
-__global__ void k_mlp_tile_features(int n, int ntiles, const float* __restrict__ x, uint8_t* __restrict__ tiles) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= ntiles * kMlpTile * kMlpInPad) return;
-    const int row = t / kMlpInPad, k = t % kMlpInPad;
-    const int tile = row / kMlpTile, r = row % kMlpTile;
-    const float v = (row < n && k < kMlpIn) ? x[(size_t)row * kMlpIn + k] : 0.f;
-    reinterpret_cast<__nv_bfloat16*>(tiles + (size_t)tile * kTileBytes)[interleaved_offset(r, k, kMlpInPad) / 2] =
-        __float2bfloat16_rn(v);
-}
-
 // ---------------------------------------------------------------------------
 // tcgen05 / bulk-copy / mbarrier helpers (inline PTX, sm_100a)
 // ---------------------------------------------------------------------------
@@ -179,10 +167,7 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // ---------------------------------------------------------------------------
-// Inference: one CTA (4 warps) per 128-row tile, grid-strided over tiles.
-//   out_mode 0: y[row] = (y0, y1, y2, 0)
-//   out_mode 1: e[row] += scale[row] * (y0, y1, y2)   (learned smoothing sweep)
-// err (optional): set to 1 when a bounded wait ran out; the kernel then stops.
+// Inference: one CTA per 128-row tile, grid-strided over tiles.
 // ---------------------------------------------------------------------------
 constexpr int kMlpThreads = 256;   // 8 warps: warp w serves TMEM lanes 32 (w % 4).. and hidden columns 32 (w / 4)..
 constexpr int kTmemCols = 256;     // D1 cols [0,64), D2 [64,128), D3 [128,144)
@@ -364,15 +349,27 @@ __device__ __forceinline__ bool mlp_tile_layers(MlpSmem& S, uint32_t tmem, uint3
     return ok;
 }
 
-// Inference over feature tiles in global memory: one CTA (4 warps) per
-// 128-row tile, grid-strided.
-//   out_mode 0: y[row] = (y0, y1, y2, 0)
-//   out_mode 1: e[row] += scale[row] * (y0, y1, y2)
-// err (optional): set to 1 when a bounded wait ran out; the kernel then stops.
-__global__ void __launch_bounds__(kMlpThreads) k_mlp_tc(int n, int ntiles, const uint8_t* __restrict__ tiles,
-                                                        const uint8_t* __restrict__ img, int out_mode,
-                                                        float4* __restrict__ y, float4* __restrict__ e,
-                                                        const float* __restrict__ scale, int32_t* __restrict__ err) {
+// One row of FP32 features into the BF16 operand tile (K padded 9 -> 16 with zeros).
+__device__ __forceinline__ void mlp_store_features(uint8_t* tile, int row_in_tile, const float (&f)[kMlpIn]) {
+    uint32_t w[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const float lo = 2 * i < kMlpIn ? f[2 * i] : 0.f;
+        const float hi = 2 * i + 1 < kMlpIn ? f[2 * i + 1] : 0.f;
+        const __nv_bfloat162 two = __floats2bfloat162_rn(lo, hi);
+        w[i] = *reinterpret_cast<const uint32_t*>(&two);
+    }
+    uint8_t* base = tile + interleaved_offset(row_in_tile, 0, kMlpInPad);
+    *reinterpret_cast<uint4*>(base) = make_uint4(w[0], w[1], w[2], w[3]);
+    *reinterpret_cast<uint4*>(base + 128) = make_uint4(w[4], w[5], w[6], w[7]);
+}
+
+// Inference on row-major features x[n][9], outputs y[n][3]: one CTA per 128-row tile, grid-strided; a thread per row
+// rounds the row's features straight into the operand tile.  err: set to 1 when a bounded wait ran out; the kernel
+// then stops.
+__global__ void __launch_bounds__(kMlpThreads) k_mlp_tc(int n, int ntiles, const float* __restrict__ x,
+                                                        const uint8_t* __restrict__ img, float* __restrict__ y,
+                                                        int32_t* __restrict__ err) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     MlpSmem& S = *reinterpret_cast<MlpSmem*>(smem_raw);
     WaitState ws;
@@ -382,30 +379,26 @@ __global__ void __launch_bounds__(kMlpThreads) k_mlp_tc(int n, int ntiles, const
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         __syncthreads();
         if (S.stop) break;
-        if (threadIdx.x == 0) {
-            mbar_expect_tx(&S.bar_load, kTileBytes);
-            bulk_g2s(S.x, tiles + (size_t)tile * kTileBytes, kTileBytes, &S.bar_load);
+        const int row = tile * kMlpTile + row_in_tile;
+        if (row_in_tile < kMlpTile) {
+            float f[kMlpIn];
+#pragma unroll
+            for (int k = 0; k < kMlpIn; ++k) f[k] = row < n ? x[(size_t)row * kMlpIn + k] : 0.f;
+            mlp_store_features(S.x, row_in_tile, f);
         }
-        bool ok = wait_bar(ws, &S.bar_load, ph_load);
-        ph_load ^= 1;
+        fence_async_shared();
+        tc_fence_before();
+        __syncthreads();
         float out[3];
-        ok = mlp_tile_layers(S, tmem, ph_mma, ws, ok, out);
+        const bool ok = mlp_tile_layers(S, tmem, ph_mma, ws, true, out);
         if (!ok) {
             S.stop = 1;
             if (err) atomicExch(err, 1);
         }
-        const int row = tile * kMlpTile + row_in_tile;
         if (ok && row_in_tile < kMlpTile && row < n) {
-            if (out_mode == 0) {
-                y[row] = make_float4(out[0], out[1], out[2], 0.f);
-            } else {
-                const float sc = scale[row];
-                float4 q = e[row];
-                q.x += sc * out[0];
-                q.y += sc * out[1];
-                q.z += sc * out[2];
-                e[row] = q;
-            }
+            y[3 * (size_t)row] = out[0];
+            y[3 * (size_t)row + 1] = out[1];
+            y[3 * (size_t)row + 2] = out[2];
         }
     }
     mlp_cta_teardown(S, tmem, ws);

@@ -126,7 +126,8 @@ struct mgsb_solver {
     int stage_idx = 0;
     // pinned host buffer for readbacks (N0 x 16 bytes: positions, velocities, flags)
     char* readback = nullptr;
-    float* xpack = nullptr;   // positions as packed xyz (mgsb_get_frame_view)
+    float* xpack = nullptr;   // positions as packed xyz, for the frames that are copied in pieces (mgsb_get_frame)
+    cudaEvent_t piece_ev[2] = {nullptr, nullptr};
     // ---- state (kept across rebuilds)
     float4 *x = nullptr, *xb = nullptr, *v = nullptr, *s = nullptr, *last = nullptr, *prev = nullptr;
     int32_t* cflag = nullptr;
@@ -185,9 +186,9 @@ struct mgsb_solver {
     std::vector<int> nrm_f_off, nrm_nf, nrm_sv_off, nrm_nsv;
     std::vector<int32_t> nrm_sv_host;
     int nrm_max_f = 0, nrm_max_sv = 0;
-    float4 *nrm_face = nullptr, *nrm_out = nullptr;   // scratch: triangle normals, vertex normals
-    // energy reduction scratch: per-block partials and the five results
-    double *energy_part = nullptr, *energy_out = nullptr;
+    float4* nrm_face = nullptr;   // scratch: triangle normals
+    // energy reduction scratch: per-block partials
+    double* energy_part = nullptr;
     std::vector<LevelDev> lev;   // lev[0] = finest
     float *A0dense = nullptr, *B0dense = nullptr, *Lfac = nullptr, *Ldinv = nullptr, *c_prev = nullptr;
     int2* range = nullptr;
@@ -266,6 +267,8 @@ mgsb_solver::~mgsb_solver() {
         if (stage_ev[k]) cudaEventDestroy(stage_ev[k]);
     }
     if (readback) cudaFreeHost(readback);
+    for (cudaEvent_t e : piece_ev)
+        if (e) cudaEventDestroy(e);
     if (staged_dev) cudaFree(staged_dev);
     if (aux_stream) cudaStreamDestroy(aux_stream);
     if (ev0) cudaEventDestroy(ev0);
@@ -511,7 +514,6 @@ mgsb_status upload_normals_data(mgsb_solver* h, std::vector<DevMem>& pool) {
     TRY(dupload(h, pool, &h->nrm_ptr, ptr_all));
     TRY(dupload(h, pool, &h->nrm_fidx, fidx_all));
     TRY(dalloc(h, pool, &h->nrm_face, (size_t)std::max(1, h->nrm_max_f)));
-    TRY(dalloc(h, pool, &h->nrm_out, (size_t)std::max(1, h->nrm_max_sv)));
     return MGSB_OK;
 }
 
@@ -795,7 +797,6 @@ mgsb_status rebuild(mgsb_solver* h) {
         CUDA_TRY(h, cudaDeviceGetAttribute(&h->sm_count, cudaDevAttrMultiProcessorCount, h->device));
     }
     TRY(dalloc(h, pool, &h->energy_part, (size_t)kEnergyBlocks * kEnergyTerms));
-    TRY(dalloc(h, pool, &h->energy_out, kEnergyTerms));
     h->dirty = false;
     return MGSB_OK;
 }
@@ -1989,8 +1990,7 @@ mgsb_status push_tool(mgsb_solver* h) {
     const size_t nb = h->bodies.size() * sizeof(BodyDev);
     std::memcpy(h->stage[k], h->bodies_host, nb);
     std::memcpy(h->stage[k] + nb, h->spheres_host, sizeof(SphereSet));
-    CUDA_TRY(h, cudaMemcpyAsync(h->bodies_dev, h->stage[k], nb, cudaMemcpyHostToDevice, h->stream));
-    CUDA_TRY(h, cudaMemcpyAsync(h->spheres_dev, h->stage[k] + nb, sizeof(SphereSet), cudaMemcpyHostToDevice, h->stream));
+    CUDA_TRY(h, cudaMemcpyAsync(h->bodies_dev, h->stage[k], nb + sizeof(SphereSet), cudaMemcpyHostToDevice, h->stream));
     CUDA_TRY(h, cudaEventRecord(h->stage_ev[k], h->stream));
     return MGSB_OK;
 }
@@ -2142,9 +2142,9 @@ mgsb_status create_impl(int32_t nbodies, const mgsb_mesh* meshes, const mgsb_par
     }
     auto& pool = h->state_mem;
     const int N0 = h->N0;
-    // pinned readback: N0 float4 rows (or, for mgsb_get_frame_view, N0 packed xyz + N0 contact
-    // flags), then the non-finite flag that every readback fetches with its data (at N0 x 16 B)
-    CUDA_TRY(hp, cudaMallocHost((void**)&h->readback, (size_t)std::max(N0, 1) * sizeof(float4) + 16));
+    // pinned readback: N0 float4 rows (or N0 packed xyz + N0 contact flags), then the non-finite flag that every
+    // readback fetches with its data (at N0 x 16 B) and the energies
+    CUDA_TRY(hp, cudaMallocHost((void**)&h->readback, (size_t)std::max(N0, 1) * sizeof(float4) + 16 + kEnergyTerms * sizeof(double)));
     TRY(dalloc(hp, pool, &h->x, N0));
     TRY(dalloc(hp, pool, &h->xpack, (size_t)3 * std::max(N0, 1)));
     TRY(dalloc(hp, pool, &h->xb, N0));
@@ -2165,8 +2165,13 @@ mgsb_status create_impl(int32_t nbodies, const mgsb_mesh* meshes, const mgsb_par
         CUDA_TRY(hp, cudaMemcpy(h->x64, x.data(), N0 * sizeof(double4), cudaMemcpyHostToDevice));
         CUDA_TRY(hp, cudaMemset(h->v64, 0, N0 * sizeof(double4)));
     }
-    TRY(dalloc(hp, pool, &h->bodies_dev, nbodies));
-    TRY(dalloc(hp, pool, &h->spheres_dev, 1));
+    {   // the body table and the spheres in one piece: one copy per frame
+        static_assert(sizeof(BodyDev) % alignof(SphereSet) == 0, "the spheres follow the body table");
+        char* table = nullptr;
+        TRY(dalloc(hp, pool, &table, nbodies * sizeof(BodyDev) + sizeof(SphereSet)));
+        h->bodies_dev = reinterpret_cast<BodyDev*>(table);
+        h->spheres_dev = reinterpret_cast<SphereSet*>(table + nbodies * sizeof(BodyDev));
+    }
     {
         std::vector<float4> x4(N0);
         for (const BodyHost& B : h->bodies)
@@ -2188,63 +2193,67 @@ mgsb_status create_impl(int32_t nbodies, const mgsb_mesh* meshes, const mgsb_par
     return MGSB_OK;
 }
 
-// Device -> pinned readback buffer, together with the non-finite flag, in one
-// stream synchronisation: MGSB_DIVERGED when the flag is set (the caller then
-// writes nothing).
-mgsb_status readback_checked(mgsb_solver* h, const void* src, size_t bytes) {
-    CUDA_TRY(h, cudaSetDevice(h->device));
-    int32_t* flag = reinterpret_cast<int32_t*>(h->readback + (size_t)std::max(h->N0, 1) * sizeof(float4));
-    CUDA_TRY(h, cudaMemcpyAsync(flag, h->nonfinite, sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
-    if (bytes) CUDA_TRY(h, cudaMemcpyAsync(h->readback, src, bytes, cudaMemcpyDeviceToHost, h->stream));
+// The non-finite flag's word of the pinned readback buffer (after N0 x 16 bytes).
+int32_t* readback_flag(mgsb_solver* h) {
+    return reinterpret_cast<int32_t*>(h->readback + (size_t)std::max(h->N0, 1) * sizeof(float4));
+}
+
+// After a readback kernel: one synchronisation, and MGSB_DIVERGED when the flag that came with the data is set (the
+// caller then writes nothing).
+mgsb_status readback_done(mgsb_solver* h) {
+    CUDA_TRY(h, cudaGetLastError());
     CUDA_TRY(h, cudaStreamSynchronize(h->stream));
-    if (*flag) return set_err(h, MGSB_DIVERGED, "non-finite positions detected");
+    if (*readback_flag(h)) return set_err(h, MGSB_DIVERGED, "non-finite positions detected");
     return MGSB_OK;
 }
 
-template <typename F>
-mgsb_status copy_body_f4(mgsb_solver* h, int32_t body, const float4* src, F&& sink) {
+// Rows [off, off + n) of the positions or velocities as packed xyz in the pinned readback buffer, with the contact
+// flags after them when asked for.
+mgsb_status read_rows(mgsb_solver* h, const float4* src, int off, int n, bool flags) {
+    CUDA_TRY(h, cudaSetDevice(h->device));
+    float* out = reinterpret_cast<float*>(h->readback);
+    k_read_frame<<<std::max(1, grid_for((n + 3) / 4)), kBlock, 0, h->stream>>>(
+        n, src + off, flags ? h->cflag + off : nullptr, h->nonfinite, out, reinterpret_cast<int32_t*>(out + 3 * (size_t)n),
+        readback_flag(h));
+    return readback_done(h);
+}
+
+// n words of device memory into the pinned readback buffer.
+mgsb_status read_words(mgsb_solver* h, const void* src, int n) {
+    CUDA_TRY(h, cudaSetDevice(h->device));
+    k_read_words<<<std::max(1, grid_for(n)), kBlock, 0, h->stream>>>(n, static_cast<const int32_t*>(src), h->nonfinite,
+                                                                   reinterpret_cast<int32_t*>(h->readback), readback_flag(h));
+    return readback_done(h);
+}
+
+mgsb_status copy_rows(mgsb_solver* h, int32_t body, const float4* src, float* out) {
     TRY(check_body(h, body));
     const BodyHost& B = h->bodies[body];
-    TRY(readback_checked(h, src + B.v_off, B.V * sizeof(float4)));
-    const float4* tmp = reinterpret_cast<const float4*>(h->readback);
-    for (int i = 0; i < B.V; ++i) sink(i, tmp[i]);
+    TRY(read_rows(h, src, B.v_off, B.V, false));
+    std::memcpy(out, h->readback, (size_t)B.V * 3 * sizeof(float));
     return MGSB_OK;
 }
 
-// Surface normals of one body from the current positions: triangle normals
-// into fscratch (>= the body's triangle count), vertex normals of the
-// surface vertices into vscratch (>= its surface-vertex count), then a copy
-// to the host and a scatter into out[3V] (zero for interior vertices).  The
-// copy lands in host_stage (>= the surface-vertex count of float4) when one is
-// given, else in a temporary host vector.
-mgsb_status run_normals(mgsb_solver* h, int32_t body, float4* fscratch, float4* vscratch, float4* host_stage,
-                        float* out) {
+// Surface normals of one body from the current positions: triangle normals into fscratch (>= the body's triangle
+// count), vertex normals of the surface vertices into the pinned readback buffer, then a scatter into out[3V] (zero
+// for interior vertices).
+mgsb_status run_normals(mgsb_solver* h, int32_t body, float4* fscratch, float* out) {
     const BodyHost& B = h->bodies[body];
     const int nf = h->nrm_nf[body], nsv = h->nrm_nsv[body];
     const int f_off = h->nrm_f_off[body], sv_off = h->nrm_sv_off[body];
+    const float4* nrm = reinterpret_cast<const float4*>(h->readback);
     CUDA_TRY(h, cudaSetDevice(h->device));
-    if (nf > 0) {
-        k_tri_normals<<<(nf + 255) / 256, 256, 0, h->stream>>>(nf, h->nrm_tris + f_off, h->x, fscratch);
-        k_vert_normals<<<(nsv + 255) / 256, 256, 0, h->stream>>>(nsv, h->nrm_ptr + sv_off, h->nrm_fidx, fscratch, vscratch);
-        CUDA_TRY(h, cudaGetLastError());
-    }
-    std::vector<float4> tmp;
-    if (!host_stage) {
-        tmp.resize(nsv);
-        host_stage = tmp.data();
-    }
-    if (nsv > 0)
-        CUDA_TRY(h, cudaMemcpyAsync(host_stage, vscratch, nsv * sizeof(float4), cudaMemcpyDeviceToHost, h->stream));
-    CUDA_TRY(h, cudaStreamSynchronize(h->stream));
-    int32_t nf_flag = 0;
-    CUDA_TRY(h, cudaMemcpy(&nf_flag, h->nonfinite, sizeof(int32_t), cudaMemcpyDeviceToHost));
-    if (nf_flag) return set_err(h, MGSB_DIVERGED, "non-finite positions detected");
+    if (nf > 0) k_tri_normals<<<(nf + 255) / 256, 256, 0, h->stream>>>(nf, h->nrm_tris + f_off, h->x, fscratch);
+    k_vert_normals<<<std::max(1, (nsv + 255) / 256), 256, 0, h->stream>>>(
+        nsv, h->nrm_ptr + sv_off, h->nrm_fidx, fscratch, reinterpret_cast<float4*>(h->readback), h->nonfinite,
+        readback_flag(h));
+    TRY(readback_done(h));
     std::fill(out, out + 3 * (size_t)B.V, 0.f);
     for (int j = 0; j < nsv; ++j) {
         const int i = h->nrm_sv_host[sv_off + j] - B.v_off;
-        out[3 * i] = host_stage[j].x;
-        out[3 * i + 1] = host_stage[j].y;
-        out[3 * i + 2] = host_stage[j].z;
+        out[3 * i] = nrm[j].x;
+        out[3 * i + 1] = nrm[j].y;
+        out[3 * i + 2] = nrm[j].z;
     }
     return MGSB_OK;
 }
@@ -2417,11 +2426,7 @@ mgsb_status mgsb_synchronize(mgsb_solver* h) {
 mgsb_status mgsb_get_positions(mgsb_solver* h, int32_t body, float* out) {
     if (!out) return MGSB_INVALID_ARG;
     TRY(check_body(h, body));
-    return copy_body_f4(h, body, h->x, [&](int i, float4 v) {
-        out[3 * i] = v.x;
-        out[3 * i + 1] = v.y;
-        out[3 * i + 2] = v.z;
-    });
+    return copy_rows(h, body, h->x, out);
 }
 
 mgsb_status mgsb_get_velocities(mgsb_solver* h, int32_t body, float* out) {
@@ -2439,22 +2444,13 @@ mgsb_status mgsb_get_velocities(mgsb_solver* h, int32_t body, float* out) {
         }
         return MGSB_OK;
     }
-    return copy_body_f4(h, body, h->v, [&](int i, float4 v) {
-        out[3 * i] = v.x;
-        out[3 * i + 1] = v.y;
-        out[3 * i + 2] = v.z;
-    });
+    return copy_rows(h, body, h->v, out);
 }
 
 mgsb_status mgsb_get_all_positions(mgsb_solver* h, float* out) {
     if (!h || !out) return MGSB_INVALID_ARG;
-    TRY(readback_checked(h, h->x, h->N0 * sizeof(float4)));
-    const float4* tmp = reinterpret_cast<const float4*>(h->readback);
-    for (int i = 0; i < h->N0; ++i) {
-        out[3 * i] = tmp[i].x;
-        out[3 * i + 1] = tmp[i].y;
-        out[3 * i + 2] = tmp[i].z;
-    }
+    TRY(read_rows(h, h->x, 0, h->N0, false));
+    std::memcpy(out, h->readback, (size_t)h->N0 * 3 * sizeof(float));
     return MGSB_OK;
 }
 
@@ -2478,44 +2474,71 @@ mgsb_status mgsb_get_contact_flags(mgsb_solver* h, int32_t body, int32_t* out) {
     if (!out) return MGSB_INVALID_ARG;
     TRY(check_body(h, body));
     const BodyHost& B = h->bodies[body];
-    TRY(readback_checked(h, h->cflag + B.v_off, B.V * sizeof(int32_t)));
+    TRY(read_words(h, h->cflag + B.v_off, B.V));
     std::memcpy(out, h->readback, B.V * sizeof(int32_t));
     return MGSB_OK;
 }
 
 mgsb_status mgsb_get_all_contact_flags(mgsb_solver* h, int32_t* out) {
     if (!h || !out) return MGSB_INVALID_ARG;
-    TRY(readback_checked(h, h->cflag, h->N0 * sizeof(int32_t)));
+    TRY(read_words(h, h->cflag, h->N0));
     std::memcpy(out, h->readback, h->N0 * sizeof(int32_t));
     return MGSB_OK;
 }
 
+// Frames above this many vertices are copied in pieces, each from the pinned buffer to the caller's arrays while the
+// next one crosses the bus; one piece costs less below it (a piece's event and copy launches: 5 us).
+constexpr int kFramePiece = 65536;
+
 mgsb_status mgsb_get_frame(mgsb_solver* h, float* positions, int32_t* contact_flags) {
     if (!h || !positions || !contact_flags) return MGSB_INVALID_ARG;
-    const float* pos = nullptr;
-    const int32_t* flags = nullptr;
-    TRY(mgsb_get_frame_view(h, &pos, &flags));
     const size_t n = (size_t)h->N0;
-    std::memcpy(positions, pos, n * 3 * sizeof(float));
-    std::memcpy(contact_flags, flags, n * sizeof(int32_t));
+    if (n <= kFramePiece) {
+        const float* pos = nullptr;
+        const int32_t* flags = nullptr;
+        TRY(mgsb_get_frame_view(h, &pos, &flags));
+        std::memcpy(positions, pos, n * 3 * sizeof(float));
+        std::memcpy(contact_flags, flags, n * sizeof(int32_t));
+        return MGSB_OK;
+    }
+    CUDA_TRY(h, cudaSetDevice(h->device));
+    for (cudaEvent_t& e : h->piece_ev)
+        if (!e) CUDA_TRY(h, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    // the flag comes first: a diverged frame writes nothing
+    k_read_frame<<<grid_for((int)((n + 3) / 4)), kBlock, 0, h->stream>>>((int)n, h->x, nullptr, h->nonfinite, h->xpack,
+                                                                         nullptr, readback_flag(h));
+    CUDA_TRY(h, cudaGetLastError());
+    float* pos = reinterpret_cast<float*>(h->readback);
+    int32_t* flags = reinterpret_cast<int32_t*>(pos + 3 * n);
+    const size_t pieces = (n + kFramePiece - 1) / kFramePiece;
+    auto first = [&](size_t k) { return std::min(n, k * kFramePiece); };
+    auto send = [&](size_t k) -> mgsb_status {
+        const size_t a = first(k), m = first(k + 1) - a;
+        CUDA_TRY(h, cudaMemcpyAsync(pos + 3 * a, h->xpack + 3 * a, m * 3 * sizeof(float), cudaMemcpyDeviceToHost, h->stream));
+        CUDA_TRY(h, cudaMemcpyAsync(flags + a, h->cflag + a, m * sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
+        CUDA_TRY(h, cudaEventRecord(h->piece_ev[k & 1], h->stream));
+        return MGSB_OK;
+    };
+    TRY(send(0));
+    for (size_t k = 0; k < pieces; ++k) {
+        if (k + 1 < pieces) TRY(send(k + 1));
+        CUDA_TRY(h, cudaEventSynchronize(h->piece_ev[k & 1]));
+        if (*readback_flag(h)) {
+            CUDA_TRY(h, cudaStreamSynchronize(h->stream));
+            return set_err(h, MGSB_DIVERGED, "non-finite positions detected");
+        }
+        const size_t a = first(k), m = first(k + 1) - a;
+        std::memcpy(positions + 3 * a, pos + 3 * a, m * 3 * sizeof(float));
+        std::memcpy(contact_flags + a, flags + a, m * sizeof(int32_t));
+    }
     return MGSB_OK;
 }
 
 mgsb_status mgsb_get_frame_view(mgsb_solver* h, const float** positions, const int32_t** contact_flags) {
     if (!h || !positions || !contact_flags) return MGSB_INVALID_ARG;
-    const size_t n = (size_t)h->N0;
-    float* pos = reinterpret_cast<float*>(h->readback);                           // [0, 12 N)
-    int32_t* flags = reinterpret_cast<int32_t*>(h->readback + n * 3 * sizeof(float));   // [12 N, 16 N)
-    CUDA_TRY(h, cudaSetDevice(h->device));
-    if (n) {
-        k_pack_xyz<<<grid_for((int)n), kBlock, 0, h->stream>>>((int)n, h->x, h->xpack);
-        CUDA_TRY(h, cudaGetLastError());
-        CUDA_TRY(h, cudaMemcpyAsync(pos, h->xpack, n * 3 * sizeof(float), cudaMemcpyDeviceToHost, h->stream));
-        CUDA_TRY(h, cudaMemcpyAsync(flags, h->cflag, n * sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
-    }
-    TRY(readback_checked(h, nullptr, 0));   // the non-finite flag (at 16 N) and one synchronisation
-    *positions = pos;
-    *contact_flags = flags;
+    TRY(read_rows(h, h->x, 0, h->N0, true));   // [0, 12 N) positions, [12 N, 16 N) flags
+    *positions = reinterpret_cast<const float*>(h->readback);
+    *contact_flags = reinterpret_cast<const int32_t*>(h->readback + (size_t)h->N0 * 3 * sizeof(float));
     return MGSB_OK;
 }
 
@@ -2539,9 +2562,9 @@ mgsb_status mgsb_get_contacts(mgsb_solver* h, int32_t body, int32_t* idx, size_t
 mgsb_status mgsb_get_collision_depth(mgsb_solver* h, int32_t body, float* out) {
     if (!out) return MGSB_INVALID_ARG;
     TRY(check_body(h, body));
-    TRY(sync_check(h));
     const BodyHost& B = h->bodies[body];
-    CUDA_TRY(h, cudaMemcpy(out, h->cdepth + B.v_off, B.V * sizeof(float), cudaMemcpyDeviceToHost));
+    TRY(read_words(h, h->cdepth + B.v_off, B.V));
+    std::memcpy(out, h->readback, B.V * sizeof(float));
     return MGSB_OK;
 }
 
@@ -2556,7 +2579,7 @@ mgsb_status mgsb_get_normals(mgsb_solver* h, int32_t body, float* out) {
     if (!out) return MGSB_INVALID_ARG;
     TRY(check_body(h, body));
     TRY(ensure_ready(h));
-    return run_normals(h, body, h->nrm_face, h->nrm_out, nullptr, out);
+    return run_normals(h, body, h->nrm_face, out);
 }
 
 mgsb_status mgsb_set_state(mgsb_solver* h, int32_t body, const float* positions, const float* velocities) {
@@ -2592,7 +2615,6 @@ mgsb_status mgsb_get_energy(mgsb_solver* h, int32_t body, double out[5]) {
     if (!out) return MGSB_INVALID_ARG;
     TRY(check_body(h, body));
     TRY(ensure_ready(h));
-    TRY(sync_check(h));
     const BodyHost& B = h->bodies[body];
     const mgsb_params& p = h->p;
     EnergyArgs a{};
@@ -2639,10 +2661,11 @@ mgsb_status mgsb_get_energy(mgsb_solver* h, int32_t body, double out[5]) {
     const int nblk = std::max(1, std::min(kEnergyBlocks, (work + kEnergyThreads - 1) / kEnergyThreads));
     CUDA_TRY(h, cudaSetDevice(h->device));
     k_energy_partial<<<nblk, kEnergyThreads, 0, h->stream>>>(a, h->energy_part);
-    k_energy_final<<<1, kEnergyThreads, 0, h->stream>>>(h->energy_part, nblk, h->energy_out);
-    CUDA_TRY(h, cudaGetLastError());
-    CUDA_TRY(h, cudaMemcpyAsync(out, h->energy_out, kEnergyTerms * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-    CUDA_TRY(h, cudaStreamSynchronize(h->stream));
+    // the five results and the non-finite flag straight into pinned memory, past the readback buffer's flag word
+    double* res = reinterpret_cast<double*>(reinterpret_cast<char*>(readback_flag(h)) + 16);
+    k_energy_final<<<1, kEnergyThreads, 0, h->stream>>>(h->energy_part, nblk, res, h->nonfinite, readback_flag(h));
+    TRY(readback_done(h));
+    std::memcpy(out, res, kEnergyTerms * sizeof(double));
     return MGSB_OK;
 }
 
@@ -3126,11 +3149,11 @@ constexpr int kNoAllocMaxTris = 65536;        // triangle normals of one body
 constexpr int kNoAllocMaxSurfVerts = 65536;   // surface-vertex normals of one body
 constexpr int kNoAllocMaxDevices = 64;
 
-// 131,072 float4 = 2 MiB: triangle normals in [0, kNoAllocMaxTris), vertex
-// normals after them.  Every GPU that loads the library holds this array until
-// the process exits.  Nothing in it needs to start at zero: each call writes
-// every triangle slot it reads and every vertex slot it copies out.
-static __device__ __align__(256) float4 g_noalloc_scratch[kNoAllocMaxTris + kNoAllocMaxSurfVerts];
+// 65,536 float4 = 1 MiB of triangle normals (the vertex normals go to the
+// solver's pinned readback buffer).  Every GPU that loads the library holds this
+// array until the process exits.  Nothing in it needs to start at zero: each call
+// writes every triangle slot it reads.
+static __device__ __align__(256) float4 g_noalloc_scratch[kNoAllocMaxTris];
 
 // The driver's cuCtxGetCurrent, fetched through the runtime (no link against
 // libcuda): the context a cached symbol address belongs to.
@@ -3196,8 +3219,7 @@ extern "C" mgsb_status mgsb_get_normals_noalloc(mgsb_solver* h, int32_t body, fl
                        body, nf, nsv, kNoAllocMaxTris, kNoAllocMaxSurfVerts);
     float4* scratch = nullptr;
     TRY(noalloc_scratch(h, &scratch));
-    // the solver's pinned readback buffer (N0 float4, allocated at create) takes the copy
-    return run_normals(h, body, scratch, scratch + kNoAllocMaxTris, reinterpret_cast<float4*>(h->readback), out);
+    return run_normals(h, body, scratch, out);
 }
 
 // ===========================================================================
