@@ -1052,7 +1052,9 @@ __global__ void __launch_bounds__(1024) k_coarse_vcycle_dsm(const CoarseArgs A) 
 constexpr int kMaxCluster = 16;
 constexpr int kStagedStaticSmem = 1024;   // the barrier, and the alignment of the dynamic part
 constexpr int kStagedThreads = 512;       // at most: 128 registers a thread hold a phase's operator entries
-constexpr int kStagedHeld = 6;            // entries of a lane held in registers; longer rows read the rest in a loop
+// entries of a lane held in registers; longer rows read the rest in a loop
+template <int G>
+constexpr int kStagedHeld = G == kLanesL0 ? kHeldL0 : kHeldC;
 
 enum StagedKind : int {
     kStRestrict,   // right-hand side = restriction of the finer residual, correction = dinv of it
@@ -1096,6 +1098,12 @@ struct StagedPlan {
     int ainv;                     // the own rows of the coarsest inverse
     int phases, phase_at;         // the same in every CTA
     int bytes, block;
+    // level 0 too: its phases before and after the coarse levels' (0: the coarse levels alone)
+    int pre0, post0;
+    float4 *x, *b;                // in and out; right-hand side
+    int gather;                   // b = b0 + slots first
+    const float4 *b0, *slots;
+    const int32_t* slot_ptr;
 };
 
 __device__ __forceinline__ void cluster_st(uint32_t a, float4 v) {
@@ -1111,6 +1119,9 @@ __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_async8(uint32_t dst, const void* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
@@ -1136,26 +1147,42 @@ __device__ __forceinline__ float4 staged_dense_row(const T* a, int n, int lane, 
     return make_float4((float)ax, (float)ay, (float)az, 0.f);
 }
 
-// What a slice of 4 rows (8 lanes per row) needs of the image in one phase, in registers.
+// What a slice of 32 / G rows (G lanes per row: 8 on the coarse levels, 4 on level 0) needs of the image in one phase,
+// in registers.
+template <int G>
 struct StagedSlice {
+    static constexpr int kTo = kMaxCluster / G;   // CTAs that a lane stores its row to
     int row, li;   // this lane's row and its place among the own rows (0 when the row is not one)
     bool valid;
     int t, T;      // this lane's first and last step
-    int idx[kStagedHeld];
-    float val[kStagedHeld];
-    uint32_t d0, d1;   // where the row goes in this lane's two CTAs; 0: it does not
+    int idx[kStagedHeld<G>];
+    float val[kStagedHeld<G>];
+    uint32_t d[kTo];   // where the row goes in this lane's CTAs; 0: it does not
 };
 
-__device__ __forceinline__ void staged_load(StagedSlice& s, const StagedPhase& P, const unsigned char* smb, int g, int lane,
-                                            uint32_t peer0, uint32_t peer1) {
-    constexpr int S = 32 / kLanesC;
+// Shared memory of this lane's CTAs (of up to 16; a CTA beyond the cluster has an empty window).
+template <int G>
+__device__ __forceinline__ void staged_peers(uint32_t (&peer)[kMaxCluster / G], uint32_t base, int lane, int cs, int rank) {
+#pragma unroll
+    for (int j = 0; j < kMaxCluster / G; ++j) {
+        const int c = lane / (32 / G) + j * G;
+        peer[j] = cluster_addr(base, c < cs ? c : rank);
+    }
+}
+
+template <int G>
+__device__ __forceinline__ void staged_load(StagedSlice<G>& s, const StagedPhase& P, const unsigned char* smb, int g, int lane,
+                                            const uint32_t (&peer)[kMaxCluster / G]) {
+    constexpr int S = 32 / G;
     s.row = P.first + g * S + lane % S;
     s.valid = s.row >= P.rb && s.row < P.re;
     s.li = s.valid ? s.row - P.rb : 0;
     const int2* win = reinterpret_cast<const int2*>(smb + P.win) + lane / S;
-    const int2 w0 = win[0], w1 = win[kLanesC];
-    s.d0 = s.valid && (unsigned)(s.row - w0.x) < (unsigned)w0.y ? peer0 + P.dst + 16 * (s.row - w0.x) : 0u;
-    s.d1 = s.valid && (unsigned)(s.row - w1.x) < (unsigned)w1.y ? peer1 + P.dst + 16 * (s.row - w1.x) : 0u;
+#pragma unroll
+    for (int j = 0; j < kMaxCluster / G; ++j) {
+        const int2 w = win[j * G];
+        s.d[j] = s.valid && (unsigned)(s.row - w.x) < (unsigned)w.y ? peer[j] + P.dst + 16 * (s.row - w.x) : 0u;
+    }
     s.t = s.T = 0;
     if (P.kind == kStProlong) return;
     const int* ptr = reinterpret_cast<const int*>(smb + P.ptr);
@@ -1163,7 +1190,7 @@ __device__ __forceinline__ void staged_load(StagedSlice& s, const StagedPhase& P
     s.T = ptr[g + 1];
     const bool wide = P.src < 0;
 #pragma unroll
-    for (int k = 0; k < kStagedHeld; ++k) {
+    for (int k = 0; k < kStagedHeld<G>; ++k) {
         const int e = min(s.t + k, s.T - 1) * 32 + lane;   // past the end: the last entry with coefficient 0
         s.idx[k] = wide ? reinterpret_cast<const int*>(smb + P.idx)[e] : (int)reinterpret_cast<const uint16_t*>(smb + P.idx)[e];
         s.val[k] = s.t + k < s.T ? reinterpret_cast<const float*>(smb + P.val)[e] : 0.f;
@@ -1171,26 +1198,27 @@ __device__ __forceinline__ void staged_load(StagedSlice& s, const StagedPhase& P
 }
 
 // Sum of the slice's entries, reduced over each row's lanes.
-__device__ __forceinline__ float4 staged_sum(const StagedSlice& s, const StagedPhase& P, const unsigned char* smb, int lane) {
-    constexpr int S = 32 / kLanesC;
-    float4 v[kStagedHeld];
+template <int G>
+__device__ __forceinline__ float4 staged_sum(const StagedSlice<G>& s, const StagedPhase& P, const unsigned char* smb, int lane) {
+    constexpr int S = 32 / G;
+    float4 v[kStagedHeld<G>];
     if (P.src < 0) {
         const float4* x = P.gsrc;
 #pragma unroll
-        for (int k = 0; k < kStagedHeld; ++k) v[k] = __ldg(x + s.idx[k]);
+        for (int k = 0; k < kStagedHeld<G>; ++k) v[k] = __ldg(x + s.idx[k]);
     } else {
         const float4* x = reinterpret_cast<const float4*>(smb + P.src);
 #pragma unroll
-        for (int k = 0; k < kStagedHeld; ++k) v[k] = x[s.idx[k]];
+        for (int k = 0; k < kStagedHeld<G>; ++k) v[k] = x[s.idx[k]];
     }
     float ax = 0.f, ay = 0.f, az = 0.f;
 #pragma unroll
-    for (int k = 0; k < kStagedHeld; ++k) {
+    for (int k = 0; k < kStagedHeld<G>; ++k) {
         ax = fmaf(s.val[k], v[k].x, ax);
         ay = fmaf(s.val[k], v[k].y, ay);
         az = fmaf(s.val[k], v[k].z, az);
     }
-    for (int t = s.t + kStagedHeld; t < s.T; ++t) {
+    for (int t = s.t + kStagedHeld<G>; t < s.T; ++t) {
         const int e = t * 32 + lane;
         const float a = reinterpret_cast<const float*>(smb + P.val)[e];
         const float4 x = P.src < 0 ? __ldg(P.gsrc + reinterpret_cast<const int*>(smb + P.idx)[e])
@@ -1208,17 +1236,19 @@ __device__ __forceinline__ float4 staged_sum(const StagedSlice& s, const StagedP
     return make_float4(ax, ay, az, 0.f);
 }
 
-__device__ __forceinline__ void staged_store(const StagedSlice& s, const StagedPhase& P, int lane, float4 q) {
+template <int G>
+__device__ __forceinline__ void staged_store(const StagedSlice<G>& s, const StagedPhase& P, int lane, float4 q) {
     if (P.out) {
-        if (s.valid && lane < 32 / kLanesC) P.gout[s.row] = q;
+        if (s.valid && lane < 32 / G) P.gout[s.row] = q;
         return;
     }
-    if (s.d0) cluster_st(s.d0, q);
-    if (s.d1) cluster_st(s.d1, q);
+#pragma unroll
+    for (int j = 0; j < kMaxCluster / G; ++j)
+        if (s.d[j]) cluster_st(s.d[j], q);
 }
 
 // The slice's rows from their sum, for the phases that restrict.
-__device__ __forceinline__ void staged_restricted(const StagedSlice& s, const StagedPhase& P, unsigned char* smb, int lane,
+__device__ __forceinline__ void staged_restricted(const StagedSlice<kLanesC>& s, const StagedPhase& P, unsigned char* smb, int lane,
                                                   float4 r) {
     if (P.kind == kStRestrict) {
         if (s.valid && lane < 32 / kLanesC) reinterpret_cast<float4*>(smb + P.rhs)[s.li] = r;
@@ -1228,9 +1258,68 @@ __device__ __forceinline__ void staged_restricted(const StagedSlice& s, const St
     staged_store(s, P, lane, r);
 }
 
+template <int G>
+__device__ __forceinline__ void staged_sweep(StagedSlice<G>& s, const StagedPhase& P, unsigned char* smb, int lane, int warp,
+                                             int nwarp, const uint32_t (&peer)[kMaxCluster / G]) {
+    const int kind = P.kind;
+    for (int g = warp; g < P.many; g += nwarp) {
+        if (g != warp) staged_load(s, P, smb, g, lane, peer);
+        const float4 x = reinterpret_cast<const float4*>(smb + P.self)[s.valid ? s.row - P.lo : 0];
+        const float4 b = reinterpret_cast<const float4*>(smb + P.rhs)[s.li];
+        const float D = reinterpret_cast<const float*>(smb + P.dd)[s.li];
+        const float w = reinterpret_cast<const float*>(smb + P.dd)[P.re - P.rb + s.li];
+        const float4 a = staged_sum(s, P, smb, lane);
+        const float rx = b.x - fmaf(D, x.x, a.x), ry = b.y - fmaf(D, x.y, a.y), rz = b.z - fmaf(D, x.z, a.z);
+        staged_store(s, P, lane, kind == kStResidual
+                                     ? make_float4(rx, ry, rz, 0.f)
+                                     : make_float4(fmaf(w, rx, x.x), fmaf(w, ry, x.y), fmaf(w, rz, x.z), 0.f));
+    }
+}
+
+template <int G>
+__device__ __forceinline__ void staged_prolong(StagedSlice<G>& s, const StagedPhase& P, unsigned char* smb, int lane, int warp,
+                                               int nwarp, const uint32_t (&peer)[kMaxCluster / G]) {
+    const int kind = P.kind;
+    for (int g = warp; g < P.many; g += nwarp) {
+        if (g != warp) staged_load(s, P, smb, g, lane, peer);
+        const float4* ec = reinterpret_cast<const float4*>(smb + P.src);
+        const int4 id = reinterpret_cast<const int4*>(smb + P.par)[2 * s.li];
+        const float4 pw = reinterpret_cast<const float4*>(smb + P.par)[2 * s.li + 1];
+        const float4 c0 = ec[id.x], c1 = ec[id.y], c2 = ec[id.z], c3 = ec[id.w];
+        const float4 pe = make_float4(pw.x * c0.x + pw.y * c1.x + pw.z * c2.x + pw.w * c3.x,
+                                      pw.x * c0.y + pw.y * c1.y + pw.z * c2.y + pw.w * c3.y,
+                                      pw.x * c0.z + pw.y * c1.z + pw.z * c2.z + pw.w * c3.z, 0.f);
+        float4 x = reinterpret_cast<const float4*>(smb + P.self)[s.valid ? s.row - P.lo : 0];
+        if (kind == kStProlongSweep) {
+            // A (x + pe) = A x + D pe + OP e: the sweep from the residual at x
+            const float4 b = reinterpret_cast<const float4*>(smb + P.rhs)[s.valid ? s.row - P.rhs0 : 0];
+            const float D = reinterpret_cast<const float*>(smb + P.dd)[s.li];
+            const float w = reinterpret_cast<const float*>(smb + P.dd)[P.re - P.rb + s.li];
+            const float4 a = staged_sum(s, P, smb, lane);
+            const float rx = b.x - fmaf(D, pe.x, a.x), ry = b.y - fmaf(D, pe.y, a.y), rz = b.z - fmaf(D, pe.z, a.z);
+            x.x += pe.x;
+            x.y += pe.y;
+            x.z += pe.z;
+            x = make_float4(fmaf(w, rx, x.x), fmaf(w, ry, x.y), fmaf(w, rz, x.z), 0.f);
+        } else {
+            __syncwarp();   // in place: every lane of the row has read it
+            x.x += pe.x;
+            x.y += pe.y;
+            x.z += pe.z;
+        }
+        staged_store(s, P, lane, x);
+    }
+}
+
+// kTop: level 0 too, its phases (8 rows to a slice, 4 lanes per row, as its own kernels) Q.pre0 before and Q.post0 after
+// the coarse levels': x over the window and the right-hand side are fetched behind the launch, and the result goes back
+// into x, which every CTA has read by then.  1,025 vertices, 3 levels, 2+2 sweeps: 15.1 us per V-cycle, 19.6 us with
+// level 0 in five launches and 28 us before the coarse levels' operators lay in shared memory.
+template <bool kTop>
 __global__ void __launch_bounds__(kStagedThreads, 1) k_coarse_vcycle_staged(const StagedPlan Q, const float* __restrict__ Ainv,
                                                                          const double* __restrict__ Ainv64,
-                                                                         const int32_t* __restrict__ dense_off) {
+                                                                         const int32_t* __restrict__ dense_off,
+                                                                         int32_t* __restrict__ nonfinite) {
     pdl_trigger();
     extern __shared__ __align__(128) unsigned char smb[];
     __shared__ __align__(8) uint64_t bar;
@@ -1248,22 +1337,54 @@ __global__ void __launch_bounds__(kStagedThreads, 1) k_coarse_vcycle_staged(cons
     }
     __syncthreads();
     cluster_arrive();   // matched below: every CTA of the cluster runs before it is written to
-    // this lane's two CTAs (of up to 16; a CTA beyond the cluster has an empty window): their shared memory
     const uint32_t base = smem_u32(smb);
-    const uint32_t peer0 = cluster_addr(base, sub < cs ? sub : rank),
-                   peer1 = cluster_addr(base, sub + kLanesC < cs ? sub + kLanesC : rank);
+    uint32_t peer[kMaxCluster / kLanesC];
+    staged_peers<kLanesC>(peer, base, lane, cs, rank);
     const int dense0 = __ldg(dense_off + blockIdx.x / cs);
-    // the image; when it does not arrive the CTA takes part in the barriers only, and the frame ends non-finite
+    // the image; when it does not arrive the CTA takes part in the barriers only, and the frame ends marked non-finite
     const bool ok = mbar_wait(&bar, 0, kMaxPolls);
     const StagedHead& head = *reinterpret_cast<const StagedHead*>(smb);
     const int nc = head.coarse_n;
     auto phase = [&](int p) -> const StagedPhase& {
         return *reinterpret_cast<const StagedPhase*>(smb + Q.phase_at + p * sizeof(StagedPhase));
     };
-    StagedSlice s;
+    StagedSlice<kLanesC> s;
+    StagedSlice<kLanesL0> s0;
+    uint32_t peer_l0[kMaxCluster / kLanesL0];
     float4 sum = f4z();
     const bool busy = ok && warp < phase(0).many;
-    if (busy) staged_load(s, phase(0), smb, warp, lane, peer0, peer1);
+    // the level-0 phases p .. end - 1, then the first slice of the coarse phase that follows them
+    auto level0 = [&](int p, int end) {
+        for (; p < end; ++p) {
+            const StagedPhase& P = phase(p);
+            if (ok && (P.kind == kStSweep || P.kind == kStResidual))
+                staged_sweep<kLanesL0>(s0, P, smb, lane, warp, nwarp, peer_l0);
+            else if (ok)
+                staged_prolong<kLanesL0>(s0, P, smb, lane, warp, nwarp, peer_l0);
+            if (p + 1 == Q.phases) return;
+            cluster_arrive();
+            if (ok && warp < phase(p + 1).many) {
+                if (p + 1 < end)
+                    staged_load(s0, phase(p + 1), smb, warp, lane, peer_l0);
+                else
+                    staged_load(s, phase(p + 1), smb, warp, lane, peer);
+            }
+            cluster_wait();
+        }
+    };
+    if (kTop) staged_peers<kLanesL0>(peer_l0, base, lane, cs, rank);
+    if (busy) {
+        if (kTop)
+            staged_load(s0, phase(0), smb, warp, lane, peer_l0);
+        else
+            staged_load(s, phase(0), smb, warp, lane, peer);
+    }
+    int slot0 = 0, slot1 = 0;   // this warp's first slice of slots
+    if (kTop && busy && Q.gather) {
+        const int slice = phase(0).first / (32 / kLanesL0) + warp;
+        slot0 = __ldg(Q.slot_ptr + slice);
+        slot1 = __ldg(Q.slot_ptr + slice + 1);
+    }
     pdl_wait();
     if (ok) {   // this frame's data: diagonals, and the inverse's rows behind the first phases
         for (int i = 0; i < head.loads; ++i) {
@@ -1273,6 +1394,13 @@ __global__ void __launch_bounds__(kStagedThreads, 1) k_coarse_vcycle_staged(cons
                 cp_async4(base + d.dd + 4 * (d.count + r), d.dinv + d.rb + r);
             }
         }
+        if (kTop) {   // x over the window, the right-hand side of the own rows
+            const StagedPhase& P = phase(0);
+            const int2 w = reinterpret_cast<const int2*>(smb + P.win)[rank];
+            for (int r = threadIdx.x; r < w.y; r += blockDim.x) cp_async16(base + P.self + 16 * r, Q.x + w.x + r);
+            if (!Q.gather)
+                for (int r = P.rb + threadIdx.x; r < P.re; r += blockDim.x) cp_async16(base + P.rhs + 16 * (r - P.rb), Q.b + r);
+        }
         asm volatile("cp.async.commit_group;" ::: "memory");
         const size_t first = (size_t)(head.coarse_rb - head.coarse_off) * nc + dense0;
         const int many = (head.coarse_re - head.coarse_rb) * nc;
@@ -1281,63 +1409,43 @@ __global__ void __launch_bounds__(kStagedThreads, 1) k_coarse_vcycle_staged(cons
         else
             for (int i = threadIdx.x; i < many; i += blockDim.x) cp_async4(base + Q.ainv + 4 * i, Ainv + first + i);
         asm volatile("cp.async.commit_group;" ::: "memory");
-        if (busy) sum = staged_sum(s, phase(0), smb, lane);   // the first phase's rows, while the diagonals arrive
+        if (!kTop) {
+            if (busy) sum = staged_sum(s, phase(0), smb, lane);   // the first phase's rows, while the diagonals arrive
+        } else if (Q.gather) {
+            const StagedPhase& P = phase(0);
+            constexpr int S0 = 32 / kLanesL0;
+            for (int g = warp; g < P.many; g += nwarp) {
+                const int slice = P.first / S0 + g, row = slice * S0 + lane % S0;
+                const bool valid = row < P.re;   // a body's first row starts a slice: one body
+                const float4 bb = valid ? __ldg(Q.b0 + row) : f4z();
+                const bool first = g == warp;
+                const float4 sl = rg_slot_sum<kLanesL0>(lane, first ? slot0 : __ldg(Q.slot_ptr + slice),
+                                                        first ? slot1 : __ldg(Q.slot_ptr + slice + 1), Q.slots);
+                if (!valid || lane >= S0) continue;
+                const float4 bi = make_float4(bb.x + sl.x, bb.y + sl.y, bb.z + sl.z, 0.f);
+                reinterpret_cast<float4*>(smb + P.rhs)[row - P.rb] = bi;
+                Q.b[row] = bi;
+            }
+        }
         asm volatile("cp.async.wait_group 1;" ::: "memory");
     }
     cluster_wait();
     __syncthreads();   // the diagonals of this CTA
-    for (int p = 0; p < Q.phases; ++p) {
+    if (kTop) level0(0, Q.pre0);
+    const int stop = kTop ? Q.phases - Q.post0 : Q.phases;
+    for (int p = kTop ? Q.pre0 : 0; p < stop; ++p) {
         const StagedPhase& P = phase(p);
         const int kind = ok ? P.kind : -1;
         if (kind == kStRestrict || kind == kStWhole) {
             for (int g = warp; g < P.many; g += nwarp) {
-                if (g != warp) staged_load(s, P, smb, g, lane, peer0, peer1);
-                staged_restricted(s, P, smb, lane, p == 0 && g == warp ? sum : staged_sum(s, P, smb, lane));
+                if (g != warp) staged_load(s, P, smb, g, lane, peer);
+                staged_restricted(s, P, smb, lane, !kTop && p == 0 && g == warp ? sum : staged_sum(s, P, smb, lane));
             }
             if (kind == kStWhole) asm volatile("cp.async.wait_all;" ::: "memory");
         } else if (kind == kStSweep || kind == kStResidual) {
-            for (int g = warp; g < P.many; g += nwarp) {
-                if (g != warp) staged_load(s, P, smb, g, lane, peer0, peer1);
-                const float4 x = reinterpret_cast<const float4*>(smb + P.self)[s.valid ? s.row - P.lo : 0];
-                const float4 b = reinterpret_cast<const float4*>(smb + P.rhs)[s.li];
-                const float D = reinterpret_cast<const float*>(smb + P.dd)[s.li];
-                const float w = reinterpret_cast<const float*>(smb + P.dd)[P.re - P.rb + s.li];
-                const float4 a = staged_sum(s, P, smb, lane);
-                const float rx = b.x - fmaf(D, x.x, a.x), ry = b.y - fmaf(D, x.y, a.y), rz = b.z - fmaf(D, x.z, a.z);
-                staged_store(s, P, lane, kind == kStResidual
-                                             ? make_float4(rx, ry, rz, 0.f)
-                                             : make_float4(fmaf(w, rx, x.x), fmaf(w, ry, x.y), fmaf(w, rz, x.z), 0.f));
-            }
+            staged_sweep<kLanesC>(s, P, smb, lane, warp, nwarp, peer);
         } else if (kind == kStProlongSweep || kind == kStProlong) {
-            for (int g = warp; g < P.many; g += nwarp) {
-                if (g != warp) staged_load(s, P, smb, g, lane, peer0, peer1);
-                const float4* ec = reinterpret_cast<const float4*>(smb + P.src);
-                const int4 id = reinterpret_cast<const int4*>(smb + P.par)[2 * s.li];
-                const float4 pw = reinterpret_cast<const float4*>(smb + P.par)[2 * s.li + 1];
-                const float4 c0 = ec[id.x], c1 = ec[id.y], c2 = ec[id.z], c3 = ec[id.w];
-                const float4 pe = make_float4(pw.x * c0.x + pw.y * c1.x + pw.z * c2.x + pw.w * c3.x,
-                                              pw.x * c0.y + pw.y * c1.y + pw.z * c2.y + pw.w * c3.y,
-                                              pw.x * c0.z + pw.y * c1.z + pw.z * c2.z + pw.w * c3.z, 0.f);
-                float4 x = reinterpret_cast<const float4*>(smb + P.self)[s.valid ? s.row - P.lo : 0];
-                if (kind == kStProlongSweep) {
-                    // A (x + pe) = A x + D pe + OP e: the sweep from the residual at x
-                    const float4 b = reinterpret_cast<const float4*>(smb + P.rhs)[s.valid ? s.row - P.rhs0 : 0];
-                    const float D = reinterpret_cast<const float*>(smb + P.dd)[s.li];
-                    const float w = reinterpret_cast<const float*>(smb + P.dd)[P.re - P.rb + s.li];
-                    const float4 a = staged_sum(s, P, smb, lane);
-                    const float rx = b.x - fmaf(D, pe.x, a.x), ry = b.y - fmaf(D, pe.y, a.y), rz = b.z - fmaf(D, pe.z, a.z);
-                    x.x += pe.x;
-                    x.y += pe.y;
-                    x.z += pe.z;
-                    x = make_float4(fmaf(w, rx, x.x), fmaf(w, ry, x.y), fmaf(w, rz, x.z), 0.f);
-                } else {
-                    __syncwarp();   // in place: every lane of the row has read it
-                    x.x += pe.x;
-                    x.y += pe.y;
-                    x.z += pe.z;
-                }
-                staged_store(s, P, lane, x);
-            }
+            staged_prolong<kLanesC>(s, P, smb, lane, warp, nwarp, peer);
         } else if (kind == kStDense) {
             // coarsest: e = A^-1 r for the own rows, to every CTA (or out, when it is the only level)
             for (int i = warp; i < P.re - P.rb; i += nwarp) {
@@ -1350,19 +1458,29 @@ __global__ void __launch_bounds__(kStagedThreads, 1) k_coarse_vcycle_staged(cons
                     if (lane == 0) P.gout[row] = e;
                 } else if (lane % S == 0) {
                     const int to = P.dst + 16 * (row - head.coarse_off);
-                    if (sub < cs) cluster_st(peer0 + to, e);
-                    if (sub + kLanesC < cs) cluster_st(peer1 + to, e);
+#pragma unroll
+                    for (int j = 0; j < kMaxCluster / kLanesC; ++j)
+                        if (sub + j * kLanesC < cs) cluster_st(peer[j] + to, e);
                 }
             }
         }
         if (p + 1 == Q.phases) break;
         cluster_arrive();
         // the next phase's operator, behind the barrier
-        if (ok && warp < phase(p + 1).many) staged_load(s, phase(p + 1), smb, warp, lane, peer0, peer1);
+        if (ok && warp < phase(p + 1).many) {
+            if (kTop && p + 1 == stop)
+                staged_load(s0, phase(p + 1), smb, warp, lane, peer_l0);
+            else
+                staged_load(s, phase(p + 1), smb, warp, lane, peer);
+        }
         cluster_wait();
     }
+    if (kTop) level0(stop, Q.phases);
     // no remote store follows the last barrier; a copy that never arrived is waited for again before the CTA ends
-    if (!ok) mbar_wait(&bar, 0, kMaxPolls);
+    if (!ok) {
+        if (threadIdx.x == 0) atomicOr(nonfinite, 1);
+        mbar_wait(&bar, 0, kMaxPolls);
+    }
 }
 
 // ---------------------------------------------------------------------------

@@ -341,6 +341,11 @@ size_t coarse_smem_bytes(const mgsb_solver* h, int cs, int split);
 // Largest body's rows on a coarse level below which it stays in the cluster
 // kernel by default; larger levels run as grid-wide kernels over all SMs.
 constexpr int kClusterLevelRows = 1024;
+// A body of at most this many vertices has level 0 in the cluster kernel too: 5 phases of about 1 us in place of 5
+// launches, until a CTA's share of the rows makes its phases longer than a launch over all SMs.  Frames of FP32 beams,
+// with it and with level 0 grid-wide: 126 and 162 us at 176 vertices, 187 and 226 at 525, 199 and 232 at 1,025, 234 and
+// 261 at 1,836, 311 and 300 at 2,254, 320 and 310 at 2,989; mixed, two passes: 447 and 507 at 1,836, 584 and 589 at 2,254.
+constexpr int kClusterL0Rows = 2000;
 
 // The dense coarse operator can start at level `split`: one body, at most
 // dop_cap rows there, and the apply kernel's shared memory (the split level's
@@ -665,11 +670,17 @@ mgsb_status rebuild(mgsb_solver* h) {
         h->range_host = P.range;
         if (L > kMaxLevels) return set_err(h, MGSB_NOT_SUPPORTED, "at most %d levels", kMaxLevels);
         h->coarse_host.assign(L, LevelHost{});
-        for (int l = 1; l < L; ++l) {   // the plan's arrays are not needed after their upload
+        // the plan's arrays are not needed after their upload (level 0's only where the cluster kernel can take it)
+        for (int l = h->bodies.size() == 1 && P.levels[0].n <= kClusterL0Rows ? 0 : 1; l < L; ++l) {
             PlanLevel& pl = P.levels[l];
             LevelHost& H = h->coarse_host[l];
-            H.slice_ptr = std::move(pl.slice_ptr);
-            H.ell_col = std::move(pl.ell_col);
+            if (l == 0) {   // read again below
+                H.slice_ptr = pl.slice_ptr;
+                H.ell_col = pl.ell_col;
+            } else {
+                H.slice_ptr = std::move(pl.slice_ptr);
+                H.ell_col = std::move(pl.ell_col);
+            }
             H.ell_val = std::move(pl.ell_val);
             H.rptr = std::move(pl.rptr);
             H.rcol = std::move(pl.rcol);
@@ -687,9 +698,11 @@ mgsb_status rebuild(mgsb_solver* h) {
                                          h->max_smem_optin));
         CUDA_TRY(h, cudaFuncSetAttribute(k_coarse_vcycle_cta, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          h->max_smem_optin));
-        CUDA_TRY(h, cudaFuncSetAttribute(k_coarse_vcycle_staged, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-        CUDA_TRY(h, cudaFuncSetAttribute(k_coarse_vcycle_staged, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         h->max_smem_optin - kStagedStaticSmem));
+        for (auto k : {k_coarse_vcycle_staged<false>, k_coarse_vcycle_staged<true>}) {
+            CUDA_TRY(h, cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+            CUDA_TRY(h, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             h->max_smem_optin - kStagedStaticSmem));
+        }
         CUDA_TRY(h, cudaFuncSetAttribute(k_coarse_apply, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          h->max_smem_optin));
         TRY(dupload(h, pool, &h->dense_off_d, P.dense_off));
@@ -900,8 +913,11 @@ size_t coarse_smem_bytes(const mgsb_solver* h, int cs, int split) {
 // CTA's image and vectors fit its shared memory; k_coarse_vcycle_dsm, which reads the operators from L2 in every
 // phase, runs the shapes that do not, numberings whose rows reach far among them.  Leaves h->staged.bytes 0 if it
 // does not fit or the device cannot schedule the cluster.
+bool coarse_shape_feasible(mgsb_solver* h, int cs, int block, int fused, int split);
+
 void plan_staged(mgsb_solver* h, int cs, int split) {
-    constexpr int S = kSliceCoarse, G = kLanesC;
+    auto slice = [](int l) { return l ? kSliceCoarse : 32 / kLanesL0; };   // rows
+    const bool top = split == 0;
     const int L = h->p.levels, lc = L - 1, nb = (int)h->bodies.size();
     struct Entries {
         std::vector<int> idx;
@@ -921,6 +937,7 @@ void plan_staged(mgsb_solver* h, int cs, int split) {
     for (int bi = 0; bi < nb; ++bi) {
         for (int l = split; l < L; ++l) {
             const int2 rg = h->range_host[(size_t)bi * L + l];
+            const int S = slice(l);
             const int g0 = rg.x / S, g1 = (rg.x + rg.y + S - 1) / S, per = (g1 - g0 + cs - 1) / cs;
             for (int k = 0; k < cs; ++k) {
                 Part& o = part(bi, k, l);
@@ -935,6 +952,7 @@ void plan_staged(mgsb_solver* h, int cs, int split) {
         }
         for (int l = split; l < L; ++l) {
             const LevelHost& H = h->coarse_host[l];
+            const int S = slice(l);
             for (int k = 0; k < cs; ++k) {
                 Part& o = part(bi, k, l);
                 int2 w{o.rb, o.re};
@@ -950,8 +968,9 @@ void plan_staged(mgsb_solver* h, int cs, int split) {
                     if (l > split) {
                         const LevelHost& U = h->coarse_host[l - 1];
                         const Part& u = part(bi, k, l - 1);
+                        const int T = slice(l - 1);
                         for (int i = u.rb; i < u.re; ++i) {
-                            for (int e = U.op_slice_ptr[i / S] + i % S; e < U.op_slice_ptr[i / S + 1]; e += S) add(U.op_col[e]);
+                            for (int e = U.op_slice_ptr[i / T] + i % T; e < U.op_slice_ptr[i / T + 1]; e += T) add(U.op_col[e]);
                             for (int c : {U.pid[i].x, U.pid[i].y, U.pid[i].z, U.pid[i].w}) add(c);
                         }
                     }
@@ -960,10 +979,11 @@ void plan_staged(mgsb_solver* h, int cs, int split) {
             }
         }
     }
-    // entries: slices of 4 rows, 8 lanes per row, 32 entries per step, at least one step per slice; a lane without an
+    // entries: slices of 4 (level 0: 8) rows, 8 (4) lanes per row, 32 entries per step, at least one step per slice; a lane without an
     // entry reads the vector's first row with coefficient 0
-    auto steps = [&](const Part& o, auto&& row_entries, std::vector<int32_t>& ptr, Entries& ent) {
-        std::vector<std::pair<int, float>> row[S];
+    auto steps = [&](const Part& o, int S, auto&& row_entries, std::vector<int32_t>& ptr, Entries& ent) {
+        const int G = 32 / S;
+        std::vector<std::pair<int, float>> row[8];
         ptr.assign(1, 0);
         for (int g = 0; g < o.slices; ++g) {
             int T = 1;
@@ -994,11 +1014,13 @@ void plan_staged(mgsb_solver* h, int cs, int split) {
             for (int l = split; l < L; ++l) {
                 Part& o = part(bi, k, l);
                 const LevelHost& H = h->coarse_host[l];
+                const int S = slice(l);
                 using Row = std::vector<std::pair<int, float>>;
-                steps(o, [&](int i, Row& out) {
-                    for (int e = H.rptr[i]; e < H.rptr[i + 1]; ++e)
-                        out.emplace_back(l == split ? H.rcol[e] : at(part(bi, k, l - 1), H.rcol[e]), H.rw[e]);
-                }, o.rp, o.re_);
+                if (l > 0)
+                    steps(o, S, [&](int i, Row& out) {
+                        for (int e = H.rptr[i]; e < H.rptr[i + 1]; ++e)
+                            out.emplace_back(l == split ? H.rcol[e] : at(part(bi, k, l - 1), H.rcol[e]), H.rw[e]);
+                    }, o.rp, o.re_);
                 Most& m = most[l];
                 m.rows = std::max(m.rows, (size_t)(o.re - o.rb));
                 m.slices = std::max(m.slices, (size_t)o.slices);
@@ -1009,14 +1031,15 @@ void plan_staged(mgsb_solver* h, int cs, int split) {
                     continue;
                 }
                 const Part& n = part(bi, k, l + 1);
-                // the padding (a zero on the row itself, on its first parent) is left out: the row reads both anyway
-                steps(o, [&](int i, Row& out) {
+                // the padding (a zero on the row itself, at the end on its first parent) is left out: the row reads both anyway
+                steps(o, S, [&](int i, Row& out) {
                     for (int e = H.slice_ptr[i / S] + i % S; e < H.slice_ptr[i / S + 1]; e += S)
                         if (H.ell_col[e] != i) out.emplace_back(at(o, H.ell_col[e]), H.ell_val[e]);
                 }, o.ep, o.ee);
-                steps(o, [&](int i, Row& out) {
+                steps(o, S, [&](int i, Row& out) {
                     for (int e = H.op_slice_ptr[i / S] + i % S; e < H.op_slice_ptr[i / S + 1]; e += S)
-                        if (H.op_val[e] != 0.f || H.op_col[e] != H.pid[i].x) out.emplace_back(at(n, H.op_col[e]), H.op_val[e]);
+                        out.emplace_back(at(n, H.op_col[e]), H.op_val[e]);
+                    while (!out.empty() && out.back() == std::make_pair(at(n, H.pid[i].x), 0.f)) out.pop_back();
                 }, o.op, o.oe);
                 for (int i = o.rb; i < o.re; ++i) {
                     const int4 id = H.pid[i];
@@ -1040,6 +1063,9 @@ void plan_staged(mgsb_solver* h, int cs, int split) {
         return (int)std::min<size_t>(a, 1u << 30);
     };
     const int pre = h->p.pre_sweeps, post = h->p.post_sweeps;
+    // level 0's sweeps before the coarse levels: the mixed kind's outer residual makes the first one
+    const bool mixed = h->p.precision == MGSB_PRECISION_MIXED;
+    const int pre_l0 = mixed ? std::max(pre, 1) - 1 : pre;
     const bool fused = h->fuse_prolong && post > 0;
     const int levels = lc - split;   // levels above the coarsest
     const int most_phases = levels * (1 + std::max(pre, 1) + 1 + post) + 2;
@@ -1074,7 +1100,7 @@ void plan_staged(mgsb_solver* h, int cs, int split) {
         s.res = room(16 * m.W);
         s.dd = room(8 * m.rows);
     }
-    q.ainv = room(ainv * (h->p.precision == MGSB_PRECISION_MIXED ? 8 : 4));
+    q.ainv = room(ainv * (mixed ? 8 : 4));
     if (bytes > (size_t)(h->max_smem_optin - kStagedStaticSmem)) return;
     q.image_bytes = (int)image;
     q.phase_at = phase_at;
@@ -1095,7 +1121,8 @@ void plan_staged(mgsb_solver* h, int cs, int split) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int nclusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&nclusters, k_coarse_vcycle_staged, &cfg) != cudaSuccess) {
+    const auto kernel = top ? k_coarse_vcycle_staged<true> : k_coarse_vcycle_staged<false>;
+    if (cudaOccupancyMaxActiveClusters(&nclusters, kernel, &cfg) != cudaSuccess) {
         cudaGetLastError();
         return;
     }
@@ -1151,17 +1178,20 @@ void plan_staged(mgsb_solver* h, int cs, int split) {
                     const int2 w = part(bi, j, l).win, window{w.x, w.y - w.x};
                     std::memcpy(img + lay[l].win + j * sizeof(int2), &window, sizeof window);
                 }
-                put(lay[l].rp, o.rp);
-                put_entries(lay[l].ri, lay[l].rv, o.re_, l == split);
-                StagedPhase& R = phase(l, l == lc ? kStWhole : kStRestrict);
-                R.ptr = lay[l].rp;
-                R.idx = lay[l].ri;
-                R.val = lay[l].rv;
-                R.src = l == split ? -1 : lay[l - 1].res;
-                R.gsrc = l == split ? h->lev[l - 1].res : nullptr;
-                R.rhs = lay[l].r;
-                R.dst = l == lc ? lay[l].r : lay[l].e;
                 cur[l] = lay[l].e;
+                if (l > 0) {
+                    put(lay[l].rp, o.rp);
+                    put_entries(lay[l].ri, lay[l].rv, o.re_, l == split);
+                    StagedPhase& R = phase(l, l == lc ? kStWhole : kStRestrict);
+                    R.ptr = lay[l].rp;
+                    R.idx = lay[l].ri;
+                    R.val = lay[l].rv;
+                    R.src = l == split ? -1 : lay[l - 1].res;
+                    R.gsrc = l == split ? h->lev[l - 1].res : nullptr;
+                    R.rhs = lay[l].r;
+                    R.dst = l == lc ? lay[l].r : lay[l].e;
+                    R.zero = pre == 0;
+                }
                 if (l == lc) break;
                 put(lay[l].ep, o.ep);
                 put_entries(lay[l].ei, lay[l].ev, o.ee, false);
@@ -1172,12 +1202,12 @@ void plan_staged(mgsb_solver* h, int cs, int split) {
                     std::memcpy(img + lay[l].par + 32 * r + 16, &o.pw[r], 16);
                 }
                 loads.push_back(StagedLoad{o.rb, o.re - o.rb, lay[l].dd, 0, h->lev[l].dfull, h->lev[l].dinv});
-                R.zero = pre == 0;
-                for (int j = 1; j < pre; ++j) {
+                for (int j = l ? 1 : 0; j < (l ? pre : pre_l0); ++j) {
                     sweep(l, cur[l], other(l, cur[l]), kStSweep);
                     cur[l] = other(l, cur[l]);
                 }
                 sweep(l, cur[l], lay[l].res, kStResidual);
+                if (l == 0) q.pre0 = (int)ph.size();
             }
             {
                 StagedPhase& P = phase(lc, kStDense);
@@ -1186,6 +1216,7 @@ void plan_staged(mgsb_solver* h, int cs, int split) {
                 P.dst = lay[lc].e;
             }
             for (int l = lc - 1; l >= split; --l) {
+                if (l == 0) q.post0 = -(int)ph.size();
                 StagedPhase& P = phase(l, fused ? kStProlongSweep : kStProlong);
                 P.ptr = lay[l].op;
                 P.idx = lay[l].oi;
@@ -1201,15 +1232,40 @@ void plan_staged(mgsb_solver* h, int cs, int split) {
                 }
             }
             ph.back().out = 1;
-            ph.back().gout = h->lev[split].e;
+            ph.back().gout = top ? h->d : h->lev[split].e;
             const Part& c = part(bi, k, lc);
             const StagedHead head{(int)loads.size(), load_at, c.off, c.n, c.rb, c.re, {0, 0}};
             q.phases = (int)ph.size();
+            if (top) q.post0 += q.phases;
             std::memcpy(img, &head, sizeof head);
             put(phase_at, ph);
             put(load_at, loads);
         }
+    if (top) {
+        q.x = h->d;
+        q.b = mixed ? h->r32 : h->b;
+        q.b0 = h->b0;
+        q.slots = h->slots;
+        q.slot_ptr = h->slot_ptr;
+    }
     h->staged = q;
+}
+
+// The whole V-cycle in the cluster kernel, for a small body whose kernel shape is the solver's own choice, over as many
+// CTAs as have 16 rows of level 0 (1,025 vertices: 199 us per frame over 16, 254 over 8, 324 over 4).  Without
+// pre-smoothing the FP32 kind's right-hand side is summed by its own kernel, in another order.
+void plan_top(mgsb_solver* h) {
+    if (h->p.precision != MGSB_PRECISION_MIXED && h->p.pre_sweeps == 0) return;
+    if (h->tune_fuse >= 0 || h->tune_split > 0 || h->split != 1 || h->ls_net || h->coarse_host[0].slice_ptr.empty()) return;
+    for (int cs : {16, 8, 4, 2}) {
+        if (cs > 2 && cs * 16 > h->maxv[0]) continue;
+        // mgsb_vcycle_residuals and mgsb_smoother_pairs run the coarse levels alone
+        if (!coarse_shape_feasible(h, cs, h->coarse_block, 0, 1)) continue;
+        plan_staged(h, cs, 0);
+        if (!h->staged.bytes) continue;
+        h->cluster = cs;
+        return;
+    }
 }
 
 // The staged kernel's plan and images for the current shape, if they are not there yet; the copy goes on the stream:
@@ -1226,8 +1282,10 @@ mgsb_status ready_staged(mgsb_solver* h) {
         if (h->tune_cluster > 1) {
             plan_staged(h, h->cluster, h->split);
         } else if (h->tune_cluster == 0) {
+            plan_top(h);
             const int most = std::min(kMaxCluster, (h->maxv[h->split] + 15) / 16);
             for (int cs : {16, 8, 4, 2}) {
+                if (h->staged.bytes) break;
                 if (cs > most && cs > 2) continue;
                 plan_staged(h, cs, h->split);
                 if (!h->staged.bytes) continue;
@@ -1294,7 +1352,7 @@ bool coarse_shape_feasible(mgsb_solver* h, int cs, int block, int fused, int spl
     return nclusters > 0;
 }
 
-mgsb_status launch_coarse_cluster(mgsb_solver* h, const CoarseArgs& args);
+mgsb_status launch_coarse_cluster(mgsb_solver* h, const CoarseArgs& args, bool top = false, bool gather = false);
 
 // Coarse part of one V-cycle: from the level-0 residual lv[0].res to the
 // level-1 correction lv[1].e.  Levels 1..split-1 run as grid-wide kernels
@@ -1385,13 +1443,13 @@ mgsb_status launch_coarse(mgsb_solver* h, const CoarseArgs& args_in) {
     return MGSB_OK;
 }
 
-mgsb_status launch_coarse_cluster(mgsb_solver* h, const CoarseArgs& args) {
+// top: the whole V-cycle from the right-hand side and displacement of level 0 (gather: the former from the slots).
+mgsb_status launch_coarse_cluster(mgsb_solver* h, const CoarseArgs& args, bool top, bool gather) {
+    const bool staged = h->staged.bytes && top == (h->staged.pre0 > 0);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(h->bodies.size() * h->cluster));
-    cfg.blockDim = dim3((unsigned)(h->staged.bytes ? h->staged.block : h->coarse_block));
-    cfg.dynamicSmemBytes = h->fuse_l0       ? 0
-                           : h->staged.bytes ? (size_t)h->staged.bytes
-                                             : coarse_smem_bytes(h, h->cluster, args.first);
+    cfg.blockDim = dim3((unsigned)(staged ? h->staged.block : h->coarse_block));
+    cfg.dynamicSmemBytes = h->fuse_l0 ? 0 : staged ? (size_t)h->staged.bytes : coarse_smem_bytes(h, h->cluster, args.first);
     if (cfg.dynamicSmemBytes > (size_t)h->max_smem_optin) {
         h->enqueue_status = set_err(h, MGSB_NOT_SUPPORTED,
                                     "coarse kernel shape (cluster %d, split %d) needs %zu B of shared memory per CTA (max %d)",
@@ -1416,14 +1474,18 @@ mgsb_status launch_coarse_cluster(mgsb_solver* h, const CoarseArgs& args) {
     // fused: global-memory kernel that also owns the level-0 residual and prolongation;
     // one CTA: every owned level in one CTA's shared memory; else the
     // distributed-shared-memory kernels over the cluster, with the operators staged where they fit
-    const int reps = prof_begin(h, "k_coarse_vcycle");
+    StagedPlan plan = h->staged;
+    plan.gather = gather ? 1 : 0;
+    const char* name = top ? "k_vcycle" : "k_coarse_vcycle";
+    const int reps = prof_begin(h, name);
     cudaError_t e = cudaSuccess;
     for (int r = 0; r < reps && e == cudaSuccess; ++r)
         e = h->fuse_l0 ? cudaLaunchKernelEx(&cfg, k_coarse_vcycle, args)
-            : one_cta         ? cudaLaunchKernelEx(&cfg, k_coarse_vcycle_cta, args)
-            : h->staged.bytes ? cudaLaunchKernelEx(&cfg, k_coarse_vcycle_staged, h->staged, args.Ainv, args.Ainv64, args.dense_off)
-                              : cudaLaunchKernelEx(&cfg, k_coarse_vcycle_dsm, args);
-    prof_end(h, "k_coarse_vcycle");
+            : one_cta  ? cudaLaunchKernelEx(&cfg, k_coarse_vcycle_cta, args)
+            : staged   ? cudaLaunchKernelEx(&cfg, top ? k_coarse_vcycle_staged<true> : k_coarse_vcycle_staged<false>, plan,
+                                            args.Ainv, args.Ainv64, args.dense_off, h->nonfinite)
+                       : cudaLaunchKernelEx(&cfg, k_coarse_vcycle_dsm, args);
+    prof_end(h, name);
     ++h->launches;
     if (e != cudaSuccess) {
         h->enqueue_status = set_err(h, MGSB_CUDA_ERROR, "coarse V-cycle launch failed: %s", cudaGetErrorString(e));
@@ -1819,6 +1881,10 @@ float4* enqueue_mg_solve(mgsb_solver* h, bool learned, const LearnedFallback& fb
             continue;
         }
         for (int pass = 0; pass < p.refinement_passes; ++pass) {
+            if (h->staged.pre0 > 0) {
+                launch_coarse_cluster(h, ca, true, pass == 0);
+                continue;
+            }
             bool gathered = pass > 0;
             for (int k = 0; k < l0_pre; ++k) {
                 LAUNCH(h, k_l0_sweep_rg, g0, kBlock, 0, n0, lv[0].slice_ptr, lv[0].ell_col, lv[0].ell_val, lv[0].dfull,
@@ -1933,6 +1999,11 @@ void enqueue_mixed_solve(mgsb_solver* h, bool learned, const LearnedFallback& fb
                 enqueue_learned_vcycle(h, ea, h->r32, true, ca, c, false, true, last ? nullptr : h->dd64,
                                        last ? nullptr : h->d32);
                 if (last) enqueue_learned_guard(h, ea, h->r32, c, true, fb, h->dd64, h->d32);
+                continue;
+            }
+            if (h->staged.pre0 > 0) {
+                launch_coarse_cluster(h, ca, true, false);
+                LAUNCH(h, k_mx_update, grid_for(n0), kBlock, 0, n0, ea, h->dd64, h->d32);
                 continue;
             }
             for (int k = 1; k < l0_pre; ++k) {
@@ -2953,6 +3024,8 @@ mgsb_status mgsb_autotune(mgsb_solver* h, int32_t frames, int32_t* chosen) {
     if (nb == 1)
         for (int sp = 1; sp < L; ++sp)
             if (dense_eligible(h, sp)) cands.push_back({1, 256, 0, sp, 1});
+    // the solver's own choice, where it takes the whole V-cycle into the cluster kernel
+    if (h->staged.pre0 > 0) cands.push_back({0, 512, -1, 0, 0});
     float best = 1e30f;
     Cand bestc = {h->cluster, h->coarse_block, h->fuse_l0, h->split, h->dense_op ? 1 : 0};
     cudaEvent_t a, b;
@@ -3003,7 +3076,7 @@ mgsb_status mgsb_autotune(mgsb_solver* h, int32_t frames, int32_t* chosen) {
     h->coarse_block = bestc.block;
     apply_tuning(h);
     invalidate_graph(h);
-    const mgsb_status st2 = MGSB_OK;
+    const mgsb_status st2 = ready_staged(h);
     cudaMemsetAsync(h->fac_valid, 0, h->bodies.size() * sizeof(int32_t), h->stream);
     restore();
     cudaStreamSynchronize(h->stream);
@@ -3014,9 +3087,9 @@ mgsb_status mgsb_autotune(mgsb_solver* h, int32_t frames, int32_t* chosen) {
     if (st != MGSB_OK) return st;
     if (st2 != MGSB_OK) return st2;
     if (chosen) {
-        chosen[0] = bestc.cluster;
+        chosen[0] = h->cluster;
         chosen[1] = bestc.block;
-        chosen[2] = bestc.fuse;
+        chosen[2] = h->fuse_l0;
     }
     return MGSB_OK;
 }
