@@ -197,9 +197,9 @@ constexpr int kLsPerThread = 8;    // ELL entries a thread loads ahead (2 thread
 // Dynamic shared memory of k_ls_sweep_tc: the MLP's operands and barriers, then
 // the residual window; at least 80 KiB (two CTAs per SM at most, so that
 // tcgen05.alloc never waits).
-inline size_t ls_sweep_smem_bytes() {
-    const size_t b = ((sizeof(MlpSmem) + 127) / 128) * 128 + (size_t)kLsWinRows * sizeof(float4);
-    return b > 80 * 1024 ? b : (size_t)80 * 1024;
+inline size_t ls_sweep_smem_bytes(int win_rows) {
+    const size_t b = ((sizeof(MlpSmem) + 127) / 128) * 128 + (size_t)win_rows * sizeof(float4);
+    return b > kMlpMinSmem ? b : kMlpMinSmem;
 }
 
 // One learned sweep in a single kernel: per 128-row tile, each thread forms its

@@ -170,7 +170,7 @@ __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.
 // Inference: one CTA per 128-row tile, grid-strided over tiles.
 // ---------------------------------------------------------------------------
 constexpr int kMlpThreads = 256;   // 8 warps: warp w serves TMEM lanes 32 (w % 4).. and hidden columns 32 (w / 4)..
-constexpr int kTmemCols = 256;     // D1 cols [0,64), D2 [64,128), D3 [128,144)
+constexpr int kTmemCols = 128;     // D1 cols [0,64), D2 [64,128), D3 [0,16): D1 has been read by then
 constexpr int kMaxPolls = 1 << 22;
 
 struct MlpSmem {
@@ -182,9 +182,10 @@ struct MlpSmem {
     int stop;
 };
 
-// Dynamic shared memory of k_mlp_tc: at least 80 KiB, so that at most two CTAs
-// (2 x 256 TMEM columns) are resident per SM and tcgen05.alloc never waits.
-inline size_t mlp_tc_smem_bytes() { return sizeof(MlpSmem) > 80 * 1024 ? sizeof(MlpSmem) : (size_t)80 * 1024; }
+// Dynamic shared memory of the kernels with tensor-core tiles: at least 48 KiB, so that at most four CTAs (4 x 128 TMEM
+// columns) are resident per SM, of one kernel or of several, and tcgen05.alloc never waits.
+constexpr size_t kMlpMinSmem = 48 * 1024;
+inline size_t mlp_tc_smem_bytes() { return sizeof(MlpSmem) > kMlpMinSmem ? sizeof(MlpSmem) : kMlpMinSmem; }
 
 // Bounded waits of one thread; the first wait that ran out is remembered so
 // that it can be retried once before TMEM is released (no copy or MMA of the
@@ -202,7 +203,7 @@ __device__ __forceinline__ bool wait_bar(WaitState& ws, uint64_t* bar, uint32_t 
     return done;
 }
 
-// CTA prologue: barriers, TMEM (256 columns, warp 0) and the weight image.
+// CTA prologue: barriers, TMEM (128 columns, warp 0) and the weight image.
 // With wait_weights = false the copy is left in flight (the caller overlaps it
 // with other work and calls mlp_wait_weights before the first MMA).
 __device__ __forceinline__ uint32_t mlp_cta_setup(MlpSmem& S, const uint8_t* img, WaitState& ws, uint32_t& ph_load,
@@ -332,7 +333,7 @@ __device__ __forceinline__ bool mlp_tile_layers(MlpSmem& S, uint32_t tmem, uint3
     if (threadIdx.x == 0 && ok) {
 #pragma unroll
         for (int k = 0; k < kMlpHid / 16; ++k)
-            umma_bf16(tmem + 128, umma_desc(S.h + k * 256, 128, 1024), umma_desc(S.w + kImgW3 + k * 256, 128, 1024),
+            umma_bf16(tmem, umma_desc(S.h + k * 256, 128, 1024), umma_desc(S.w + kImgW3 + k * 256, 128, 1024),
                       id16, k > 0 ? 1u : 0u);
         umma_commit(&S.bar_mma);
     }
@@ -340,7 +341,7 @@ __device__ __forceinline__ bool mlp_tile_layers(MlpSmem& S, uint32_t tmem, uint3
     ph_mma ^= 1;
     tc_fence_after();
     float v[16];
-    tmem_ld16(tmem + lane_base + 128, v);   // every warp (the .sync.aligned load is warp-wide); warps 0-3 use it
+    tmem_ld16(tmem + lane_base, v);   // every warp (the .sync.aligned load is warp-wide); warps 0-3 use it
     tmem_wait_ld();
     tc_fence_before();
     y[0] = v[0] + bias[2 * kMlpHid];

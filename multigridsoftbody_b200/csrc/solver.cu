@@ -230,7 +230,7 @@ struct mgsb_solver {
     const mgsb_mlp* ls_net = nullptr;
     cudaStream_t aux_stream = nullptr;   // captures the bodies of conditional graph nodes
     float ls_gamma = 0.5f;
-    int ls_ntiles = 0, ls_nblk = 0, sm_count = 148;
+    int ls_win_rows = 0, ls_ntiles = 0, ls_nblk = 0, sm_count = 148;
     uint8_t* ls_tiles = nullptr;
     float* ls_scale = nullptr;
     float4 *ls_r = nullptr, *ls_save = nullptr, *ls_dpost = nullptr;
@@ -770,6 +770,7 @@ mgsb_status rebuild(mgsb_solver* h) {
     if (mg) {
         // learned-smoother level-0 buffers (used when a network is attached)
         h->ls_ntiles = (N0 + kMlpTile - 1) / kMlpTile;
+        h->ls_win_rows = 0;
         h->ls_nblk = grid_rows(N0, h->lev[0].S);
         TRY(dalloc(h, pool, &h->ls_tiles, (size_t)h->ls_ntiles * kTileBytes));
         TRY(dalloc(h, pool, &h->ls_scale, (size_t)N0));
@@ -790,6 +791,7 @@ mgsb_status rebuild(mgsb_solver* h) {
                     }
                 }
                 win[t] = (hi - lo <= kLsWinRows) ? int2{lo, hi} : int2{0, 0};
+                h->ls_win_rows = std::max(h->ls_win_rows, win[t].y - win[t].x);
             }
             TRY(dupload(h, pool, &h->ls_win, win));
         }
@@ -806,7 +808,7 @@ mgsb_status rebuild(mgsb_solver* h) {
         CUDA_TRY(h, cudaMemset(h->ls_gate, 0, sizeof(int32_t)));
         CUDA_TRY(h, cudaMemset(h->ls_werr, 0, sizeof(int32_t)));
         CUDA_TRY(h, cudaFuncSetAttribute(k_ls_sweep_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)ls_sweep_smem_bytes()));
+                                         (int)ls_sweep_smem_bytes(kLsWinRows)));
         CUDA_TRY(h, cudaDeviceGetAttribute(&h->sm_count, cudaDevAttrMultiProcessorCount, h->device));
     }
     TRY(dalloc(h, pool, &h->energy_part, (size_t)kEnergyBlocks * kEnergyTerms));
@@ -1547,7 +1549,7 @@ void enqueue_learned_vcycle(mgsb_solver* h, float4* d, const float4* b, bool fro
     const int g0 = h->ls_nblk;
     const uint8_t* img = mlp_device_image(h->ls_net);
     const int mgrid = std::min(h->ls_ntiles, 2 * h->sm_count);
-    const size_t msmem = ls_sweep_smem_bytes();
+    const size_t msmem = ls_sweep_smem_bytes(h->ls_win_rows);
     float4* bw = const_cast<float4*>(b);
     (void)from_zero;
     // pre-smoothing (with gather_b the right-hand side b = b0 + slots is assembled here first;
