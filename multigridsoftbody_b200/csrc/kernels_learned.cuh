@@ -159,7 +159,7 @@ __global__ void __launch_bounds__(kLsThreads) k_ls_row_consts(int n, const int32
     const bool valid = row < n;
     // the row's entries and its contact-free diagonal are set-up data: loaded before the wait
     HeldEntries<kHeldL0> he;
-    hold_ell_row<G>(he, row, valid, lane, sp, col, val);
+    hold_warp_slice<G>(he, warp, n, lane, sp, col, val);
     const float L = (valid && lane < S) ? __ldg(diag0 + row) : 0.f;
     pdl_wait();
     float sa = 0.f, sd = 0.f;   // the entries in the order of the row's ELL loop

@@ -162,27 +162,29 @@ struct HeldEntries {
     int next, end, stride;   // first entry not held, the row's end, entry stride
 };
 
-// This lane's entries of `row` of a sliced-ELL matrix (slice height 32 / G).
-template <int G, int K>
-__device__ __forceinline__ void hold_ell_row(HeldEntries<K>& h, int row, bool valid, int lane,
-                                             const int32_t* __restrict__ sp, const int32_t* __restrict__ col,
-                                             const float* __restrict__ val) {
-    constexpr int S = 32 / G;
-    int e = 0, end = 0;
-    if (valid) {
-        const int slice = row / S;
-        end = __ldg(sp + slice + 1);
-        e = __ldg(sp + slice) + (lane / S) * S + (row - slice * S);
-    }
+// This lane's entries of its row (valid: there is one) in a slice of a sliced-ELL matrix, 32 entries per step.
+template <int K>
+__device__ __forceinline__ void hold_slice(HeldEntries<K>& h, int beg, int end, bool valid, int lane,
+                                           const int32_t* __restrict__ col, const float* __restrict__ val) {
+    const int e = beg + lane;
+    h.end = valid ? end : 0;
+    h.stride = 32;
 #pragma unroll
     for (int k = 0; k < K; ++k) {
-        const bool ok = e + 32 * k < end;
+        const bool ok = e + 32 * k < h.end;
         h.c[k] = ok ? __ldg(col + e + 32 * k) : -1;
         h.v[k] = ok ? __ldg(val + e + 32 * k) : 0.f;
     }
     h.next = e + 32 * K;
-    h.end = end;
-    h.stride = 32;
+}
+
+// The same of slice `s`, its pointers read once for the warp.
+template <int G, int K>
+__device__ __forceinline__ void hold_warp_slice(HeldEntries<K>& h, int s, int n, int lane, const int32_t* __restrict__ sp,
+                                                const int32_t* __restrict__ col, const float* __restrict__ val) {
+    constexpr int S = 32 / G;
+    const bool any = s * S < n;
+    hold_slice(h, any ? __ldg(sp + s) : 0, any ? __ldg(sp + s + 1) : 0, s * S + lane % S < n, lane, col, val);
 }
 
 // This lane's entries [beg, end) of a CSR row split across G lanes.
@@ -235,6 +237,11 @@ __device__ __forceinline__ float4 held_sum(const HeldEntries<K>& h, int lane, co
     return make_float4(ax, ay, az, 0.f);
 }
 
+// CTAs of 256 threads per SM of the kernels with a slice per warp: 40 registers a thread hold the slice's entries and the
+// row's own data, which are loaded together (loaded behind the sum they cost a second latency: 3.0 to 2.7 us per level-0
+// sweep of the 12x120x12 beam, 2.2 to 2.1 us per restriction).
+constexpr int kRowCtas = 6;
+
 constexpr int kHeldL0 = 4;   // level-0 entries held per lane (4 lanes per row: 16 per row)
 constexpr int kHeldC = 6;    // coarse-level entries held per lane (8 lanes per row: 48 per row)
 
@@ -266,62 +273,63 @@ __device__ __forceinline__ float4 rg_slot_sum(int lane, int beg, int end, const 
 // With gather != 0 the RHS is assembled first (b = b0 + slots) and stored.
 // One warp per 8 rows, 4 lanes per row.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_l0_sweep_rg(int n, const int32_t* __restrict__ sp, const int32_t* __restrict__ col,
-                                                     const float* __restrict__ val, const float* __restrict__ dfull,
-                                                     const float* __restrict__ dinv, const float4* __restrict__ din,
-                                                     float4* __restrict__ dout, float4* __restrict__ b,
-                                                     const float4* __restrict__ b0, const int32_t* __restrict__ slot_ptr,
-                                                     const float4* __restrict__ slots, int gather,
-                                                     const int32_t* __restrict__ gate = nullptr) {
+__global__ void __launch_bounds__(256, kRowCtas) k_l0_sweep_rg(int n, const int32_t* __restrict__ sp,
+                                                               const int32_t* __restrict__ col, const float* __restrict__ val,
+                                                               const float* __restrict__ dfull, const float* __restrict__ dinv,
+                                                               const float4* __restrict__ din, float4* __restrict__ dout,
+                                                               float4* __restrict__ b, const float4* __restrict__ b0,
+                                                               const int32_t* __restrict__ slot_ptr,
+                                                               const float4* __restrict__ slots, int gather) {
     pdl_trigger();
     constexpr int G = kLanesL0, S = 32 / G;
     const int lane = threadIdx.x & 31;
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int row = warp * S + (lane % S);
+    const int row = warp * S + lane % S;
     const bool valid = row < n;
     HeldEntries<kHeldL0> he;
-    hold_ell_row<G>(he, row, valid, lane, sp, col, val);
-    const bool slice = gather && warp * S < n;
-    const int sbeg = slice ? __ldg(slot_ptr + warp) : 0, send = slice ? __ldg(slot_ptr + warp + 1) : 0;
+    hold_warp_slice<G>(he, warp, n, lane, sp, col, val);
+    const bool any = gather && warp * S < n;
+    const int sbeg = any ? __ldg(slot_ptr + warp) : 0, send = any ? __ldg(slot_ptr + warp + 1) : 0;
     pdl_wait();
-    if (gate && __ldg(gate) == 0) return;   // gated launches run only when the learned V-cycle was rejected
+    const int r = valid ? row : 0;
+    // the row's own data before the sums that wait for the gathers
+    const float4 di4 = __ldg(din + r);
+    const float D = __ldg(dfull + r), w = __ldg(dinv + r);
     float4 bi;
     if (gather) {
+        const float4 bb = __ldg(b0 + r);
         const float4 sl = rg_slot_sum<G>(lane, sbeg, send, slots);
-        const float4 bb = valid ? __ldg(b0 + row) : f4z();
         bi = make_float4(bb.x + sl.x, bb.y + sl.y, bb.z + sl.z, 0.f);
         if (valid && lane < S) b[row] = bi;
     } else {
-        bi = valid ? b[row] : f4z();
+        bi = b[r];
     }
     const float4 off = held_sum<G>(he, lane, col, val, din);
     if (!valid || lane >= S) return;
-    const float4 di4 = __ldg(din + row);
-    const float D = __ldg(dfull + row), w = __ldg(dinv + row);
     dout[row] = make_float4(fmaf(w, bi.x - fmaf(D, di4.x, off.x), di4.x), fmaf(w, bi.y - fmaf(D, di4.y, off.y), di4.y),
                             fmaf(w, bi.z - fmaf(D, di4.z, off.z), di4.z), 0.f);
 }
 
 // Level-0 residual res = b - A d (used when the coarse kernel does not fuse it).
-__global__ void __launch_bounds__(256) k_l0_residual_rg(int n, const int32_t* __restrict__ sp, const int32_t* __restrict__ col,
-                                                        const float* __restrict__ val, const float* __restrict__ dfull,
-                                                        const float4* __restrict__ dvec, const float4* __restrict__ b,
-                                                        float4* __restrict__ res, const int32_t* __restrict__ gate = nullptr) {
+__global__ void __launch_bounds__(256, kRowCtas) k_l0_residual_rg(int n, const int32_t* __restrict__ sp, const int32_t* __restrict__ col,
+                                                  const float* __restrict__ val, const float* __restrict__ dfull,
+                                                  const float4* __restrict__ x, const float4* __restrict__ b,
+                                                  float4* __restrict__ res) {
     pdl_trigger();
     constexpr int G = kLanesL0, S = 32 / G;
     const int lane = threadIdx.x & 31;
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int row = warp * S + (lane % S);
+    const int row = warp * S + lane % S;
     const bool valid = row < n;
     HeldEntries<kHeldL0> he;
-    hold_ell_row<G>(he, row, valid, lane, sp, col, val);
+    hold_warp_slice<G>(he, warp, n, lane, sp, col, val);
     pdl_wait();
-    if (gate && __ldg(gate) == 0) return;
-    const float4 off = held_sum<G>(he, lane, col, val, dvec);
+    const int q = valid ? row : 0;
+    const float4 xi = __ldg(x + q), bi = __ldg(b + q);
+    const float D = __ldg(dfull + q);
+    const float4 off = held_sum<G>(he, lane, col, val, x);
     if (!valid || lane >= S) return;
-    const float4 x = __ldg(dvec + row), bi = __ldg(b + row);
-    const float D = __ldg(dfull + row);
-    res[row] = make_float4(bi.x - fmaf(D, x.x, off.x), bi.y - fmaf(D, x.y, off.y), bi.z - fmaf(D, x.z, off.z), 0.f);
+    res[row] = make_float4(bi.x - fmaf(D, xi.x, off.x), bi.y - fmaf(D, xi.y, off.y), bi.z - fmaf(D, xi.z, off.z), 0.f);
 }
 
 // Level-0 prolongation d += P e1 (used when the coarse kernel does not fuse it).
@@ -353,7 +361,7 @@ __global__ void k_l0_prolong(int n, const int4* __restrict__ pid, const float4* 
 __global__ void __launch_bounds__(256) k_lvl_restrict(int n, const int32_t* __restrict__ rptr, const int32_t* __restrict__ rcol,
                                                       const float* __restrict__ rw, const float4* __restrict__ res_fine,
                                                       const float* __restrict__ dinv, float4* __restrict__ r,
-                                                      float4* __restrict__ e, const int32_t* __restrict__ gate) {
+                                                      float4* __restrict__ e) {
     pdl_trigger();
     constexpr int G = kLanesC, S = 32 / G;
     const int lane = threadIdx.x & 31;
@@ -364,11 +372,10 @@ __global__ void __launch_bounds__(256) k_lvl_restrict(int n, const int32_t* __re
     HeldEntries<kHeldC> he;
     hold_csr_row<G>(he, valid, lane, beg, end, rcol, rw);
     pdl_wait();
-    if (gate && __ldg(gate) == 0) return;
+    const float di = dinv && valid ? __ldg(dinv + row) : 0.f;
     const float4 s = held_sum<G>(he, lane, rcol, rw, res_fine);
     if (!valid || lane >= S) return;
     r[row] = s;
-    const float di = dinv ? __ldg(dinv + row) : 0.f;
     e[row] = make_float4(di * s.x, di * s.y, di * s.z, 0.f);
 }
 
@@ -431,49 +438,48 @@ __global__ void __launch_bounds__(256) k_lvl_restrict_res0(int n, const int32_t*
 }
 
 // eout = ein + dinv (r - A ein)
-__global__ void __launch_bounds__(256) k_lvl_sweep(int n, const int32_t* __restrict__ sp, const int32_t* __restrict__ col,
-                                                   const float* __restrict__ val, const float* __restrict__ dfull,
-                                                   const float* __restrict__ dinv, const float4* __restrict__ r,
-                                                   const float4* __restrict__ ein, float4* __restrict__ eout,
-                                                   const int32_t* __restrict__ gate) {
+__global__ void __launch_bounds__(256, kRowCtas) k_lvl_sweep(int n, const int32_t* __restrict__ sp, const int32_t* __restrict__ col,
+                                                             const float* __restrict__ val, const float* __restrict__ dfull,
+                                                             const float* __restrict__ dinv, const float4* __restrict__ r,
+                                                             const float4* __restrict__ ein, float4* __restrict__ eout) {
     pdl_trigger();
     constexpr int G = kLanesC, S = 32 / G;
     const int lane = threadIdx.x & 31;
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int row = warp * S + (lane % S);
+    const int row = warp * S + lane % S;
     const bool valid = row < n;
     HeldEntries<kHeldC> he;
-    hold_ell_row<G>(he, row, valid, lane, sp, col, val);
+    hold_warp_slice<G>(he, warp, n, lane, sp, col, val);
     pdl_wait();
-    if (gate && __ldg(gate) == 0) return;
+    const int q = valid ? row : 0;
+    const float4 x = __ldg(ein + q), ri = __ldg(r + q);
+    const float D = __ldg(dfull + q), w = __ldg(dinv + q);
     const float4 off = held_sum<G>(he, lane, col, val, ein);
     if (!valid || lane >= S) return;
-    const float4 x = __ldg(ein + row), ri = __ldg(r + row);
-    const float D = __ldg(dfull + row), w = __ldg(dinv + row);
     eout[row] = make_float4(fmaf(w, ri.x - fmaf(D, x.x, off.x), x.x), fmaf(w, ri.y - fmaf(D, x.y, off.y), x.y),
                             fmaf(w, ri.z - fmaf(D, x.z, off.z), x.z), 0.f);
 }
 
-// res = r - A e
-__global__ void __launch_bounds__(256) k_lvl_residual(int n, const int32_t* __restrict__ sp, const int32_t* __restrict__ col,
-                                                      const float* __restrict__ val, const float* __restrict__ dfull,
-                                                      const float4* __restrict__ r, const float4* __restrict__ e,
-                                                      float4* __restrict__ res, const int32_t* __restrict__ gate) {
+// res = b - A x
+__global__ void __launch_bounds__(256, kRowCtas) k_lvl_residual(int n, const int32_t* __restrict__ sp, const int32_t* __restrict__ col,
+                                                  const float* __restrict__ val, const float* __restrict__ dfull,
+                                                  const float4* __restrict__ b, const float4* __restrict__ x,
+                                                  float4* __restrict__ res) {
     pdl_trigger();
     constexpr int G = kLanesC, S = 32 / G;
     const int lane = threadIdx.x & 31;
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int row = warp * S + (lane % S);
+    const int row = warp * S + lane % S;
     const bool valid = row < n;
     HeldEntries<kHeldC> he;
-    hold_ell_row<G>(he, row, valid, lane, sp, col, val);
+    hold_warp_slice<G>(he, warp, n, lane, sp, col, val);
     pdl_wait();
-    if (gate && __ldg(gate) == 0) return;
-    const float4 off = held_sum<G>(he, lane, col, val, e);
+    const int q = valid ? row : 0;
+    const float4 xi = __ldg(x + q), bi = __ldg(b + q);
+    const float D = __ldg(dfull + q);
+    const float4 off = held_sum<G>(he, lane, col, val, x);
     if (!valid || lane >= S) return;
-    const float4 x = __ldg(e + row), ri = __ldg(r + row);
-    const float D = __ldg(dfull + row);
-    res[row] = make_float4(ri.x - fmaf(D, x.x, off.x), ri.y - fmaf(D, x.y, off.y), ri.z - fmaf(D, x.z, off.z), 0.f);
+    res[row] = make_float4(bi.x - fmaf(D, xi.x, off.x), bi.y - fmaf(D, xi.y, off.y), bi.z - fmaf(D, xi.z, off.z), 0.f);
 }
 
 // dst = cur + P ec (P: 4 coarse parents per row); dst may be cur.
@@ -494,6 +500,41 @@ __global__ void k_lvl_prolong(int n, const int4* __restrict__ pid, const float4*
     dst[i] = v;
 }
 
+// The slices of a sliced-ELL matrix over a grid's warps: wait() once, the first slice's entries loaded before it, then
+// row(slice, entries) for every slice of this warp, with the next slice's entries and the slice pointers after those
+// on their way.  Where the rows outnumber the warps that the SMs hold (a batch's 330,000 rows), a warp with one slice
+// spends its life in three dependent loads (pointer, entries, gathered vector), and DRAM ran at 31-32 % of its rate;
+// a few warps per scheduler that stream keep all three kinds of load in flight.
+template <int G, int K, typename Wait, typename Row>
+__device__ __forceinline__ void each_slice(int n, const int32_t* __restrict__ sp, const int32_t* __restrict__ col,
+                                           const float* __restrict__ val, Wait&& wait, Row&& row) {
+    constexpr int S = 32 / G;
+    const int lane = threadIdx.x & 31, slices = (n + S - 1) / S;
+    const int step = gridDim.x * (blockDim.x >> 5);
+    int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    int beg = 0, end = 0;   // the next slice
+    auto pointers = [&](int t) {
+        beg = t < slices ? __ldg(sp + t) : 0;
+        end = t < slices ? __ldg(sp + t + 1) : 0;
+    };
+    auto entries = [&](HeldEntries<K>& h, int t) { hold_slice(h, beg, end, t * S + lane % S < n, lane, col, val); };
+    HeldEntries<K> he;
+    pointers(s);
+    entries(he, s);
+    pointers(s + step);
+    wait();
+    for (; s < slices; s += step) {
+        HeldEntries<K> hn = he;
+        if (s + step < slices) {
+            entries(hn, s + step);
+            pointers(s + 2 * step);
+        }
+        row(s, he);
+        he = hn;
+    }
+}
+constexpr int kProlongCtas = 3;   // CTAs of 256 threads per SM (80 registers a thread)
+
 // ---------------------------------------------------------------------------
 // Prolongation fused with the first post-smoothing sweep.  With the level's
 // operator A = D + Off, pe = P e_c (this row's 4 parents on the coarser level)
@@ -510,58 +551,55 @@ __global__ void k_lvl_prolong(int n, const int4* __restrict__ pid, const float4*
 // be dout.
 // ---------------------------------------------------------------------------
 template <int G>
-__global__ void __launch_bounds__(256) k_prolong_sweep(int n, const int4* __restrict__ pid, const float4* __restrict__ pw,
-                                                       const float4* __restrict__ ec, const int32_t* __restrict__ sp,
-                                                       const int32_t* __restrict__ col, const float* __restrict__ val,
-                                                       const float* __restrict__ dfull, const float* __restrict__ dinv,
-                                                       const float4* __restrict__ res, const float4* din, float4* dout,
-                                                       const float* __restrict__ fixf, float4* __restrict__ ls_r,
-                                                       const int32_t* __restrict__ gate, const float4* __restrict__ b,
-                                                       const int32_t* __restrict__ sp0, const int32_t* __restrict__ col0,
-                                                       const float* __restrict__ val0) {
+__global__ void __launch_bounds__(256, kProlongCtas)
+    k_prolong_sweep(int n, const int4* __restrict__ pid, const float4* __restrict__ pw, const float4* __restrict__ ec,
+                    const int32_t* __restrict__ sp, const int32_t* __restrict__ col, const float* __restrict__ val,
+                    const float* __restrict__ dfull, const float* __restrict__ dinv, const float4* __restrict__ res,
+                    const float4* din, float4* dout, const float* __restrict__ fixf, float4* __restrict__ ls_r,
+                    const float4* __restrict__ b, const int32_t* __restrict__ sp0, const int32_t* __restrict__ col0,
+                    const float* __restrict__ val0) {
     pdl_trigger();
-    constexpr int S = 32 / G;
+    constexpr int S = 32 / G, K = G == kLanesL0 ? kHeldL0 : kHeldC;
     const bool form_res = res == nullptr;   // uniform over the launch
     const int lane = threadIdx.x & 31;
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int row = warp * S + (lane % S);
-    const bool valid = row < n;
-    HeldEntries<G == kLanesL0 ? kHeldL0 : kHeldC> he, ha;
-    hold_ell_row<G>(he, row, valid, lane, sp, col, val);
-    if (form_res) hold_ell_row<G>(ha, row, valid, lane, sp0, col0, val0);
-    const bool own = valid && lane < S;
-    const int4 id = own ? __ldg(pid + row) : make_int4(0, 0, 0, 0);
-    const float4 w = own ? __ldg(pw + row) : f4z();
-    pdl_wait();
-    if (gate && __ldg(gate) == 0) return;
-    const float4 q = held_sum<G>(he, lane, col, val, ec);
-    const float4 offd = form_res ? held_sum<G>(ha, lane, col0, val0, din) : f4z();
-    if (!own) return;
-    const float4 e0 = __ldg(ec + id.x), e1 = __ldg(ec + id.y), e2 = __ldg(ec + id.z), e3 = __ldg(ec + id.w);
-    const float4 pe = make_float4(w.x * e0.x + w.y * e1.x + w.z * e2.x + w.w * e3.x,
-                                  w.x * e0.y + w.y * e1.y + w.z * e2.y + w.w * e3.y,
-                                  w.x * e0.z + w.y * e1.z + w.z * e2.z + w.w * e3.z, 0.f);
-    const float D = __ldg(dfull + row);
-    float4 r0;
-    if (form_res) {
-        const float4 xd = __ldg(din + row), bi = __ldg(b + row);
-        r0 = make_float4(bi.x - fmaf(D, xd.x, offd.x), bi.y - fmaf(D, xd.y, offd.y), bi.z - fmaf(D, xd.z, offd.z), 0.f);
-    } else {
-        r0 = __ldg(res + row);
-    }
-    const float rx = r0.x - fmaf(D, pe.x, q.x), ry = r0.y - fmaf(D, pe.y, q.y), rz = r0.z - fmaf(D, pe.z, q.z);
-    float4 x = din[row];
-    x.x += pe.x;
-    x.y += pe.y;
-    x.z += pe.z;
-    if (ls_r) {
-        const float fx = __ldg(fixf + row);
-        ls_r[row] = make_float4(fx * rx, fx * ry, fx * rz, 0.f);
-        dout[row] = x;
-    } else {
-        const float wi = __ldg(dinv + row);
-        dout[row] = make_float4(fmaf(wi, rx, x.x), fmaf(wi, ry, x.y), fmaf(wi, rz, x.z), 0.f);
-    }
+    const int first = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int row0 = first * S + lane % S;
+    // the first row's parents: set-up data
+    int4 id = row0 < n ? __ldg(pid + row0) : make_int4(0, 0, 0, 0);
+    float4 w = row0 < n ? __ldg(pw + row0) : f4z();
+    each_slice<G, K>(n, sp, col, val, [] { pdl_wait(); }, [&](int s, const HeldEntries<K>& he) {
+        const int row = s * S + lane % S;
+        const bool valid = row < n;
+        const int r = valid ? row : 0;
+        if (s != first) {
+            id = __ldg(pid + r);
+            w = __ldg(pw + r);
+        }
+        // the row's own data before the sum that waits for the gathers
+        float4 x = din[r];
+        float4 r0 = __ldg((form_res ? b : res) + r);
+        const float D = __ldg(dfull + r), k = ls_r ? __ldg(fixf + r) : __ldg(dinv + r);
+        const float4 e0 = __ldg(ec + id.x), e1 = __ldg(ec + id.y), e2 = __ldg(ec + id.z), e3 = __ldg(ec + id.w);
+        const float4 q = held_sum<G>(he, lane, col, val, ec);
+        if (form_res) {
+            const float4 offd = rg_offdiag<G>(row, valid, lane, sp0, col0, val0, din);
+            r0 = make_float4(r0.x - fmaf(D, x.x, offd.x), r0.y - fmaf(D, x.y, offd.y), r0.z - fmaf(D, x.z, offd.z), 0.f);
+        }
+        if (!valid || lane >= S) return;
+        const float4 pe = make_float4(w.x * e0.x + w.y * e1.x + w.z * e2.x + w.w * e3.x,
+                                      w.x * e0.y + w.y * e1.y + w.z * e2.y + w.w * e3.y,
+                                      w.x * e0.z + w.y * e1.z + w.z * e2.z + w.w * e3.z, 0.f);
+        const float rx = r0.x - fmaf(D, pe.x, q.x), ry = r0.y - fmaf(D, pe.y, q.y), rz = r0.z - fmaf(D, pe.z, q.z);
+        x.x += pe.x;
+        x.y += pe.y;
+        x.z += pe.z;
+        if (ls_r) {
+            ls_r[row] = make_float4(k * rx, k * ry, k * rz, 0.f);
+            dout[row] = x;
+        } else {
+            dout[row] = make_float4(fmaf(k, rx, x.x), fmaf(k, ry, x.y), fmaf(k, rz, x.z), 0.f);
+        }
+    });
 }
 
 // ---------------------------------------------------------------------------

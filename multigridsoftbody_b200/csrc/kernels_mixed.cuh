@@ -183,7 +183,8 @@ __global__ void __launch_bounds__(kMxThreads, 3) k_mx_residual(int n, const int3
     const double4 xown = own ? d[row] : d4z();
     const double Down = own ? D0 + (double)__ldg(c + row) : 0.0;
     const float wown = (own && first_sweep) ? __ldg(dinv + row) : 0.f;
-    double4 bi = d4z(), bprev = d4z();
+    double4 bi = own ? (b0 ? b0[row] : b[row]) : d4z();
+    const double4 bprev = own && b0 && part_end ? b[row] : d4z();   // the previous iteration's right-hand side, before it is replaced
     if (b0) {   // uniform over the block: the row's slots split over its G lanes, FP64 sums
         double sx = 0.0, sy = 0.0, sz = 0.0;
 #pragma unroll
@@ -206,9 +207,7 @@ __global__ void __launch_bounds__(kMxThreads, 3) k_mx_residual(int n, const int3
             sy += __shfl_xor_sync(0xffffffffu, sy, o);
             sz += __shfl_xor_sync(0xffffffffu, sz, o);
         }
-        if (valid && lane < RW) {
-            if (part_end) bprev = b[row];   // the previous iteration's right-hand side, before it is replaced
-            bi = b0[row];
+        if (own) {
             bi.x += sx;
             bi.y += sy;
             bi.z += sz;
@@ -241,7 +240,6 @@ __global__ void __launch_bounds__(kMxThreads, 3) k_mx_residual(int n, const int3
     float rr = 0.f, re = 0.f;
     if (own) {
         const double4 x = xown;
-        if (!b0) bi = b[row];
         const double D = Down;
         const float rx = (float)(bi.x - fma(D, x.x, ax)), ry = (float)(bi.y - fma(D, x.y, ay)), rz = (float)(bi.z - fma(D, x.z, az));
         if (part_end) {

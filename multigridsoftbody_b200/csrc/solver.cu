@@ -35,6 +35,8 @@ inline int grid_for(int n) { return (n + kBlock - 1) / kBlock; }
 inline int grid_ref_vertex(int n) { return (n + kRefVertexThreads - 1) / kRefVertexThreads; }
 // blocks of kBlock threads for a row-group kernel (32/S lanes per row, slices of S rows)
 inline int grid_rows(int n, int S) { return ((n + S - 1) / S * 32 + kBlock - 1) / kBlock; }
+// Of the kernels that stream slices (each_slice): one wave at most.
+inline int grid_slices(int n, int S, int sms, int ctas) { return std::min(grid_rows(n, S), sms * ctas); }
 
 // Device allocation owned by the solver.
 struct DevMem {
@@ -1378,13 +1380,13 @@ mgsb_status launch_coarse(mgsb_solver* h, const CoarseArgs& args_in) {
                    C.r, C.e, gate);
         else
             LAUNCH(h, k_lvl_restrict, g, kBlock, 0, C.n, C.rptr, C.rcol, C.rw, args.lv[l - 1].res,
-                   args.pre > 0 ? C.dinv : nullptr, C.r, C.e, gate);
+                   args.pre > 0 ? C.dinv : nullptr, C.r, C.e);
         float4 *a = C.e, *b = C.e2;
         for (int k = 1; k < args.pre; ++k) {
-            LAUNCH(h, k_lvl_sweep, g, kBlock, 0, C.n, C.slice_ptr, C.col, C.val, C.dfull, C.dinv, C.r, a, b, gate);
+            LAUNCH(h, k_lvl_sweep, g, kBlock, 0, C.n, C.slice_ptr, C.col, C.val, C.dfull, C.dinv, C.r, a, b);
             std::swap(a, b);
         }
-        LAUNCH(h, k_lvl_residual, g, kBlock, 0, C.n, C.slice_ptr, C.col, C.val, C.dfull, C.r, a, C.res, gate);
+        LAUNCH(h, k_lvl_residual, g, kBlock, 0, C.n, C.slice_ptr, C.col, C.val, C.dfull, C.r, a, C.res);
         cur[l] = a;
     }
     if (h->dense_op) {   // levels F..L-1: the restriction to level F and the dense operator, one launch
@@ -1425,11 +1427,10 @@ mgsb_status launch_coarse(mgsb_solver* h, const CoarseArgs& args_in) {
             // prolongation + first post-sweep in one launch (from the residual C.res of the descent)
             float4* a = ((args.post - 1) % 2 == 0) ? C.e : C.e2;
             float4* b = (a == C.e) ? C.e2 : C.e;
-            LAUNCH(h, k_prolong_sweep<kLanesC>, g, kBlock, 0, C.n, Cc.pid, Cc.pw, Cc.e, C.op_slice_ptr, C.op_col,
-                   C.op_val, C.dfull, C.dinv, C.res, cur[l], a, nullptr, nullptr, gate, nullptr, nullptr, nullptr,
-                   nullptr);
+            LAUNCH(h, k_prolong_sweep<kLanesC>, grid_slices(C.n, 32 / kLanesC, h->sm_count, kProlongCtas), kBlock, 0, C.n,
+                   Cc.pid, Cc.pw, Cc.e, C.op_slice_ptr, C.op_col, C.op_val, C.dfull, C.dinv, C.res, cur[l], a, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr);
             for (int k = 1; k < args.post; ++k) {
-                LAUNCH(h, k_lvl_sweep, g, kBlock, 0, C.n, C.slice_ptr, C.col, C.val, C.dfull, C.dinv, C.r, a, b, gate);
+                LAUNCH(h, k_lvl_sweep, g, kBlock, 0, C.n, C.slice_ptr, C.col, C.val, C.dfull, C.dinv, C.r, a, b);
                 std::swap(a, b);
             }
             continue;
@@ -1438,7 +1439,7 @@ mgsb_status launch_coarse(mgsb_solver* h, const CoarseArgs& args_in) {
         float4* b = (a == C.e) ? C.e2 : C.e;
         LAUNCH(h, k_lvl_prolong, grid_for(C.n), kBlock, 0, C.n, Cc.pid, Cc.pw, Cc.e, cur[l], a, gate);
         for (int k = 0; k < args.post; ++k) {
-            LAUNCH(h, k_lvl_sweep, g, kBlock, 0, C.n, C.slice_ptr, C.col, C.val, C.dfull, C.dinv, C.r, a, b, gate);
+            LAUNCH(h, k_lvl_sweep, g, kBlock, 0, C.n, C.slice_ptr, C.col, C.val, C.dfull, C.dinv, C.r, a, b);
             std::swap(a, b);
         }
     }
@@ -1505,6 +1506,20 @@ bool res0_fused(const mgsb_solver* h) {
            h->lev[1].ro_ptr != nullptr;
 }
 
+// A Jacobi sweep on level 0, from -> to; gather: the right-hand side b = b0 + slots first.
+void enqueue_l0_sweep(mgsb_solver* h, const float4* from, float4* to, float4* b, bool gather = false) {
+    const LevelDev& l = h->lev[0];
+    LAUNCH(h, k_l0_sweep_rg, grid_rows(h->N0, l.S), kBlock, 0, h->N0, l.slice_ptr, l.ell_col, l.ell_val,
+           l.dfull, l.dinv, from, to, b, h->b0, h->slot_ptr, h->slots, gather ? 1 : 0);
+}
+
+// The level-0 residual b - A x.
+void enqueue_l0_residual(mgsb_solver* h, const float4* x, const float4* b) {
+    const LevelDev& l = h->lev[0];
+    LAUNCH(h, k_l0_residual_rg, grid_rows(h->N0, l.S), kBlock, 0, h->N0, l.slice_ptr, l.ell_col, l.ell_val,
+           l.dfull, x, b, l.res);
+}
+
 // Level-0 prolongation d += P e1 and the post-smoothing sweeps (ping-pong
 // xa -> xb; on return xa holds the result): the first sweep fused with the
 // prolongation (k_prolong_sweep, from the level-0 residual lv[0].res of the
@@ -1516,11 +1531,11 @@ void enqueue_l0_post(mgsb_solver* h, float4*& xa, float4*& xb, float4* b, const 
     const int n0 = h->N0;
     const LevelDev& l0 = h->lev[0];
     const LevelDev& l1 = h->lev[1];
-    const int g0 = grid_rows(n0, l0.S);
     int k0 = 0;
     if (h->fuse_prolong && post > 0) {
-        LAUNCH(h, k_prolong_sweep<kLanesL0>, g0, kBlock, 0, n0, l1.pid, l1.pw, l1.e, l0.op_slice_ptr, l0.op_col,
-               l0.op_val, l0.dfull, l0.dinv, form_res ? nullptr : l0.res, xa, xb, nullptr, nullptr, gate,
+        LAUNCH(h, k_prolong_sweep<kLanesL0>, grid_slices(n0, l0.S, h->sm_count, kProlongCtas), kBlock, 0, n0, l1.pid, l1.pw,
+               l1.e, l0.op_slice_ptr, l0.op_col, l0.op_val, l0.dfull, l0.dinv, form_res ? nullptr : l0.res, xa, xb, nullptr,
+               nullptr,
                form_res ? b : nullptr, l0.slice_ptr, l0.ell_col, l0.ell_val);
         std::swap(xa, xb);
         k0 = 1;
@@ -1528,8 +1543,7 @@ void enqueue_l0_post(mgsb_solver* h, float4*& xa, float4*& xb, float4* b, const 
         LAUNCH(h, k_l0_prolong, grid_for(n0), kBlock, 0, n0, l1.pid, l1.pw, l1.e, xa, gate);
     }
     for (int k = k0; k < post; ++k) {
-        LAUNCH(h, k_l0_sweep_rg, g0, kBlock, 0, n0, l0.slice_ptr, l0.ell_col, l0.ell_val, l0.dfull, l0.dinv, xa, xb, b,
-               h->b0, h->slot_ptr, h->slots, 0, gate);
+        enqueue_l0_sweep(h, xa, xb, b);
         std::swap(xa, xb);
     }
 }
@@ -1565,8 +1579,7 @@ void enqueue_learned_vcycle(mgsb_solver* h, float4* d, const float4* b, bool fro
     // takes b and d, the post-smoothing kernel forms its rows into ls_dpost's sweep)
     const bool fr = res0_fused(h);
     if (!fr)
-        LAUNCH(h, k_l0_residual_rg, g0, kBlock, 0, n0, l0.slice_ptr, l0.ell_col, l0.ell_val, l0.dfull, d, b, l0.res,
-               nullptr);
+        enqueue_l0_residual(h, d, b);
     ca.d = d;
     ca.gate = nullptr;
     ca.res0_b = fr ? b : nullptr;
@@ -1574,8 +1587,9 @@ void enqueue_learned_vcycle(mgsb_solver* h, float4* d, const float4* b, bool fro
     // post-smoothing: d += P e1 and the residual the learned sweep starts from
     float4* dpost = fr ? h->ls_dpost : d;
     if (h->fuse_prolong) {
-        LAUNCH(h, k_prolong_sweep<kLanesL0>, g0, kBlock, 0, n0, lv[1].pid, lv[1].pw, lv[1].e, l0.op_slice_ptr,
-               l0.op_col, l0.op_val, l0.dfull, l0.dinv, fr ? nullptr : l0.res, d, dpost, h->fixf, h->ls_r, nullptr,
+        LAUNCH(h, k_prolong_sweep<kLanesL0>, grid_slices(n0, l0.S, h->sm_count, kProlongCtas), kBlock, 0, n0, lv[1].pid,
+               lv[1].pw, lv[1].e, l0.op_slice_ptr, l0.op_col, l0.op_val, l0.dfull, l0.dinv, fr ? nullptr : l0.res, d, dpost,
+               h->fixf, h->ls_r,
                fr ? b : nullptr, l0.slice_ptr, l0.ell_col, l0.ell_val);
     } else {
         LAUNCH(h, k_l0_prolong, grid_for(n0), kBlock, 0, n0, lv[1].pid, lv[1].pw, lv[1].e, d, nullptr);
@@ -1889,16 +1903,14 @@ float4* enqueue_mg_solve(mgsb_solver* h, bool learned, const LearnedFallback& fb
             }
             bool gathered = pass > 0;
             for (int k = 0; k < l0_pre; ++k) {
-                LAUNCH(h, k_l0_sweep_rg, g0, kBlock, 0, n0, lv[0].slice_ptr, lv[0].ell_col, lv[0].ell_val, lv[0].dfull,
-                       lv[0].dinv, xa, xb, h->b, h->b0, h->slot_ptr, h->slots, gathered ? 0 : 1, nullptr);
+                enqueue_l0_sweep(h, xa, xb, h->b, !gathered);
                 gathered = true;
                 std::swap(xa, xb);
             }
             if (!gathered) LAUNCH(h, k_gather_rhs, grid_for(n0), kBlock, 0, n0, h->b, h->b0, h->slot_ptr, h->slots);
             const bool fr = res0_fused(h);
             if (!h->fuse_l0 && !fr)
-                LAUNCH(h, k_l0_residual_rg, g0, kBlock, 0, n0, lv[0].slice_ptr, lv[0].ell_col, lv[0].ell_val,
-                       lv[0].dfull, xa, h->b, lv[0].res, nullptr);
+                enqueue_l0_residual(h, xa, h->b);
             ca.d = xa;
             ca.res0_b = fr ? h->b : nullptr;
             launch_coarse(h, ca);
@@ -1906,8 +1918,7 @@ float4* enqueue_mg_solve(mgsb_solver* h, bool learned, const LearnedFallback& fb
                 enqueue_l0_post(h, xa, xb, h->b, nullptr, l0_post, fr);
             } else {
                 for (int k = 0; k < l0_post; ++k) {
-                    LAUNCH(h, k_l0_sweep_rg, g0, kBlock, 0, n0, lv[0].slice_ptr, lv[0].ell_col, lv[0].ell_val,
-                           lv[0].dfull, lv[0].dinv, xa, xb, h->b, h->b0, h->slot_ptr, h->slots, 0, nullptr);
+                    enqueue_l0_sweep(h, xa, xb, h->b);
                     std::swap(xa, xb);
                 }
             }
@@ -2009,14 +2020,12 @@ void enqueue_mixed_solve(mgsb_solver* h, bool learned, const LearnedFallback& fb
                 continue;
             }
             for (int k = 1; k < l0_pre; ++k) {
-                LAUNCH(h, k_l0_sweep_rg, g0, kBlock, 0, n0, lv[0].slice_ptr, lv[0].ell_col, lv[0].ell_val, lv[0].dfull,
-                       lv[0].dinv, ea, eb, h->r32, h->b0, h->slot_ptr, h->slots, 0, nullptr);
+                enqueue_l0_sweep(h, ea, eb, h->r32);
                 std::swap(ea, eb);
             }
             const bool fr = res0_fused(h);
             if (!fr)
-                LAUNCH(h, k_l0_residual_rg, g0, kBlock, 0, n0, lv[0].slice_ptr, lv[0].ell_col, lv[0].ell_val,
-                       lv[0].dfull, ea, h->r32, lv[0].res, nullptr);
+                enqueue_l0_residual(h, ea, h->r32);
             ca.d = ea;
             ca.res0_b = fr ? h->r32 : nullptr;
             launch_coarse(h, ca);
@@ -3395,7 +3404,7 @@ extern "C" mgsb_status mgsb_smoother_pairs(mgsb_solver* h, int32_t sweeps, float
         cudaMemsetAsync(xa, 0, (size_t)n0 * sizeof(float4), st);
         for (int k = 0; k < k_sweeps; ++k) {
             k_l0_sweep_rg<<<g0, kBlock, 0, st>>>(n0, l0.slice_ptr, l0.ell_col, l0.ell_val, l0.dfull, l0.dinv, xa, xb,
-                                                 const_cast<float4*>(rhs), h->b0, h->slot_ptr, h->slots, 0, nullptr);
+                                                 const_cast<float4*>(rhs), h->b0, h->slot_ptr, h->slots, 0);
             std::swap(xa, xb);
         }
         return xa;
@@ -3441,7 +3450,7 @@ extern "C" mgsb_status mgsb_smoother_pairs(mgsb_solver* h, int32_t sweeps, float
     // (2) the residual after plain pre-smoothing and the coarse correction (a
     //     post-smoothing input): e = sweeps(r) + P V_c(P^T (r - A e)), r2 = r - A e
     float4* e = sweeps_from_zero(h->ls_r, p.pre_sweeps);
-    k_l0_residual_rg<<<g0, kBlock, 0, st>>>(n0, l0.slice_ptr, l0.ell_col, l0.ell_val, l0.dfull, e, h->ls_r, l0.res, nullptr);
+    k_l0_residual_rg<<<g0, kBlock, 0, st>>>(n0, l0.slice_ptr, l0.ell_col, l0.ell_val, l0.dfull, e, h->ls_r, l0.res);
     ca.d = e;
     TRY(launch_coarse(h, ca));
     k_l0_prolong<<<grid_for(n0), kBlock, 0, st>>>(n0, lv[1].pid, lv[1].pw, lv[1].e, e, nullptr);
@@ -3526,18 +3535,17 @@ extern "C" mgsb_status mgsb_vcycle_residuals(mgsb_solver* h, int32_t cycles, int
             float4* xb = tmp;
             for (int k = 0; k < pre; ++k) {
                 k_l0_sweep_rg<<<g0, kBlock, 0, st>>>(n0, l0.slice_ptr, l0.ell_col, l0.ell_val, l0.dfull, l0.dinv, xa, xb,
-                                                     rhs, h->b0, h->slot_ptr, h->slots, 0, nullptr);
+                                                     rhs, h->b0, h->slot_ptr, h->slots, 0);
                 std::swap(xa, xb);
             }
-            k_l0_residual_rg<<<g0, kBlock, 0, st>>>(n0, l0.slice_ptr, l0.ell_col, l0.ell_val, l0.dfull, xa, rhs, l0.res,
-                                                    nullptr);
+            k_l0_residual_rg<<<g0, kBlock, 0, st>>>(n0, l0.slice_ptr, l0.ell_col, l0.ell_val, l0.dfull, xa, rhs, l0.res);
             ca.d = xa;
             ca.gate = nullptr;
             TRY(launch_coarse(h, ca));
             k_l0_prolong<<<grid_for(n0), kBlock, 0, st>>>(n0, lv[1].pid, lv[1].pw, lv[1].e, xa, nullptr);
             for (int k = 0; k < post; ++k) {
                 k_l0_sweep_rg<<<g0, kBlock, 0, st>>>(n0, l0.slice_ptr, l0.ell_col, l0.ell_val, l0.dfull, l0.dinv, xa, xb,
-                                                     rhs, h->b0, h->slot_ptr, h->slots, 0, nullptr);
+                                                     rhs, h->b0, h->slot_ptr, h->slots, 0);
                 std::swap(xa, xb);
             }
             if (xa != e) CUDA_TRY(h, cudaMemcpyAsync(e, xa, (size_t)n0 * sizeof(float4), cudaMemcpyDeviceToDevice, st));
