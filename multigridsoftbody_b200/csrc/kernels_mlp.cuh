@@ -411,7 +411,7 @@ __global__ void __launch_bounds__(kMlpThreads) k_mlp_tc(int n, int ntiles, const
 // backward).  Loss = mean over samples and the 3 outputs of (y - t)^2.
 //
 // A step is a chain of two launches.  k_mlp_fwd_bwd takes 32 samples per CTA (a
-// sample per lane, 8 hidden units per warp) and leaves the rows that the weight
+// sample per lane, 4 hidden units per warp) and leaves the rows that the weight
 // gradients multiply -- features, dZ1, H1, dZ2, H2, dY -- in global scratch, a
 // row per unit over all samples.  k_mlp_grad gives each CTA a tile of
 // parameters: their rows arrive in shared memory by bulk copies, a thread forms
@@ -423,7 +423,8 @@ __global__ void __launch_bounds__(kMlpThreads) k_mlp_tc(int n, int ntiles, const
 // take 3.2 ms (the upload of the pairs included).  Every sum runs in the order of
 // that form: the same bits.
 // ---------------------------------------------------------------------------
-constexpr int kTrainThreads = 256;            // 8 warps of 8 hidden units each
+constexpr int kTrainThreads = 512;            // 16 warps of 4 hidden units each
+constexpr int kTrainUnits = 4;
 constexpr int kTrainSamples = 32;             // per CTA
 constexpr int kGradBlock = 128;               // samples of one dot product
 constexpr int kGradLd = kGradBlock + 4;       // its place in a scratch row: 16-byte reads of 8 blocks miss no bank
@@ -436,8 +437,8 @@ __host__ __device__ inline int train_blocks(int n) { return (n + kGradBlock - 1)
 
 struct TrainSmem {
     float w1[kMlpIn][kMlpHid];     // [k][j]
-    float w2t[kMlpHid][kMlpHid + 4];   // [k][j], forward (the transposing stores meet 4 to a bank)
-    float w2[kMlpHid][kMlpHid];    // [j][k], backward
+    float w2t[kMlpHid][kMlpHid + 4];   // [k][j], forward
+    float w2[kMlpHid][kMlpHid + 4];    // [j][k], backward
     float w3[kMlpOut][kMlpHid];
     float b1[kMlpHid], b2[kMlpHid], b3[kMlpOut + 1];
     float x[kMlpIn][kTrainSamples];
@@ -467,7 +468,7 @@ __global__ void __launch_bounds__(kTrainThreads) k_mlp_fwd_bwd(int nb, SampleOf 
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     extern __shared__ __align__(16) unsigned char train_smem[];
     TrainSmem& S = *reinterpret_cast<TrainSmem*>(train_smem);
-    const int s = threadIdx.x & 31, warp = threadIdx.x >> 5, j0 = 8 * warp;
+    const int s = threadIdx.x & 31, warp = threadIdx.x >> 5, j0 = kTrainUnits * warp;
     const int gs = blockIdx.x * kTrainSamples + s;
     const bool valid = gs < nb;
     // the samples are not written by any kernel of a training run: read before the wait
@@ -476,10 +477,21 @@ __global__ void __launch_bounds__(kTrainThreads) k_mlp_fwd_bwd(int nb, SampleOf 
     const float target = valid && warp < kMlpOut ? T[(size_t)row * kMlpOut + warp] : 0.f;
     asm volatile("griddepcontrol.wait;" ::: "memory");
     // weights, BF16-rounded, and exact biases
-    for (int q = threadIdx.x; q < kMlpHid * kMlpHid; q += kTrainThreads) {
-        const float w = bf16r(prm[kOffW2 + q]);
-        S.w2[q / kMlpHid][q % kMlpHid] = w;
-        S.w2t[q % kMlpHid][q / kMlpHid] = w;
+    {   // a thread per row of 64 and 4 columns at a time: the stores to both copies miss no bank
+        static_assert(kOffW2 % 4 == 0 && kTrainThreads == 8 * kMlpHid, "16-byte reads, 8 columns a thread");
+        const int j = threadIdx.x % kMlpHid, k0 = threadIdx.x / kMlpHid * 8;
+        const float4* from = reinterpret_cast<const float4*>(prm + kOffW2 + j * kMlpHid + k0);
+        const float4 q[2] = {from[0], from[1]};
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const float4 w = make_float4(bf16r(q[h].x), bf16r(q[h].y), bf16r(q[h].z), bf16r(q[h].w));
+            const int k = k0 + 4 * h;
+            *reinterpret_cast<float4*>(&S.w2[j][k]) = w;
+            S.w2t[k][j] = w.x;
+            S.w2t[k + 1][j] = w.y;
+            S.w2t[k + 2][j] = w.z;
+            S.w2t[k + 3][j] = w.w;
+        }
     }
     for (int q = threadIdx.x; q < kMlpHid * kMlpIn; q += kTrainThreads) S.w1[q % kMlpIn][q / kMlpIn] = bf16r(prm[kOffW1 + q]);
     if (threadIdx.x < kMlpOut * kMlpHid) S.w3[threadIdx.x / kMlpHid][threadIdx.x % kMlpHid] = bf16r(prm[kOffW3 + threadIdx.x]);
@@ -489,41 +501,40 @@ __global__ void __launch_bounds__(kTrainThreads) k_mlp_fwd_bwd(int nb, SampleOf 
     }
     if (threadIdx.x < kMlpOut) S.b3[threadIdx.x] = prm[kOffB3 + threadIdx.x];
     __syncthreads();
-    auto row8 = [](const float* p, float (&w)[8]) {
-        const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
+    auto row_units = [](const float* p, float (&w)[kTrainUnits]) {
+        const float4 a = *reinterpret_cast<const float4*>(p);
         w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w;
-        w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
     };
     // place of this sample in the scratch rows
     float* at = act + (size_t)(gs / kGradBlock) * kGradLd + gs % kGradBlock;
     for (int k = warp; k < kMlpIn; k += kTrainThreads / 32) at[(size_t)(kActX + k) * ld] = S.x[k][s];
     // ---- forward
-    float z1[8], z2[8], w[8];
-    row8(S.b1 + j0, z1);
+    float z1[kTrainUnits], z2[kTrainUnits], w[kTrainUnits];
+    row_units(S.b1 + j0, z1);
 #pragma unroll
     for (int k = 0; k < kMlpIn; ++k) {
-        row8(&S.w1[k][j0], w);
+        row_units(&S.w1[k][j0], w);
         const float x = S.x[k][s];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) z1[u] = fmaf(w[u], x, z1[u]);
+        for (int u = 0; u < kTrainUnits; ++u) z1[u] = fmaf(w[u], x, z1[u]);
     }
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
+    for (int u = 0; u < kTrainUnits; ++u) {
         const float h = bf16r(gelu(z1[u]));
         S.h1[j0 + u][s] = h;
         at[(size_t)(kActH1 + j0 + u) * ld] = h;
     }
     __syncthreads();
-    row8(S.b2 + j0, z2);
+    row_units(S.b2 + j0, z2);
 #pragma unroll 8
     for (int k = 0; k < kMlpHid; ++k) {
-        row8(&S.w2t[k][j0], w);
+        row_units(&S.w2t[k][j0], w);
         const float h = S.h1[k][s];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) z2[u] = fmaf(w[u], h, z2[u]);
+        for (int u = 0; u < kTrainUnits; ++u) z2[u] = fmaf(w[u], h, z2[u]);
     }
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
+    for (int u = 0; u < kTrainUnits; ++u) {
         const float h = bf16r(gelu(z2[u]));
         S.h2[j0 + u][s] = h;
         at[(size_t)(kActH2 + j0 + u) * ld] = h;
@@ -551,7 +562,7 @@ __global__ void __launch_bounds__(kTrainThreads) k_mlp_fwd_bwd(int nb, SampleOf 
     }
     // ---- backward through layers 3 and 2
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
+    for (int u = 0; u < kTrainUnits; ++u) {
         float a = 0.f;
 #pragma unroll
         for (int o = 0; o < kMlpOut; ++o) a = fmaf(S.dy[o][s], S.w3[o][j0 + u], a);
@@ -560,18 +571,18 @@ __global__ void __launch_bounds__(kTrainThreads) k_mlp_fwd_bwd(int nb, SampleOf 
         at[(size_t)(kActZ2 + j0 + u) * ld] = z;
     }
     __syncthreads();
-    float a1[8];
+    float a1[kTrainUnits];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) a1[u] = 0.f;
+    for (int u = 0; u < kTrainUnits; ++u) a1[u] = 0.f;
 #pragma unroll 8
     for (int j = 0; j < kMlpHid; ++j) {
-        row8(&S.w2[j][j0], w);
+        row_units(&S.w2[j][j0], w);
         const float z = S.z2[j][s];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) a1[u] = fmaf(z, w[u], a1[u]);
+        for (int u = 0; u < kTrainUnits; ++u) a1[u] = fmaf(z, w[u], a1[u]);
     }
 #pragma unroll
-    for (int u = 0; u < 8; ++u) at[(size_t)(kActZ1 + j0 + u) * ld] = a1[u] * gelu_grad(z1[u]);
+    for (int u = 0; u < kTrainUnits; ++u) at[(size_t)(kActZ1 + j0 + u) * ld] = a1[u] * gelu_grad(z1[u]);
 }
 
 // Adam (Kingma & Ba 2015) on one FP32 master parameter.
