@@ -47,47 +47,38 @@ struct BodyDev {
 
 // calculateST (PDSolver.cu:72-116); external force is always zero in the
 // reference's frame and is omitted.
+struct RefPredict {
+    float damping, gx, gy, gz;
+};
+__device__ __forceinline__ void ref_predict(float4& p, float4& vel, float fix, const RefPredict& a, float dt) {
+    vel.x *= a.damping * fix; vel.y *= a.damping * fix; vel.z *= a.damping * fix;
+    vel.x += a.gx * dt * fix; vel.y += a.gy * dt * fix; vel.z += a.gz * dt * fix;
+    p.x += vel.x * dt * fix; p.y += vel.y * dt * fix; p.z += vel.z * dt * fix;
+}
 __global__ void k_ref_predict(int n, float4* __restrict__ x, float4* __restrict__ v, float4* __restrict__ s,
                               float4* __restrict__ prev, float4* __restrict__ last, const float* __restrict__ fixf,
-                              float damping, float dt, float gx, float gy, float gz) {
+                              RefPredict a, float dt) {
     pdl_enter();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     float4 p = x[i], vel = v[i];
     last[i] = p;
-    const float fix = fixf[i];
-    vel.x *= damping * fix; vel.y *= damping * fix; vel.z *= damping * fix;
-    vel.x += gx * dt * fix; vel.y += gy * dt * fix; vel.z += gz * dt * fix;
-    p.x += vel.x * dt * fix; p.y += vel.y * dt * fix; p.z += vel.z * dt * fix;
+    ref_predict(p, vel, fixf[i], a, dt);
     x[i] = p;
     v[i] = vel;
     s[i] = p;
     prev[i] = p;
 }
 
-// Local step, one thread per tet: F = Ds Dm^-1, R by the invariant polar
+// A tet's local step: F = Ds Dm^-1, R by the invariant polar
 // decomposition, per (i,j): val = sum_k (R-F)_ik Ac_kj, NaN->0, clamp +-10,
-// c = val*V*k, |c| < 1e-5 dropped (PDSolverAc.cu:447-662).  The four corner
-// contributions go to their RHS slots (float4 each).
-__global__ void __launch_bounds__(256) k_ref_local(int T, const int4* __restrict__ tets, const float4* __restrict__ invA,
-                                                   const float4* __restrict__ invB, const float2* __restrict__ invC,
-                                                   const float4* __restrict__ x, const int4* __restrict__ slot_of,
-                                                   float4* __restrict__ slots, float stiffness, int drop_small = 1) {
-    pdl_trigger();
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= T) {
-        pdl_wait();
-        return;
-    }
-    // the tet's set-up data is written by no kernel: loaded before the dependency wait
-    const int4 id = __ldg(tets + t);
-    const float4 a = __ldg(invA + t), b = __ldg(invB + t);
-    const float2 c = __ldg(invC + t);
-    const int4 so = __ldg(slot_of + t);
-    pdl_wait();
+// c = val*V*k, |c| < 1e-5 dropped (PDSolverAc.cu:447-662).  out: the four
+// corners' contributions.  a, b, c: Dm^-1 by rows and the volume.
+__device__ __forceinline__ void ref_tet(const float4 a, const float4 b, const float2 c, const float4 p0, const float4 p1,
+                                        const float4 p2, const float4 p3, float stiffness, int drop_small,
+                                        float4 (&out4)[4]) {
     const float inv[9] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, c.x};
     const float vol = c.y;
-    const float4 p0 = __ldg(x + id.x), p1 = __ldg(x + id.y), p2 = __ldg(x + id.z), p3 = __ldg(x + id.w);
     const float D[9] = {p1.x - p0.x, p2.x - p0.x, p3.x - p0.x, p1.y - p0.y, p2.y - p0.y,
                         p3.y - p0.y, p1.z - p0.z, p2.z - p0.z, p3.z - p0.z};
     float F[9];
@@ -109,7 +100,6 @@ __global__ void __launch_bounds__(256) k_ref_local(int T, const int4* __restrict
         Ac[r * 4 + 2] = inv[r + 3];
         Ac[r * 4 + 3] = inv[r + 6];
     }
-    const int sid[4] = {so.x, so.y, so.z, so.w};
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         float out[3];
@@ -124,13 +114,103 @@ __global__ void __launch_bounds__(256) k_ref_local(int T, const int4* __restrict
             if (drop_small && (double)fabsf(res) < 1e-5) res = 0.f;
             out[i] = res;
         }
-        slots[sid[j]] = make_float4(out[0], out[1], out[2], 0.f);
+        out4[j] = make_float4(out[0], out[1], out[2], 0.f);
     }
 }
 
-// Per vertex: gather the elastic force from the slots, sphere DCD
-// (DCDByPoint_sphere, PDSolver.cu:277-331), then the under-relaxed Jacobi
-// step with Chebyshev acceleration (calculatePOS, PDSolver.cu:192-235).
+// Local step, one thread per tet: the corners' contributions go to their RHS slots (float4 each).
+__global__ void __launch_bounds__(256) k_ref_local(int T, const int4* __restrict__ tets, const float4* __restrict__ invA,
+                                                   const float4* __restrict__ invB, const float2* __restrict__ invC,
+                                                   const float4* __restrict__ x, const int4* __restrict__ slot_of,
+                                                   float4* __restrict__ slots, float stiffness, int drop_small = 1) {
+    pdl_trigger();
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= T) {
+        pdl_wait();
+        return;
+    }
+    // the tet's set-up data is written by no kernel: loaded before the dependency wait
+    const int4 id = __ldg(tets + t);
+    const float4 a = __ldg(invA + t), b = __ldg(invB + t);
+    const float2 c = __ldg(invC + t);
+    const int4 so = __ldg(slot_of + t);
+    pdl_wait();
+    float4 out[4];
+    ref_tet(a, b, c, __ldg(x + id.x), __ldg(x + id.y), __ldg(x + id.z), __ldg(x + id.w), stiffness, drop_small, out);
+    slots[so.x] = out[0];
+    slots[so.y] = out[1];
+    slots[so.z] = out[2];
+    slots[so.w] = out[3];
+}
+
+// What the vertex step finds of contact.
+struct RefContact {
+    float cd[3] = {0.f, 0.f, 0.f}, cf[3] = {0.f, 0.f, 0.f};   // diagonal and force
+    int flag = 0;
+    float depth = 0.f, energy = 0.f;
+};
+
+// Sphere DCD of a vertex at p (DCDByPoint_sphere, PDSolver.cu:277-331).
+__device__ __forceinline__ void ref_contact(const float4 p4, RefContact& c, const SphereSet* spheres, float kc) {
+    const float p[3] = {p4.x, p4.y, p4.z};
+    float(&cd)[3] = c.cd;
+    float(&cf)[3] = c.cf;
+    const int nsph = spheres->count;
+    for (int q = 0; q < nsph; ++q) {
+        if (!spheres->active[q]) continue;
+        const float cx = spheres->cx[q], cy = spheres->cy[q], cz = spheres->cz[q];
+        float radius = spheres->r[q];
+        const float cp[3] = {p[0] - cx, p[1] - cy, p[2] - cz};
+        const float len = sqrtf(cp[0] * cp[0] + cp[1] * cp[1] + cp[2] * cp[2]);
+        const float dir[3] = {cp[0] / len, cp[1] / len, cp[2] / len};
+        const float distance = len;
+        const float oldRadius = radius;
+        radius *= 1.5f;
+        if (distance < radius) {
+            const float bq = 2 * (cp[0] * dir[0] + cp[1] * dir[1] + cp[2] * dir[2]);
+            const float cq = (cp[0] * cp[0] + cp[1] * cp[1] + cp[2] * cp[2]) - radius * radius;
+            float t = (-bq + sqrtf(bq * bq - 4 * 1 * cq)) / (2 * 1);
+            if (t > 0.5f * oldRadius) {
+                c.flag = 1;
+                c.depth = t - 0.5f * oldRadius;
+            }
+            t = t / 2.0f;
+            const float colP[3] = {p[0] + dir[0] * t, p[1] + dir[1] * t, p[2] + dir[2] * t};
+            const float cc[3] = {colP[0] - cx, colP[1] - cy, colP[2] - cz};
+            const float lc = sqrtf(cc[0] * cc[0] + cc[1] * cc[1] + cc[2] * cc[2]);
+            const float nrm[3] = {cc[0] / lc, cc[1] / lc, cc[2] / lc};
+            const float ndd = nrm[0] * dir[0] + nrm[1] * dir[1] + nrm[2] * dir[2];
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                cd[a] += kc * nrm[a] * nrm[a];
+                cf[a] += kc * t * ndd * nrm[a];
+            }
+            const float pe = (p[0] - colP[0]) * nrm[0] + (p[1] - colP[1]) * nrm[1] + (p[2] - colP[2]) * nrm[2];
+            c.energy += kc * pe * pe;
+        }
+    }
+}
+
+// The under-relaxed Jacobi step with Chebyshev acceleration of a vertex at p with elastic force f (calculatePOS,
+// PDSolver.cu:192-235).
+__device__ __forceinline__ float4 ref_vertex(const float4 p4, const float4 s4, const float4 pv4, const float4 f,
+                                             const RefContact& c, float dc, float vd, float fix, float omega, double relax) {
+    const float p[3] = {p4.x, p4.y, p4.z};
+    const float sv[3] = {s4.x, s4.y, s4.z}, pv[3] = {pv4.x, pv4.y, pv4.z};
+    const float fe[3] = {f.x, f.y, f.z};
+    float nx[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const float el = fe[a] + c.cf[a];
+        float nxt = (dc * (sv[a] - p[a]) + el) / (vd + c.cd[a] + dc) * fix + p[a];
+        nxt = (float)((double)(nxt - p[a]) * relax + (double)p[a]);
+        nxt = omega * (nxt - pv[a]) + pv[a];
+        nx[a] = nxt;
+    }
+    return make_float4(nx[0], nx[1], nx[2], 0.f);
+}
+
+// Per vertex: gather the elastic force from the slots, contact, then ref_vertex.
 // On the last iteration also v = (x - last)/dt (calculateV, PDSolver.cu:245).
 // Latency bound: what no kernel of a frame writes (the slots' place, mass,
 // diagonal, fix flag; the spheres, copied before the frame) is read before the
@@ -166,10 +246,7 @@ __global__ void __launch_bounds__(kRefVertexThreads) k_ref_vertex(
         const float4 c = __ldg(slots + e);
         fx += c.x; fy += c.y; fz += c.z;
     }
-    const float p[3] = {p4.x, p4.y, p4.z};
-    float cd[3] = {0.f, 0.f, 0.f}, cf[3] = {0.f, 0.f, 0.f};
-    int flag = 0;
-    float depth = 0.f, ce = 0.f;
+    RefContact ct;
     if (tri_push) {
         // collision from the surface triangles around this vertex (the coarse level of
         // the two-level schedule): k_c per contact on every axis, k_c (c - hit) as force
@@ -182,59 +259,16 @@ __global__ void __launch_bounds__(kRefVertexThreads) k_ref_vertex(
             mz += q.z;
             cnt += q.w;
         }
-        cd[0] = cd[1] = cd[2] = kc * cnt;
-        cf[0] = kc * mx;
-        cf[1] = kc * my;
-        cf[2] = kc * mz;
-        flag = (int)cnt;
+        ct.cd[0] = ct.cd[1] = ct.cd[2] = kc * cnt;
+        ct.cf[0] = kc * mx;
+        ct.cf[1] = kc * my;
+        ct.cf[2] = kc * mz;
+        ct.flag = (int)cnt;
+    } else {
+        ref_contact(p4, ct, spheres, kc);
     }
-    const int nsph = tri_push ? 0 : spheres->count;
-    for (int q = 0; q < nsph; ++q) {
-        if (!spheres->active[q]) continue;
-        const float cx = spheres->cx[q], cy = spheres->cy[q], cz = spheres->cz[q];
-        float radius = spheres->r[q];
-        const float cp[3] = {p[0] - cx, p[1] - cy, p[2] - cz};
-        const float len = sqrtf(cp[0] * cp[0] + cp[1] * cp[1] + cp[2] * cp[2]);
-        const float dir[3] = {cp[0] / len, cp[1] / len, cp[2] / len};
-        const float distance = len;
-        const float oldRadius = radius;
-        radius *= 1.5f;
-        if (distance < radius) {
-            const float bq = 2 * (cp[0] * dir[0] + cp[1] * dir[1] + cp[2] * dir[2]);
-            const float cq = (cp[0] * cp[0] + cp[1] * cp[1] + cp[2] * cp[2]) - radius * radius;
-            float t = (-bq + sqrtf(bq * bq - 4 * 1 * cq)) / (2 * 1);
-            if (t > 0.5f * oldRadius) {
-                flag = 1;
-                depth = t - 0.5f * oldRadius;
-            }
-            t = t / 2.0f;
-            const float colP[3] = {p[0] + dir[0] * t, p[1] + dir[1] * t, p[2] + dir[2] * t};
-            const float cc[3] = {colP[0] - cx, colP[1] - cy, colP[2] - cz};
-            const float lc = sqrtf(cc[0] * cc[0] + cc[1] * cc[1] + cc[2] * cc[2]);
-            const float nrm[3] = {cc[0] / lc, cc[1] / lc, cc[2] / lc};
-            const float ndd = nrm[0] * dir[0] + nrm[1] * dir[1] + nrm[2] * dir[2];
-#pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                cd[a] += kc * nrm[a] * nrm[a];
-                cf[a] += kc * t * ndd * nrm[a];
-            }
-            const float pe = (p[0] - colP[0]) * nrm[0] + (p[1] - colP[1]) * nrm[1] + (p[2] - colP[2]) * nrm[2];
-            ce += kc * pe * pe;
-        }
-    }
-    const float sv[3] = {s4.x, s4.y, s4.z}, pv[3] = {pv4.x, pv4.y, pv4.z};
-    const float fe[3] = {fx, fy, fz};
-    float nx[3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        const float el = fe[a] + cf[a];
-        float nxt = (dc * (sv[a] - p[a]) + el) / (vd + cd[a] + dc) * fix + p[a];
-        nxt = (float)((double)(nxt - p[a]) * relax + (double)p[a]);
-        nxt = omega * (nxt - pv[a]) + pv[a];
-        nx[a] = nxt;
-    }
+    const float4 xn = ref_vertex(p4, s4, pv4, make_float4(fx, fy, fz, 0.f), ct, dc, vd, fix, omega, relax);
     prev[i] = p4;
-    const float4 xn = make_float4(nx[0], nx[1], nx[2], 0.f);
     x[i] = xn;
     // last_iter: bit 0 = velocity, bit 1 = contact outputs and the finiteness check
     if (last_iter & 1) {
@@ -242,9 +276,9 @@ __global__ void __launch_bounds__(kRefVertexThreads) k_ref_vertex(
         v[i] = make_float4((xn.x - l4.x) / dt, (xn.y - l4.y) / dt, (xn.z - l4.z) / dt, 0.f);
     }
     if (last_iter & 2) {
-        cflag[i] = flag;
-        cdepth[i] = depth;
-        cenergy[i] = ce;
+        cflag[i] = ct.flag;
+        cdepth[i] = ct.depth;
+        cenergy[i] = ct.energy;
         if (!isfinite(xn.x) || !isfinite(xn.y) || !isfinite(xn.z)) atomicOr(nonfinite, 1);
     }
 }

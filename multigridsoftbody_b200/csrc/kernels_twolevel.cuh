@@ -18,13 +18,7 @@ namespace mgsb {
 // triangle's sum and counts 1.  The reference scatters k_c and k_c (c - hit)
 // into the three vertices with float atomics (PDSolver.cu:462-501); here the
 // vertex kernel gathers the per-triangle sums through a vertex->triangle CSR.
-__global__ void __launch_bounds__(256) k_ref_tri_dcd(int nf, const int4* __restrict__ tris, const float4* __restrict__ x,
-                                                     const SphereSet* __restrict__ spheres, float4* __restrict__ push) {
-    pdl_enter();
-    const int f = blockIdx.x * blockDim.x + threadIdx.x;
-    if (f >= nf) return;
-    const int4 t = __ldg(tris + f);
-    const float4 a4 = x[t.x], b4 = x[t.y], c4 = x[t.z];
+__device__ __forceinline__ float4 ref_tri_push(const float4 a4, const float4 b4, const float4 c4, const SphereSet* spheres) {
     const float V[3][3] = {{a4.x, a4.y, a4.z}, {b4.x, b4.y, b4.z}, {c4.x, c4.y, c4.z}};
     const float* A = V[0];
     float n[3];
@@ -115,7 +109,16 @@ __global__ void __launch_bounds__(256) k_ref_tri_dcd(int nf, const int4* __restr
         mz += ctr[2] - hit[2];
         cnt += 1.f;
     }
-    push[f] = make_float4(mx, my, mz, cnt);
+    return make_float4(mx, my, mz, cnt);
+}
+
+__global__ void __launch_bounds__(256) k_ref_tri_dcd(int nf, const int4* __restrict__ tris, const float4* __restrict__ x,
+                                                     const SphereSet* __restrict__ spheres, float4* __restrict__ push) {
+    pdl_enter();
+    const int f = blockIdx.x * blockDim.x + threadIdx.x;
+    if (f >= nf) return;
+    const int4 t = __ldg(tris + f);
+    push[f] = ref_tri_push(x[t.x], x[t.y], x[t.z], spheres);
 }
 
 // x = prev = sum_k w_k src[id_k] (updatePointInTet, PDSolver.cu:724-743): the

@@ -20,6 +20,7 @@
 #include "kernels_mg.cuh"
 #include "kernels_mixed.cuh"
 #include "kernels_contact.cuh"
+#include "kernels_refcluster.cuh"
 #include "mesh.hpp"
 #include "mlp.hpp"
 #include "plan.hpp"
@@ -147,6 +148,11 @@ struct mgsb_solver {
     float4 *tA = nullptr, *tB = nullptr;
     float2* tC = nullptr;
     int4* slot_of = nullptr;
+    // reference kind: k_ref_iterations' layout (bytes 0: the body does not take it), and the surface triangles of the
+    // two-level schedule's coarse level, with the triangles of each vertex
+    RefPlan ref{};
+    std::vector<int4> ref_tris;
+    std::vector<int32_t> ref_tri_ptr, ref_tri_idx;
     int32_t* slot_ptr = nullptr;
     float4* slots = nullptr;
     // multigrid: the local step's blocks, and the mixed kind's slots
@@ -527,6 +533,177 @@ mgsb_status upload_normals_data(mgsb_solver* h, std::vector<DevMem>& pool) {
 // ---------------------------------------------------------------------------
 // Derived data (rebuilt when fixed set / material / params change)
 // ---------------------------------------------------------------------------
+// Layout and images of k_ref_iterations, for a body small enough that a CTA's share of the tets takes less than the two
+// launches that it replaces, over 16 CTAs (8 if the device cannot schedule 16).
+// Frames of 20 iterations with it and with its launches: 57 and 119 us at 375 vertices, 62 and 124 at 1,025, 98 and 145
+// at 2,009, 126 and 159 at 2,989, 159 and 165 at 4,050.
+constexpr int kRefClusterVerts = 3500;
+
+mgsb_status plan_ref(mgsb_solver* h, std::vector<DevMem>& pool, const Plan& P) {
+    h->ref = RefPlan{};
+    const int n = P.N0, T = P.T;
+    if (n > kRefClusterVerts || h->bodies.size() != 1 || h->p.iterations < 1) return MGSB_OK;
+    const int nf = (int)h->ref_tris.size();
+    int most_smem = 0;
+    CUDA_TRY(h, cudaDeviceGetAttribute(&most_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device));
+    CUDA_TRY(h, cudaFuncSetAttribute(k_ref_iterations, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    CUDA_TRY(h, cudaFuncSetAttribute(k_ref_iterations, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     most_smem - kStagedStaticSmem));
+    struct Part {
+        int first = 0, own = 0, lo = 0, hi = 0;
+        std::vector<int> tets, tris;
+    };
+    for (int cs : {16, 8}) {
+        const int per = (n + cs - 1) / cs;
+        if (per > kRefThreads) continue;
+        std::vector<Part> part(cs);
+        for (int k = 0; k < cs; ++k) {
+            part[k].first = part[k].lo = std::min(n, k * per);
+            part[k].hi = std::min(n, (k + 1) * per);
+            part[k].own = part[k].hi - part[k].first;
+        }
+        auto share = [&](int id, const int* c, int nc, std::vector<int> Part::*list) {   // to every CTA that owns a corner
+            for (int a = 0; a < nc; ++a) {
+                Part& o = part[c[a] / per];
+                if (!(o.*list).empty() && (o.*list).back() == id) continue;
+                (o.*list).push_back(id);
+                for (int b = 0; b < nc; ++b) {
+                    o.lo = std::min(o.lo, c[b]);
+                    o.hi = std::max(o.hi, c[b] + 1);
+                }
+            }
+        };
+        for (int t = 0; t < T; ++t) {
+            const int c[4] = {P.tets[t].x, P.tets[t].y, P.tets[t].z, P.tets[t].w};
+            share(t, c, 4, &Part::tets);
+        }
+        for (int f = 0; f < nf; ++f) {
+            const int c[3] = {h->ref_tris[f].x, h->ref_tris[f].y, h->ref_tris[f].z};
+            share(f, c, 3, &Part::tris);
+        }
+        // contributions of each vertex, tets ascending
+        std::vector<int> deg(n, 0);
+        int depth = 0;
+        for (int t = 0; t < T; ++t)
+            for (int c : {P.tets[t].x, P.tets[t].y, P.tets[t].z, P.tets[t].w}) depth = std::max(depth, ++deg[c]);
+        size_t tets = 0, tris = 0, win = 0, refs = 0;
+        for (const Part& o : part) {
+            tets = std::max(tets, o.tets.size());
+            tris = std::max(tris, o.tris.size());
+            win = std::max(win, (size_t)(o.hi - o.lo));
+            if (nf) refs = std::max(refs, (size_t)(h->ref_tri_ptr[o.first + o.own] - h->ref_tri_ptr[o.first]));
+        }
+        if ((size_t)depth * per >= 0xffff || tris > 0xffff || refs > 0xffff) continue;
+        RefPlan q{};
+        size_t bytes = sizeof(RefHead);
+        auto room = [&](size_t b) {
+            const size_t a = bytes;
+            bytes += (b + 15) / 16 * 16;
+            return (int)std::min<size_t>(a, 1u << 30);
+        };
+        q.inv_a = room(16 * tets);
+        q.inv_b = room(16 * tets);
+        q.inv_c = room(8 * tets);
+        q.corner = room(8 * tets);
+        q.slot = room(8 * tets);
+        q.deg = room(2 * per);
+        q.to = room(2 * per);
+        q.tri = room(8 * tris);
+        q.tri_ptr = room(2 * (per + 1));
+        q.tri_idx = room(2 * refs);
+        const size_t image = bytes;
+        q.win[0] = room(16 * win);
+        q.win[1] = room(16 * win);
+        q.slots = room((size_t)16 * depth * per);
+        q.push = room(16 * tris);
+        if (bytes > (size_t)(most_smem - kStagedStaticSmem)) continue;
+        q.image_bytes = (int)image;
+        q.stride = per;
+        q.bytes = (int)bytes;
+        q.cluster = cs;
+        q.block = (int)std::min<size_t>(kRefThreads, (std::max<size_t>(tets, 32) + 31) / 32 * 32 + ((size_t)per + 31) / 32 * 32);
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)cs);
+        cfg.blockDim = dim3((unsigned)q.block);
+        cfg.dynamicSmemBytes = bytes;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)cs;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int nclusters = 0;
+        if (cudaOccupancyMaxActiveClusters(&nclusters, k_ref_iterations, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            continue;
+        }
+        if (nclusters < 1) continue;
+        std::vector<unsigned char> img((size_t)cs * image, 0);
+        std::vector<int> fill(n, 0), at(std::max(nf, 1), 0);
+        for (int k = 0; k < cs; ++k) {
+            const Part& o = part[k];
+            unsigned char* m = img.data() + (size_t)k * image;
+            RefHead head{};
+            head.tets = (int)o.tets.size();
+            head.own = o.own;
+            head.first = o.first;
+            head.tris = (int)o.tris.size();
+            head.win_lo = o.lo;
+            head.win_n = o.hi - o.lo;
+            for (int j = 0; j < cs; ++j) head.peer_lo[j] = part[j].lo;
+            std::memcpy(m, &head, sizeof head);
+            for (int r = 0; r < head.tets; ++r) {
+                const int t = o.tets[r], c[4] = {P.tets[t].x, P.tets[t].y, P.tets[t].z, P.tets[t].w};
+                uint16_t corner[4], slot[4];
+                for (int a = 0; a < 4; ++a) {
+                    const int v = c[a] - o.first;
+                    corner[a] = (uint16_t)(c[a] - o.lo);
+                    slot[a] = v >= 0 && v < o.own ? (uint16_t)(fill[c[a]]++ * per + v) : (uint16_t)0xffff;
+                }
+                reinterpret_cast<float4*>(m + q.inv_a)[r] = P.tA[t];
+                reinterpret_cast<float4*>(m + q.inv_b)[r] = P.tB[t];
+                reinterpret_cast<float2*>(m + q.inv_c)[r] = P.tC[t];
+                std::memcpy(m + q.corner + 8 * r, corner, 8);
+                std::memcpy(m + q.slot + 8 * r, slot, 8);
+            }
+            for (int v = 0; v < o.own; ++v) {
+                const int i = o.first + v;
+                uint32_t to = 0;
+                for (int j = 0; j < cs; ++j)
+                    if (i >= part[j].lo && i < part[j].hi) to |= 1u << j;
+                reinterpret_cast<uint16_t*>(m + q.deg)[v] = (uint16_t)deg[i];
+                reinterpret_cast<uint16_t*>(m + q.to)[v] = (uint16_t)to;
+            }
+            for (int r = 0; r < head.tris; ++r) {
+                const int4 f = h->ref_tris[o.tris[r]];
+                const uint16_t c[4] = {(uint16_t)(f.x - o.lo), (uint16_t)(f.y - o.lo), (uint16_t)(f.z - o.lo), 0};
+                std::memcpy(m + q.tri + 8 * r, c, 8);
+                at[o.tris[r]] = r;
+            }
+            if (nf)
+                for (int v = 0, e = 0; v <= o.own; ++v) {
+                    reinterpret_cast<uint16_t*>(m + q.tri_ptr)[v] = (uint16_t)e;
+                    if (v == o.own) break;
+                    for (int b = h->ref_tri_ptr[o.first + v]; b < h->ref_tri_ptr[o.first + v + 1]; ++b)
+                        reinterpret_cast<uint16_t*>(m + q.tri_idx)[e++] = (uint16_t)at[h->ref_tri_idx[b]];
+                }
+        }
+        std::vector<float> omega(h->p.iterations);
+        float w = 1.0f;
+        for (float& o : omega) o = w = 4 / (4 - h->p.cheb_rho * h->p.cheb_rho * w);
+        unsigned char* dimg = nullptr;
+        float* dom = nullptr;
+        TRY(dupload(h, pool, &dimg, img));
+        TRY(dupload(h, pool, &dom, omega));
+        q.image = dimg;
+        q.omega = dom;
+        h->ref = q;
+        return MGSB_OK;
+    }
+    return MGSB_OK;
+}
+
 mgsb_status rebuild(mgsb_solver* h) {
     CUDA_TRY(h, cudaSetDevice(h->device));
     CUDA_TRY(h, cudaStreamSynchronize(h->stream));
@@ -588,6 +765,7 @@ mgsb_status rebuild(mgsb_solver* h) {
         h->local_blocks = (int)P.lblock.size();
     } else {
         TRY(dupload(h, pool, &h->slot_of, P.slot_of));
+        TRY(plan_ref(h, pool, P));
     }
     h->h_inv = P.h_inv;
     h->h_ac = P.h_ac;
@@ -874,22 +1052,74 @@ void launch_kernel(mgsb_solver* h, void (*kernel)(KArgs...), dim3 grid, int bloc
         ++(h)->launches;                                                             \
     } while (0)
 
-void enqueue_ref_frame(mgsb_solver* h) {
+// The iterations of a reference-faithful frame.  drop_small: of k_ref_local; last_iter: of k_ref_vertex.  tris: contact
+// with the surface triangles, whose pushes go to push (else with the vertices).  predict (cluster kernel only): the
+// frame's prediction first.
+struct RefTris {
+    int n = 0;
+    const int4* tris = nullptr;
+    const int32_t *ptr = nullptr, *idx = nullptr;
+    float4* push = nullptr;
+};
+
+void enqueue_ref_iterations(mgsb_solver* h, int drop_small, int last_iter, const RefTris& tris, const RefPredict* predict) {
     const int n = h->N0, T = h->T;
     const mgsb_params& p = h->p;
-    const BodyHost& B = h->bodies[0];
-    LAUNCH(h, k_ref_predict, grid_for(n), kBlock, 0, n, h->x, h->v, h->s, h->prev, h->last, h->fixf, B.damping, p.dt,
-           B.gravity[0], B.gravity[1], B.gravity[2]);
+    if (h->ref.bytes) {
+        const RefPlan& q = h->ref;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)q.cluster);
+        cfg.blockDim = dim3((unsigned)q.block);
+        cfg.dynamicSmemBytes = (size_t)q.bytes;
+        cfg.stream = h->stream;
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)q.cluster;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = h->pdl ? 2 : 1;
+        const int reps = prof_begin(h, "k_ref_iterations");
+        cudaError_t e = cudaSuccess;
+        for (int r = 0; r < reps && e == cudaSuccess; ++r)
+            e = cudaLaunchKernelEx(&cfg, k_ref_iterations, q, (int)p.iterations, predict ? 1 : 0,
+                                   predict ? *predict : RefPredict{}, h->x, h->prev, h->s, h->last, h->v, (const float*)h->fixf, (const float*)h->mass,
+                                   (const float*)h->vdiag, (const SphereSet*)h->spheres_dev, p.volume_stiffness, drop_small,
+                                   p.collision_stiffness, p.dt, (double)p.relaxation, tris.push ? 1 : 0, last_iter, h->cflag,
+                                   h->cdepth, h->cenergy, h->nonfinite);
+        prof_end(h, "k_ref_iterations");
+        ++h->launches;
+        if (e != cudaSuccess && h->enqueue_status == MGSB_OK)
+            h->enqueue_status = set_err(h, MGSB_CUDA_ERROR, "reference iterations launch failed: %s", cudaGetErrorString(e));
+        return;
+    }
     float omega = 1.0f;
     for (int it = 0; it < p.iterations; ++it) {
         LAUNCH(h, k_ref_local, grid_for(T), kBlock, 0, T, h->tets, h->tA, h->tB, h->tC, h->x, h->slot_of, h->slots,
-               p.volume_stiffness, 1);
+               p.volume_stiffness, drop_small);
+        if (tris.n)
+            LAUNCH(h, k_ref_tri_dcd, grid_for(tris.n), kBlock, 0, tris.n, tris.tris, h->x, h->spheres_dev, tris.push);
         omega = 4 / (4 - p.cheb_rho * p.cheb_rho * omega);
         LAUNCH(h, k_ref_vertex, grid_ref_vertex(n), kRefVertexThreads, 0, n, h->x, h->prev, h->s, h->last, h->v, h->fixf, h->mass,
                h->vdiag, h->slot_ptr, h->slots, h->spheres_dev, p.collision_stiffness, p.dt, omega,
-               (double)p.relaxation, it == p.iterations - 1 ? 3 : 0, h->cflag, h->cdepth, h->cenergy,
-               h->nonfinite, nullptr, nullptr, nullptr);
+               (double)p.relaxation, it == p.iterations - 1 ? last_iter : 0, h->cflag, h->cdepth, h->cenergy,
+               h->nonfinite, tris.ptr, tris.idx, tris.push);
     }
+}
+
+void enqueue_ref_frame(mgsb_solver* h) {
+    const int n = h->N0;
+    const mgsb_params& p = h->p;
+    const BodyHost& B = h->bodies[0];
+    const RefPredict a{B.damping, B.gravity[0], B.gravity[1], B.gravity[2]};
+    if (h->ref.bytes) {
+        enqueue_ref_iterations(h, 1, 3, RefTris{}, &a);
+        return;
+    }
+    LAUNCH(h, k_ref_predict, grid_for(n), kBlock, 0, n, h->x, h->v, h->s, h->prev, h->last, h->fixf, a, p.dt);
+    enqueue_ref_iterations(h, 1, 3, RefTris{}, nullptr);
     if (p.iterations == 0) {
         // velocity only
         LAUNCH(h, k_velocity, grid_for(n), kBlock, 0, n, h->x, h->last, h->v, p.dt, h->nonfinite);
@@ -3623,32 +3853,13 @@ void enqueue_two_level_frame(mgsb_two_level* t) {
     C->launches = F->launches = 0;
     const BodyHost& BC = C->bodies[0];
     const BodyHost& BF = F->bodies[0];
-    LAUNCH(C, k_ref_predict, grid_for(t->nc), kBlock, 0, t->nc, C->x, C->v, C->s, C->prev, C->last, C->fixf, BC.damping,
-           pc.dt, BC.gravity[0], BC.gravity[1], BC.gravity[2]);
-    LAUNCH(F, k_ref_predict, grid_for(t->nf), kBlock, 0, t->nf, F->x, F->v, F->s, F->prev, F->last, F->fixf, BF.damping,
-           pf.dt, BF.gravity[0], BF.gravity[1], BF.gravity[2]);
-    float omega = 1.0f;
-    for (int it = 0; it < pc.iterations; ++it) {
-        LAUNCH(C, k_ref_local, grid_for(C->T), kBlock, 0, C->T, C->tets, C->tA, C->tB, C->tC, C->x, C->slot_of, C->slots,
-               pc.volume_stiffness, 0);
-        LAUNCH(C, k_ref_tri_dcd, grid_for(t->ntri), kBlock, 0, t->ntri, t->tris, C->x, C->spheres_dev, t->push);
-        omega = 4 / (4 - pc.cheb_rho * pc.cheb_rho * omega);
-        LAUNCH(C, k_ref_vertex, grid_ref_vertex(t->nc), kRefVertexThreads, 0, t->nc, C->x, C->prev, C->s, C->last, C->v, C->fixf, C->mass,
-               C->vdiag, C->slot_ptr, C->slots, C->spheres_dev, pc.collision_stiffness, pc.dt, omega,
-               (double)pc.relaxation, it == pc.iterations - 1 ? 2 : 0, C->cflag, C->cdepth, C->cenergy, C->nonfinite,
-               t->tri_ptr, t->tri_idx, t->push);
-    }
+    const RefPredict ac{BC.damping, BC.gravity[0], BC.gravity[1], BC.gravity[2]};
+    const RefPredict af{BF.damping, BF.gravity[0], BF.gravity[1], BF.gravity[2]};
+    LAUNCH(C, k_ref_predict, grid_for(t->nc), kBlock, 0, t->nc, C->x, C->v, C->s, C->prev, C->last, C->fixf, ac, pc.dt);
+    LAUNCH(F, k_ref_predict, grid_for(t->nf), kBlock, 0, t->nf, F->x, F->v, F->s, F->prev, F->last, F->fixf, af, pf.dt);
+    enqueue_ref_iterations(C, 0, 2, RefTris{t->ntri, t->tris, t->tri_ptr, t->tri_idx, t->push}, nullptr);
     LAUNCH(F, k_tl_transfer, grid_for(t->nf), kBlock, 0, t->nf, t->f_ids, t->f_w, C->x, F->x, F->prev);
-    omega = 1.0f;
-    for (int it = 0; it < pf.iterations; ++it) {
-        LAUNCH(F, k_ref_local, grid_for(F->T), kBlock, 0, F->T, F->tets, F->tA, F->tB, F->tC, F->x, F->slot_of, F->slots,
-               pf.volume_stiffness, 0);
-        omega = 4 / (4 - pf.cheb_rho * pf.cheb_rho * omega);
-        LAUNCH(F, k_ref_vertex, grid_ref_vertex(t->nf), kRefVertexThreads, 0, t->nf, F->x, F->prev, F->s, F->last, F->v, F->fixf, F->mass,
-               F->vdiag, F->slot_ptr, F->slots, F->spheres_dev, pf.collision_stiffness, pf.dt, omega,
-               (double)pf.relaxation, it == pf.iterations - 1 ? 2 : 0, F->cflag, F->cdepth, F->cenergy, F->nonfinite,
-               nullptr, nullptr, nullptr);
-    }
+    enqueue_ref_iterations(F, 0, 2, RefTris{}, nullptr);
     LAUNCH(C, k_tl_transfer, grid_for(t->nc), kBlock, 0, t->nc, t->c_ids, t->c_w, F->x, C->x, C->prev);
     LAUNCH(F, k_tl_update_mapping, grid_for(t->nf), kBlock, 0, t->nf, F->x, t->f_ids, C->x, t->f_w);
     LAUNCH(C, k_velocity, grid_for(t->nc), kBlock, 0, t->nc, C->x, C->last, C->v, pc.dt, C->nonfinite);
@@ -3715,6 +3926,9 @@ mgsb_status mgsb_mg2_create(const mgsb_mesh* coarse, const mgsb_mesh* fine, cons
     std::vector<int32_t> fill(ptr.begin(), ptr.end() - 1);
     for (int f = 0; f < t->ntri; ++f)
         for (int q = 0; q < 3; ++q) idx[fill[tris[3 * f + q]]++] = f;
+    t->coarse->ref_tris = t4;
+    t->coarse->ref_tri_ptr = ptr;
+    t->coarse->ref_tri_idx = idx;
     TRY(tl_upload(t.get(), &t->tris, t4.data(), t4.size()));
     TRY(tl_upload(t.get(), &t->tri_ptr, ptr.data(), ptr.size()));
     TRY(tl_upload(t.get(), &t->tri_idx, idx.data(), idx.size()));
