@@ -1,4 +1,5 @@
-// Every iteration of the reference-faithful frame of a small body in one launch, by one thread-block cluster.
+// Every iteration of the reference-faithful frame of a body in one launch: of a small one by one thread-block cluster, of
+// a larger one by a cooperative launch over every SM.
 #pragma once
 
 #include "kernels.cuh"
@@ -12,10 +13,10 @@ namespace {
 // k_ref_local and k_ref_vertex alternate, 2.8-3.0 us each on a small body whatever
 // they do: the latency of a launch, of its loads and of its end.  Here CTA `rank`
 // of the cluster owns consecutive vertices and runs all iterations on them:
-//   - the tets around its vertices (some of them in other CTAs too), their
-//     constants, and where each corner's contribution goes lie in shared memory,
-//     one image per CTA, laid out by the host and brought by one bulk copy before
-//     the dependency wait;
+//   - the tets around its vertices (some of them in other CTAs too), and where
+//     each corner's contribution goes, lie in shared memory, one image per CTA,
+//     laid out by the host and brought by one bulk copy before the dependency
+//     wait; the tets' constants follow it there;
 //   - x over the window of vertices that those tets read (contiguous in the
 //     numbering) is double buffered: the owner of a vertex stores its new position
 //     into the other buffer of every CTA whose window holds it, and one cluster
@@ -27,7 +28,24 @@ namespace {
 // With triangles (the coarse level of the two-level schedule) a CTA also forms the
 // pushes of the surface triangles around its vertices (k_ref_tri_dcd).
 // ---------------------------------------------------------------------------
+// On a body too large for one cluster (kGrid) the same runs as a cooperative launch
+// of one CTA per SM: positions go through L2 (two buffers, for the same reason), and
+// a barrier over the grid, one atomic add per CTA and one thread of each polling,
+// ends the iteration.
 constexpr int kRefThreads = 512;   // at most; a thread per own vertex, and tets in turn
+constexpr int kRefPolls = 1 << 22;   // of a grid barrier; then the frame is given up and marked non-finite
+
+__device__ __forceinline__ void grid_arrive(int32_t* count) {   // thread 0, behind a barrier of the CTA
+    asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(count) : "memory");
+}
+__device__ __forceinline__ bool grid_reached(const int32_t* count, int target) {
+    for (int polls = 0; polls < kRefPolls; ++polls) {
+        int32_t c;
+        asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(c) : "l"(count) : "memory");
+        if (c >= target) return true;
+    }
+    return false;
+}
 
 struct RefHead {   // at the start of the image
     int tets, own, first, tris;
@@ -37,15 +55,43 @@ struct RefHead {   // at the start of the image
 struct RefPlan {   // offsets: bytes in the CTA's dynamic shared memory, the same in every CTA
     const unsigned char* image;
     int image_bytes;
-    int inv_a, inv_b, inv_c, corner, slot;   // per tet; corner: among the window, slot: 0xffff where another CTA owns it
+    int id;                                  // per tet
     int deg, to;                             // per own vertex: contributions, the CTAs that read it (one bit each)
     int tri, tri_ptr, tri_idx;               // triangles among the window; per own vertex, its triangles
-    int win[2], slots, push;                 // what the kernel writes
+    int corner, slot;                        // per tet, the image's last part (k_ref_image): corners among the window,
+                                             // contributions, 0xffff where another CTA owns the vertex
+    int inv_a, inv_b, inv_c, win[2], slots, push;   // what the kernel writes: the tets' constants, positions, contributions
+    const float4 *from_a, *from_b;           // the constants of all tets
+    const float2* from_c;
     int stride;                              // contribution k of own vertex v at slots[k * stride + v]
-    int bytes, block, cluster;
+    int bytes, block, ctas, grid;            // grid: a cooperative launch, not a cluster
     const float* omega;                      // Chebyshev factor of each iteration
+    float4* pos[2];                          // grid: the positions that odd and even iterations leave
+    int32_t* barrier;                        // grid: arrivals, CTAs that are done; both 0 between launches
 };
 
+// The images' corners and contributions, at set-up: contribution k of a vertex is its k-th slot.
+__global__ void k_ref_image(RefPlan Q, unsigned char* images, const int4* __restrict__ tets, const int4* __restrict__ slot_of,
+                            const int32_t* __restrict__ slot_ptr) {
+    unsigned char* image = images + (size_t)blockIdx.x * Q.image_bytes;
+    const RefHead& head = *reinterpret_cast<const RefHead*>(image);
+    for (int r = threadIdx.x; r < head.tets; r += blockDim.x) {
+        const int t = reinterpret_cast<const int32_t*>(image + Q.id)[r];
+        const int4 id = __ldg(tets + t), so = __ldg(slot_of + t);
+        auto contribution = [&](int i, int at) -> uint16_t {
+            const int v = i - head.first;
+            if (v < 0 || v >= head.own) return (uint16_t)0xffff;
+            return (uint16_t)((at - __ldg(slot_ptr + i / kSlotSlice) - i % kSlotSlice) / kSlotSlice * Q.stride + v);
+        };
+        reinterpret_cast<ushort4*>(image + Q.corner)[r] =
+            make_ushort4((uint16_t)(id.x - head.win_lo), (uint16_t)(id.y - head.win_lo), (uint16_t)(id.z - head.win_lo),
+                         (uint16_t)(id.w - head.win_lo));
+        reinterpret_cast<ushort4*>(image + Q.slot)[r] = make_ushort4(contribution(id.x, so.x), contribution(id.y, so.y),
+                                                                     contribution(id.z, so.z), contribution(id.w, so.w));
+    }
+}
+
+template <bool kGrid>
 __global__ void __launch_bounds__(kRefThreads, 1) k_ref_iterations(
     const RefPlan Q, int iterations, int predict, const RefPredict pa, float4* __restrict__ x, float4* __restrict__ prev,
     float4* __restrict__ s, float4* __restrict__ last, float4* __restrict__ v, const float* __restrict__ fixf, const float* __restrict__ mass,
@@ -56,8 +102,10 @@ __global__ void __launch_bounds__(kRefThreads, 1) k_ref_iterations(
     extern __shared__ __align__(128) unsigned char smb[];
     __shared__ __align__(8) uint64_t bar;
     __shared__ SphereSet spheres;
-    const int rank = (int)blockIdx.x, tid = threadIdx.x;   // one cluster
+    __shared__ int stop;
+    const int rank = (int)blockIdx.x, tid = threadIdx.x;   // one cluster, or the grid
     if (tid == 0) {
+        stop = 0;
         mbar_init(&bar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         mbar_expect_tx(&bar, (uint32_t)Q.image_bytes);
@@ -79,6 +127,12 @@ __global__ void __launch_bounds__(kRefThreads, 1) k_ref_iterations(
     const int deg = mine ? reinterpret_cast<const uint16_t*>(smb + Q.deg)[vert] : 0;
     const uint32_t to = mine ? reinterpret_cast<const uint16_t*>(smb + Q.to)[vert] : 0;
     const uint32_t base = smem_u32(smb);
+    for (int t = tid; t < tets; t += blockDim.x) {   // written by no kernel of a frame
+        const int q = reinterpret_cast<const int32_t*>(smb + Q.id)[t];
+        reinterpret_cast<float4*>(smb + Q.inv_a)[t] = __ldg(Q.from_a + q);
+        reinterpret_cast<float4*>(smb + Q.inv_b)[t] = __ldg(Q.from_b + q);
+        reinterpret_cast<float2*>(smb + Q.inv_c)[t] = __ldg(Q.from_c + q);
+    }
     pdl_wait();
     {
         float4* w = reinterpret_cast<float4*>(smb + Q.win[0]);
@@ -106,12 +160,34 @@ __global__ void __launch_bounds__(kRefThreads, 1) k_ref_iterations(
         pv4 = prev[i];
         l4 = last[i];
     }
-    cluster_arrive();   // every CTA runs before it is written to, and has read x before it is written
-    cluster_wait();
+    int target = 0;
+    // every CTA has read what it needs and written what the others read; false: one did not arrive in time
+    auto together = [&]() -> bool {
+        if (!kGrid) {
+            cluster_arrive();
+            cluster_wait();
+            return true;
+        }
+        target += gridDim.x;
+        __syncthreads();
+        if (tid == 0) {
+            grid_arrive(Q.barrier);
+            if (!grid_reached(Q.barrier, target)) stop = 1;
+        }
+        __syncthreads();
+        return !stop;
+    };
+    // cluster: every CTA runs before it is written to; both: x has been read before it is written
+    bool on = kGrid && iterations > 1 ? (__syncthreads(), true) : together();
     float4* slots = reinterpret_cast<float4*>(smb + Q.slots);
-    for (int it = 0; it < iterations; ++it) {
+    for (int it = 0; it < iterations && on; ++it) {
         const float omega = __ldg(Q.omega + it);
-        const float4* w = reinterpret_cast<const float4*>(smb + Q.win[it & 1]);
+        float4* w = reinterpret_cast<float4*>(smb + Q.win[kGrid ? 0 : it & 1]);
+        if (kGrid && it > 0) {
+            const int n = ok ? head.win_n : 0;
+            for (int k = tid; k < n; k += blockDim.x) w[k] = __ldcg(Q.pos[it & 1] + head.win_lo + k);
+            __syncthreads();
+        }
         RefContact ct;
         const float4 p4 = mine ? w[i - head.win_lo] : s4;
         if (mine && !with_tris) ref_contact(p4, ct, &spheres, kc);
@@ -158,7 +234,9 @@ __global__ void __launch_bounds__(kRefThreads, 1) k_ref_iterations(
             }
             const float4 xn = ref_vertex(p4, s4, pv4, make_float4(fx, fy, fz, 0.f), ct, dc, vd, fix, omega, relax);
             pv4 = p4;
-            if (it + 1 < iterations) {
+            if (kGrid && it + 1 < iterations) {
+                __stcg(Q.pos[(it + 1) & 1] + i, xn);
+            } else if (it + 1 < iterations) {
                 for (uint32_t m = to; m; m &= m - 1) {
                     const int c = __ffs(m) - 1;
                     cluster_st(cluster_addr(base + Q.win[(it + 1) & 1] + 16 * (i - head.peer_lo[c]), c), xn);
@@ -179,8 +257,14 @@ __global__ void __launch_bounds__(kRefThreads, 1) k_ref_iterations(
             }
         }
         if (it + 1 == iterations) break;
-        cluster_arrive();   // the new positions are in the windows, the contributions have been read
-        cluster_wait();
+        on = together();   // the new positions are there, the contributions have been read
+    }
+    if (kGrid && tid == 0) {
+        if (!on) atomicOr(nonfinite, 1);
+        if (atomicAdd(Q.barrier + 1, 1) == (int)gridDim.x - 1) {   // every other CTA has left: ready for the next launch
+            Q.barrier[0] = 0;
+            Q.barrier[1] = 0;
+        }
     }
     if (!ok) {   // a copy that never arrived is waited for again before the CTA ends
         if (tid == 0) atomicOr(nonfinite, 1);

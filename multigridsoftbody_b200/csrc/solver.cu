@@ -533,31 +533,44 @@ mgsb_status upload_normals_data(mgsb_solver* h, std::vector<DevMem>& pool) {
 // ---------------------------------------------------------------------------
 // Derived data (rebuilt when fixed set / material / params change)
 // ---------------------------------------------------------------------------
-// Layout and images of k_ref_iterations, for a body small enough that a CTA's share of the tets takes less than the two
-// launches that it replaces, over 16 CTAs (8 if the device cannot schedule 16).
-// Frames of 20 iterations with it and with its launches: 57 and 119 us at 375 vertices, 62 and 124 at 1,025, 98 and 145
-// at 2,009, 126 and 159 at 2,989, 159 and 165 at 4,050.
-constexpr int kRefClusterVerts = 3500;
+// Layout and images of k_ref_iterations: one cluster of 16 CTAs (8 if the device cannot schedule 16) up to
+// kRefClusterVerts vertices, a CTA per SM above that while a CTA's tets, those of its neighbours included, take at most
+// kRefRounds turns of its threads; larger bodies, and numberings whose vertices reach too far, run k_ref_local and
+// k_ref_vertex.  Frames of 20 iterations by cluster, grid and launches: 58, 75 and 119 us at 375 vertices, 62, 76 and 124
+// at 1,025, 88, 76 and 130 at 1,476, 98, 77 and 142 at 2,009; by grid and launches: 85 and 165 us at 4,050, 110 and 170
+// at 7,100, 160 and 191 at 19,097 (4 turns), 189 and 199 at 22,022 (5 turns), 231 and 236 at 31,725.
+constexpr int kRefClusterVerts = 1200, kRefRounds = 5;
 
 mgsb_status plan_ref(mgsb_solver* h, std::vector<DevMem>& pool, const Plan& P) {
     h->ref = RefPlan{};
     const int n = P.N0, T = P.T;
-    if (n > kRefClusterVerts || h->bodies.size() != 1 || h->p.iterations < 1) return MGSB_OK;
+    if (h->bodies.size() != 1 || h->p.iterations < 1) return MGSB_OK;
+    std::vector<float> omega(h->p.iterations);   // Chebyshev factors
+    float* dom = nullptr;
+    float wi = 1.0f;
+    for (float& o : omega) o = wi = 4 / (4 - h->p.cheb_rho * h->p.cheb_rho * wi);
+    TRY(dupload(h, pool, &dom, omega));
     const int nf = (int)h->ref_tris.size();
     int most_smem = 0;
     CUDA_TRY(h, cudaDeviceGetAttribute(&most_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device));
-    CUDA_TRY(h, cudaFuncSetAttribute(k_ref_iterations, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    CUDA_TRY(h, cudaFuncSetAttribute(k_ref_iterations, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     most_smem - kStagedStaticSmem));
+    int sms = 0, coop = 0;
+    CUDA_TRY(h, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
+    CUDA_TRY(h, cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, h->device));
+    CUDA_TRY(h, cudaFuncSetAttribute(k_ref_iterations<false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    for (auto k : {k_ref_iterations<false>, k_ref_iterations<true>})
+        CUDA_TRY(h, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most_smem - kStagedStaticSmem));
     struct Part {
         int first = 0, own = 0, lo = 0, hi = 0;
         std::vector<int> tets, tris;
     };
-    for (int cs : {16, 8}) {
+    for (int cs : {16, 8, sms}) {
+        const bool grid = cs == sms;
+        if (grid ? !coop : n > kRefClusterVerts) continue;
         const int per = (n + cs - 1) / cs;
         if (per > kRefThreads) continue;
         std::vector<Part> part(cs);
         for (int k = 0; k < cs; ++k) {
+            part[k].tets.reserve((size_t)T / cs * 3 + 64);
             part[k].first = part[k].lo = std::min(n, k * per);
             part[k].hi = std::min(n, (k + 1) * per);
             part[k].own = part[k].hi - part[k].first;
@@ -593,7 +606,8 @@ mgsb_status plan_ref(mgsb_solver* h, std::vector<DevMem>& pool, const Plan& P) {
             win = std::max(win, (size_t)(o.hi - o.lo));
             if (nf) refs = std::max(refs, (size_t)(h->ref_tri_ptr[o.first + o.own] - h->ref_tri_ptr[o.first]));
         }
-        if ((size_t)depth * per >= 0xffff || tris > 0xffff || refs > 0xffff) continue;
+        if (grid && tets > (size_t)kRefRounds * kRefThreads) continue;
+        if ((size_t)depth * per >= 0xffff || tris > 0xffff || refs > 0xffff || win > 0x10000) continue;
         RefPlan q{};
         size_t bytes = sizeof(RefHead);
         auto room = [&](size_t b) {
@@ -601,49 +615,59 @@ mgsb_status plan_ref(mgsb_solver* h, std::vector<DevMem>& pool, const Plan& P) {
             bytes += (b + 15) / 16 * 16;
             return (int)std::min<size_t>(a, 1u << 30);
         };
-        q.inv_a = room(16 * tets);
-        q.inv_b = room(16 * tets);
-        q.inv_c = room(8 * tets);
-        q.corner = room(8 * tets);
-        q.slot = room(8 * tets);
+        q.id = room(4 * tets);
         q.deg = room(2 * per);
         q.to = room(2 * per);
         q.tri = room(8 * tris);
         q.tri_ptr = room(2 * (per + 1));
         q.tri_idx = room(2 * refs);
+        const size_t from_host = bytes;
+        q.corner = room(8 * tets);
+        q.slot = room(8 * tets);
         const size_t image = bytes;
+        q.inv_a = room(16 * tets);
+        q.inv_b = room(16 * tets);
+        q.inv_c = room(8 * tets);
+        q.from_a = h->tA;
+        q.from_b = h->tB;
+        q.from_c = h->tC;
         q.win[0] = room(16 * win);
-        q.win[1] = room(16 * win);
+        q.win[1] = grid ? 0 : room(16 * win);
         q.slots = room((size_t)16 * depth * per);
         q.push = room(16 * tris);
         if (bytes > (size_t)(most_smem - kStagedStaticSmem)) continue;
         q.image_bytes = (int)image;
         q.stride = per;
         q.bytes = (int)bytes;
-        q.cluster = cs;
+        q.ctas = cs;
+        q.grid = grid;
         q.block = (int)std::min<size_t>(kRefThreads, (std::max<size_t>(tets, 32) + 31) / 32 * 32 + ((size_t)per + 31) / 32 * 32);
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)cs);
-        cfg.blockDim = dim3((unsigned)q.block);
-        cfg.dynamicSmemBytes = bytes;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = (unsigned)cs;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        int nclusters = 0;
-        if (cudaOccupancyMaxActiveClusters(&nclusters, k_ref_iterations, &cfg) != cudaSuccess) {
-            cudaGetLastError();
-            continue;
+        int fit = 0;
+        if (grid) {
+            CUDA_TRY(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, k_ref_iterations<true>, q.block, bytes));
+        } else {
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3((unsigned)cs);
+            cfg.blockDim = dim3((unsigned)q.block);
+            cfg.dynamicSmemBytes = bytes;
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = (unsigned)cs;
+            attr[0].val.clusterDim.y = 1;
+            attr[0].val.clusterDim.z = 1;
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+            if (cudaOccupancyMaxActiveClusters(&fit, k_ref_iterations<false>, &cfg) != cudaSuccess) {
+                cudaGetLastError();
+                continue;
+            }
         }
-        if (nclusters < 1) continue;
-        std::vector<unsigned char> img((size_t)cs * image, 0);
-        std::vector<int> fill(n, 0), at(std::max(nf, 1), 0);
+        if (fit < 1) continue;
+        std::vector<unsigned char> img((size_t)cs * from_host, 0);
+        std::vector<int> at(std::max(nf, 1), 0);
         for (int k = 0; k < cs; ++k) {
             const Part& o = part[k];
-            unsigned char* m = img.data() + (size_t)k * image;
+            unsigned char* m = img.data() + (size_t)k * from_host;
             RefHead head{};
             head.tets = (int)o.tets.size();
             head.own = o.own;
@@ -651,26 +675,13 @@ mgsb_status plan_ref(mgsb_solver* h, std::vector<DevMem>& pool, const Plan& P) {
             head.tris = (int)o.tris.size();
             head.win_lo = o.lo;
             head.win_n = o.hi - o.lo;
-            for (int j = 0; j < cs; ++j) head.peer_lo[j] = part[j].lo;
+            for (int j = 0; j < cs && !grid; ++j) head.peer_lo[j] = part[j].lo;
             std::memcpy(m, &head, sizeof head);
-            for (int r = 0; r < head.tets; ++r) {
-                const int t = o.tets[r], c[4] = {P.tets[t].x, P.tets[t].y, P.tets[t].z, P.tets[t].w};
-                uint16_t corner[4], slot[4];
-                for (int a = 0; a < 4; ++a) {
-                    const int v = c[a] - o.first;
-                    corner[a] = (uint16_t)(c[a] - o.lo);
-                    slot[a] = v >= 0 && v < o.own ? (uint16_t)(fill[c[a]]++ * per + v) : (uint16_t)0xffff;
-                }
-                reinterpret_cast<float4*>(m + q.inv_a)[r] = P.tA[t];
-                reinterpret_cast<float4*>(m + q.inv_b)[r] = P.tB[t];
-                reinterpret_cast<float2*>(m + q.inv_c)[r] = P.tC[t];
-                std::memcpy(m + q.corner + 8 * r, corner, 8);
-                std::memcpy(m + q.slot + 8 * r, slot, 8);
-            }
+            std::memcpy(m + q.id, o.tets.data(), 4 * o.tets.size());
             for (int v = 0; v < o.own; ++v) {
                 const int i = o.first + v;
                 uint32_t to = 0;
-                for (int j = 0; j < cs; ++j)
+                for (int j = 0; j < cs && !grid; ++j)
                     if (i >= part[j].lo && i < part[j].hi) to |= 1u << j;
                 reinterpret_cast<uint16_t*>(m + q.deg)[v] = (uint16_t)deg[i];
                 reinterpret_cast<uint16_t*>(m + q.to)[v] = (uint16_t)to;
@@ -689,15 +700,20 @@ mgsb_status plan_ref(mgsb_solver* h, std::vector<DevMem>& pool, const Plan& P) {
                         reinterpret_cast<uint16_t*>(m + q.tri_idx)[e++] = (uint16_t)at[h->ref_tri_idx[b]];
                 }
         }
-        std::vector<float> omega(h->p.iterations);
-        float w = 1.0f;
-        for (float& o : omega) o = w = 4 / (4 - h->p.cheb_rho * h->p.cheb_rho * w);
         unsigned char* dimg = nullptr;
-        float* dom = nullptr;
-        TRY(dupload(h, pool, &dimg, img));
-        TRY(dupload(h, pool, &dom, omega));
+        TRY(dalloc(h, pool, &dimg, (size_t)cs * image));
+        CUDA_TRY(h, cudaMemcpy2D(dimg, image, img.data(), from_host, from_host, cs, cudaMemcpyHostToDevice));
+        // behind the copies of its inputs, on their stream
+        k_ref_image<<<cs, kBlock>>>(q, dimg, h->tets, h->slot_of, h->slot_ptr);
+        CUDA_TRY(h, cudaGetLastError());
+        CUDA_TRY(h, cudaStreamSynchronize(nullptr));
         q.image = dimg;
         q.omega = dom;
+        if (grid) {
+            for (float4*& b : q.pos) TRY(dalloc(h, pool, &b, (size_t)n));
+            TRY(dalloc(h, pool, &q.barrier, 2));
+            CUDA_TRY(h, cudaMemset(q.barrier, 0, 2 * sizeof(int32_t)));
+        }
         h->ref = q;
         return MGSB_OK;
     }
@@ -1068,23 +1084,28 @@ void enqueue_ref_iterations(mgsb_solver* h, int drop_small, int last_iter, const
     if (h->ref.bytes) {
         const RefPlan& q = h->ref;
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)q.cluster);
+        cfg.gridDim = dim3((unsigned)q.ctas);
         cfg.blockDim = dim3((unsigned)q.block);
         cfg.dynamicSmemBytes = (size_t)q.bytes;
         cfg.stream = h->stream;
         cudaLaunchAttribute attr[2];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = (unsigned)q.cluster;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
+        if (q.grid) {
+            attr[0].id = cudaLaunchAttributeCooperative;
+            attr[0].val.cooperative = 1;
+        } else {
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = (unsigned)q.ctas;
+            attr[0].val.clusterDim.y = 1;
+            attr[0].val.clusterDim.z = 1;
+        }
         attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
-        cfg.numAttrs = h->pdl ? 2 : 1;
+        cfg.numAttrs = h->pdl && !q.grid ? 2 : 1;
         const int reps = prof_begin(h, "k_ref_iterations");
         cudaError_t e = cudaSuccess;
         for (int r = 0; r < reps && e == cudaSuccess; ++r)
-            e = cudaLaunchKernelEx(&cfg, k_ref_iterations, q, (int)p.iterations, predict ? 1 : 0,
+            e = cudaLaunchKernelEx(&cfg, q.grid ? k_ref_iterations<true> : k_ref_iterations<false>, q, (int)p.iterations, predict ? 1 : 0,
                                    predict ? *predict : RefPredict{}, h->x, h->prev, h->s, h->last, h->v, (const float*)h->fixf, (const float*)h->mass,
                                    (const float*)h->vdiag, (const SphereSet*)h->spheres_dev, p.volume_stiffness, drop_small,
                                    p.collision_stiffness, p.dt, (double)p.relaxation, tris.push ? 1 : 0, last_iter, h->cflag,
