@@ -195,8 +195,8 @@ constexpr int kLsWinRows = 3072;   // 48 KiB of float4
 constexpr int kLsPerThread = 8;    // ELL entries a thread loads ahead (2 threads per row: rows up to 16 wide)
 
 // Dynamic shared memory of k_ls_sweep_tc: the MLP's operands and barriers, then
-// the residual window; at least 80 KiB (two CTAs per SM at most, so that
-// tcgen05.alloc never waits).
+// the residual window; at least 48 KiB (four CTAs per SM at most, 128 TMEM columns
+// each, so that tcgen05.alloc never waits).
 inline size_t ls_sweep_smem_bytes(int win_rows) {
     const size_t b = ((sizeof(MlpSmem) + 127) / 128) * 128 + (size_t)win_rows * sizeof(float4);
     return b > kMlpMinSmem ? b : kMlpMinSmem;
