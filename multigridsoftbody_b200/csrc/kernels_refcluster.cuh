@@ -65,6 +65,7 @@ struct RefPlan {   // offsets: bytes in the CTA's dynamic shared memory, the sam
     const float2* from_c;
     int stride;                              // contribution k of own vertex v at slots[k * stride + v]
     int bytes, block, ctas, grid;            // grid: a cooperative launch, not a cluster
+    int with_tris;                           // surface triangles that the images hold
     const float* omega;                      // Chebyshev factor of each iteration
     float4* pos[2];                          // grid: the positions that odd and even iterations leave
     int32_t* barrier;                        // grid: arrivals, CTAs that are done; both 0 between launches

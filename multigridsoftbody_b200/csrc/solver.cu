@@ -148,9 +148,10 @@ struct mgsb_solver {
     float4 *tA = nullptr, *tB = nullptr;
     float2* tC = nullptr;
     int4* slot_of = nullptr;
-    // reference kind: k_ref_iterations' layout (bytes 0: the body does not take it), and the surface triangles of the
-    // two-level schedule's coarse level, with the triangles of each vertex
+    // reference kind: k_ref_iterations' layout (bytes 0: the body does not take it), whether it is older than the set-up
+    // or the triangles, and the surface triangles of the two-level schedule's coarse level, with the triangles of each vertex
     RefPlan ref{};
+    bool ref_stale = false;
     std::vector<int4> ref_tris;
     std::vector<int32_t> ref_tri_ptr, ref_tri_idx;
     int32_t* slot_ptr = nullptr;
@@ -541,10 +542,11 @@ mgsb_status upload_normals_data(mgsb_solver* h, std::vector<DevMem>& pool) {
 // at 7,100, 160 and 191 at 19,097 (4 turns), 189 and 199 at 22,022 (5 turns), 231 and 236 at 31,725.
 constexpr int kRefClusterVerts = 1200, kRefRounds = 5;
 
-mgsb_status plan_ref(mgsb_solver* h, std::vector<DevMem>& pool, const Plan& P) {
-    h->ref = RefPlan{};
-    const int n = P.N0, T = P.T;
+mgsb_status plan_ref(mgsb_solver* h) {
+    std::vector<DevMem>& pool = h->derived_mem;
+    const int n = h->N0, T = h->T;
     if (h->bodies.size() != 1 || h->p.iterations < 1) return MGSB_OK;
+    const int32_t* corners = h->bodies[0].tets.data();
     std::vector<float> omega(h->p.iterations);   // Chebyshev factors
     float* dom = nullptr;
     float wi = 1.0f;
@@ -586,10 +588,7 @@ mgsb_status plan_ref(mgsb_solver* h, std::vector<DevMem>& pool, const Plan& P) {
                 }
             }
         };
-        for (int t = 0; t < T; ++t) {
-            const int c[4] = {P.tets[t].x, P.tets[t].y, P.tets[t].z, P.tets[t].w};
-            share(t, c, 4, &Part::tets);
-        }
+        for (int t = 0; t < T; ++t) share(t, corners + 4 * (size_t)t, 4, &Part::tets);
         for (int f = 0; f < nf; ++f) {
             const int c[3] = {h->ref_tris[f].x, h->ref_tris[f].y, h->ref_tris[f].z};
             share(f, c, 3, &Part::tris);
@@ -597,8 +596,7 @@ mgsb_status plan_ref(mgsb_solver* h, std::vector<DevMem>& pool, const Plan& P) {
         // contributions of each vertex, tets ascending
         std::vector<int> deg(n, 0);
         int depth = 0;
-        for (int t = 0; t < T; ++t)
-            for (int c : {P.tets[t].x, P.tets[t].y, P.tets[t].z, P.tets[t].w}) depth = std::max(depth, ++deg[c]);
+        for (size_t c = 0; c < 4 * (size_t)T; ++c) depth = std::max(depth, ++deg[corners[c]]);
         size_t tets = 0, tris = 0, win = 0, refs = 0;
         for (const Part& o : part) {
             tets = std::max(tets, o.tets.size());
@@ -641,6 +639,7 @@ mgsb_status plan_ref(mgsb_solver* h, std::vector<DevMem>& pool, const Plan& P) {
         q.bytes = (int)bytes;
         q.ctas = cs;
         q.grid = grid;
+        q.with_tris = nf;
         q.block = (int)std::min<size_t>(kRefThreads, (std::max<size_t>(tets, 32) + 31) / 32 * 32 + ((size_t)per + 31) / 32 * 32);
         int fit = 0;
         if (grid) {
@@ -781,7 +780,8 @@ mgsb_status rebuild(mgsb_solver* h) {
         h->local_blocks = (int)P.lblock.size();
     } else {
         TRY(dupload(h, pool, &h->slot_of, P.slot_of));
-        TRY(plan_ref(h, pool, P));
+        h->ref = RefPlan{};
+        h->ref_stale = true;   // planned before the next frame, by when a coarse level has its triangles
     }
     h->h_inv = P.h_inv;
     h->h_ac = P.h_ac;
@@ -1078,10 +1078,13 @@ struct RefTris {
     float4* push = nullptr;
 };
 
+// One launch for all of them: the plan is there, and has the triangles that the frame asks for.
+bool ref_one_launch(const mgsb_solver* h, const RefTris& tris) { return h->ref.bytes && (!tris.push || h->ref.with_tris == tris.n); }
+
 void enqueue_ref_iterations(mgsb_solver* h, int drop_small, int last_iter, const RefTris& tris, const RefPredict* predict) {
     const int n = h->N0, T = h->T;
     const mgsb_params& p = h->p;
-    if (h->ref.bytes) {
+    if (ref_one_launch(h, tris)) {
         const RefPlan& q = h->ref;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)q.ctas);
@@ -1135,7 +1138,7 @@ void enqueue_ref_frame(mgsb_solver* h) {
     const mgsb_params& p = h->p;
     const BodyHost& B = h->bodies[0];
     const RefPredict a{B.damping, B.gravity[0], B.gravity[1], B.gravity[2]};
-    if (h->ref.bytes) {
+    if (ref_one_launch(h, RefTris{})) {
         enqueue_ref_iterations(h, 1, 3, RefTris{}, &a);
         return;
     }
@@ -2311,8 +2314,19 @@ void enqueue_frame(mgsb_solver* h) {
         enqueue_ref_frame(h);
 }
 
+// k_ref_iterations' plan, if it is older than the set-up or the triangles.
+mgsb_status ready_ref(mgsb_solver* h) {
+    if (!h->ref_stale) return MGSB_OK;
+    CUDA_TRY(h, cudaSetDevice(h->device));
+    h->ref = RefPlan{};
+    TRY(plan_ref(h));
+    h->ref_stale = false;
+    return MGSB_OK;
+}
+
 mgsb_status ensure_ready(mgsb_solver* h) {
     if (h->dirty) TRY(rebuild(h));
+    TRY(ready_ref(h));
     return ready_staged(h);
 }
 
@@ -3874,11 +3888,12 @@ void enqueue_two_level_frame(mgsb_two_level* t) {
     C->launches = F->launches = 0;
     const BodyHost& BC = C->bodies[0];
     const BodyHost& BF = F->bodies[0];
+    const RefTris tris{t->ntri, t->tris, t->tri_ptr, t->tri_idx, t->push};
     const RefPredict ac{BC.damping, BC.gravity[0], BC.gravity[1], BC.gravity[2]};
     const RefPredict af{BF.damping, BF.gravity[0], BF.gravity[1], BF.gravity[2]};
     LAUNCH(C, k_ref_predict, grid_for(t->nc), kBlock, 0, t->nc, C->x, C->v, C->s, C->prev, C->last, C->fixf, ac, pc.dt);
     LAUNCH(F, k_ref_predict, grid_for(t->nf), kBlock, 0, t->nf, F->x, F->v, F->s, F->prev, F->last, F->fixf, af, pf.dt);
-    enqueue_ref_iterations(C, 0, 2, RefTris{t->ntri, t->tris, t->tri_ptr, t->tri_idx, t->push}, nullptr);
+    enqueue_ref_iterations(C, 0, 2, tris, nullptr);
     LAUNCH(F, k_tl_transfer, grid_for(t->nf), kBlock, 0, t->nf, t->f_ids, t->f_w, C->x, F->x, F->prev);
     enqueue_ref_iterations(F, 0, 2, RefTris{}, nullptr);
     LAUNCH(C, k_tl_transfer, grid_for(t->nc), kBlock, 0, t->nc, t->c_ids, t->c_w, F->x, C->x, C->prev);
@@ -3950,6 +3965,7 @@ mgsb_status mgsb_mg2_create(const mgsb_mesh* coarse, const mgsb_mesh* fine, cons
     t->coarse->ref_tris = t4;
     t->coarse->ref_tri_ptr = ptr;
     t->coarse->ref_tri_idx = idx;
+    t->coarse->ref_stale = true;
     TRY(tl_upload(t.get(), &t->tris, t4.data(), t4.size()));
     TRY(tl_upload(t.get(), &t->tri_ptr, ptr.data(), ptr.size()));
     TRY(tl_upload(t.get(), &t->tri_idx, idx.data(), idx.size()));
