@@ -4028,9 +4028,17 @@ mgsb_status mgsb_mg2_step(mgsb_two_level* t) {
         t->graph = nullptr;
         if (cudaStreamBeginCapture(t->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
             return tl_err(t, MGSB_CUDA_ERROR, "graph capture could not start");
+        C->enqueue_status = F->enqueue_status = MGSB_OK;
         enqueue_two_level_frame(t);
-        if (cudaStreamEndCapture(t->stream, &t->graph) != cudaSuccess ||
-            cudaGraphInstantiate(&t->exec, t->graph, 0) != cudaSuccess)
+        const cudaError_t e = cudaStreamEndCapture(t->stream, &t->graph);
+        for (mgsb_solver* s : {C, F})
+            if (s->enqueue_status != MGSB_OK) {   // a refused launch: the frame lacks that level's iterations
+                if (e == cudaSuccess) cudaGraphDestroy(t->graph);
+                t->graph = nullptr;
+                cudaGetLastError();
+                return tl_err(t, s->enqueue_status, s->err.c_str());
+            }
+        if (e != cudaSuccess || cudaGraphInstantiate(&t->exec, t->graph, 0) != cudaSuccess)
             return tl_err(t, MGSB_CUDA_ERROR, "graph capture of the two-level frame failed");
         t->graph_valid = true;
     }

@@ -1,0 +1,43 @@
+"""What the solvers' host code does when the runtime refuses a launch, and when set-up changes behind a captured frame:
+the library over a stand-in for the CUDA runtime."""
+import pytest
+
+import multigridsoftbody_b200 as mg
+from multigridsoftbody_b200 import _lib as L
+
+from .common import beam
+from .host_only import CAPTURES, GRAPH_LAUNCHES, Host, build_host_only
+
+
+@pytest.fixture(scope="module")
+def host_library(tmp_path_factory):
+    return Host(build_host_only(str(tmp_path_factory.mktemp("host"))))
+
+
+@pytest.fixture
+def host(host_library, monkeypatch):
+    monkeypatch.setattr(L, "_lib", host_library.lib)
+    host_library.reset()
+    return host_library
+
+
+def _two_level():
+    (c, cf), (f, ff) = beam(2, 20, 2), beam(4, 40, 4)
+    t = mg.TwoLevel(c, f, mg.default_params(mg.SOLVER_REFERENCE_JACOBI))
+    t.set_fixed(cf, ff)
+    return t
+
+
+def test_refused_launch_fails_the_two_level_step(host):
+    t = _two_level()
+    host.refuse("k_ref_iterations")
+    for _ in range(2):   # not kept as a frame without its iterations either
+        with pytest.raises(mg.MgsbError, match="reference iterations launch failed"):
+            t.step()
+    assert host.count(GRAPH_LAUNCHES) == 0
+    host.refuse("")
+    host.reset()
+    t.step()
+    t.step()
+    assert host.count(CAPTURES) == 1 and host.count(GRAPH_LAUNCHES) == 2 and len(host.launches("k_ref_iterations")) == 2
+    t.close()
