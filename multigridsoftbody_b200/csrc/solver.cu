@@ -101,6 +101,7 @@ struct mgsb_solver {
     std::vector<BodyHost> bodies;
     int N0 = 0, T = 0;
     bool dirty = true;          // derived data must be rebuilt before the next step
+    uint64_t revision = 0;      // counts what makes a captured frame out of date: set-ups, and changes of its launches
     bool graph_valid = false;
     cudaGraphExec_t graph_exec = nullptr;
     cudaGraph_t graph = nullptr;
@@ -396,6 +397,7 @@ void apply_tuning(mgsb_solver* h) {
 }
 
 void invalidate_graph(mgsb_solver* h) {
+    ++h->revision;
     if (h->graph_exec) {
         cudaGraphExecDestroy(h->graph_exec);
         h->graph_exec = nullptr;
@@ -731,6 +733,7 @@ mgsb_status rebuild(mgsb_solver* h) {
         h->graph = nullptr;
     }
     h->graph_valid = false;
+    ++h->revision;
     free_pool(h->derived_mem);
     h->lev.clear();
     auto& pool = h->derived_mem;
@@ -3849,6 +3852,7 @@ struct mgsb_two_level {
     int32_t *tri_ptr = nullptr, *tri_idx = nullptr;   // coarse vertex -> its triangles
     float4* push = nullptr;    // per-triangle push sum and contact count
     bool graph_valid = false;
+    uint64_t revision[2] = {0, 0};   // of the levels (fine, coarse) when the graph was captured
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     ~mgsb_two_level() {
@@ -4015,9 +4019,10 @@ mgsb_status mgsb_mg2_step(mgsb_two_level* t) {
     if (!t) return MGSB_INVALID_ARG;
     mgsb_solver* C = t->coarse;
     mgsb_solver* F = t->fine;
-    if (C->dirty || F->dirty) t->graph_valid = false;
     TRY(ensure_ready(C));
     TRY(ensure_ready(F));
+    // a level may have been set up again by a call on its own handle since the capture: its buffers are others then
+    if (t->revision[0] != F->revision || t->revision[1] != C->revision) t->graph_valid = false;
     if (cudaSetDevice(t->device) != cudaSuccess) return tl_err(t, MGSB_CUDA_ERROR, "cudaSetDevice failed");
     TRY(push_tool(C));
     TRY(push_tool(F));
@@ -4040,6 +4045,8 @@ mgsb_status mgsb_mg2_step(mgsb_two_level* t) {
             }
         if (e != cudaSuccess || cudaGraphInstantiate(&t->exec, t->graph, 0) != cudaSuccess)
             return tl_err(t, MGSB_CUDA_ERROR, "graph capture of the two-level frame failed");
+        t->revision[0] = F->revision;
+        t->revision[1] = C->revision;
         t->graph_valid = true;
     }
     if (cudaGraphLaunch(t->exec, t->stream) != cudaSuccess) return tl_err(t, MGSB_CUDA_ERROR, "graph launch failed");

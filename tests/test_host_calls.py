@@ -41,3 +41,20 @@ def test_refused_launch_fails_the_two_level_step(host):
     t.step()
     assert host.count(CAPTURES) == 1 and host.count(GRAPH_LAUNCHES) == 2 and len(host.launches("k_ref_iterations")) == 2
     t.close()
+
+
+@pytest.mark.parametrize("level", [0, 1])
+def test_level_set_up_by_its_own_handle_is_captured_again(host, level):
+    (c, cf), (f, ff) = beam(2, 20, 2), beam(4, 40, 4)
+    t = _two_level()
+    t.step()
+    own = t.levels[level]
+    own.set_fixed((ff, cf)[level])
+    own.normals()        # sets the level up again: the captured frame's buffers are gone
+    t.step()
+    assert host.count(CAPTURES) == 2
+    own.set_launch_overlap(False)
+    t.step()
+    t.step()
+    assert host.count(CAPTURES) == 3
+    t.close()
