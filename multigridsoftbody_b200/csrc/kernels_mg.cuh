@@ -1380,7 +1380,7 @@ __global__ void __launch_bounds__(kStagedThreads, 1) k_coarse_vcycle_staged(cons
     staged_peers<kLanesC>(peer, base, lane, cs, rank);
     const int dense0 = __ldg(dense_off + blockIdx.x / cs);
     // the image; when it does not arrive the CTA takes part in the barriers only, and the frame ends marked non-finite
-    const bool ok = mbar_wait(&bar, 0, kMaxPolls);
+    const bool ok = cta_wait(&bar, 0, kMaxPolls);
     const StagedHead& head = *reinterpret_cast<const StagedHead*>(smb);
     const int nc = head.coarse_n;
     auto phase = [&](int p) -> const StagedPhase& {

@@ -119,6 +119,11 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int ma
     }
     return false;
 }
+// The same for every thread of a CTA: false in all of them when the bound ran out in any, so that they go on together
+// and whichever thread reports it has seen it.
+__device__ __forceinline__ bool cta_wait(uint64_t* bar, uint32_t parity, int max_polls) {
+    return __syncthreads_and(mbar_wait(bar, parity, max_polls)) != 0;
+}
 // 1-D bulk async copy global -> shared, completion counted on `bar` (16-byte
 // aligned addresses, size a multiple of 16).
 __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
@@ -747,7 +752,7 @@ __global__ void __launch_bounds__(kGradThreads) k_mlp_grad(int nblk, const float
             }
             S.loss[lane] = t;
         }
-        ok = mbar_wait(&S.bar, phase, kMaxPolls);
+        ok = cta_wait(&S.bar, phase, kMaxPolls);
         if (ok && lane < nb) {
             if (kind == 2)
                 grad_tile<4, 5>(S, lane, 4 * half, U, U, V, 4 * half, 0, bias >= 0);

@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(kRefThreads, 1) k_ref_iterations(
         reinterpret_cast<int32_t*>(&spheres)[k] = reinterpret_cast<const int32_t*>(sphere_set)[k];
     __syncthreads();
     // when the image does not arrive the CTA takes part in the barriers only, and the frame ends marked non-finite
-    const bool ok = mbar_wait(&bar, 0, kMaxPolls);
+    const bool ok = cta_wait(&bar, 0, kMaxPolls);
     const RefHead& head = *reinterpret_cast<const RefHead*>(smb);
     const int tets = ok ? head.tets : 0, tris = ok && with_tris ? head.tris : 0, own = ok ? head.own : 0;
     // the vertices' threads come last: where the tets leave them free they look for contact meanwhile
