@@ -3283,13 +3283,14 @@ mgsb_status mgsb_autotune(mgsb_solver* h, int32_t frames, int32_t* chosen) {
     struct Cand {
         int cluster, block, fuse, split, dense;
     };
-    std::vector<Cand> cands;
+    // the solver's own choice first: what an untuned solver runs, and a tie leaves it
+    std::vector<Cand> cands{{0, 512, -1, 0, 0}};
     const int nb = (int)h->bodies.size();
     const int L = h->p.levels;
     const int cls[] = {1, 2, 4, 8, 12, 16};
     for (int c : cls) {
         if (nb > 1 && c > 2) continue;   // many bodies: small clusters, one per body
-        for (int blk : {256, 512, 1024}) {
+        for (int blk : {512, 256, 1024}) {
             // split: the cluster kernel's first level; skip clusters with < 32 of its rows per CTA
             for (int sp = 1; sp < L; ++sp)
                 if ((c == 1 || h->maxv[sp] >= 32 * c) && coarse_shape_feasible(h, c, blk, 0, sp))
@@ -3303,15 +3304,15 @@ mgsb_status mgsb_autotune(mgsb_solver* h, int32_t frames, int32_t* chosen) {
     if (nb == 1)
         for (int sp = 1; sp < L; ++sp)
             if (dense_eligible(h, sp)) cands.push_back({1, 256, 0, sp, 1});
-    // the solver's own choice, where it takes the whole V-cycle into the cluster kernel
-    if (h->staged.pre0 > 0) cands.push_back({0, 512, -1, 0, 0});
     float best = 1e30f;
     Cand bestc = {h->cluster, h->coarse_block, h->fuse_l0, h->split, h->dense_op ? 1 : 0};
     cudaEvent_t a, b;
     cudaEventCreate(&a);
     cudaEventCreate(&b);
     mgsb_status st = MGSB_OK;
+    bool seen[kMaxCluster + 1][kMaxLevels] = {};   // shapes that the staged kernel took: it picks its own block size
     for (const Cand& c : cands) {
+        if (!c.dense && c.fuse == 0 && seen[c.cluster][c.split]) continue;
         h->tune_cluster = c.cluster;
         h->tune_fuse = c.fuse;
         h->tune_split = c.split;
@@ -3320,7 +3321,7 @@ mgsb_status mgsb_autotune(mgsb_solver* h, int32_t frames, int32_t* chosen) {
         apply_tuning(h);
         invalidate_graph(h);
         if ((st = ready_staged(h)) != MGSB_OK) break;
-        if (h->staged.bytes && c.block != 512) continue;   // it picks its own block size
+        if (h->staged.bytes && c.cluster) seen[c.cluster][c.split] = true;
         cudaMemsetAsync(h->fac_valid, 0, h->bodies.size() * sizeof(int32_t), h->stream);
         restore();
         st = step_once(h);   // warm-up: capture + coarsest factorisation

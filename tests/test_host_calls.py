@@ -58,3 +58,23 @@ def test_level_set_up_by_its_own_handle_is_captured_again(host, level):
     t.step()
     assert host.count(CAPTURES) == 3
     t.close()
+
+
+@pytest.mark.parametrize("dims,levels,bodies", [((6, 60, 6), 3, 1), ((8, 80, 8), 3, 1), ((4, 40, 4), 3, 1), ((4, 40, 4), 3, 2)])
+def test_autotune_offers_the_solvers_own_choice(host, dims, levels, bodies):
+    m, fixed = beam(*dims)
+    s = mg.Solver([m] * bodies, mg.default_params(mg.SOLVER_MULTIGRID, levels=levels))
+    for b in range(bodies):
+        s.set_fixed(fixed, body=b)
+    s.step()
+    own = host.launches("k_coarse_vcycle")[0]
+    frame = s.launches_per_frame()
+    host.reset()
+    s.autotune(1)
+    tried = host.launches("k_coarse_vcycle")
+    assert own in tried and len(set(tried)) > 1
+    # every candidate takes as long here: the own choice stays
+    host.reset()
+    s.step()
+    assert host.launches("k_coarse_vcycle")[0] == own and s.launches_per_frame() == frame
+    s.close()
