@@ -149,10 +149,12 @@ struct mgsb_solver {
     float4 *tA = nullptr, *tB = nullptr;
     float2* tC = nullptr;
     int4* slot_of = nullptr;
-    // reference kind: k_ref_iterations' layout (bytes 0: the body does not take it), whether it is older than the set-up
-    // or the triangles, and the surface triangles of the two-level schedule's coarse level, with the triangles of each vertex
+    // reference kind: k_ref_iterations' layout (bytes 0: the body does not take it), which depends on the mesh alone and is
+    // kept over set-ups, with its device memory; whether it is older than the triangles, and what it holds of the set-up
+    // older than that; and the surface triangles of the two-level schedule's coarse level, with the triangles of each vertex
     RefPlan ref{};
-    bool ref_stale = false;
+    std::vector<DevMem> ref_mem;
+    bool ref_planned = false, ref_stale = false;
     std::vector<int4> ref_tris;
     std::vector<int32_t> ref_tri_ptr, ref_tri_idx;
     int32_t* slot_ptr = nullptr;
@@ -268,6 +270,7 @@ mgsb_solver::~mgsb_solver() {
     if (graph_exec) cudaGraphExecDestroy(graph_exec);
     if (graph) cudaGraphDestroy(graph);
     for (auto& m : derived_mem) cudaFree(m.p);
+    for (auto& m : ref_mem) cudaFree(m.p);
     for (auto& m : state_mem) cudaFree(m.p);
     for (auto& m : pair_mem) cudaFree(m.p);
     delete[] bodies_host;
@@ -545,15 +548,12 @@ mgsb_status upload_normals_data(mgsb_solver* h, std::vector<DevMem>& pool) {
 constexpr int kRefClusterVerts = 1200, kRefRounds = 5;
 
 mgsb_status plan_ref(mgsb_solver* h) {
-    std::vector<DevMem>& pool = h->derived_mem;
+    std::vector<DevMem>& pool = h->ref_mem;
+    free_pool(pool);
+    h->ref = RefPlan{};
     const int n = h->N0, T = h->T;
-    if (h->bodies.size() != 1 || h->p.iterations < 1) return MGSB_OK;
+    if (h->bodies.size() != 1) return MGSB_OK;
     const int32_t* corners = h->bodies[0].tets.data();
-    std::vector<float> omega(h->p.iterations);   // Chebyshev factors
-    float* dom = nullptr;
-    float wi = 1.0f;
-    for (float& o : omega) o = wi = 4 / (4 - h->p.cheb_rho * h->p.cheb_rho * wi);
-    TRY(dupload(h, pool, &dom, omega));
     const int nf = (int)h->ref_tris.size();
     int most_smem = 0;
     CUDA_TRY(h, cudaDeviceGetAttribute(&most_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device));
@@ -628,9 +628,6 @@ mgsb_status plan_ref(mgsb_solver* h) {
         q.inv_a = room(16 * tets);
         q.inv_b = room(16 * tets);
         q.inv_c = room(8 * tets);
-        q.from_a = h->tA;
-        q.from_b = h->tB;
-        q.from_c = h->tC;
         q.win[0] = room(16 * win);
         q.win[1] = grid ? 0 : room(16 * win);
         q.slots = room((size_t)16 * depth * per);
@@ -709,11 +706,9 @@ mgsb_status plan_ref(mgsb_solver* h) {
         CUDA_TRY(h, cudaGetLastError());
         CUDA_TRY(h, cudaStreamSynchronize(nullptr));
         q.image = dimg;
-        q.omega = dom;
         if (grid) {
             for (float4*& b : q.pos) TRY(dalloc(h, pool, &b, (size_t)n));
             TRY(dalloc(h, pool, &q.barrier, 2));
-            CUDA_TRY(h, cudaMemset(q.barrier, 0, 2 * sizeof(int32_t)));
         }
         h->ref = q;
         return MGSB_OK;
@@ -783,8 +778,7 @@ mgsb_status rebuild(mgsb_solver* h) {
         h->local_blocks = (int)P.lblock.size();
     } else {
         TRY(dupload(h, pool, &h->slot_of, P.slot_of));
-        h->ref = RefPlan{};
-        h->ref_stale = true;   // planned before the next frame, by when a coarse level has its triangles
+        h->ref_stale = true;   // brought up to date before the next frame, by when a coarse level has its triangles
     }
     h->h_inv = P.h_inv;
     h->h_ac = P.h_ac;
@@ -1082,7 +1076,9 @@ struct RefTris {
 };
 
 // One launch for all of them: the plan is there, and has the triangles that the frame asks for.
-bool ref_one_launch(const mgsb_solver* h, const RefTris& tris) { return h->ref.bytes && (!tris.push || h->ref.with_tris == tris.n); }
+bool ref_one_launch(const mgsb_solver* h, const RefTris& tris) {
+    return h->ref.bytes && h->p.iterations > 0 && (!tris.push || h->ref.with_tris == tris.n);
+}
 
 void enqueue_ref_iterations(mgsb_solver* h, int drop_small, int last_iter, const RefTris& tris, const RefPredict* predict) {
     const int n = h->N0, T = h->T;
@@ -2317,18 +2313,37 @@ void enqueue_frame(mgsb_solver* h) {
         enqueue_ref_frame(h);
 }
 
-// k_ref_iterations' plan, if it is older than the set-up or the triangles.
+// k_ref_iterations' plan, if it is older than the triangles, and what it holds of the set-up, if older than that.
 mgsb_status ready_ref(mgsb_solver* h) {
     if (!h->ref_stale) return MGSB_OK;
     CUDA_TRY(h, cudaSetDevice(h->device));
-    h->ref = RefPlan{};
-    TRY(plan_ref(h));
+    if (!h->ref_planned && h->p.iterations > 0) {
+        TRY(plan_ref(h));
+        h->ref_planned = true;
+    }
+    RefPlan& q = h->ref;
+    if (q.bytes) {
+        q.from_a = h->tA;
+        q.from_b = h->tB;
+        q.from_c = h->tC;
+        std::vector<float> omega(h->p.iterations);   // Chebyshev factors
+        float wi = 1.0f;
+        for (float& o : omega) o = wi = 4 / (4 - h->p.cheb_rho * h->p.cheb_rho * wi);
+        float* dom = nullptr;
+        TRY(dupload(h, h->derived_mem, &dom, omega));
+        q.omega = dom;
+        if (q.grid) CUDA_TRY(h, cudaMemset(q.barrier, 0, 2 * sizeof(int32_t)));
+    }
     h->ref_stale = false;
     return MGSB_OK;
 }
 
+// For calls that look at what was set up.
+mgsb_status ensure_set_up(mgsb_solver* h) { return h->dirty ? rebuild(h) : MGSB_OK; }
+
+// For calls that run a frame: the plans of its kernels too.
 mgsb_status ensure_ready(mgsb_solver* h) {
-    if (h->dirty) TRY(rebuild(h));
+    TRY(ensure_set_up(h));
     TRY(ready_ref(h));
     return ready_staged(h);
 }
@@ -2928,7 +2943,7 @@ mgsb_status mgsb_get_device_positions(mgsb_solver* h, int32_t body, const float*
 mgsb_status mgsb_get_normals(mgsb_solver* h, int32_t body, float* out) {
     if (!out) return MGSB_INVALID_ARG;
     TRY(check_body(h, body));
-    TRY(ensure_ready(h));
+    TRY(ensure_set_up(h));
     return run_normals(h, body, h->nrm_face, out);
 }
 
@@ -2964,7 +2979,7 @@ mgsb_status mgsb_set_state(mgsb_solver* h, int32_t body, const float* positions,
 mgsb_status mgsb_get_energy(mgsb_solver* h, int32_t body, double out[5]) {
     if (!out) return MGSB_INVALID_ARG;
     TRY(check_body(h, body));
-    TRY(ensure_ready(h));
+    TRY(ensure_set_up(h));
     const BodyHost& B = h->bodies[body];
     const mgsb_params& p = h->p;
     EnergyArgs a{};
@@ -3185,7 +3200,7 @@ mgsb_status mgsb_set_broad_phase(mgsb_solver* h, int32_t on) {
     if (!is_mg(h)) return set_err(h, MGSB_NOT_SUPPORTED, "the broad phase applies to the multigrid kinds");
     if (on && h->tri_contact)
         return set_err(h, MGSB_NOT_SUPPORTED, "the broad phase bins vertices only: turn the triangle contact off first");
-    TRY(ensure_ready(h));
+    TRY(ensure_set_up(h));
     CUDA_TRY(h, cudaSetDevice(h->device));
     h->broad_phase = on != 0;
     invalidate_graph(h);
@@ -3224,7 +3239,7 @@ mgsb_status mgsb_set_launch_overlap(mgsb_solver* h, int32_t on) {
 mgsb_status mgsb_set_coarse_dense(mgsb_solver* h, int32_t on) {
     if (!h || (on != 0 && on != 1)) return MGSB_INVALID_ARG;
     if (!is_mg(h)) return set_err(h, MGSB_NOT_SUPPORTED, "the coarse operator applies to the multigrid kind");
-    TRY(ensure_ready(h));
+    TRY(ensure_set_up(h));
     if (on && (h->fuse_l0 || !dense_eligible(h, h->split)))
         return set_err(h, MGSB_NOT_SUPPORTED,
                        "the dense coarse operator needs one body, at most %d rows on the coarse split's level "
@@ -3238,7 +3253,7 @@ mgsb_status mgsb_set_coarse_dense(mgsb_solver* h, int32_t on) {
 
 mgsb_status mgsb_get_coarse_dense(mgsb_solver* h, int32_t* on) {
     if (!h || !on) return MGSB_INVALID_ARG;
-    TRY(ensure_ready(h));
+    TRY(ensure_set_up(h));
     *on = h->dense_op ? 1 : 0;
     return MGSB_OK;
 }
@@ -3246,7 +3261,7 @@ mgsb_status mgsb_get_coarse_dense(mgsb_solver* h, int32_t* on) {
 mgsb_status mgsb_get_coarse_split(mgsb_solver* h, int32_t* split) {
     if (!h || !split) return MGSB_INVALID_ARG;
     if (!is_mg(h)) return set_err(h, MGSB_NOT_SUPPORTED, "the coarse split applies to the multigrid kind");
-    TRY(ensure_ready(h));
+    TRY(ensure_set_up(h));
     *split = h->fuse_l0 ? 1 : h->split;
     return MGSB_OK;
 }
@@ -3423,7 +3438,7 @@ mgsb_status mgsb_launches_per_frame(const mgsb_solver* h, int32_t* n) {
 
 mgsb_status mgsb_get_precompute(mgsb_solver* h, float* inv_dm, float* ac, float* volume, float* mass, float* diag) {
     if (!h) return MGSB_INVALID_ARG;
-    TRY(ensure_ready(h));
+    TRY(ensure_set_up(h));
     if (inv_dm) std::copy(h->h_inv.begin(), h->h_inv.end(), inv_dm);
     if (ac) std::copy(h->h_ac.begin(), h->h_ac.end(), ac);
     if (volume) std::copy(h->h_vol.begin(), h->h_vol.end(), volume);
@@ -3434,7 +3449,7 @@ mgsb_status mgsb_get_precompute(mgsb_solver* h, float* inv_dm, float* ac, float*
 
 mgsb_status mgsb_level_size(mgsb_solver* h, int32_t level, int32_t* num_verts, int32_t* nnz_offdiag) {
     if (!h || !num_verts || !nnz_offdiag) return MGSB_INVALID_ARG;
-    TRY(ensure_ready(h));
+    TRY(ensure_set_up(h));
     if (level < 0 || level >= (int32_t)h->lev.size()) return set_err(h, MGSB_INVALID_ARG, "level %d out of range", level);
     *num_verts = h->lev[level].n;
     *nnz_offdiag = h->lev[level].nnz;
@@ -3460,7 +3475,7 @@ mgsb_status mgsb_level_info(mgsb_solver* h, int32_t level, int32_t info[8]) {
 mgsb_status mgsb_body_level_size(mgsb_solver* h, int32_t body, int32_t level, int32_t* n) {
     if (!h || !n) return MGSB_INVALID_ARG;
     TRY(check_body(h, body));
-    TRY(ensure_ready(h));
+    TRY(ensure_set_up(h));
     if (!is_mg(h)) return set_err(h, MGSB_NOT_SUPPORTED, "levels exist in the multigrid kinds only");
     if (level < 0 || level >= h->p.levels) return set_err(h, MGSB_INVALID_ARG, "level %d out of range", level);
     *n = h->range_host[(size_t)body * h->p.levels + level].y;
@@ -3970,6 +3985,7 @@ mgsb_status mgsb_mg2_create(const mgsb_mesh* coarse, const mgsb_mesh* fine, cons
     t->coarse->ref_tris = t4;
     t->coarse->ref_tri_ptr = ptr;
     t->coarse->ref_tri_idx = idx;
+    t->coarse->ref_planned = false;
     t->coarse->ref_stale = true;
     TRY(tl_upload(t.get(), &t->tris, t4.data(), t4.size()));
     TRY(tl_upload(t.get(), &t->tri_ptr, ptr.data(), ptr.size()));

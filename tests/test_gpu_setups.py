@@ -1,0 +1,43 @@
+"""Plans that are kept over set-ups: a solver whose masks, stiffness and iterations change between frames moves in the
+bits of one that was made anew for each frame."""
+import numpy as np
+import pytest
+
+import multigridsoftbody_b200 as mg
+
+from .common import beam
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dims", [(3, 12, 3), (8, 42, 8), (16, 160, 16)])   # one cluster, the grid, launches
+def test_reference_frames_over_set_ups(lib, dims):
+    m, fixed = beam(*dims)
+    half = (m.positions[:, 1] > 0).astype(np.uint8)
+    steps = [dict(), dict(mask=half), dict(iterations=3), dict(iterations=0), dict(volume_stiffness=2000.0),
+             dict(iterations=9, cheb_rho=0.9), dict(mask=fixed, dt=0.01)]
+    params = dict(iterations=5, gravity=(0.0, -9.8, 0.0))
+    make = lambda: mg.Solver(m, mg.default_params(mg.SOLVER_REFERENCE_JACOBI, **params))
+    s, mask = make(), fixed
+    s.set_fixed(mask)
+    flags = np.zeros(len(m.positions), np.int32)
+    x, v = m.positions, np.zeros_like(m.positions)
+    for k, change in enumerate(steps):
+        mask = change.pop("mask", mask)
+        params.update(change)
+        if change:
+            s.set_params(**change)
+        s.set_fixed(mask)
+        fresh = make()
+        fresh.set_fixed(mask)
+        fresh.set_state(x, v)
+        for q in (s, fresh):
+            q.set_spheres([[1.5 - 0.03 * k, -3.0, 0.0]], [0.8])
+            q.step()
+        x, v = s.positions(), s.velocities()
+        assert np.array_equal(x, fresh.positions()) and np.array_equal(v, fresh.velocities()), (k, change)
+        if params["iterations"]:   # a frame without iterations finds no contact: the flags stay the last ones
+            flags = fresh.contact_flags()
+        assert np.array_equal(s.contact_flags(), flags)
+        fresh.close()
+    s.close()

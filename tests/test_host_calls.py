@@ -6,7 +6,7 @@ import multigridsoftbody_b200 as mg
 from multigridsoftbody_b200 import _lib as L
 
 from .common import beam
-from .host_only import CAPTURES, GRAPH_LAUNCHES, Host, build_host_only
+from .host_only import CAPTURES, GRAPH_LAUNCHES, UPLOADED, Host, build_host_only
 
 
 @pytest.fixture(scope="module")
@@ -78,3 +78,46 @@ def test_autotune_offers_the_solvers_own_choice(host, dims, levels, bodies):
     s.step()
     assert host.launches("k_coarse_vcycle")[0] == own and s.launches_per_frame() == frame
     s.close()
+
+
+def test_reference_plan_is_made_once_and_for_frames_only(host):
+    m, fixed = beam(4, 40, 4)
+    p = mg.default_params(mg.SOLVER_REFERENCE_JACOBI)
+    s = mg.Solver(m, p)
+    s.set_fixed(fixed)
+    s.normals()
+    s.energy()
+    assert not host.launches("k_ref_image")
+    s.step()
+    assert len(host.launches("k_ref_image")) == 1 and len(host.launches("k_ref_iterations")) == 1
+    for change in range(3):   # it depends on the mesh alone
+        s.set_fixed(fixed if change else 1 - fixed)
+        if change == 1:
+            s.set_params(mg.default_params(mg.SOLVER_REFERENCE_JACOBI, iterations=7))
+        s.step()
+    assert len(host.launches("k_ref_image")) == 1 and len(host.launches("k_ref_iterations")) == 4
+    s.close()
+    host.reset()
+    t = _two_level()
+    assert not host.launches("k_ref_image")
+    t.step()
+    assert len(host.launches("k_ref_image")) == 2
+    t.close()
+
+
+@pytest.mark.parametrize("call", ["normals", "energy", "coarse_dense", "coarse_split", "precompute", "set_coarse_dense"])
+def test_coarse_images_are_made_for_frames_only(host, call):
+    m, fixed = beam(4, 40, 4)
+    uploaded = []
+    for first in (call, "step"):
+        s = mg.Solver(m, mg.default_params(mg.SOLVER_MULTIGRID, levels=3))
+        s.set_fixed(fixed)
+        host.reset()
+        {"set_coarse_dense": lambda: s.set_coarse_dense(False)}.get(first, getattr(s, first))()
+        uploaded.append(host.count(UPLOADED))
+        if first != "step":   # the rest is made by the first frame
+            s.step()
+            uploaded.append(host.count(UPLOADED))
+        s.close()
+    own, frame, whole = uploaded
+    assert frame == whole and own < whole - 100_000
