@@ -76,7 +76,96 @@ void build_ell(const std::vector<int32_t>& ptr, const std::vector<int32_t>& col,
     }
 }
 
-bool build_plan(std::vector<PlanBody>& bodies, const mgsb_params& p, Plan& P, std::string& err) {
+// The places of the right-hand-side slots, from the meshes alone.
+static bool build_slots(const std::vector<PlanBody>& bodies, bool mg, Plan& P, std::string& err) {
+    const int N0 = P.N0, T = P.T;
+    // RHS slots, sliced like the matrices: slot k of vertex i at slot_ptr[i / 8] + 8 k + i % 8, so that neighbouring
+    // lanes read neighbouring slots; a slice is as deep as its deepest vertex (the slots past a vertex's own stay zero).
+    std::vector<int32_t> depth(N0, 0), fill;
+    auto place_slots = [&]() -> bool {   // from depth: slot_ptr and the vertices' first slots
+        const int ns = (N0 + kSlotSlice - 1) / kSlotSlice;
+        P.slot_ptr.assign(ns + 1, 0);
+        int64_t total = 0;
+        for (int s = 0; s < ns; ++s) {
+            int w = 0;
+            for (int i = s * kSlotSlice; i < std::min(N0, (s + 1) * kSlotSlice); ++i) w = std::max(w, depth[i]);
+            total += (int64_t)w * kSlotSlice;
+            if (total > INT32_MAX) {
+                err = "too many right-hand-side slots";
+                return false;
+            }
+            P.slot_ptr[s + 1] = (int32_t)total;
+        }
+        fill.resize(N0);
+        for (int i = 0; i < N0; ++i) fill[i] = P.slot_ptr[i / kSlotSlice] + i % kSlotSlice;
+        return true;
+    };
+    auto next_slot = [&](int i) {
+        const int32_t q = fill[i];
+        fill[i] += kSlotSlice;
+        return q;
+    };
+    if (!mg) {   // one per (tet, corner), tets ascending within a vertex
+        P.slot_of.assign(T, int4{0, 0, 0, 0});
+        for (int t = 0; t < T; ++t)
+            for (int i : {P.tets[t].x, P.tets[t].y, P.tets[t].z, P.tets[t].w}) ++depth[i];
+        if (!place_slots()) return false;
+        for (int t = 0; t < T; ++t) {
+            const int4 v = P.tets[t];
+            const int32_t x = next_slot(v.x), y = next_slot(v.y), z = next_slot(v.z), w = next_slot(v.w);
+            P.slot_of[t] = int4{x, y, z, w};
+        }
+    } else {     // one per vertex of a block, blocks ascending within a vertex; a block holds tets of one body
+        P.ltet.resize(T);
+        P.lent.resize(4 * (size_t)T);
+        P.lblock.reserve((size_t)T / kLocalTets + bodies.size());
+        std::vector<int32_t> local(N0, -1);   // a vertex's place among its block's, while that block is worked on
+        int32_t ids[4 * kLocalTets];
+        uint16_t corner[4 * kLocalTets], many[4 * kLocalTets], next[4 * kLocalTets];
+        for (const PlanBody& B : bodies)
+            for (int t0 = B.t_off; t0 < B.t_off + B.T; t0 += kLocalTets) {
+                const int nt = std::min(kLocalTets, B.t_off + B.T - t0);
+                int nv = 0;
+                for (int t = 0; t < nt; ++t) {
+                    const int4 v = P.tets[t0 + t];
+                    const int c[4] = {v.x, v.y, v.z, v.w};
+                    for (int a = 0; a < 4; ++a) {
+                        int32_t l = local[c[a]];
+                        if (l < 0) {
+                            l = local[c[a]] = nv;
+                            ids[nv] = c[a];
+                            many[nv++] = 0;
+                        }
+                        corner[4 * t + a] = (uint16_t)l;
+                        ++many[l];
+                    }
+                    P.ltet[t0 + t] = ushort4{corner[4 * t], corner[4 * t + 1], corner[4 * t + 2], corner[4 * t + 3]};
+                }
+                const size_t at = P.lv_id.size();
+                P.lblock.push_back(int4{t0, nt, (int)at, nv});
+                P.max_local = std::max(P.max_local, nv);
+                P.lv_id.resize(at + nv);
+                P.lv_range.resize(at + nv);
+                for (int k = 0, beg = 0; k < nv; ++k) {
+                    next[k] = (uint16_t)beg;
+                    P.lv_id[at + k] = ids[k];
+                    P.lv_range[at + k] = ushort2{(uint16_t)beg, (uint16_t)(beg + many[k])};
+                    beg += many[k];
+                    ++depth[ids[k]];
+                    local[ids[k]] = -1;
+                }
+                uint16_t* ent = &P.lent[4 * (size_t)t0];
+                for (int t = 0; t < nt; ++t)
+                    for (int a = 0; a < 4; ++a) ent[next[corner[4 * t + a]]++] = (uint16_t)(a * kLocalTets + t);
+            }
+        if (!place_slots()) return false;
+        P.lv_slot.resize(P.lv_id.size());
+        for (size_t k = 0; k < P.lv_id.size(); ++k) P.lv_slot[k] = next_slot(P.lv_id[k]);
+    }
+    return true;
+}
+
+bool build_plan(std::vector<PlanBody>& bodies, const mgsb_params& p, Plan& P, std::string& err, bool with_slots) {
     const bool mg = p.solver == MGSB_SOLVER_MULTIGRID;
     P = Plan();
     int N0 = 0, T = 0;
@@ -166,83 +255,7 @@ bool build_plan(std::vector<PlanBody>& bodies, const mgsb_params& p, Plan& P, st
             }
         }
     }
-    // RHS slots, sliced like the matrices: slot k of vertex i at slot_ptr[i / 8] + 8 k + i % 8, so that neighbouring
-    // lanes read neighbouring slots; a slice is as deep as its deepest vertex (the slots past a vertex's own stay zero).
-    std::vector<int32_t> depth(N0, 0), fill;
-    auto place_slots = [&]() -> bool {   // from depth: slot_ptr and the vertices' first slots
-        const int ns = (N0 + kSlotSlice - 1) / kSlotSlice;
-        P.slot_ptr.assign(ns + 1, 0);
-        int64_t total = 0;
-        for (int s = 0; s < ns; ++s) {
-            int w = 0;
-            for (int i = s * kSlotSlice; i < std::min(N0, (s + 1) * kSlotSlice); ++i) w = std::max(w, depth[i]);
-            total += (int64_t)w * kSlotSlice;
-            if (total > INT32_MAX) {
-                err = "too many right-hand-side slots";
-                return false;
-            }
-            P.slot_ptr[s + 1] = (int32_t)total;
-        }
-        fill.resize(N0);
-        for (int i = 0; i < N0; ++i) fill[i] = P.slot_ptr[i / kSlotSlice] + i % kSlotSlice;
-        return true;
-    };
-    auto next_slot = [&](int i) {
-        const int32_t q = fill[i];
-        fill[i] += kSlotSlice;
-        return q;
-    };
-    if (!mg) {   // one per (tet, corner), tets ascending within a vertex
-        P.slot_of.assign(T, int4{0, 0, 0, 0});
-        for (int t = 0; t < T; ++t)
-            for (int i : {P.tets[t].x, P.tets[t].y, P.tets[t].z, P.tets[t].w}) ++depth[i];
-        if (!place_slots()) return false;
-        for (int t = 0; t < T; ++t) {
-            const int4 v = P.tets[t];
-            const int32_t x = next_slot(v.x), y = next_slot(v.y), z = next_slot(v.z), w = next_slot(v.w);
-            P.slot_of[t] = int4{x, y, z, w};
-        }
-    } else {     // one per vertex of a block, blocks ascending within a vertex; a block holds tets of one body
-        P.ltet.resize(T);
-        P.lent.resize(4 * (size_t)T);
-        std::vector<int32_t> local(N0, -1), ids;
-        std::vector<std::vector<uint16_t>> contrib;
-        for (const PlanBody& B : bodies)
-            for (int t0 = B.t_off; t0 < B.t_off + B.T; t0 += kLocalTets) {
-                const int nt = std::min(kLocalTets, B.t_off + B.T - t0);
-                ids.clear();
-                for (int t = 0; t < nt; ++t) {
-                    const int4 v = P.tets[t0 + t];
-                    const int c[4] = {v.x, v.y, v.z, v.w};
-                    uint16_t l[4];
-                    for (int a = 0; a < 4; ++a) {
-                        if (local[c[a]] < 0) {
-                            local[c[a]] = (int32_t)ids.size();
-                            ids.push_back(c[a]);
-                            if (contrib.size() < ids.size()) contrib.emplace_back();
-                        }
-                        l[a] = (uint16_t)local[c[a]];
-                        contrib[l[a]].push_back((uint16_t)(a * kLocalTets + t));
-                    }
-                    P.ltet[t0 + t] = ushort4{l[0], l[1], l[2], l[3]};
-                }
-                P.lblock.push_back(int4{t0, nt, (int)P.lv_id.size(), (int)ids.size()});
-                P.max_local = std::max(P.max_local, (int)ids.size());
-                int at = 0;
-                for (size_t k = 0; k < ids.size(); ++k) {
-                    const int beg = at;
-                    for (uint16_t e : contrib[k]) P.lent[4 * (size_t)t0 + at++] = e;
-                    contrib[k].clear();
-                    P.lv_id.push_back(ids[k]);
-                    P.lv_range.push_back(ushort2{(uint16_t)beg, (uint16_t)at});
-                    ++depth[ids[k]];
-                    local[ids[k]] = -1;
-                }
-            }
-        if (!place_slots()) return false;
-        P.lv_slot.resize(P.lv_id.size());
-        for (size_t k = 0; k < P.lv_id.size(); ++k) P.lv_slot[k] = next_slot(P.lv_id[k]);
-    }
+    if (with_slots && !build_slots(bodies, mg, P, err)) return false;
     if (!mg) return true;
 
     // CSR of the off-diagonal part of the level built last, and the first row

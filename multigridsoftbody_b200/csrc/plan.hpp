@@ -106,6 +106,6 @@ constexpr int kSliceCoarse = 4;   // 8 lanes per row on coarse levels
 mgsb_status make_body(const mgsb_mesh& m, const mgsb_params& p, bool multigrid, PlanBody& B, std::string& err);
 
 // Builds the plan; also (re)builds each body's multigrid hierarchy.
-bool build_plan(std::vector<PlanBody>& bodies, const mgsb_params& p, Plan& out, std::string& err);
+bool build_plan(std::vector<PlanBody>& bodies, const mgsb_params& p, Plan& out, std::string& err, bool with_slots = true);
 
 }  // namespace mgsb

@@ -157,8 +157,11 @@ struct mgsb_solver {
     bool ref_planned = false, ref_stale = false;
     std::vector<int4> ref_tris;
     std::vector<int32_t> ref_tri_ptr, ref_tri_idx;
+    // right-hand-side slots and their places, which depend on the mesh alone and are kept over set-ups, in mesh_mem
     int32_t* slot_ptr = nullptr;
     float4* slots = nullptr;
+    std::vector<DevMem> mesh_mem;
+    bool mesh_ready = false;
     // multigrid: the local step's blocks, and the mixed kind's slots
     LocalArgs local{};
     int local_blocks = 0;
@@ -271,6 +274,7 @@ mgsb_solver::~mgsb_solver() {
     if (graph) cudaGraphDestroy(graph);
     for (auto& m : derived_mem) cudaFree(m.p);
     for (auto& m : ref_mem) cudaFree(m.p);
+    for (auto& m : mesh_mem) cudaFree(m.p);
     for (auto& m : state_mem) cudaFree(m.p);
     for (auto& m : pair_mem) cudaFree(m.p);
     delete[] bodies_host;
@@ -716,6 +720,42 @@ mgsb_status plan_ref(mgsb_solver* h) {
     return MGSB_OK;
 }
 
+// Right-hand-side slots (zero: those past a vertex's own stay so), their places, and the multigrid kinds' local blocks.
+mgsb_status upload_slots(mgsb_solver* h, const Plan& P) {
+    auto& pool = h->mesh_mem;
+    free_pool(pool);
+    const size_t n = (size_t)P.slot_ptr.back();
+    TRY(dupload(h, pool, &h->slot_ptr, P.slot_ptr));
+    if (is_mg(h) && h->p.precision == MGSB_PRECISION_MIXED) {
+        TRY(dalloc(h, pool, &h->slots64, n));
+        CUDA_TRY(h, cudaMemset(h->slots64, 0, n * sizeof(double4)));
+    } else {
+        TRY(dalloc(h, pool, &h->slots, n));
+        CUDA_TRY(h, cudaMemset(h->slots, 0, n * sizeof(float4)));
+    }
+    if (is_mg(h)) {
+        LocalArgs& A = h->local;
+        auto up = [&](auto& out, const auto& v) {
+            std::remove_const_t<std::remove_pointer_t<std::remove_reference_t<decltype(out)>>>* p = nullptr;
+            const mgsb_status st = dupload(h, pool, &p, v);
+            out = p;
+            return st;
+        };
+        TRY(up(A.block, P.lblock));
+        TRY(up(A.tet, P.ltet));
+        TRY(up(A.id, P.lv_id));
+        TRY(up(A.slot, P.lv_slot));
+        TRY(up(A.range, P.lv_range));
+        TRY(up(A.ent, P.lent));
+        A.most = P.max_local;
+        h->local_blocks = (int)P.lblock.size();
+    } else {
+        TRY(dupload(h, pool, &h->slot_of, P.slot_of));
+    }
+    h->mesh_ready = true;
+    return MGSB_OK;
+}
+
 mgsb_status rebuild(mgsb_solver* h) {
     CUDA_TRY(h, cudaSetDevice(h->device));
     CUDA_TRY(h, cudaStreamSynchronize(h->stream));
@@ -735,7 +775,7 @@ mgsb_status rebuild(mgsb_solver* h) {
     const bool mg = is_mg(h);
     Plan P;
     std::string perr;
-    if (!build_plan(h->bodies, h->p, P, perr)) return set_err(h, MGSB_INVALID_ARG, "%s", perr.c_str());
+    if (!build_plan(h->bodies, h->p, P, perr, !h->mesh_ready)) return set_err(h, MGSB_INVALID_ARG, "%s", perr.c_str());
     const int N0 = P.N0;
     TRY(dupload(h, pool, &h->body_of, P.body_of));
     TRY(dupload(h, pool, &h->fixf, P.fixf));
@@ -745,39 +785,16 @@ mgsb_status rebuild(mgsb_solver* h) {
     TRY(dupload(h, pool, &h->tA, P.tA));
     TRY(dupload(h, pool, &h->tB, P.tB));
     TRY(dupload(h, pool, &h->tC, P.tC));
-    TRY(dupload(h, pool, &h->slot_ptr, P.slot_ptr));
-    if (mg && h->p.precision == MGSB_PRECISION_MIXED) {
-        TRY(dalloc(h, pool, &h->slots64, (size_t)P.slot_ptr.back()));
-        CUDA_TRY(h, cudaMemset(h->slots64, 0, (size_t)P.slot_ptr.back() * sizeof(double4)));
-    } else {
-        TRY(dalloc(h, pool, &h->slots, (size_t)P.slot_ptr.back()));
-        CUDA_TRY(h, cudaMemset(h->slots, 0, (size_t)P.slot_ptr.back() * sizeof(float4)));
-    }
+    if (!h->mesh_ready) TRY(upload_slots(h, P));
     if (mg) {
-        LocalArgs& A = h->local;
-        auto up = [&](auto& out, const auto& v) {
-            std::remove_const_t<std::remove_pointer_t<std::remove_reference_t<decltype(out)>>>* p = nullptr;
-            const mgsb_status st = dupload(h, pool, &p, v);
-            out = p;
-            return st;
-        };
-        TRY(up(A.block, P.lblock));
-        TRY(up(A.tet, P.ltet));
-        TRY(up(A.id, P.lv_id));
-        TRY(up(A.slot, P.lv_slot));
-        TRY(up(A.range, P.lv_range));
-        TRY(up(A.ent, P.lent));
-        A.gA = h->tA;
-        A.gB = h->tB;
-        A.gC = h->tC;
-        A.most = P.max_local;
+        h->local.gA = h->tA;
+        h->local.gB = h->tB;
+        h->local.gC = h->tC;
         CUDA_TRY(h, cudaFuncSetAttribute(k_mg_local, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)local_smem_bytes(4 * kLocalTets)));
         CUDA_TRY(h, cudaFuncSetAttribute(k_mg_local64, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)local_smem_bytes(4 * kLocalTets)));
-        h->local_blocks = (int)P.lblock.size();
     } else {
-        TRY(dupload(h, pool, &h->slot_of, P.slot_of));
         h->ref_stale = true;   // brought up to date before the next frame, by when a coarse level has its triangles
     }
     h->h_inv = P.h_inv;

@@ -41,3 +41,32 @@ def test_reference_frames_over_set_ups(lib, dims):
         assert np.array_equal(s.contact_flags(), flags)
         fresh.close()
     s.close()
+
+
+@pytest.mark.parametrize("precision", [mg.PRECISION_FP32, mg.PRECISION_MIXED])
+@pytest.mark.parametrize("dims", [[(3, 12, 3)], [(7, 35, 6)], [(2, 5, 2), (4, 19, 3)]])   # whole V-cycle, coarse part, batch
+def test_multigrid_frames_over_set_ups(lib, dims, precision):
+    bodies = [beam(*d) for d in dims]
+    steps = [dict(), dict(flip=True), dict(iterations=3), dict(youngs=4e4), dict(iterations=6, pre_sweeps=1, dt=0.01)]
+    params = dict(iterations=4, levels=3, gravity=(0.0, -9.8, 0.0), precision=precision)
+    make = lambda: mg.Solver([m for m, _ in bodies], mg.default_params(mg.SOLVER_MULTIGRID, **params))
+    s, flip, youngs = make(), False, None
+    state = [(m.positions, np.zeros_like(m.positions)) for m, _ in bodies]
+    for change in steps:
+        flip, youngs = change.pop("flip", flip), change.pop("youngs", youngs)
+        params.update(change)
+        if change:
+            s.set_params(**change)
+        fresh = make()
+        for q in (s, fresh):
+            for b, (m, fixed) in enumerate(bodies):
+                q.set_fixed(1 - fixed if flip else fixed, body=b)
+                if youngs:
+                    q.set_material(youngs, 0.3, body=b)
+                q.set_state(*state[b], body=b)
+            q.step(2)
+        state = [(s.positions(b), s.velocities(b)) for b in range(len(bodies))]
+        for b, (x, v) in enumerate(state):
+            assert np.isfinite(x).all() and np.array_equal(x, fresh.positions(b)) and np.array_equal(v, fresh.velocities(b))
+        fresh.close()
+    s.close()

@@ -121,3 +121,18 @@ def test_coarse_images_are_made_for_frames_only(host, call):
         s.close()
     own, frame, whole = uploaded
     assert frame == whole and own < whole - 100_000
+
+
+@pytest.mark.parametrize("solver,precision", [(mg.SOLVER_REFERENCE_JACOBI, 0), (mg.SOLVER_MULTIGRID, mg.PRECISION_FP32),
+                                              (mg.SOLVER_MULTIGRID, mg.PRECISION_MIXED)])
+def test_slots_are_placed_once(host, solver, precision):
+    m, fixed = beam(4, 40, 4)
+    s = mg.Solver(m, mg.default_params(solver, precision=precision))
+    state = (5 * 16 + 32 * precision) * m.num_verts   # positions, predictions and earlier ones; FP64 ones of the mixed kind
+    made = host.count(UPLOADED) - state
+    host.reset()
+    s.set_fixed(fixed)
+    s.normals()
+    # 16 bytes per tet of the reference kind; 8 + 8 of the multigrid kinds and more per vertex of a block
+    assert 0 < host.count(UPLOADED) <= made - 16 * m.num_tets
+    s.close()
