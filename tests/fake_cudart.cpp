@@ -19,7 +19,7 @@ struct Launch {
 std::map<const void*, std::string> kernels;
 std::vector<Launch> launches;
 std::string refused;
-long counts[4];   // captures, graph launches, stream synchronisations, bytes copied to the device
+long counts[5];   // captures, graph launches, stream synchronisations, bytes copied to the device, pinned allocations
 cudaError_t last = cudaSuccess;
 char token[8];    // what handles point at
 
@@ -89,7 +89,7 @@ cudaError_t cudaMalloc(void** p, size_t n) {
     *p = aligned_alloc(256, size);
     return *p ? memset(*p, 0, size), cudaSuccess : cudaErrorMemoryAllocation;
 }
-cudaError_t cudaMallocHost(void** p, size_t n) { return cudaMalloc(p, n); }
+cudaError_t cudaMallocHost(void** p, size_t n) { return ++counts[4], cudaMalloc(p, n); }
 cudaError_t cudaFree(void* p) { return free(p), cudaSuccess; }
 cudaError_t cudaFreeHost(void* p) { return free(p), cudaSuccess; }
 cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind k, cudaStream_t) {

@@ -1,12 +1,14 @@
 """What the solvers' host code does when the runtime refuses a launch, and when set-up changes behind a captured frame:
 the library over a stand-in for the CUDA runtime."""
+import numpy as np
 import pytest
 
 import multigridsoftbody_b200 as mg
 from multigridsoftbody_b200 import _lib as L
+from multigridsoftbody_b200.learned import MLP
 
 from .common import beam
-from .host_only import CAPTURES, GRAPH_LAUNCHES, UPLOADED, Host, build_host_only
+from .host_only import CAPTURES, GRAPH_LAUNCHES, PINNED, UPLOADED, Host, build_host_only
 
 
 @pytest.fixture(scope="module")
@@ -136,3 +138,11 @@ def test_slots_are_placed_once(host, solver, precision):
     # 16 bytes per tet of the reference kind; 8 + 8 of the multigrid kinds and more per vertex of a block
     assert 0 < host.count(UPLOADED) <= made - 16 * m.num_tets
     s.close()
+
+
+@pytest.mark.parametrize("rows", [1, 128, 100_000])
+def test_inference_pins_no_memory(host, rows):
+    net = MLP(device=0, seed=0)
+    y = net.forward(np.zeros((rows, 9), np.float32))
+    assert y.shape == (rows, 3) and host.count(PINNED) == 0
+    net.close()
