@@ -54,7 +54,6 @@ struct CoarseArgs {
     const double* Ainv64;    // FP64 coarsest inverse (mixed precision), else null
     const float4* b;         // level-0 right-hand side
     float4* d;               // level-0 unknown (displacement)
-    const int32_t* gate;     // if set, the kernel runs only when *gate != 0 (learned-smoother fallback)
     // level-1 right-hand side straight from level 0 (host launches only): with res0_b set, level 1's
     // restriction forms R (res0_b - D0 d) - RO d, RO = R Off(level 0), and lv[0].res is not read
     const float4* res0_b;
@@ -334,9 +333,8 @@ __global__ void __launch_bounds__(256, kRowCtas) k_l0_residual_rg(int n, const i
 
 // Level-0 prolongation d += P e1 (used when the coarse kernel does not fuse it).
 __global__ void k_l0_prolong(int n, const int4* __restrict__ pid, const float4* __restrict__ pw,
-                             const float4* __restrict__ ec, float4* __restrict__ v, const int32_t* __restrict__ gate = nullptr) {
+                             const float4* __restrict__ ec, float4* __restrict__ v) {
     pdl_enter();
-    if (gate && __ldg(gate) == 0) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int4 id = __ldg(pid + i);
@@ -394,8 +392,7 @@ __global__ void __launch_bounds__(256) k_lvl_restrict_res0(int n, const int32_t*
                                                            const float* __restrict__ roval,
                                                            const float4* __restrict__ b0, const float* __restrict__ dfull0,
                                                            const float4* __restrict__ d0, const float* __restrict__ dinv,
-                                                           float4* __restrict__ r, float4* __restrict__ e,
-                                                           const int32_t* __restrict__ gate) {
+                                                           float4* __restrict__ r, float4* __restrict__ e) {
     pdl_trigger();
     constexpr int G = kLanesC, S = 32 / G;
     const int lane = threadIdx.x & 31;
@@ -409,7 +406,6 @@ __global__ void __launch_bounds__(256) k_lvl_restrict_res0(int n, const int32_t*
     HeldEntries<kHeldRO> ho;
     hold_csr_row<G>(ho, valid, lane, obeg, oend, rocol, roval);
     pdl_wait();
-    if (gate && __ldg(gate) == 0) return;
     // R (b0 - D0 d0): this lane's children, in the order of hold_csr_row
     float ax = 0.f, ay = 0.f, az = 0.f;
     auto child = [&](int i, float w) {
@@ -484,10 +480,8 @@ __global__ void __launch_bounds__(256, kRowCtas) k_lvl_residual(int n, const int
 
 // dst = cur + P ec (P: 4 coarse parents per row); dst may be cur.
 __global__ void k_lvl_prolong(int n, const int4* __restrict__ pid, const float4* __restrict__ pw,
-                              const float4* __restrict__ ec, const float4* cur, float4* dst,
-                              const int32_t* __restrict__ gate) {
+                              const float4* __restrict__ ec, const float4* cur, float4* dst) {
     pdl_enter();
-    if (gate && __ldg(gate) == 0) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int4 id = __ldg(pid + i);
@@ -608,7 +602,6 @@ __global__ void __launch_bounds__(256, kProlongCtas)
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(1024) k_coarse_vcycle(const CoarseArgs A) {
     pdl_enter();
-    if (A.gate && __ldg(A.gate) == 0) return;   // uniform over the cluster, before any barrier
     cg::cluster_group cluster = cg::this_cluster();
     const int cs = (int)cluster.num_blocks();
     const int rank = (int)cluster.block_rank();
@@ -833,7 +826,6 @@ __host__ __device__ inline int coarse_smem_float4(const int* nl, int L, int firs
 
 __global__ void __launch_bounds__(1024) k_coarse_vcycle_dsm(const CoarseArgs A) {
     pdl_enter();
-    if (A.gate && __ldg(A.gate) == 0) return;   // uniform over the cluster, before any barrier
     extern __shared__ float4 smv[];
     cg::cluster_group cluster = cg::this_cluster();
     const int cs = (int)cluster.num_blocks();
@@ -1640,7 +1632,6 @@ __host__ __device__ inline int coarse_cta_smem_float4(const int* nl, int L, int 
 
 __global__ void __launch_bounds__(1024) k_coarse_vcycle_cta(const CoarseArgs A) {
     pdl_enter();
-    if (A.gate && __ldg(A.gate) == 0) return;
     const int body = blockIdx.x;
     extern __shared__ float4 smv[];
     constexpr int P = kCtaRowGroups;
@@ -2069,8 +2060,7 @@ __global__ void __launch_bounds__(kDenseApplyThreads, 1) k_coarse_apply(int nf, 
                                                                        const float* __restrict__ rw,
                                                                        const float4* __restrict__ res_fine,
                                                                        const float* __restrict__ M,
-                                                                       float4* __restrict__ e,
-                                                                       const int32_t* __restrict__ gate) {
+                                                                       float4* __restrict__ e) {
     pdl_trigger();
     cg::cluster_group cluster = cg::this_cluster();
     extern __shared__ float4 apply_smem[];
@@ -2092,7 +2082,6 @@ __global__ void __launch_bounds__(kDenseApplyThreads, 1) k_coarse_apply(int nf, 
         cw[k] = q < end ? __ldg(rw + q) : 0.f;
     }
     pdl_wait();
-    if (gate && __ldg(gate) == 0) return;   // uniform over the launch: every CTA of the cluster leaves
     const int i = blockIdx.x * kDenseApplyRows + warp;   // this warp's row of M
     float mr[kApplyMRegs];
 #pragma unroll

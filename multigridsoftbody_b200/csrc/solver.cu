@@ -1639,7 +1639,6 @@ mgsb_status launch_coarse(mgsb_solver* h, const CoarseArgs& args_in) {
     const int F = h->fuse_l0 ? 1 : h->split;
     args.first = F;
     args.fuse_prolong = h->fuse_prolong ? 1 : 0;
-    const int32_t* gate = args.gate;
     float4* cur[kMaxLevels] = {};
     for (int l = 1; l < F; ++l) {
         const LevelView& C = args.lv[l];
@@ -1647,7 +1646,7 @@ mgsb_status launch_coarse(mgsb_solver* h, const CoarseArgs& args_in) {
         if (l == 1 && args.res0_b)
             LAUNCH(h, k_lvl_restrict_res0, g, kBlock, 0, C.n, C.rptr, C.rcol, C.rw, args.ro_ptr, args.ro_col,
                    args.ro_val, args.res0_b, args.lv[0].dfull, (const float4*)args.d, args.pre > 0 ? C.dinv : nullptr,
-                   C.r, C.e, gate);
+                   C.r, C.e);
         else
             LAUNCH(h, k_lvl_restrict, g, kBlock, 0, C.n, C.rptr, C.rcol, C.rw, args.lv[l - 1].res,
                    args.pre > 0 ? C.dinv : nullptr, C.r, C.e);
@@ -1680,7 +1679,7 @@ mgsb_status launch_coarse(mgsb_solver* h, const CoarseArgs& args_in) {
         for (int r = 0; r < reps && e == cudaSuccess; ++r)
             e = cudaLaunchKernelEx(&cfg, k_coarse_apply, C.n, (const int32_t*)C.rptr, (const int32_t*)C.rcol,
                                    (const float*)C.rw, (const float4*)args.lv[F - 1].res,
-                                   (const float*)h->dop_result, C.e, gate);
+                                   (const float*)h->dop_result, C.e);
         prof_end(h, "k_coarse_apply");
         ++h->launches;
         if (e != cudaSuccess)
@@ -1707,7 +1706,7 @@ mgsb_status launch_coarse(mgsb_solver* h, const CoarseArgs& args_in) {
         }
         float4* a = (args.post % 2 == 0) ? C.e : C.e2;
         float4* b = (a == C.e) ? C.e2 : C.e;
-        LAUNCH(h, k_lvl_prolong, grid_for(C.n), kBlock, 0, C.n, Cc.pid, Cc.pw, Cc.e, cur[l], a, gate);
+        LAUNCH(h, k_lvl_prolong, grid_for(C.n), kBlock, 0, C.n, Cc.pid, Cc.pw, Cc.e, cur[l], a);
         for (int k = 0; k < args.post; ++k) {
             LAUNCH(h, k_lvl_sweep, g, kBlock, 0, C.n, C.slice_ptr, C.col, C.val, C.dfull, C.dinv, C.r, a, b);
             std::swap(a, b);
@@ -1794,8 +1793,7 @@ void enqueue_l0_residual(mgsb_solver* h, const float4* x, const float4* b) {
 // xa -> xb; on return xa holds the result): the first sweep fused with the
 // prolongation (k_prolong_sweep, from the level-0 residual lv[0].res of the
 // descent) unless disabled.  b: the right-hand side of the sweeps.
-void enqueue_l0_post(mgsb_solver* h, float4*& xa, float4*& xb, float4* b, const int32_t* gate, int post = -1,
-                     bool form_res = false) {
+void enqueue_l0_post(mgsb_solver* h, float4*& xa, float4*& xb, float4* b, int post = -1, bool form_res = false) {
     const mgsb_params& p = h->p;
     if (post < 0) post = p.post_sweeps;
     const int n0 = h->N0;
@@ -1805,12 +1803,11 @@ void enqueue_l0_post(mgsb_solver* h, float4*& xa, float4*& xb, float4* b, const 
     if (h->fuse_prolong && post > 0) {
         LAUNCH(h, k_prolong_sweep<kLanesL0>, grid_slices(n0, l0.S, h->sm_count, kProlongCtas), kBlock, 0, n0, l1.pid, l1.pw,
                l1.e, l0.op_slice_ptr, l0.op_col, l0.op_val, l0.dfull, l0.dinv, form_res ? nullptr : l0.res, xa, xb, nullptr,
-               nullptr,
-               form_res ? b : nullptr, l0.slice_ptr, l0.ell_col, l0.ell_val);
+               nullptr, form_res ? b : nullptr, l0.slice_ptr, l0.ell_col, l0.ell_val);
         std::swap(xa, xb);
         k0 = 1;
     } else {
-        LAUNCH(h, k_l0_prolong, grid_for(n0), kBlock, 0, n0, l1.pid, l1.pw, l1.e, xa, gate);
+        LAUNCH(h, k_l0_prolong, grid_for(n0), kBlock, 0, n0, l1.pid, l1.pw, l1.e, xa);
     }
     for (int k = k0; k < post; ++k) {
         enqueue_l0_sweep(h, xa, xb, b);
@@ -1851,7 +1848,6 @@ void enqueue_learned_vcycle(mgsb_solver* h, float4* d, const float4* b, bool fro
     if (!fr)
         enqueue_l0_residual(h, d, b);
     ca.d = d;
-    ca.gate = nullptr;
     ca.res0_b = fr ? b : nullptr;
     launch_coarse(h, ca);
     // post-smoothing: d += P e1 and the residual the learned sweep starts from
@@ -1862,7 +1858,7 @@ void enqueue_learned_vcycle(mgsb_solver* h, float4* d, const float4* b, bool fro
                h->fixf, h->ls_r,
                fr ? b : nullptr, l0.slice_ptr, l0.ell_col, l0.ell_val);
     } else {
-        LAUNCH(h, k_l0_prolong, grid_for(n0), kBlock, 0, n0, lv[1].pid, lv[1].pw, lv[1].e, d, nullptr);
+        LAUNCH(h, k_l0_prolong, grid_for(n0), kBlock, 0, n0, lv[1].pid, lv[1].pw, lv[1].e, d);
         LAUNCH(h, k_ls_residual, g0, kLsThreads, 0, n0, l0.slice_ptr, l0.ell_col, l0.ell_val, l0.dfull, h->fixf, d, b,
                h->ls_r, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr);
     }
@@ -2185,7 +2181,7 @@ float4* enqueue_mg_solve(mgsb_solver* h, bool learned, const LearnedFallback& fb
             ca.res0_b = fr ? h->b : nullptr;
             launch_coarse(h, ca);
             if (!h->fuse_l0) {   // the shared-memory kernel leaves the level-1 correction in lv[1].e
-                enqueue_l0_post(h, xa, xb, h->b, nullptr, l0_post, fr);
+                enqueue_l0_post(h, xa, xb, h->b, l0_post, fr);
             } else {
                 for (int k = 0; k < l0_post; ++k) {
                     enqueue_l0_sweep(h, xa, xb, h->b);
@@ -2299,7 +2295,7 @@ void enqueue_mixed_solve(mgsb_solver* h, bool learned, const LearnedFallback& fb
             ca.d = ea;
             ca.res0_b = fr ? h->r32 : nullptr;
             launch_coarse(h, ca);
-            enqueue_l0_post(h, ea, eb, h->r32, nullptr, l0_post, fr);
+            enqueue_l0_post(h, ea, eb, h->r32, l0_post, fr);
             LAUNCH(h, k_mx_update, grid_for(n0), kBlock, 0, n0, ea, h->dd64, h->d32);
         }
     }
@@ -3754,7 +3750,7 @@ extern "C" mgsb_status mgsb_smoother_pairs(mgsb_solver* h, int32_t sweeps, float
     k_l0_residual_rg<<<g0, kBlock, 0, st>>>(n0, l0.slice_ptr, l0.ell_col, l0.ell_val, l0.dfull, e, h->ls_r, l0.res);
     ca.d = e;
     TRY(launch_coarse(h, ca));
-    k_l0_prolong<<<grid_for(n0), kBlock, 0, st>>>(n0, lv[1].pid, lv[1].pw, lv[1].e, e, nullptr);
+    k_l0_prolong<<<grid_for(n0), kBlock, 0, st>>>(n0, lv[1].pid, lv[1].pw, lv[1].e, e);
     k_ls_residual<<<g0, kLsThreads, 0, st>>>(n0, l0.slice_ptr, l0.ell_col, l0.ell_val, l0.dfull, h->fixf, e, h->ls_r,
                                              h->ls_save, nullptr, nullptr);
     TRY(collect(h->ls_save));
@@ -3841,9 +3837,8 @@ extern "C" mgsb_status mgsb_vcycle_residuals(mgsb_solver* h, int32_t cycles, int
             }
             k_l0_residual_rg<<<g0, kBlock, 0, st>>>(n0, l0.slice_ptr, l0.ell_col, l0.ell_val, l0.dfull, xa, rhs, l0.res);
             ca.d = xa;
-            ca.gate = nullptr;
             TRY(launch_coarse(h, ca));
-            k_l0_prolong<<<grid_for(n0), kBlock, 0, st>>>(n0, lv[1].pid, lv[1].pw, lv[1].e, xa, nullptr);
+            k_l0_prolong<<<grid_for(n0), kBlock, 0, st>>>(n0, lv[1].pid, lv[1].pw, lv[1].e, xa);
             for (int k = 0; k < post; ++k) {
                 k_l0_sweep_rg<<<g0, kBlock, 0, st>>>(n0, l0.slice_ptr, l0.ell_col, l0.ell_val, l0.dfull, l0.dinv, xa, xb,
                                                      rhs, h->b0, h->slot_ptr, h->slots, 0);
