@@ -94,15 +94,14 @@ __device__ __forceinline__ float ls_row_features(int row, float sx, float sy, fl
     return (fx != 0.f && s > 0.f) ? s / D : 0.f;
 }
 
-// Features of every row into the BF16 tensor-core tiles and the update scale
-// s_i / D_i (0 for fixed vertices or a zero residual); optionally the FP32
-// features row-major into xf[n][9].  4 lanes per row.
+// For training pairs: the FP32 features of every row, row-major into xf[n][9],
+// and the update scale s_i / D_i (0 for fixed vertices or a zero residual).  4
+// lanes per row.
 __global__ void __launch_bounds__(kLsThreads) k_ls_features(int n, const int32_t* __restrict__ sp,
                                                             const int32_t* __restrict__ col, const float* __restrict__ val,
                                                             const float* __restrict__ dfull, const float* __restrict__ diag0,
                                                             const float* __restrict__ fixf, const float4* __restrict__ r,
-                                                            uint8_t* __restrict__ tiles, float* __restrict__ scale,
-                                                            float* __restrict__ xf) {
+                                                            float* __restrict__ scale, float* __restrict__ xf) {
     pdl_enter();
     constexpr int G = kLanesL0, S = 32 / G;
     const int lane = threadIdx.x & 31;
@@ -136,9 +135,7 @@ __global__ void __launch_bounds__(kLsThreads) k_ls_features(int n, const int32_t
     if (!valid || lane >= S) return;
     float f[kMlpIn];
     scale[row] = ls_row_features(row, sx, sy, sz, sa, sd, dfull, diag0, fixf, r, f);
-    if (tiles) mlp_store_features(tiles + (size_t)(row / kMlpTile) * kTileBytes, row % kMlpTile, f);
-    if (xf)
-        for (int k = 0; k < kMlpIn; ++k) xf[(size_t)row * kMlpIn + k] = f[k];
+    for (int k = 0; k < kMlpIn; ++k) xf[(size_t)row * kMlpIn + k] = f[k];
 }
 
 // Per-frame row constants of the learned sweep's features, from this frame's

@@ -32,6 +32,9 @@ using namespace mgsb;
 namespace {
 
 constexpr int kBlock = 256;
+// Frames above this many vertices are copied in pieces, each from the pinned buffer to the caller's arrays while the
+// next one crosses the bus; one piece costs less below it (a piece's event and copy launches: 5 us).
+constexpr int kFramePiece = 65536;
 inline int grid_for(int n) { return (n + kBlock - 1) / kBlock; }
 inline int grid_ref_vertex(int n) { return (n + kRefVertexThreads - 1) / kRefVertexThreads; }
 // blocks of kBlock threads for a row-group kernel (32/S lanes per row, slices of S rows)
@@ -246,7 +249,6 @@ struct mgsb_solver {
     cudaStream_t aux_stream = nullptr;   // captures the bodies of conditional graph nodes
     float ls_gamma = 0.5f;
     int ls_win_rows = 0, ls_ntiles = 0, ls_nblk = 0, sm_count = 148;
-    uint8_t* ls_tiles = nullptr;
     float* ls_scale = nullptr;
     float4 *ls_r = nullptr, *ls_save = nullptr, *ls_dpost = nullptr;
     float4* ls_rc = nullptr;    // per-frame row constants of the sweep's features (k_ls_row_consts)
@@ -982,7 +984,6 @@ mgsb_status rebuild(mgsb_solver* h) {
         h->ls_ntiles = (N0 + kMlpTile - 1) / kMlpTile;
         h->ls_win_rows = 0;
         h->ls_nblk = grid_rows(N0, h->lev[0].S);
-        TRY(dalloc(h, pool, &h->ls_tiles, (size_t)h->ls_ntiles * kTileBytes));
         TRY(dalloc(h, pool, &h->ls_scale, (size_t)N0));
         TRY(dalloc(h, pool, &h->ls_r, (size_t)N0));
         TRY(dalloc(h, pool, &h->ls_dpost, (size_t)N0));
@@ -2524,7 +2525,7 @@ mgsb_status create_impl(int32_t nbodies, const mgsb_mesh* meshes, const mgsb_par
     // readback fetches with its data (at N0 x 16 B) and the energies
     CUDA_TRY(hp, cudaMallocHost((void**)&h->readback, (size_t)std::max(N0, 1) * sizeof(float4) + 16 + kEnergyTerms * sizeof(double)));
     TRY(dalloc(hp, pool, &h->x, N0));
-    TRY(dalloc(hp, pool, &h->xpack, (size_t)3 * std::max(N0, 1)));
+    if (N0 > kFramePiece) TRY(dalloc(hp, pool, &h->xpack, (size_t)3 * N0));
     TRY(dalloc(hp, pool, &h->xb, N0));
     TRY(dalloc(hp, pool, &h->v, N0));
     TRY(dalloc(hp, pool, &h->s, N0));
@@ -2863,10 +2864,6 @@ mgsb_status mgsb_get_all_contact_flags(mgsb_solver* h, int32_t* out) {
     std::memcpy(out, h->readback, h->N0 * sizeof(int32_t));
     return MGSB_OK;
 }
-
-// Frames above this many vertices are copied in pieces, each from the pinned buffer to the caller's arrays while the
-// next one crosses the bus; one piece costs less below it (a piece's event and copy launches: 5 us).
-constexpr int kFramePiece = 65536;
 
 mgsb_status mgsb_get_frame(mgsb_solver* h, float* positions, int32_t* contact_flags) {
     if (!h || !positions || !contact_flags) return MGSB_INVALID_ARG;
@@ -3709,7 +3706,7 @@ extern "C" mgsb_status mgsb_smoother_pairs(mgsb_solver* h, int32_t sweeps, float
     // one set of pairs for residual r: features of r against `sweeps` Jacobi sweeps
     auto collect = [&](const float4* r) -> mgsb_status {
         k_ls_features<<<g0, kLsThreads, 0, st>>>(n0, l0.slice_ptr, l0.ell_col, l0.ell_val, l0.dfull, h->vdiag, h->fixf, r,
-                                                 nullptr, h->ls_scale, h->ls_xf);
+                                                 h->ls_scale, h->ls_xf);
         const float4* ek = sweeps_from_zero(r, sweeps);
         CUDA_TRY(h, cudaMemsetAsync(h->ls_ec, 0, (size_t)n0 * sizeof(float4), st));   // no coarse part
         k_ls_targets<<<grid_for(n0), kBlock, 0, st>>>(n0, h->ls_scale, l0.dfull, ek, h->ls_ec, h->ls_t, h->ls_mask,
