@@ -25,6 +25,7 @@ struct PlanBody {
     float gravity[3] = {0, 0, 0};
     float damping = 1.f;
     std::vector<TetRest> tr;
+    std::vector<int32_t> tet_order;   // the mesh's tet at each place of the plan's arrays; empty: its own
     std::vector<CoarseLevel> levels;  // multigrid levels 1..L-1
 };
 

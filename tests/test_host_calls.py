@@ -146,3 +146,22 @@ def test_inference_pins_no_memory(host, rows):
     y = net.forward(np.zeros((rows, 9), np.float32))
     assert y.shape == (rows, 3) and host.count(PINNED) == 0
     net.close()
+
+
+@pytest.mark.parametrize("dims,levels", [((4, 40, 4), 3), ((9, 50, 9), 4)])
+def test_blocks_of_shuffled_tets_are_compact(host, dims, levels):
+    """The local step's shared memory grows with the vertices of its largest block."""
+    m, fixed = beam(*dims)
+    need = []
+    for order in (np.arange(m.num_tets), np.random.default_rng(1).permutation(m.num_tets)):
+        host.reset()
+        s = mg.Solver([m, mg.TetMesh(m.positions, np.ascontiguousarray(m.tets[order]))],
+                      mg.default_params(mg.SOLVER_MULTIGRID, levels=levels))
+        for _ in range(2):
+            s.step()
+            s.set_fixed(fixed)
+        launches = host.launches("k_mg_local")
+        assert len({x[1:] for x in launches}) == 1
+        need.append(launches[0][5])
+        s.close()
+    assert need[1] < 1.25 * need[0]
