@@ -546,12 +546,16 @@ mgsb_status upload_normals_data(mgsb_solver* h, std::vector<DevMem>& pool) {
 // Derived data (rebuilt when fixed set / material / params change)
 // ---------------------------------------------------------------------------
 // Layout and images of k_ref_iterations: one cluster of 16 CTAs (8 if the device cannot schedule 16) up to
-// kRefClusterVerts vertices, a CTA per SM above that while a CTA's tets, those of its neighbours included, take at most
-// kRefRounds turns of its threads; larger bodies, and numberings whose vertices reach too far, run k_ref_local and
-// k_ref_vertex.  Frames of 20 iterations by cluster, grid and launches: 58, 75 and 119 us at 375 vertices, 62, 76 and 124
-// at 1,025, 88, 76 and 130 at 1,476, 98, 77 and 142 at 2,009; by grid and launches: 85 and 165 us at 4,050, 110 and 170
-// at 7,100, 160 and 191 at 19,097 (4 turns), 189 and 199 at 22,022 (5 turns), 231 and 236 at 31,725.
-constexpr int kRefClusterVerts = 1200, kRefRounds = 5;
+// kRefClusterVerts vertices; above that a CTA per SM, while the fullest CTA's tets, those that its neighbours work on too
+// included, are at most kRefTets (three and a half turns of its threads), its window at most kRefWindow vertices (read
+// again in every iteration) and both fit its shared memory; else k_ref_local and k_ref_vertex.  Frames of 20 iterations
+// in us by cluster, grid and launches: 58, 75 and 119 at 375 vertices, 62, 76 and 124 at 1,025, 88, 76 and 130 at 1,476,
+// 98, 77 and 142 at 2,009.  By grid and launches, beams, 1, 2, 5 and 20 iterations: 18, 21, 32, 90 and 22, 29, 52, 167 at
+// 4,050 vertices (0.7 turns); 23, 27, 51, 166 and 23, 31, 60, 201 at 19,097 (3.0); 25, 31, 59, 193 and 22, 31, 59, 203 at
+// 22,022 (3.4); 25, 31, 61, 202 and 23, 31, 59, 197 at 25,676 (3.8); 26, 33, 68, 229 and 24, 33, 63, 210 at 29,596 (4.2).
+// With shuffled vertices, whose windows are the whole body, 2 and 20 iterations: 24, 117 and 26, 140 at 2,009; 27, 147
+// and 26, 143 at 3,483; 33, 204 and 27, 169 at 7,100.
+constexpr int kRefClusterVerts = 1200, kRefTets = 1792, kRefWindow = 3072;
 
 mgsb_status plan_ref(mgsb_solver* h) {
     std::vector<DevMem>& pool = h->ref_mem;
@@ -596,7 +600,14 @@ mgsb_status plan_ref(mgsb_solver* h) {
                 }
             }
         };
-        for (int t = 0; t < T; ++t) share(t, corners + 4 * (size_t)t, 4, &Part::tets);
+        const size_t most_tets = grid ? kRefTets : SIZE_MAX;
+        bool full = false;
+        for (int t = 0; t < T && !full; ++t) {
+            const int32_t* c = corners + 4 * (size_t)t;
+            share(t, c, 4, &Part::tets);
+            full = part[c[0] / per].tets.size() > most_tets;
+        }
+        if (full) continue;
         for (int f = 0; f < nf; ++f) {
             const int c[3] = {h->ref_tris[f].x, h->ref_tris[f].y, h->ref_tris[f].z};
             share(f, c, 3, &Part::tris);
@@ -612,7 +623,7 @@ mgsb_status plan_ref(mgsb_solver* h) {
             win = std::max(win, (size_t)(o.hi - o.lo));
             if (nf) refs = std::max(refs, (size_t)(h->ref_tri_ptr[o.first + o.own] - h->ref_tri_ptr[o.first]));
         }
-        if (grid && tets > (size_t)kRefRounds * kRefThreads) continue;
+        if (tets > most_tets || (grid && win > (size_t)kRefWindow)) continue;
         if ((size_t)depth * per >= 0xffff || tris > 0xffff || refs > 0xffff || win > 0x10000) continue;
         RefPlan q{};
         size_t bytes = sizeof(RefHead);

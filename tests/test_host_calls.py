@@ -165,3 +165,21 @@ def test_blocks_of_shuffled_tets_are_compact(host, dims, levels):
         need.append(launches[0][5])
         s.close()
     assert need[1] < 1.25 * need[0]
+
+
+@pytest.mark.parametrize("dims,shuffled,one", [
+    ((4, 40, 4), True, True), ((6, 40, 6), True, True), ((8, 49, 8), False, True), ((8, 49, 8), True, False),
+    ((12, 112, 12), False, True), ((13, 120, 12), False, True), ((13, 130, 13), False, False), ((16, 160, 16), False, False),
+])
+def test_reference_bodies_in_one_launch(host, dims, shuffled, one):
+    """Up to 1,792 tets in the fullest of 148 CTAs (1,752 at 22,022 vertices, 1,966 at 25,676), and windows of 3,072
+    vertices (a shuffled body's are the whole of it)."""
+    m, _ = beam(*dims)
+    if shuffled:
+        to = np.random.default_rng(3).permutation(m.num_verts).astype(np.int32)
+        m = mg.TetMesh(np.ascontiguousarray(m.positions[np.argsort(to)]), np.ascontiguousarray(to[m.tets]))
+    s = mg.Solver(m, mg.default_params(mg.SOLVER_REFERENCE_JACOBI))
+    s.step()
+    assert len(host.launches("k_ref_iterations")) == one and len(host.launches("k_ref_local")) == (0 if one else 20)
+    assert len(host.launches("k_ref_image")) == one
+    s.close()
