@@ -2,12 +2,14 @@
 // BF16 weights and activations as tensor-core operands, FP32 accumulation.
 //
 //   inference  k_mlp_tc: tcgen05.mma (kind::f16, BF16 x BF16 -> FP32 in TMEM),
-//              operands staged in shared memory by bulk async copies (TMA
-//              engine), one CTA per 128-row tile, the three layers chained
-//              through TMEM -> registers (bias, GELU) -> shared memory.
+//              the weights staged in shared memory by a bulk async copy (TMA
+//              engine), the rows' features rounded into the operand tile, one CTA
+//              per 128-row tile, the three layers chained through TMEM ->
+//              registers (bias, GELU) -> shared memory.
 //   training   k_mlp_fwd_bwd: SIMT forward + hand-written backward with the same
 //              BF16 rounding of the weights and activations, FP32 math;
-//              per-block gradient partials summed in a fixed order.
+//              k_mlp_grad: the weight gradients from its rows, summed in a fixed
+//              order, and the Adam step.
 //
 // Parameter vector (FP32 master copy, 4,995 floats):
 //   W1[64][9]  b1[64]  W2[64][64]  b2[64]  W3[3][64]  b3[3]
@@ -425,7 +427,7 @@ __global__ void __launch_bounds__(kMlpThreads) k_mlp_tc(int n, int ntiles, const
 // the Adam step.  Both kernels fill the chip at 4,096 samples (128 and 127 CTAs
 // of 148 SMs); one CTA per 128 samples for everything, as before, left 116 SMs
 // idle: 100 steps on 200,000 pairs took 10.1 ms with its four small launches, and
-// take 3.2 ms (the upload of the pairs included).  Every sum runs in the order of
+// take 2.65 ms (the upload of the pairs included).  Every sum runs in the order of
 // that form: the same bits.
 // ---------------------------------------------------------------------------
 constexpr int kTrainThreads = 512;            // 16 warps of 4 hidden units each
