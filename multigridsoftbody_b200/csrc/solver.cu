@@ -235,7 +235,7 @@ struct mgsb_solver {
     int dop_cap = 0;                           // rows of the largest level the operator may start at
     float* dop_work = nullptr;                 // per level l: R, E, E2, RES blocks of n_l x dop_cap floats
     std::vector<size_t> dop_off;               // offset of level l's four blocks in dop_work (SIZE_MAX: none)
-    const float* dop_result = nullptr;         // the frame's M (n_F x n_F, row-major): in dop_work, or the coarsest inverse
+    const float* dop_result = nullptr;         // null until formed for the present shape; the frame's M (n_F x n_F, row-major): in dop_work, or the coarsest inverse
     std::vector<int> maxv;   // largest body's rows on each level
     std::vector<int2> range_host;
     int max_smem_optin = 0;
@@ -403,6 +403,7 @@ void apply_tuning(mgsb_solver* h) {
     }
     h->staged = StagedPlan{};
     h->staged_stale = true;   // planned for this shape before the next launch
+    h->dop_result = nullptr;  // formed for another shape
 }
 
 void invalidate_graph(mgsb_solver* h) {
@@ -3699,6 +3700,7 @@ extern "C" mgsb_status mgsb_smoother_pairs(mgsb_solver* h, int32_t sweeps, float
     const int launches = h->launches;   // not part of a frame
     CoarseArgs ca;
     fill_coarse_args(h, ca);
+    if (!h->dop_result) enqueue_coarse_operator(h, ca);   // the shape has changed since the last frame
     std::vector<float> hx((size_t)n0 * kMlpIn), ht((size_t)n0 * kMlpOut), hs(n0);
     std::vector<uint8_t> hm(n0);
     int64_t cnt = 0;
@@ -3831,6 +3833,7 @@ extern "C" mgsb_status mgsb_vcycle_residuals(mgsb_solver* h, int32_t cycles, int
     const bool prof = h->profiling;
     const int launches = h->launches;   // this measurement is not part of a frame
     h->profiling = false;
+    if (!h->dop_result) enqueue_coarse_operator(h, ca);   // the shape has changed since the last frame
     if (mode == 2) enqueue_ls_row_consts(h);
     for (int c = 0; c < cycles; ++c) {
         if (mode == 2) {

@@ -70,3 +70,20 @@ def test_multigrid_frames_over_set_ups(lib, dims, precision):
             assert np.isfinite(x).all() and np.array_equal(x, fresh.positions(b)) and np.array_equal(v, fresh.velocities(b))
         fresh.close()
     s.close()
+
+
+@pytest.mark.parametrize("dims,levels", [((6, 40, 6), 3), ((8, 80, 8), 4)])
+def test_residuals_after_a_change_of_coarse_shape(lib, dims, levels):
+    """No frame between: the dense operator is formed for the new shape, the same V-cycle up to rounding (496 products
+    of FP32 at most: 3e-5 of the first residual)."""
+    m, fixed = beam(*dims)
+    s = mg.Solver(m, mg.default_params(mg.SOLVER_MULTIGRID, levels=levels))
+    s.set_fixed(fixed)
+    s.step(2)
+    want = s.vcycle_residuals(3)
+    for split, dense in ((levels - 1, True), (levels - 2, True), (levels - 2, False), (levels - 1, True)):
+        s.set_coarse_split(split)
+        s.set_coarse_dense(dense)
+        got = s.vcycle_residuals(3)
+        assert np.abs(got - want).max() < 1e-4 * want[0], (split, dense, got, want)
+    s.close()

@@ -183,3 +183,25 @@ def test_reference_bodies_in_one_launch(host, dims, shuffled, one):
     assert len(host.launches("k_ref_iterations")) == one and len(host.launches("k_ref_local")) == (0 if one else 20)
     assert len(host.launches("k_ref_image")) == one
     s.close()
+
+
+@pytest.mark.parametrize("change", ["on", "split"])
+def test_dense_operator_belongs_to_its_shape(host, change):
+    """Residuals measured after the coarse shape changed, with no frame between: the operator is formed for it first."""
+    m, fixed = beam(6, 40, 6)
+    s = mg.Solver(m, mg.default_params(mg.SOLVER_MULTIGRID, levels=3))
+    s.set_fixed(fixed)
+    if change == "split":
+        s.set_coarse_split(2)
+        s.set_coarse_dense(True)
+    s.step()
+    if change == "on":
+        s.set_coarse_dense(True)
+    else:
+        s.set_coarse_split(1)
+    host.reset()
+    s.vcycle_residuals(2)
+    s.vcycle_residuals(1)
+    order = [x[0] for x in host.launches("") if "k_op_init" in x[0] or "k_coarse_apply" in x[0]]
+    assert len(order) == 4 and "k_op_init" in order[0] and all("k_coarse_apply" in x for x in order[1:])
+    s.close()
