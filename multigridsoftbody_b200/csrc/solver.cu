@@ -233,7 +233,8 @@ struct mgsb_solver {
     int tune_dense = 0;
     bool dense_op = false;
     int dop_cap = 0;                           // rows of the largest level the operator may start at
-    float* dop_work = nullptr;                 // per level l: R, E, E2, RES blocks of n_l x dop_cap floats
+    float* dop_work = nullptr;                 // per level l: R, E, E2, RES blocks of n_l x dop_cap floats; null until used
+    size_t dop_size = 0;
     std::vector<size_t> dop_off;               // offset of level l's four blocks in dop_work (SIZE_MAX: none)
     const float* dop_result = nullptr;         // null until formed for the present shape; the frame's M (n_F x n_F, row-major): in dop_work, or the coarsest inverse
     std::vector<int> maxv;   // largest body's rows on each level
@@ -370,7 +371,7 @@ constexpr int kClusterL0Rows = 2000;
 // dop_cap rows there, and the apply kernel's shared memory (the split level's
 // rows and this CTA's share of them) within the device's limit.
 bool dense_eligible(const mgsb_solver* h, int split) {
-    return h->bodies.size() == 1 && split >= 1 && h->dop_work != nullptr && h->maxv[split] <= h->dop_cap &&
+    return h->bodies.size() == 1 && split >= 1 && h->dop_cap > 0 && h->maxv[split] <= h->dop_cap &&
            coarse_apply_smem_bytes(h->maxv[split]) <= (size_t)h->max_smem_optin;
 }
 
@@ -950,7 +951,7 @@ mgsb_status rebuild(mgsb_solver* h) {
                     h->dop_off[l] = tot;
                     tot += 4 * (size_t)h->maxv[l] * h->dop_cap;
                 }
-            TRY(dalloc(h, pool, &h->dop_work, tot));
+            h->dop_size = tot;
         }
         for (int l = 1; l < L; ++l)
             if (h->lev[l].S != 32 / kLanesC)
@@ -1563,6 +1564,10 @@ void plan_top(mgsb_solver* h) {
 // 189 rows take 13.5 us with two CTAs each and 14.8 us with their images copied first.
 mgsb_status ready_staged(mgsb_solver* h) {
     if (!h->staged_stale) return MGSB_OK;
+    CUDA_TRY(h, cudaSetDevice(h->device));
+    // the dense operator's blocks (4.9 MB at 496 rows) only for solvers that run it: with them a small solver's device
+    // memory filled one more of the runtime's 2 MB pieces, fetched and given back with every new solver (2-3 ms)
+    if (h->dense_op && !h->dop_work) TRY(dalloc(h, h->derived_mem, &h->dop_work, h->dop_size));
     h->staged = StagedPlan{};
     h->staged_image.clear();
     if (is_mg(h) && !h->fuse_l0 && !h->dense_op && h->bodies.size() == 1 && (int)h->coarse_host.size() == h->p.levels) {

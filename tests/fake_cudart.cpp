@@ -19,7 +19,8 @@ struct Launch {
 std::map<const void*, std::string> kernels;
 std::vector<Launch> launches;
 std::string refused;
-long counts[5];   // captures, graph launches, stream synchronisations, bytes copied to the device, pinned allocations
+long counts[6];   // captures, graph launches, stream synchronisations, bytes copied to the device, pinned allocations, bytes
+                  // of device memory
 cudaError_t last = cudaSuccess;
 char token[8];    // what handles point at
 
@@ -33,6 +34,11 @@ template <typename T>
 cudaError_t handle(T* out) {
     *out = reinterpret_cast<T>(token);
     return cudaSuccess;
+}
+cudaError_t host_malloc(void** p, size_t n) {
+    const size_t size = (n + 255) / 256 * 256 + 256;
+    *p = aligned_alloc(256, size);
+    return *p ? memset(*p, 0, size), cudaSuccess : cudaErrorMemoryAllocation;
 }
 thread_local struct { dim3 g, b; size_t smem; void* s; } config;
 }  // namespace
@@ -84,12 +90,8 @@ cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void
     }
     return launch(f, c->gridDim, c->blockDim, c->dynamicSmemBytes, cluster, cooperative);
 }
-cudaError_t cudaMalloc(void** p, size_t n) {
-    const size_t size = (n + 255) / 256 * 256 + 256;
-    *p = aligned_alloc(256, size);
-    return *p ? memset(*p, 0, size), cudaSuccess : cudaErrorMemoryAllocation;
-}
-cudaError_t cudaMallocHost(void** p, size_t n) { return ++counts[4], cudaMalloc(p, n); }
+cudaError_t cudaMalloc(void** p, size_t n) { return counts[5] += (long)n, host_malloc(p, n); }
+cudaError_t cudaMallocHost(void** p, size_t n) { return ++counts[4], host_malloc(p, n); }
 cudaError_t cudaFree(void* p) { return free(p), cudaSuccess; }
 cudaError_t cudaFreeHost(void* p) { return free(p), cudaSuccess; }
 cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind k, cudaStream_t) {

@@ -10,7 +10,7 @@ from multigridsoftbody_b200 import _lib as L
 from multigridsoftbody_b200 import build
 
 HERE = os.path.dirname(os.path.abspath(__file__))
-CAPTURES, GRAPH_LAUNCHES, SYNCHRONISATIONS, UPLOADED, PINNED = range(5)
+CAPTURES, GRAPH_LAUNCHES, SYNCHRONISATIONS, UPLOADED, PINNED, ALLOCATED = range(6)
 
 
 def build_host_only(out_dir: str) -> str:

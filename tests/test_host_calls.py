@@ -8,7 +8,7 @@ from multigridsoftbody_b200 import _lib as L
 from multigridsoftbody_b200.learned import MLP
 
 from .common import beam
-from .host_only import CAPTURES, GRAPH_LAUNCHES, PINNED, UPLOADED, Host, build_host_only
+from .host_only import ALLOCATED, CAPTURES, GRAPH_LAUNCHES, PINNED, UPLOADED, Host, build_host_only
 
 
 @pytest.fixture(scope="module")
@@ -205,3 +205,18 @@ def test_dense_operator_belongs_to_its_shape(host, change):
     order = [x[0] for x in host.launches("") if "k_op_init" in x[0] or "k_coarse_apply" in x[0]]
     assert len(order) == 4 and "k_op_init" in order[0] and all("k_coarse_apply" in x for x in order[1:])
     s.close()
+
+
+def test_dense_operator_memory_is_for_its_users(host):
+    m, _ = beam(6, 40, 6)
+    allocated = []
+    for dense in (False, True):
+        host.reset()
+        s = mg.Solver(m, mg.default_params(mg.SOLVER_MULTIGRID, levels=3))
+        s.set_coarse_dense(dense)
+        s.step()
+        assert len(host.launches("k_op_init")) == dense and len(host.launches("k_coarse_apply")) == 10 * dense
+        allocated.append(host.count(ALLOCATED))
+        blocks = 16 * s.level_size(1)[0] ** 2
+        s.close()
+    assert allocated[1] - allocated[0] > 0.75 * blocks   # a plain solver has the cluster kernel's images instead
